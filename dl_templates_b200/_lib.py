@@ -79,6 +79,20 @@ def _load() -> C.CDLL:
 lib = _load()
 
 
+def _load_native():
+    """The extension module with the host path of the call surface (argument checks, allocation, autograd nodes); it
+    links the C-ABI library next to it."""
+    try:
+        from . import _swa2d_torch
+    except ImportError as e:
+        raise RuntimeError("the extension module _swa2d_torch is missing or does not load: build it with "
+                           "`python dl_templates_b200/build.py`. This package has no fallback implementation.") from e
+    return _swa2d_torch
+
+
+native = _load_native()
+
+
 def dtype_code(dt: torch.dtype) -> int:
     try:
         return _DTYPES[dt]

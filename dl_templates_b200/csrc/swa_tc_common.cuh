@@ -499,12 +499,16 @@ __device__ __forceinline__ void trace_ev(const KParams& p, int role, int& n, boo
 #endif
 }
 
-// Record a timed-out wait (first one wins) so the host can report it.
+// Record a timed-out wait so the host can report it.  The words may be mapped host memory: plain system-visible
+// stores, the code last (of several CTAs that gave up at once, any one's record will do).
 __device__ __forceinline__ void report_abort(int32_t* status, int code, int where) {
-  if (status != nullptr && atomicCAS(status, 0, code) == 0) {
-    status[1] = blockIdx.x;
-    status[2] = blockIdx.y;
-    status[3] = where;
+  volatile int32_t* s = status;
+  if (s != nullptr && s[0] == 0) {
+    s[1] = blockIdx.x;
+    s[2] = blockIdx.y;
+    s[3] = where;
+    __threadfence_system();
+    s[0] = code;
   }
 }
 

@@ -14,11 +14,9 @@ dims ``>= 4R`` pass through.  The reference's Triton kernel substitutes (cos,sin
 """
 from __future__ import annotations
 
-import ctypes as C
-
 import torch
 
-from . import _lib
+from ._lib import native as _native
 
 
 def make_cs_table(n_rdim: int, max_len: int, theta: float = 10000.0, device=None) -> torch.Tensor:
@@ -46,18 +44,7 @@ class FusedRotaryPositionEncodingContext(torch.nn.Module):
 def rope2d_apply_(x: torch.Tensor, idx: torch.Tensor, row_cs: torch.Tensor, col_cs: torch.Tensor,
                   inverse: bool = False) -> torch.Tensor:
     """In-place rotation of ``x [batch, N, C]`` (any strides); returns ``x``."""
-    if not x.is_cuda:
-        raise RuntimeError("dl_templates_b200 runs on CUDA tensors only (sm_100a); there is no CPU path")
-    B, N, n_dim = x.shape
-    assert row_cs.shape[1] == col_cs.shape[1]
-    assert idx.shape[0] == N
-    with torch.cuda.device(x.device):
-        rope = _lib.make_rope(idx, row_cs, col_cs)
-        xs = (C.c_int64 * 3)(x.stride(0), x.stride(1), x.stride(2))
-        code = _lib.lib.rope2d_apply(_lib.dtype_code(x.dtype), x.data_ptr(), B, N, n_dim, xs, C.byref(rope),
-                                     1 if inverse else 0, _lib.stream_ptr(x.device))
-    _lib.check(code, "rope2d_apply")
-    return x
+    return _native.rope2d_(x, idx, row_cs, col_cs, int(inverse))
 
 
 def rope2d_apply_to(x: torch.Tensor, idx: torch.Tensor, row_cs: torch.Tensor, col_cs: torch.Tensor,
@@ -65,23 +52,7 @@ def rope2d_apply_to(x: torch.Tensor, idx: torch.Tensor, row_cs: torch.Tensor, co
     """``rope(x)`` (or the inverse rotation) of ``x [batch, N, C]`` in a new contiguous tensor, ``x`` untouched:
     one pass when the layout allows (fp16 / bf16, ``n_rdim % 8 == 0``, ``C % 8 == 0``, unit last stride, 16-byte
     aligned rows), else a copy followed by the in-place kernel."""
-    if not x.is_cuda:
-        raise RuntimeError("dl_templates_b200 runs on CUDA tensors only (sm_100a); there is no CPU path")
-    B, N, n_dim = x.shape
-    assert row_cs.shape[1] == col_cs.shape[1] and idx.shape[0] == N
-    y = torch.empty((B, N, n_dim), dtype=x.dtype, device=x.device)
-    rows16 = x.stride(2) == 1 and x.data_ptr() % 16 == 0 and x.stride(0) % 8 == 0 and x.stride(1) % 8 == 0
-    if x.dtype in (torch.float16, torch.bfloat16) and row_cs.shape[1] % 8 == 0 and n_dim % 8 == 0 and rows16:
-        with torch.cuda.device(x.device):
-            rope = _lib.make_rope(idx, row_cs, col_cs)
-            xs = (C.c_int64 * 3)(x.stride(0), x.stride(1), x.stride(2))
-            ys = (C.c_int64 * 3)(y.stride(0), y.stride(1), y.stride(2))
-            code = _lib.lib.rope2d_apply_to(_lib.dtype_code(x.dtype), x.data_ptr(), y.data_ptr(), B, N, n_dim, xs, ys,
-                                            C.byref(rope), 1 if inverse else 0, _lib.stream_ptr(x.device))
-        _lib.check(code, "rope2d_apply_to")
-        return y
-    y.copy_(x)
-    return rope2d_apply_(y, idx, row_cs, col_cs, inverse)
+    return _native.rope2d_to(x, idx, row_cs, col_cs, int(inverse))
 
 
 class RotaryPE2D(torch.autograd.Function):
@@ -128,6 +99,9 @@ class FusedInplaceRotaryPositionEncoding2D(torch.nn.Module):
 
     def forward(self, x: torch.Tensor, idx: torch.Tensor) -> torch.Tensor:
         # x: [B, Head, N, C]  idx: [N]
-        B, H, N, Cdim = x.shape
+        y = _native.rope2d_heads_(x, idx, self.row_buffer.cs_components, self.col_buffer.cs_components)
+        if y is not None:
+            return y
+        B, H, N, Cdim = x.shape              # x is part of a graph: the autograd function records the rotation
         x0 = x.reshape((-1, N, Cdim))
         return RotaryPE2D.apply(x0, idx, self.row_buffer.cs_components, self.col_buffer.cs_components).reshape(x.shape)
