@@ -2,6 +2,7 @@
 // maps and launches.
 #include <cudaTypedefs.h>
 
+#include <algorithm>
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
@@ -9,6 +10,7 @@
 #include <mutex>
 #include <tuple>
 #include <type_traits>
+#include <vector>
 
 #include "swa_tc.cuh"
 #include "swa_tc_bwd.cuh"
@@ -134,17 +136,15 @@ int halo_width(const swa_geom_t* g, int TW) {
 //   tensor memory (512 columns): forward  score buffers at 128-column strides (packed when they do not fit) + two O accumulators;
 //                                backward nsb pairs (S, dP) of 2N columns + the accumulators
 //   shared memory:               nxb resident-tile buffers + indicator rows + stages x (block + penalty rows [+ lse, delta])
-// `v2`: the plan is for the kernels without streamed rotation (swa_tc_fwd2.cuh / swa_tc_bwd2.cuh), whose shared-memory
-// block behind the ring differs: no fixed-size penalty tables (they are sized per plan), two more lse / delta slots.
-bool make_plan_shape(const swa_geom_t* g, int which, int TH, int TW, uint32_t tab_bytes, Plan* out, long* cost_out = nullptr,
-                     bool v2 = false) {
-  Plan pl;
+// (Kernels with streamed rotation; those without: make_strip_shape below.)
+bool make_plan_shape(const swa_geom_t* g, int which, int TH, int TW, uint32_t tab_bytes, Plan* out, long* cost_out = nullptr) {
+  Plan pl{};
   pl.ncb = 1;
   pl.tab_bytes = tab_bytes;
   pl.TH = TH;
   pl.TW = TW;
   const int hw = halo_width(g, pl.TW);
-  if (!v2 && hw > kPenCols) return false;     // the kernels with streamed rotation keep a whole halo row per block row
+  if (hw > kPenCols) return false;     // these kernels keep a whole halo row per block row
   const int halo_rows = pl.TH + 2 * g->row_size;
   const int qch = (g->d_qk + 63) / 64, vch = (g->d_v + 63) / 64;
   const uint32_t x_bytes = (which == 0 ? qch : qch + vch) * 16384u;
@@ -153,11 +153,7 @@ bool make_plan_shape(const swa_geom_t* g, int which, int TH, int TW, uint32_t ta
   const int acc_cols = which == 0 ? 0 : (which == 1 ? 64 * qch : 64 * (qch + vch));
   const int min_stages = 3;
   // alignment pad of the swizzled tiles + the kernel's barrier / exchange / penalty-table block behind the ring
-  const uint32_t slack_v1 = 1024u + (((which == 0 ? (uint32_t)sizeof(FwdShared) : (uint32_t)sizeof(BwdShared)) + 15u) & ~15u);
-  const uint32_t slack_v2 = 1024u + (((which == 0 ? (uint32_t)sizeof(Fwd2Shared) : (uint32_t)sizeof(Bwd2Shared)) + 15u) & ~15u) +
-                            (which == 0 ? 0u : 2048u);
-  // per candidate block shape: the v2 kernels' penalty tables take (halo rows + KR + KW) entries of 32 bytes
-  auto slack_for = [&](int KR, int KW, int ncb) { return v2 ? slack_v2 + (uint32_t)(halo_rows + KR + KW * ncb) * 32u : slack_v1; };
+  const uint32_t kSmemSlack = 1024u + (((which == 0 ? (uint32_t)sizeof(FwdShared) : (uint32_t)sizeof(BwdShared)) + 15u) & ~15u);
   {
     // backward: two (S, dP) pairs of 2N columns next to the accumulators (N = 64 always fits: 256 + 256 columns)
     const int nsb = 2;
@@ -168,21 +164,18 @@ bool make_plan_shape(const swa_geom_t* g, int which, int TH, int TW, uint32_t ta
     for (int nxb = which == 0 ? 2 : (kn.nxb ? kn.nxb : 2); nxb >= (which == 0 ? 2 : 1); --nxb) {
       const uint32_t fixed = nxb * x_bytes + 128u * kXRowBytes + tab_bytes;
       long best_cost = -1;
-      // ncb = column blocks per halo row: 1 whenever a block can span the halo; the kernels without streamed
-      // rotation also take halos wider than any block and walk them in several column blocks
-      for (int ncb = 1; ncb <= (v2 ? 16 : 1) && best_cost < 0; ++ncb)
-        for (int KW = (hw + ncb - 1) / ncb; KW <= kPenCols && (ncb == 1 || KW * (ncb - 1) < hw); ++KW)
-          for (int KR = 1; KR <= 16; ++KR) {
-            const int N = KW * KR;
-            if (N > nmax || N % 16) continue;
-            if (fixed + min_stages * ((uint32_t)N * row_bytes + stage_extra) + slack_for(KR, KW, ncb) > kSmemLimit) continue;
-            const long nblk = (long)((halo_rows + KR - 1) / KR) * ncb;
-            const long cost = nblk * N * 16 + nblk * 400;  // executed columns + a per-block overhead
-            if (best_cost < 0 || cost < best_cost) {
-              best_cost = cost;
-              pl.KR = KR; pl.KW = KW; pl.N = N; pl.ncb = ncb;
-            }
+      for (int KW = hw; KW <= kPenCols; ++KW)
+        for (int KR = 1; KR <= 16; ++KR) {
+          const int N = KW * KR;
+          if (N > nmax || N % 16) continue;
+          if (fixed + min_stages * ((uint32_t)N * row_bytes + stage_extra) + kSmemSlack > kSmemLimit) continue;
+          const long nblk = (halo_rows + KR - 1) / KR;
+          const long cost = nblk * N * 16 + nblk * 400;  // executed columns + a per-block overhead
+          if (best_cost < 0 || cost < best_cost) {
+            best_cost = cost;
+            pl.KR = KR; pl.KW = KW; pl.N = N;
           }
+        }
       if (best_cost < 0) continue;
       if (kn.kr) {
         pl.KR = kn.kr;
@@ -193,9 +186,6 @@ bool make_plan_shape(const swa_geom_t* g, int which, int TH, int TW, uint32_t ta
         if (pl.KW < hw || pl.KW > kPenCols || pl.KR > 16) return false;
       }
       const uint32_t stage = (uint32_t)pl.N * row_bytes + stage_extra;
-      const uint32_t kSmemSlack = slack_for(pl.KR, pl.KW, pl.ncb);
-      pl.pen_rows = halo_rows + pl.KR;
-      pl.pen_cols = pl.KW * pl.ncb;
       const int Wtok = g->t_width * g->b_size;
       pl.n_tiles_x = (Wtok + pl.TW - 1) / pl.TW;
       pl.n_tiles_y = (g->t_height + pl.TH - 1) / pl.TH;
@@ -226,6 +216,173 @@ bool make_plan_shape(const swa_geom_t* g, int which, int TH, int TW, uint32_t ta
   return false;
 }
 
+// Shared memory of the strip kernels beside resident rows, ring and tables: alignment pad of the swizzled tiles, barrier /
+// exchange block, row parts of the window mask, dK/dV the lse / delta ring.
+uint32_t strip_slack(const swa_geom_t* g, int which, int R4) {
+  const uint32_t sh = which == 0 ? (uint32_t)sizeof(Fwd2Shared) : (uint32_t)sizeof(Bwd2Shared);
+  return 1024u + ((sh + 15u) & ~15u) + row_parts_bytes(g->row_size, R4) + (which == 2 ? (kMaskRing + 2) * 1024u : 0u);
+}
+
+// ... and the mask units: three per ring entry, the unused one.
+uint32_t mask_bytes(int N) { return (uint32_t)N * 16u * (3u * kMaskRing + 1u); }
+
+// Blocks of a chunk of `nq` quarters whose first row is r0 (the kernels' strip_item).
+int strip_blocks(const swa_geom_t* g, const Plan& pl, int r0, int nq) {
+  const int q = std::min(nq, (g->t_height - r0 + pl.R4 - 1) / pl.R4);
+  const int h0 = r0 - g->row_size + pl.KR * (std::max(0, g->row_size - r0) / pl.KR);
+  const int last = std::min(r0 + q * pl.R4 - 1 + g->row_size, g->t_height - 1);
+  return ((last - h0) / pl.KR + 1) * pl.ncb;
+}
+
+// Whether quarters can slide through the slots: quarter i + 4 must not meet a block before the last one of quarter i.
+bool strip_slides(const swa_geom_t* g, int R4, int KR) {
+  for (int i = 0; i < KR; ++i)
+    if ((i * R4 + R4 - 1 + 2 * g->row_size) / KR >= (i + 4) * R4 / KR) return false;
+  return true;
+}
+
+// Chunk height in quarters.  Sliding strips: the tallest chunk has the fewest blocks per row (2 wr rows of halo are met
+// once per chunk), short ones spread a small problem over all SMs; the slowest SM's blocks decide.  The height is a
+// multiple of the block height, so that no row's blocks depend on it.
+void choose_chunk(const swa_geom_t* g, Plan* pl) {
+  const int quarters = (g->t_height + pl->R4 - 1) / pl->R4;
+  const int64_t strips = (int64_t)pl->n_tiles_x * g->B * g->H;
+  if (!strip_slides(g, pl->R4, pl->KR)) {
+    pl->nq = 4;
+  } else {
+    const int sms = sm_count();
+    int unit = 1;
+    while (unit * pl->R4 % pl->KR) ++unit;
+    const int most = std::max(1, 2048 / pl->R4);            // chunk rows the kernels' div_kr covers
+    double best = -1.;
+    for (int nq = unit; ; nq += unit) {
+      const bool whole = nq >= quarters;
+      if (nq > most && !(whole && quarters <= most)) break;
+      const int chunks = (quarters + nq - 1) / nq;
+      const int64_t items = strips * chunks;
+      double load;
+      if (items <= 8 * sms) {                                // the items as the CTAs walk them
+        std::vector<long> cta(sms, 0);
+        for (int64_t i = 0; i < items; ++i) cta[i % sms] += strip_blocks(g, *pl, (int)(i / pl->n_tiles_x % chunks) * nq * pl->R4, nq) + 2;
+        load = (double)*std::max_element(cta.begin(), cta.end());
+      } else {
+        double total = 0.;
+        for (int c = 0; c < chunks; ++c) total += strip_blocks(g, *pl, c * nq * pl->R4, nq) + 2;
+        load = total * strips / sms + 0.5 * strip_blocks(g, *pl, 0, nq);
+      }
+      if (best < 0. || load <= best) {
+        best = load;
+        pl->nq = nq;
+      }
+      if (whole) break;
+    }
+  }
+  pl->n_tiles_y = (quarters + pl->nq - 1) / pl->nq;
+  pl->chunk_rows = pl->nq * pl->R4;
+}
+
+// Plan of the kernels without streamed rotation for strips TW token columns wide (swa_tc_strip.cuh).  Halos wider than any
+// block are walked in `ncb` column blocks per row band.
+bool make_strip_shape(const swa_geom_t* g, int which, int TW, Plan* out, long* cost_out) {
+  Plan pl{};
+  pl.TW = TW;
+  pl.TH = 128 / TW;
+  pl.R4 = 32 / TW;
+  const int hw = halo_width(g, TW);
+  const int qch = (g->d_qk + 63) / 64, vch = (g->d_v + 63) / 64;
+  const uint32_t x_bytes = (which == 0 ? qch : qch + vch) * 16384u;
+  const uint32_t row_bytes = (qch + vch) * 128u;
+  const int out_chunks = which == 0 ? vch : which == 1 ? qch : qch + vch;
+  const int acc_cols = which == 0 ? 2 * 64 * vch : (which == 1 ? 64 * qch : 64 * (qch + vch));
+  const int min_stages = 3;
+  const uint32_t slack = strip_slack(g, which, pl.R4);
+  const Knobs kn = knobs();
+  int nmax = which == 0 ? 128 : std::min(128, (512 - acc_cols) / 4);
+  if (kn.nmax) nmax = kn.nmax;
+  pl.n_tiles_x = (g->t_width * g->b_size + TW - 1) / TW;
+  const int quarters = (g->t_height + pl.R4 - 1) / pl.R4;
+  // output staging for a whole quarter; for wide heads, whose quarters never follow each other block by block, one chunk (the
+  // forward kernel: none)
+  pl.stg = which == 0 ? (qch == 1 && vch == 1) : qch == 1 && vch == 1 ? out_chunks : 1;
+  const uint32_t fixed = 8192u + 4u * pl.stg * kStageChunk + slack;
+  long best_cost = -1;
+  for (int ncb = 1; ncb <= 16 && best_cost < 0; ++ncb)
+    for (int KW = (hw + ncb - 1) / ncb; KW <= 128 && (ncb == 1 || KW * (ncb - 1) < hw); ++KW)
+      for (int KR = 1; KR <= 16; ++KR) {
+        const int N = KW * KR;
+        if (N > nmax || N % 16 || N < 32) continue;            // (both compute groups need columns)
+        const bool slides = strip_slides(g, pl.R4, KR);
+        Plan c = pl;
+        c.KR = KR; c.KW = KW; c.N = N; c.ncb = ncb;
+        long blocks = 0, items = 1;                            // per strip of the whole grid height
+        if (slides) {
+          blocks = strip_blocks(g, c, 0, quarters);
+        } else {
+          items = (quarters + 3) / 4;
+          for (int q = 0; q < quarters; q += 4) blocks += strip_blocks(g, c, q * pl.R4, 4);
+        }
+        // One resident buffer leaves room for larger blocks, but nothing overlaps the load of an item's resident rows (about
+        // 3000 cycles, the time of 250 columns); sliding strips need two.
+        for (int nxb = kn.nxb && which ? kn.nxb : 2; nxb >= (kn.nxb || slides || which == 0 ? 2 : 1) && nxb >= 1; --nxb) {
+          if (fixed + nxb * x_bytes + min_stages * (uint32_t)N * row_bytes + mask_bytes(N) > kSmemLimit) continue;
+          // executed columns + what a block costs beside them: backward the latency chain of a buffer pair, as much as a
+          // hundred columns; forward the groups' work per block
+          const long cost = (blocks * (N + (which == 0 ? 40 : 100)) + (nxb == 1 ? items * 250 : 0)) * pl.n_tiles_x;
+          if (best_cost < 0 || cost < best_cost) {
+            best_cost = cost;
+            pl.KR = KR; pl.KW = KW; pl.N = N; pl.ncb = ncb; pl.nxb = nxb;
+          }
+        }
+      }
+  if (best_cost < 0) return false;
+  if (kn.kr) {
+    pl.KR = kn.kr;
+    if (kn.kw) pl.KW = kn.kw;
+    pl.N = pl.KR * pl.KW;
+    pl.ncb = 1;
+    if (pl.KW < hw || pl.KW > 128 || pl.KR > 16) return false;      // an override must still hold a whole halo row
+    pl.nxb = 2;
+  }
+  const uint32_t stage = (uint32_t)pl.N * row_bytes, rest = fixed + pl.nxb * x_bytes + mask_bytes(pl.N);
+  pl.kr_inv = (65536 + pl.KR - 1) / pl.KR;
+  pl.kw_inv = (65536 + pl.KW - 1) / pl.KW;
+  pl.tw_log = TW == 8 ? 3 : 4;
+  pl.stages = min_stages;
+  while (pl.stages < kMaxStages && rest + (pl.stages + 1) * stage <= kSmemLimit) ++pl.stages;
+  if (kn.stages) pl.stages = kn.stages;
+  pl.smem_bytes = rest + pl.stages * stage;
+  pl.nsb = 2;
+  if (which == 0) {
+    // score buffers = look-ahead of the score MMAs: 3, or 4 when the block ring is deep enough to feed them (measured); with
+    // columns of their own for P if that leaves three (swa_tc_fwd2.cuh), else P over the scores
+    const int most = kn.nsb ? kn.nsb : pl.stages >= 6 ? 4 : 3, room = 512 - acc_cols;
+    pl.p_off = std::max(3, kn.nsb) * (pl.N + pl.N / 2) <= room ? pl.N : 0;
+    const int per = pl.N + pl.p_off / 2;
+    pl.nsb = std::max(kn.nsb ? kn.nsb : 2, std::min(most, room / per));
+    pl.s_stride = per <= 128 && pl.nsb * 128 <= room ? 128 : per;
+  }
+  *out = pl;
+  *cost_out = best_cost;
+  // tensor-memory columns of the final plan (the environment overrides above included): a plan beyond the
+  // 512-column allocation is refused here, never launched
+  const uint32_t tmem_cols = (uint32_t)(which == 0 ? pl.nsb * pl.s_stride : 4 * pl.N) + (uint32_t)acc_cols;
+  return pl.smem_bytes <= kSmemLimit && pl.N % 16 == 0 && pl.N >= 16 && pl.N <= 256 && pl.N <= nmax && pl.stages >= 2 &&
+         pl.stages <= kMaxStages && pl.nsb >= 2 && pl.nsb <= 4 && tmem_cols <= 512u;
+}
+
+// Strip width by block cost.
+bool make_strip_plan(const swa_geom_t* g, int which, Plan* out) {
+  const Knobs kn = knobs();
+  const int th = kn.th[which] ? kn.th[which] : kn.th_all;
+  Plan a, b;
+  long ca = 0, cb = 0;
+  const bool oa = th != 8 && make_strip_shape(g, which, 8, &a, &ca), ob = th != 16 && make_strip_shape(g, which, 16, &b, &cb);
+  if (!oa && !ob) return false;
+  *out = oa && (!ob || ca <= cb) ? a : b;
+  choose_chunk(g, out);
+  return true;
+}
+
 // Bytes of the cos/sin tables when they are small enough to be staged in shared memory, else 0.
 uint32_t rope_table_bytes(const swa_rope_t* rope) {
   if (!rope || !rope->idx) return 0;
@@ -234,35 +391,30 @@ uint32_t rope_table_bytes(const swa_rope_t* rope) {
 }
 
 // Tile shape for one choice of staged-table bytes; *cost = the planner's block cost of the plan taken.
-static bool make_plan_tab(const swa_geom_t* g, const swa_rope_t* rope, int which, uint32_t tab, Plan* out, long* cost,
-                          bool v2 = false) {
+static bool make_plan_tab(const swa_geom_t* g, const swa_rope_t* rope, int which, uint32_t tab, Plan* out, long* cost) {
   const Knobs kn = knobs();
   const int th = kn.th[which] ? kn.th[which] : kn.th_all;
-  if (th == 8) return make_plan_shape(g, which, 8, 16, tab, out, cost, v2);
-  if (th == 16) return make_plan_shape(g, which, 16, 8, tab, out, cost, v2);
-  if (which == 2 || (which == 0 && v2)) {
+  if (th == 8) return make_plan_shape(g, which, 8, 16, tab, out, cost);
+  if (th == 16) return make_plan_shape(g, which, 16, 8, tab, out, cost);
+  if (which == 2) {
     // dK/dV (K tile resident, Q blocks streamed; its accumulators leave the narrowest blocks): the shape whose
     // blocks cost less by the planner's own measure -- 16 x 8 at the 13 x 13 window with d = 64, 8 x 16 once
     // d_v = 128 or the window grows (measured: 10 % and 13 % faster at 15 x 15 / d_v = 128 and 31 x 31 / d = 128).
-    // The forward kernel without streamed rotation: the same rule -- 8 x 16 at the 13 x 13 and 15 x 15 windows (five
-    // or six blocks instead of seven or eight), 16 x 8 at the 31 x 31 window with d = 128, where it halves the
-    // number of blocks (23 of 80 tokens instead of 38 of 48; measured 3.11 against 3.60 ms at 32 slices)
     Plan a, b;
     long ca = 0, cb = 0;
-    const bool oa = make_plan_shape(g, which, 16, 8, tab, &a, &ca, v2), ob = make_plan_shape(g, which, 8, 16, tab, &b, &cb, v2);
+    const bool oa = make_plan_shape(g, which, 16, 8, tab, &a, &ca), ob = make_plan_shape(g, which, 8, 16, tab, &b, &cb);
     if (!oa && !ob) return false;
     const bool take_a = oa && (!ob || ca <= cb);
     *out = take_a ? a : b;
     *cost = take_a ? ca : cb;
     return true;
   }
-  // measured at the 13 x 13 window: with fused RoPE 16 x 8 wins (80-token blocks, every block row shared by
-  // two rotating threads), without it 8 x 16 wins for the forward and dQ kernels (fewer, wider blocks)
-  // ... and for the dQ kernel also when at most 32 of 64 q/k dims are rotated (measured 12 % faster at d_v = 128
+  // measured at the 13 x 13 window: 16 x 8 wins (80-token blocks, every block row shared by two rotating threads),
+  // except for the dQ kernel when at most 32 of 64 q/k dims are rotated (measured 12 % faster at d_v = 128
   // with a 15 x 15 window and 3 % at the 13 x 13 window; at d_qk = 128 the 16 x 8 tile stays 27 % ahead)
-  const bool wide_first = !(rope && rope->idx) || (which == 1 && rope->n_rdim <= 8 && g->d_qk == 64);
-  return wide_first ? (make_plan_shape(g, which, 8, 16, tab, out, cost, v2) || make_plan_shape(g, which, 16, 8, tab, out, cost, v2))
-                    : (make_plan_shape(g, which, 16, 8, tab, out, cost, v2) || make_plan_shape(g, which, 8, 16, tab, out, cost, v2));
+  const bool wide_first = which == 1 && rope->n_rdim <= 8 && g->d_qk == 64;
+  return wide_first ? (make_plan_shape(g, which, 8, 16, tab, out, cost) || make_plan_shape(g, which, 16, 8, tab, out, cost))
+                    : (make_plan_shape(g, which, 16, 8, tab, out, cost) || make_plan_shape(g, which, 8, 16, tab, out, cost));
 }
 
 // The cos/sin tables are staged in shared memory when that does not cost block size: a plan with the tables is
@@ -276,7 +428,7 @@ std::map<PlanKey, std::pair<bool, Plan>> g_plan_cache;
 PlanKey plan_key(const swa_geom_t* g, const swa_rope_t* rope, int which, bool v2) {
   const bool has = rope && rope->idx;
   return PlanKey(which + (v2 ? 3 : 0), g->t_height, g->t_width, g->b_size, g->row_size, g->col_size, g->d_qk, g->d_v,
-                 has ? rope->n_rdim : 0, has ? rope->max_h : 0, has ? rope->max_w : 0, g->dtype == SWA_BF16 ? 1 : 0, 0);
+                 has ? rope->n_rdim : 0, has ? rope->max_h : 0, has ? rope->max_w : 0, g->dtype == SWA_BF16 ? 1 : 0, v2 ? g->B * g->H : 0);
 }
 bool cache_lookup(const PlanKey& k, bool* ok, Plan* out) {
   std::lock_guard<std::mutex> lock(g_plan_mu);
@@ -305,9 +457,6 @@ bool make_plan_uncached(const swa_geom_t* g, const swa_rope_t* rope, int which, 
   return ok_n;
 }
 
-// Plan of the kernels that rotate no streamed row (rotation handed on between the kernels, or no RoPE): the
-// tile shape of the problem without RoPE; the tables (read once per item, in the epilogue) are staged when that
-// costs no block size and leaves at least three stages of the ring.
 bool make_plan(const swa_geom_t* g, const swa_rope_t* rope, int which, Plan* out) {
   const PlanKey key = plan_key(g, rope, which, false);
   bool ok = false;
@@ -317,22 +466,6 @@ bool make_plan(const swa_geom_t* g, const swa_rope_t* rope, int which, Plan* out
   cache_store(key, ok, pl);
   if (ok) *out = pl;
   return ok;
-}
-
-bool make_plan_prerot_uncached(const swa_geom_t* g, const swa_rope_t* rope, int which, Plan* out) {
-  const uint32_t tab = rope_table_bytes(rope);
-  Plan with, without;
-  long cw = 0, cn = 0;
-  const bool ok_n = make_plan_tab(g, nullptr, which, 0, &without, &cn, true);
-  // (measured: a fourth or fifth stage of the ring is worth nothing here, table rows fetched from L2 inside the
-  // epilogue cost 0.2 to 0.3 ms per launch at the default workload)
-  if (ok_n && tab && make_plan_tab(g, nullptr, which, tab, &with, &cw, true) && cw <= cn &&
-      (with.stages >= without.stages || with.stages >= 3) && with.TH == without.TH) {
-    *out = with;
-    return true;
-  }
-  if (ok_n) *out = without;
-  return ok_n;
 }
 
 // Indicator value a and penalty b (powers of two, exact in fp16 and bf16) of the window mask that
@@ -346,12 +479,13 @@ bool mask_constants(float sm_scale, float* a, float* b) {
   return aa * bb >= need;
 }
 
-bool make_plan_prerot(const swa_geom_t* g, const swa_rope_t* rope, int which, Plan* out) {
-  const PlanKey key = plan_key(g, rope, which, true);
+// Plan of the kernels that rotate no streamed row (rotation handed on between the kernels, or no RoPE).
+bool make_plan_prerot(const swa_geom_t* g, int which, Plan* out) {
+  const PlanKey key = plan_key(g, nullptr, which, true);
   bool ok = false;
   if (cache_lookup(key, &ok, out)) return ok;
   Plan pl{};
-  ok = make_plan_prerot_uncached(g, rope, which, &pl);
+  ok = make_strip_plan(g, which, &pl);
   cache_store(key, ok, pl);
   if (ok) *out = pl;
   return ok;
@@ -375,6 +509,16 @@ KParams make_params(const swa_geom_t* g, const swa_rope_t* rope, const Plan& pl,
   p.pl = pl;
   p.rope = make_rope(rope);
   p.n_items = pl.n_tiles_x * pl.n_tiles_y * g->B * g->H;
+  p.div_b = g->b_size == 1 ? 0u : (uint32_t)((0x100000000ull + g->b_size - 1) / g->b_size);
+  {
+    int step = std::min(p.n_items, sm_count());                // one CTA per SM
+    p.step_tx = step % pl.n_tiles_x;
+    step /= pl.n_tiles_x;
+    p.step_cy = step % pl.n_tiles_y;
+    step /= pl.n_tiles_y;
+    p.step_hi = step % g->H;
+    p.step_bi = step / g->H;
+  }
   p.status = status;
   // the Python layer hands a 4 KiB status buffer: words 0-3 status, bytes 16.. = 4 roles x 32 clock samples
   const Knobs kn = knobs();
@@ -424,7 +568,7 @@ const char* unsupported_reason(const swa_geom_t* g, const swa_rope_t* rope, cons
   if ((int64_t)g->t_height * g->t_width * g->b_size > (1 << 30)) return "grid too large";
   Plan pl;
   const bool v2 = prerotated || !(rope && rope->idx);
-  if (!(v2 ? make_plan_prerot(g, which == 0 ? nullptr : rope, which, &pl) : make_plan(g, rope, which, &pl)))
+  if (!(v2 ? make_plan_prerot(g, which, &pl) : make_plan(g, rope, which, &pl)))
     return "no tile plan fits (window too wide for one streamed block of the kernels with streamed rotation)";
   for (int i = 0; i < n_tensors; ++i)
     if (!tensor_ok(tensors[i], g->B, g->H)) return "tensors need unit last stride, positive strides and 16-byte aligned rows";
@@ -438,20 +582,21 @@ bool describe_plan(const swa_geom_t* g, const swa_rope_t* rope, int which, int32
   const int kind = which % 3;
   const bool v2 = prerot || !(rope && rope->idx);
   Plan pl;
-  if (!(v2 ? make_plan_prerot(g, kind == 0 ? nullptr : rope, kind, &pl) : make_plan(g, rope, kind, &pl))) return false;
+  if (!(v2 ? make_plan_prerot(g, kind, &pl) : make_plan(g, rope, kind, &pl))) return false;
   const uint32_t qch = (g->d_qk + 63) / 64, vch = (g->d_v + 63) / 64, N = pl.N;
-  const uint32_t pen = v2 ? (uint32_t)(pl.pen_rows + pl.pen_cols) * 32u : 0u;   // v1: inside the kernels' shared block
+  const uint32_t xrow = v2 ? 0u : kXRowBytes;                               // window-mask bytes per streamed token of a stage
+  const uint32_t x_fixed = v2 ? 8192u + 4u * pl.stg * kStageChunk + mask_bytes(pl.N) + row_parts_bytes(g->row_size, pl.R4) : 128u * kXRowBytes;
   uint32_t used = 1023, tmem = 0;   // worst-case pad to the 1024-byte alignment of the swizzled tiles
   if (kind == 0) {
-    used += 2 * qch * 16384u + 128u * kXRowBytes + pl.stages * N * ((qch + vch) * 128u + kXRowBytes);
-    used += (((v2 ? (uint32_t)sizeof(Fwd2Shared) : (uint32_t)sizeof(FwdShared)) + 15u) & ~15u) + pen;
+    used += 2 * qch * 16384u + x_fixed + pl.stages * N * ((qch + vch) * 128u + xrow);
+    used += ((v2 ? (uint32_t)sizeof(Fwd2Shared) : (uint32_t)sizeof(FwdShared)) + 15u) & ~15u;
     const uint32_t o_cols = vch * 64u;
-    const uint32_t stride = (N <= 128u && pl.nsb * 128u + 2 * o_cols <= 512u) ? 128u : N;
+    const uint32_t stride = v2 ? (uint32_t)pl.s_stride : (N <= 128u && pl.nsb * 128u + 2 * o_cols <= 512u) ? 128u : N;
     tmem = pl.nsb * stride + 2 * o_cols;
-    if (stride < N) tmem = 1u << 30;   // a score buffer would not hold a block
+    if (stride < N + (v2 ? pl.p_off / 2 : 0)) tmem = 1u << 30;   // a score buffer would not hold a block
   } else {
-    used += pl.nxb * (qch + vch) * 16384u + 128u * kXRowBytes + pl.stages * (N * ((qch + vch) * 128u + kXRowBytes) + 1024u);
-    used += (((v2 ? (uint32_t)sizeof(Bwd2Shared) : (uint32_t)sizeof(BwdShared)) + 15u) & ~15u) + pen + (v2 ? 2048u : 0u);
+    used += pl.nxb * (qch + vch) * 16384u + x_fixed + pl.stages * (N * ((qch + vch) * 128u + xrow) + (v2 ? 0u : 1024u));
+    used += (((v2 ? (uint32_t)sizeof(Bwd2Shared) : (uint32_t)sizeof(BwdShared)) + 15u) & ~15u) + (v2 && kind == 2 ? (kMaskRing + 2) * 1024u : 0u);
     tmem = 2 * 2 * N + 64u * qch + (kind == 2 ? 64u * vch : 0u);
   }
   used += pl.tab_bytes;
@@ -507,27 +652,32 @@ int launch_fwd(const swa_geom_t* g, const swa_rope_t* rope, const swa_tensor_t* 
 int launch_fwd2(const swa_geom_t* g, const swa_tensor_t* q, const swa_tensor_t* k, const swa_tensor_t* v,
                 const swa_tensor_t* o, float* lse, int32_t* status, cudaStream_t st) {
   Plan pl;
-  if (!make_plan_prerot(g, nullptr, 0, &pl)) {      // nothing is rotated: the plan of the problem without RoPE
+  if (!make_plan_prerot(g, 0, &pl)) {      // nothing is rotated: the plan of the problem without RoPE
     snprintf(g_tc_err, sizeof(g_tc_err), "no tile plan");
     return -1;
   }
-  CUtensorMap tq, tk, tv;
-  if (!make_map(&tq, q, g, g->d_qk, pl.TW, pl.TH) || !make_map(&tk, k, g, g->d_qk, pl.KW, pl.KR) ||
-      !make_map(&tv, v, g, g->d_v, pl.KW, pl.KR))
+  CUtensorMap tq, tk, tv, to;
+  if (!make_map(&tq, q, g, g->d_qk, pl.TW, pl.R4) || !make_map(&tk, k, g, g->d_qk, pl.KW, pl.KR) ||
+      !make_map(&tv, v, g, g->d_v, pl.KW, pl.KR) || !make_map(&to, o, g, g->d_v, pl.TW, pl.R4))
     return -1;
   const KParams p = make_params(g, nullptr, pl, status);
   const int sms = sm_count();
   dim3 grid(p.n_items < sms ? p.n_items : sms), block(kFwdThreads);   // persistent: one CTA per SM walks the items
-  auto kern = g->dtype == SWA_BF16 ? fwd2_kernel<true> : fwd2_kernel<false>;
+  const bool one = p.qch == 1 && p.vch == 1;
+  using FwdKernel = void (*)(const CUtensorMap, const CUtensorMap, const CUtensorMap, const CUtensorMap, const KParams, const View4, float*);
+  static const FwdKernel table[2][2][2] = {   // [dtype][heads of at most 64][P in columns of its own]
+      {{fwd2_kernel<false, false, false>, fwd2_kernel<false, false, true>}, {fwd2_kernel<false, true, false>, fwd2_kernel<false, true, true>}},
+      {{fwd2_kernel<true, false, false>, fwd2_kernel<true, false, true>}, {fwd2_kernel<true, true, false>, fwd2_kernel<true, true, true>}}};
+  const FwdKernel kern = table[g->dtype == SWA_BF16 ? 1 : 0][one ? 1 : 0][pl.p_off ? 1 : 0];
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)pl.smem_bytes);
   if (e != cudaSuccess) {
     snprintf(g_tc_err, sizeof(g_tc_err), "cudaFuncSetAttribute(%u bytes): %s", pl.smem_bytes, cudaGetErrorString(e));
     return -1;
   }
   if (knobs().verbose)
-    fprintf(stderr, "[swa2d] fwd2 plan: tile %dx%d, block %dx%d (N=%d), stages %d, score buffers %d, smem %u, %d items on %u CTAs\n",
-            pl.TH, pl.TW, pl.KR, pl.KW, pl.N, pl.stages, pl.nsb, pl.smem_bytes, p.n_items, grid.x);
-  kern<<<grid, block, pl.smem_bytes, st>>>(tq, tk, tv, p, make_view(o), lse);
+    fprintf(stderr, "[swa2d] fwd2 plan: tile %dx%d, block %dx%d (N=%d), stages %d, score buffers %d, %d quarters per chunk, smem %u, %d items on %u CTAs\n",
+            pl.TH, pl.TW, pl.KR, pl.KW, pl.N, pl.stages, pl.nsb, pl.nq, pl.smem_bytes, p.n_items, grid.x);
+  kern<<<grid, block, pl.smem_bytes, st>>>(tq, tk, tv, to, p, make_view(o), lse);
   return 0;
 }
 
@@ -541,12 +691,13 @@ int launch_bwd(const swa_geom_t* g, const swa_rope_t* rope, bool prerotated, con
                const swa_tensor_t* out_qk, const swa_tensor_t* out_v, int32_t* status, cudaStream_t st) {
   Plan pl;
   const bool v2 = prerotated || !(rope && rope->idx);      // the kernels without streamed rotation
-  if (!(v2 ? make_plan_prerot(g, rope, DKDV ? 2 : 1, &pl) : make_plan(g, rope, DKDV ? 2 : 1, &pl))) {
+  if (!(v2 ? make_plan_prerot(g, DKDV ? 2 : 1, &pl) : make_plan(g, rope, DKDV ? 2 : 1, &pl))) {
     snprintf(g_tc_err, sizeof(g_tc_err), "no tile plan");
     return -1;
   }
   CUtensorMap mxqk, mxv, myqk, myv;
-  if (!make_map(&mxqk, xqk, g, g->d_qk, pl.TW, pl.TH) || !make_map(&mxv, xv, g, g->d_v, pl.TW, pl.TH) ||
+  const int x_rows = v2 ? pl.R4 : pl.TH;                    // the strip kernels load the resident side quarter by quarter
+  if (!make_map(&mxqk, xqk, g, g->d_qk, pl.TW, x_rows) || !make_map(&mxv, xv, g, g->d_v, pl.TW, x_rows) ||
       !make_map(&myqk, yqk, g, g->d_qk, pl.KW, pl.KR) || !make_map(&myv, yv, g, g->d_v, pl.KW, pl.KR))
     return -1;
   const KParams p = make_params(g, rope, pl, status);
@@ -554,28 +705,36 @@ int launch_bwd(const swa_geom_t* g, const swa_rope_t* rope, bool prerotated, con
   dim3 grid(p.n_items < sms ? p.n_items : sms), block(kBwdThreads);   // persistent: one CTA per SM walks the items
   using BwdKernel = void (*)(const CUtensorMap, const CUtensorMap, const CUtensorMap, const CUtensorMap, KParams, const float*,
                              const float*, View4, View4);
+  using StripKernel = void (*)(const CUtensorMap, const CUtensorMap, const CUtensorMap, const CUtensorMap, const CUtensorMap,
+                               const CUtensorMap, const KParams, const float*, const float*);
   // [dtype][tables staged][n_rdim / 8]: q / k rotated in shared memory, dQ / dK rotated back in the epilogue
   static const BwdKernel fused_table[2][2][5] = {
       {{nullptr, bwd_kernel<false, DKDV, 1, false>, bwd_kernel<false, DKDV, 2, false>, nullptr, bwd_kernel<false, DKDV, 4, false>},
        {nullptr, bwd_kernel<false, DKDV, 1, true>, bwd_kernel<false, DKDV, 2, true>, nullptr, bwd_kernel<false, DKDV, 4, true>}},
       {{nullptr, bwd_kernel<true, DKDV, 1, false>, bwd_kernel<true, DKDV, 2, false>, nullptr, bwd_kernel<true, DKDV, 4, false>},
        {nullptr, bwd_kernel<true, DKDV, 1, true>, bwd_kernel<true, DKDV, 2, true>, nullptr, bwd_kernel<true, DKDV, 4, true>}}};
-  // [dtype][n_rdim / 8]: no RoPE, or inputs already rotated and only the epilogue rotation
-  static const BwdKernel prerot_table[2][2][5] = {
+  // [dtype][heads of at most 64][n_rdim / 8]: no RoPE, or inputs already rotated and only the epilogue rotation
+  static const StripKernel prerot_table[2][2][5] = {
       {{bwd2_kernel<false, DKDV, 0, false>, bwd2_kernel<false, DKDV, 1, false>, bwd2_kernel<false, DKDV, 2, false>, nullptr,
         bwd2_kernel<false, DKDV, 4, false>},
-       {bwd2_kernel<false, DKDV, 0, false>, bwd2_kernel<false, DKDV, 1, true>, bwd2_kernel<false, DKDV, 2, true>, nullptr,
-        bwd2_kernel<false, DKDV, 4, true>}},
+       {bwd2_kernel<false, DKDV, 0, true>, bwd2_kernel<false, DKDV, 1, true>, bwd2_kernel<false, DKDV, 2, true>, nullptr, nullptr}},
       {{bwd2_kernel<true, DKDV, 0, false>, bwd2_kernel<true, DKDV, 1, false>, bwd2_kernel<true, DKDV, 2, false>, nullptr,
         bwd2_kernel<true, DKDV, 4, false>},
-       {bwd2_kernel<true, DKDV, 0, false>, bwd2_kernel<true, DKDV, 1, true>, bwd2_kernel<true, DKDV, 2, true>, nullptr,
-        bwd2_kernel<true, DKDV, 4, true>}}};
+       {bwd2_kernel<true, DKDV, 0, true>, bwd2_kernel<true, DKDV, 1, true>, bwd2_kernel<true, DKDV, 2, true>, nullptr, nullptr}}};
   const int ni = (rope && rope->idx) ? rope->n_rdim / 8 : 0;
   const int bf = g->dtype == SWA_BF16 ? 1 : 0;
-  BwdKernel kern = (prerotated || ni == 0) ? prerot_table[bf][pl.tab_bytes ? 1 : 0][ni] : fused_table[bf][pl.tab_bytes ? 1 : 0][ni];
+  const BwdKernel kern1 = v2 ? nullptr : fused_table[bf][pl.tab_bytes ? 1 : 0][ni];
+  const StripKernel kern2 = v2 ? prerot_table[bf][p.qch == 1 && p.vch == 1 ? 1 : 0][ni] : nullptr;
+  const void* kern = v2 ? (const void*)kern2 : (const void*)kern1;
   if (kern == nullptr) {
     snprintf(g_tc_err, sizeof(g_tc_err), "n_rdim %d has no tensor-core kernel", rope ? rope->n_rdim : 0);
     return -1;
+  }
+  CUtensorMap moqk, mov;                                     // outputs of the strip kernels
+  if (v2) {
+    if (!make_map(&moqk, out_qk, g, g->d_qk, pl.TW, pl.R4)) return -1;
+    mov = moqk;
+    if (DKDV && !make_map(&mov, out_v, g, g->d_v, pl.TW, pl.R4)) return -1;
   }
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)pl.smem_bytes);
   if (e != cudaSuccess) {
@@ -583,10 +742,13 @@ int launch_bwd(const swa_geom_t* g, const swa_rope_t* rope, bool prerotated, con
     return -1;
   }
   if (knobs().verbose)
-    fprintf(stderr, "[swa2d] %s plan: tile %dx%d, block %dx%d (N=%d), stages %d, nsb %d, nxb %d, tables %u, smem %u, %d items on %u CTAs\n",
-            DKDV ? "dkdv" : "dq", pl.TH, pl.TW, pl.KR, pl.KW, pl.N, pl.stages, pl.nsb, pl.nxb, pl.tab_bytes, pl.smem_bytes, p.n_items, grid.x);
-  kern<<<grid, block, pl.smem_bytes, st>>>(mxqk, mxv, myqk, myv, p, lse, delta, make_view(out_qk),
-                                          out_v ? make_view(out_v) : View4{nullptr, 0, 0, 0, 0});
+    fprintf(stderr, "[swa2d] %s plan: tile %dx%d, block %dx%d (N=%d), stages %d, nsb %d, nxb %d, %d quarters per chunk, tables %u, smem %u, %d items on %u CTAs\n",
+            DKDV ? "dkdv" : "dq", pl.TH, pl.TW, pl.KR, pl.KW, pl.N, pl.stages, pl.nsb, pl.nxb, pl.nq, pl.tab_bytes, pl.smem_bytes, p.n_items, grid.x);
+  if (v2)
+    kern2<<<grid, block, pl.smem_bytes, st>>>(mxqk, mxv, myqk, myv, moqk, mov, p, lse, delta);
+  else
+    kern1<<<grid, block, pl.smem_bytes, st>>>(mxqk, mxv, myqk, myv, p, lse, delta, make_view(out_qk),
+                                              out_v ? make_view(out_v) : View4{nullptr, 0, 0, 0, 0});
   return 0;
 }
 

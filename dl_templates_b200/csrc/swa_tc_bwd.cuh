@@ -73,7 +73,7 @@ bwd_kernel(const __grid_constant__ CUtensorMap tm_xqk, const __grid_constant__ C
   constexpr int R = 8 * NI;
   constexpr int Rd = NI > 0 ? R : 1;   // divisor that stays legal when there is no rotation
   extern __shared__ uint8_t smem_raw[];
-  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+  uint8_t* smem = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);   // an offset: the compiler keeps seeing shared memory
   const Plan& pl = p.pl;
   const int N = pl.N, nxb = pl.nxb;
   constexpr int nsb = 2;                                         // (S, dP) buffer pairs; the planner sizes N so that two fit

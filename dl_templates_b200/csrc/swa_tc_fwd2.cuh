@@ -1,128 +1,121 @@
 // tcgen05 forward kernel for inputs that need no rotation in shared memory: q and k are either not
-// rotated at all or are the rotated copies a streaming pass left behind (swa_fwd_rot).  Same mathematics,
-// tile geometry, window mask and tensor-memory layout as fwd_kernel (swa_tc_fwd.cuh); what differs is who
-// does what:
+// rotated at all or are the rotated copies a streaming pass left behind (swa_fwd_rot).  Geometry (strips, quarters,
+// slots): swa_tc_strip.cuh.
 //
-//   warp 0        TMA producer: query tile (double-buffered) and the ring of K / V halo blocks
+//   warp 0        TMA producer: K / V blocks, quarters of query rows
 //   warp 1        SCORE issuer: S = Q K^T (+ the window mask as 32 extra contraction columns)
 //   warp 2        PV issuer:    O_g += P V with P read from tensor memory
+//   warp 3        window-mask units of every streamed block
 //   warps 4-11    two softmax groups on alternate blocks, one thread per query row each, each with its own
 //                 running maximum / sum and its own accumulator O_g
-//   warps 12-15   one thread per row: window-mask penalty rows of every streamed block, and the EPILOGUE of
-//                 every item: the two groups' partial results are merged (in an order fixed by block
-//                 position), normalised and stored
+//   warps 12-15   EPILOGUE, one warp per slot: the two groups' partial results of a quarter are merged (in an order fixed by
+//                 the blocks' positions in the grid), normalised and stored
 //
-// An item has only five to seven streamed blocks.  One warp issuing every MMA ran a dependent scalar
-// instruction stream of about 2000 cycles per block while the tensor pipe needs less than half of
-// that, and an epilogue inside the softmax groups idled both at every item boundary; hence two issuers
-// (the order a single issuer gave for free becomes the barrier s_free) and epilogue warps.
+// One warp issuing every MMA ran a dependent scalar instruction stream of about 2000 cycles per block while the
+// tensor pipe needs less than half of that, and an epilogue inside the softmax groups idled both at every item
+// boundary; hence two issuers (the order a single issuer gave for free becomes the barrier s_free) and epilogue warps.
 // Measured and dropped: two threads per query row, each on half of every block's columns with the row maximum
 // exchanged through shared memory (the softmax phase of a block halves, but both groups then work on the SAME
 // block and the blocks of an item become strictly sequential: 1.47 ms per launch against 1.17 ms); rotating the
-// query tile in warps 12-15 as well (about 400 dependent instructions
-// per row cost 2700 cycles per item on the critical path, 1.1 ms per launch at the default workload,
-// against 0.1 ms for a streaming pass over q), and a single warp writing all mask rows right behind the
-// producer (four rows per lane made it the slowest role of the kernel).
+// query tile in this kernel as well (about 400 dependent instructions per row on the critical path, 1.1 ms per launch
+// at the default workload, against 0.1 ms for a streaming pass over q).
 //
 // All waits are bounded; a timed-out wait raises a CTA-wide abort flag, every role runs its loops to the
 // end without touching anything, TMEM is freed and the status word records it.
 #pragma once
 
 #include "swa_tc_fwd.cuh"
+#include "swa_tc_strip.cuh"
 
 namespace swa {
 namespace tc {
 
 struct Fwd2Shared {
   uint64_t q_full[2], q_empty[2];
-  uint64_t kv_full[kMaxStages], k_ready[kMaxStages], kv_empty[kMaxStages], kx_free[kMaxStages];
-  uint64_t s_full[4], p_full[4], s_free[4], pv_done[2], o_full, o_free, ml_full[2], ml_empty[2];
-  float ml[2][2][2][128];   // [item parity][group][maximum | sum][row]: handed to the epilogue warps
+  uint64_t kv_full[kMaxStages], kv_empty[kMaxStages], k_ready[kMaskRing], kx_free[kMaskRing];
+  uint64_t s_full[4], p_full[4], s_free[4], pv_done[2];
+  uint64_t o_full[4], o_free[4];        // per slot: the quarter in it is complete / has been read
+  // [quarter parity][slot]: running maximum and sum handed over, per group; read.  The softmax groups run up to nsb blocks ahead of
+  // the PV MMAs -- with small windows that is several quarters of a slot -- so a barrier per slot alone could complete twice
+  // before the epilogue warp looks.
+  uint64_t ml_full[2][4][2], ml_empty[2][4];
+  float ml[2][4][2][2][32];             // [quarter parity][slot][group][maximum | sum][row]
+  ItemStart start;
   uint32_t tmem_base;
   int abort_flag;
 };
 
-template <bool BF16>
+// ONE: heads of at most 64 (one 64-column chunk per tensor); OWNP: P has columns of its own behind the scores.
+template <bool BF16, bool ONE, bool OWNP>
 __global__ void __launch_bounds__(kFwdThreads, 1)
 fwd2_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
-            const __grid_constant__ CUtensorMap tm_v, KParams p, View4 o, float* __restrict__ lse) {
+            const __grid_constant__ CUtensorMap tm_v, const __grid_constant__ CUtensorMap tm_o,
+            const __grid_constant__ KParams p, const __grid_constant__ View4 o, float* __restrict__ lse) {
   using namespace ptx;
   extern __shared__ uint8_t smem_raw[];
-  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+  uint8_t* smem = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);   // an offset: the compiler keeps seeing shared memory
   const Plan& pl = p.pl;
-  const int N = pl.N;
+  const int N = pl.N, qch = ONE ? 1 : p.qch, vch = ONE ? 1 : p.vch;
   const uint32_t blk_bytes = (uint32_t)N * 128u;               // one 64-wide chunk of a streamed block
-  const uint32_t q_bytes = p.qch * 16384u;
-  const uint32_t k_stage = blk_bytes * p.qch, v_stage = blk_bytes * p.vch;
-  const uint32_t kx_stage = (uint32_t)N * kXRowBytes;           // window-mask penalty rows of a streamed block
-  const uint32_t o_cols = p.vch * 64u;                           // TMEM columns of one O accumulator
+  const uint32_t q_bytes = qch * 16384u;
+  const uint32_t k_stage = blk_bytes * qch, v_stage = blk_bytes * vch;
+  const uint32_t o_cols = vch * 64u;                           // TMEM columns of one O accumulator
   const int nsb = pl.nsb;                                        // score buffers = look-ahead of the score MMAs
-  // score buffer b at column s_stride*b (128-column strides when they fit, else packed), O_g behind them
-  const uint32_t s_stride = (N <= 128 && nsb * 128u + 2 * o_cols <= kFwdTmemCols) ? 128u : (uint32_t)N;
+  // Score buffer b at column s_stride * b, O_g behind the buffers.  P gets columns of its own behind the scores when tensor
+  // memory allows (p_off = N), so that the scores survive until it is certain that they need not be read again; else P is
+  // written over them.
+  const uint32_t s_stride = pl.s_stride, p_off = OWNP ? N : 0;
   const uint32_t o_base = nsb * s_stride;
+  const uint32_t ub = unit_bytes(pl);
   uint8_t* q_smem = smem;                                        // two buffers
-  uint8_t* qx_smem = q_smem + 2 * q_bytes;                      // window-mask indicator rows of a query tile
-  uint8_t* k_smem = qx_smem + 128 * kXRowBytes;
+  uint8_t* stg_smem = q_smem + 2 * q_bytes;                     // output staging, pl.stg chunks per epilogue warp
+  uint8_t* k_smem = stg_smem + 4 * pl.stg * kStageChunk;
   uint8_t* v_smem = k_smem + pl.stages * k_stage;
-  uint8_t* kx_smem = v_smem + pl.stages * v_stage;
-  Fwd2Shared* sh = reinterpret_cast<Fwd2Shared*>(kx_smem + pl.stages * kx_stage);
-  PenView pen;                                                   // window-mask penalty parts of the current item's halo
-  pen.row = reinterpret_cast<uint4*>(reinterpret_cast<uint8_t*>(sh) + ((sizeof(Fwd2Shared) + 15) & ~size_t(15)));
-  pen.col = pen.row + 2 * pl.pen_rows;
-  pen.n_rows = pl.pen_rows;
-  pen.n_cols = pl.pen_cols;
-  volatile int* abort_flag = &sh->abort_flag;
+  uint8_t* qx_smem = v_smem + pl.stages * v_stage;              // window mask: indicator units of the query rows,
+  uint8_t* kr_smem = qx_smem + 8192;                            // ... row units of the mask ring,
+  uint8_t* kc_smem = kr_smem + kMaskRing * ub * (pl.TH >> 3);   // ... column units,
+  uint8_t* kz_smem = kc_smem + kMaskRing * ub * (pl.TW >> 3);  // ... the unused unit
+  Fwd2Shared* sh = reinterpret_cast<Fwd2Shared*>(kz_smem + ub);
+  uint8_t* row_parts = reinterpret_cast<uint8_t*>(sh) + ((sizeof(Fwd2Shared) + 15) & ~size_t(15));
 
   const int warp = threadIdx.x >> 5;
 
+  constexpr int n_bars = offsetof(Fwd2Shared, ml) / 8, warps4 = offsetof(Fwd2Shared, p_full) / 8;   // p_full: one arrival per warp
+  for (int i = threadIdx.x; i < n_bars; i += kFwdThreads)
+    mbar_init(reinterpret_cast<uint64_t*>(sh) + i, i >= warps4 && i < warps4 + 4 ? 4 : 1);
   if (threadIdx.x == 0) {
-    for (int s = 0; s < 2; ++s) {
-      mbar_init(&sh->q_full[s], 1);
-      mbar_init(&sh->q_empty[s], 1);
-      mbar_init(&sh->pv_done[s], 1);
-      mbar_init(&sh->ml_full[s], 256);
-      mbar_init(&sh->ml_empty[s], 128);
-    }
-    for (int s = 0; s < 4; ++s) {
-      mbar_init(&sh->s_full[s], 1);
-      mbar_init(&sh->p_full[s], 128);
-      mbar_init(&sh->s_free[s], 1);
-    }
-    mbar_init(&sh->o_full, 1);
-    mbar_init(&sh->o_free, 128);
-    for (int s = 0; s < kMaxStages; ++s) {
-      mbar_init(&sh->kv_full[s], 1);
-      mbar_init(&sh->k_ready[s], 128);
-      mbar_init(&sh->kv_empty[s], 1);
-      mbar_init(&sh->kx_free[s], 1);
-    }
     sh->abort_flag = 0;
-    fence_barrier_init();
+    item_start(p, &sh->start);
   }
+  fence_barrier_init();
   if (warp == 1) {
     tmem_alloc(&sh->tmem_base, kFwdTmemCols);
     tmem_relinquish();
   }
+  build_row_parts<BF16>(row_parts, threadIdx.x, kFwdThreads, p);
+  if (threadIdx.x < 128) {
+    write_indicator_units<BF16>(qx_smem, threadIdx.x, p);
+    if ((int)threadIdx.x < N) *reinterpret_cast<uint4*>(kz_smem + threadIdx.x * 16) = make_uint4(0u, 0u, 0u, 0u);
+  }
+  fence_proxy_async_smem();
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem = sh->tmem_base;
 
-  bool ok = true;   // warp-uniform: a failed wait does not leave the loops, every later wait returns at once
+  bool ok = true;   // warp-uniform: a failed wait does not leave the loops, but nothing is waited for or touched any more
   auto wait_spin = [&](uint64_t* bar, uint32_t parity) {
-    const bool r = ok && mbar_wait<0>(bar, parity, abort_flag);
-    ok = __all_sync(0xffffffffu, r);
+    if (ok) ok = __all_sync(0xffffffffu, mbar_wait_polls<0>(smem_u32(bar), parity));
   };
   auto wait_park = [&](uint64_t* bar, uint32_t parity) {
-    const bool r = ok && mbar_wait<100>(bar, parity, abort_flag);
-    ok = __all_sync(0xffffffffu, r);
+    if (ok) ok = __all_sync(0xffffffffu, mbar_wait_polls<100>(smem_u32(bar), parity));
   };
-  const int n_items = p.n_items, tiles_per_head = pl.n_tiles_x * pl.n_tiles_y;
+  const int n_mine = sh->start.count;
 
-  // Registers follow the work: producer / issuer warpgroup 80, the two softmax warpgroups 152, the
-  // rotation + mask + epilogue warpgroup keeps 128: (80 + 2 * 152 + 128) * 128 = 64 Ki.
+  // Registers follow the work: producer / issuer / mask warpgroup 104, softmax 120, epilogue 168:
+  // (104 + 2 * 120 + 168) * 128 = 64 Ki.
   if (warp >= 4 && warp < 12) {
-    setmaxnreg_inc<152>();
+    setmaxnreg_dec<120>();
     // ------------------------------------------------------------------ softmax, one thread per query row and group
     const int lane = threadIdx.x & 31;
     const int g = (warp - 4) >> 2;                // group: takes the blocks whose stream position has parity g
@@ -133,19 +126,20 @@ fwd2_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CU
     const uint32_t o_tm = lane_base + o_base + g * o_cols;
     const float c2 = p.scale_log2;
     const int ng = N >> 4;                        // 16-column granules of a row
-    uint32_t gbase = 0;                           // stream position of the current item's block 0
+    uint32_t gbase = 0, q0 = 0;                   // stream position of the current item's block 0, quarters before it
     uint32_t own_next = g, n_own = 0;             // this group's next block in the stream; blocks done so far
     int sbuf = g % nsb, spar = 0;                 // ... its score buffer and that buffer's barrier parity
     int tn = 0;
+    float m_used = -INFINITY, l = 0.f;
+    ItemWalk w(sh->start);
 #pragma unroll 1
-    for (int it = 0, item = blockIdx.x; item < n_items; ++it, item += gridDim.x) {
-      const TilePos tp = tile_pos(p, item % tiles_per_head);
-      // rows of the grid the 32 queries of this warp can see
-      const int see_lo = tp.r0 + (quarter * 32) / pl.TW - p.wr, see_hi = tp.r0 + (quarter * 32 + 31) / pl.TW + p.wr;
-      float m_used = -INFINITY, l = 0.f;
-      int cnt = 0;                                // blocks of this item this group has handed to the PV MMA
+    for (int it = 0; it < n_mine; ++it, w.next(p)) {
+      const StripItem si = strip_item(p, w);
+      // this warp's slot holds the quarters qi, qi + 4, ...; [q_lo, q_hi] = the blocks quarter qi takes part in
+      int qi = (quarter - (int)q0) & 3;
+      int q_lo = quarter_first(p, si, qi), q_hi = quarter_last(p, si, qi);
 #pragma unroll 1
-      for (int j = (int)(own_next - gbase); j < tp.nblk; j += 2, own_next += 2, ++n_own, ++cnt) {
+      for (int j = (int)(own_next - gbase); j < si.nblk; j += 2, own_next += 2, ++n_own) {
         const uint32_t s_tm = lane_base + sbuf * s_stride;
         uint64_t* const p_bar = &sh->p_full[sbuf];
         trace_ev(p, 2 + g, tn, m == 0 && it >= p.trace_it, 0 * 16 + (j & 15));
@@ -153,205 +147,201 @@ fwd2_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CU
         trace_ev(p, 2 + g, tn, m == 0 && it >= p.trace_it, 1 * 16 + (j & 15));
         sbuf += 2;                                // two positions on in the ring of nsb buffers
         if (sbuf >= nsb) { sbuf -= nsb; spar ^= 1; }
-        int band, cblk;
-        block_pos(pl, j, band, cblk);
-        const int blk_first = tp.hr_first + band * pl.KR, blk_last = blk_first + pl.KR - 1;
-        const bool seen = !(blk_last < see_lo || blk_first > see_hi);
-        if (ok) {
-          tc_fence_after();
-          uint32_t ra[16], rb[16];
-          if (!seen) {
-#pragma unroll
-            for (int i = 0; i < 8; ++i) ra[i] = 0u;
 #pragma unroll 1
-            for (int c0 = 0; c0 < (N >> 1); c0 += 8) tmem_st8(s_tm + c0, ra);
-          } else {
-            // Two passes over the row in 16-column granules, the load of granule i+1 in flight while
-            // granule i is worked on (a TMEM load takes ~150 cycles to come back).
-            // pass 1: row maximum
+        while (qi < si.nq && q_hi < j) {          // the quarter has left the slot: its successor
+          qi += 4;
+          q_lo = quarter_first(p, si, qi);
+          q_hi = quarter_last(p, si, qi);
+        }
+        // a quarter that takes no part in the block: its rows of P are never read (umma_ts_slots)
+        const bool seen = qi < si.nq && q_lo <= j;
+        if (ok && seen) {
+          const bool first = j - q_lo < 2;        // this group's first block of the quarter
+          if (first) { m_used = -INFINITY; l = 0.f; }
+          tc_fence_after();
+          uint32_t r[16];
+          float mx = -INFINITY, bl;
+          // The row maximum is taken before the exponentials in every block when P overwrites the scores, else only in a group's
+          // first block of a quarter: the others use the running maximum and see afterwards whether it still serves: a row
+          // whose maximum has grown by more than 2^8 is done again, which is rare.  16 columns at a time, the load of the next
+          // 16 in flight while these are worked on.
+          bool exact = !OWNP || first;
+          tmem_ld16(s_tm, r);
+          if (exact) {
+            uint32_t t[16];
             float mx4[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
-            tmem_ld16(s_tm, ra);
 #pragma unroll 1
             for (int i = 0; i < ng; i += 2) {
               tmem_wait_ld();
-              if (i + 1 < ng) tmem_ld16(s_tm + 16 * (i + 1), rb);
+              if (i + 1 < ng) tmem_ld16(s_tm + 16 * (i + 1), t);
 #pragma unroll
-              for (int e = 0; e < 16; ++e) mx4[e & 3] = fmaxf(mx4[e & 3], __uint_as_float(ra[e]));
+              for (int e = 0; e < 8; ++e) mx4[e & 3] = fmaxf(mx4[e & 3], fmaxf(__uint_as_float(r[2 * e]), __uint_as_float(r[2 * e + 1])));
               if (i + 1 < ng) {
                 tmem_wait_ld();
-                if (i + 2 < ng) tmem_ld16(s_tm + 16 * (i + 2), ra);
+                if (i + 2 < ng) tmem_ld16(s_tm + 16 * (i + 2), r);
 #pragma unroll
-                for (int e = 0; e < 16; ++e) mx4[e & 3] = fmaxf(mx4[e & 3], __uint_as_float(rb[e]));
+                for (int e = 0; e < 8; ++e) mx4[e & 3] = fmaxf(mx4[e & 3], fmaxf(__uint_as_float(t[2 * e]), __uint_as_float(t[2 * e + 1])));
               }
             }
-            tmem_ld16(s_tm, ra);                            // first granule of pass 2, in flight during the bookkeeping
-            float mx = fmaxf(fmaxf(mx4[0], mx4[1]), fmaxf(mx4[2], mx4[3]));
-            if (mx < none_thresh) mx = -INFINITY;
-            // running max with lazy rescale: keep scaling by m_used until the true max exceeds it by 2^8
-            bool need = false;
-            float m_new = m_used;
-            if (mx > m_used) {
-              if (m_used == -INFINITY) m_used = mx;          // nothing accumulated yet for this row
-              else if ((mx - m_used) * c2 > kRescaleThreshold) { need = true; m_new = mx; }
-            }
-            if (__any_sync(0xffffffffu, need) && cnt > 0) {
-              // O_g must be at rest: wait for the PV MMA of this group's previous block, then scale the row
-              wait_spin(&sh->pv_done[g], (n_own - 1) & 1);
-              if (ok) {
-                tc_fence_after();
-                const float alpha = need ? exp2f((m_used - m_new) * c2) : 1.f;
-                tmem_wait_ld();
+            mx = fmaxf(fmaxf(mx4[0], mx4[1]), fmaxf(mx4[2], mx4[3]));
+            tmem_ld16(s_tm, r);                             // first 16 columns, in flight during the bookkeeping
+          }
 #pragma unroll 1
-                for (int c = 0; c < (int)o_cols; c += 16) {
-                  tmem_ld16(o_tm + c, rb);
+          while (true) {
+            if (exact) {
+              if (mx < none_thresh) mx = -INFINITY;
+              // running max with lazy rescale: keep scaling by m_used until the true max exceeds it by 2^8
+              bool need = false;
+              float m_new = m_used;
+              if (mx > m_used) {
+                if (m_used == -INFINITY) m_used = mx;       // nothing accumulated yet for this row
+                else if ((mx - m_used) * c2 > kRescaleThreshold) { need = true; m_new = mx; }
+              }
+              if (__any_sync(0xffffffffu, need) && !first) {
+                // O_g must be at rest: wait for the PV MMA of this group's previous block, then scale the row
+                wait_spin(&sh->pv_done[g], (n_own - 1) & 1);
+                if (ok) {
+                  tc_fence_after();
+                  const float alpha = need ? exp2f((m_used - m_new) * c2) : 1.f;
                   tmem_wait_ld();
+#pragma unroll 1
+                  for (int c = 0; c < (int)o_cols; c += 16) {
+                    uint32_t t[16];
+                    tmem_ld16(o_tm + c, t);
+                    tmem_wait_ld();
 #pragma unroll
-                  for (int e = 0; e < 16; ++e) rb[e] = __float_as_uint(__uint_as_float(rb[e]) * alpha);
-                  tmem_st16(o_tm + c, rb);
+                    for (int e = 0; e < 16; ++e) t[e] = __float_as_uint(__uint_as_float(t[e]) * alpha);
+                    tmem_st16(o_tm + c, t);
+                  }
+                  if (need) { m_used = m_new; l *= alpha; }
                 }
-                if (need) { m_used = m_new; l *= alpha; }
               }
             }
             const float mc = (m_used == -INFINITY) ? 0.f : m_used * c2;
-            // pass 2: P = exp2(S*c - m), row sum, packed in place (P column c/2 <- S columns c, c+1)
-            float ls4[4] = {0.f, 0.f, 0.f, 0.f};
+            const uint64_t c22 = f2_pack(c2, c2), nmc2 = f2_pack(-mc, -mc);
+            // P = exp2(S*c - m), its row sum, (OWNP) the row maximum of S*c - m; packed, two columns of P per word
+            uint64_t ls[2] = {0ull, 0ull};
+            float mx2[2] = {-INFINITY, -INFINITY};
 #pragma unroll 1
-            for (int i = 0; i < ng; i += 2) {
+            for (int i = 0; i < ng; ++i) {
+              uint64_t e[8];
+              uint32_t w[8];
               tmem_wait_ld();
-              if (i + 1 < ng) tmem_ld16(s_tm + 16 * (i + 1), rb);
+#pragma unroll
+              for (int h = 0; h < 8; ++h) e[h] = f2_fma(f2_pack(__uint_as_float(r[2 * h]), __uint_as_float(r[2 * h + 1])), c22, nmc2);
+              if (i + 1 < ng) tmem_ld16(s_tm + 16 * (i + 1), r);
 #pragma unroll
               for (int h = 0; h < 8; ++h) {
-                const float p0 = exp2f(fmaf(__uint_as_float(ra[2 * h]), c2, -mc));
-                const float p1 = exp2f(fmaf(__uint_as_float(ra[2 * h + 1]), c2, -mc));
-                ls4[h & 3] += p0 + p1;
-                ra[h] = pack2<BF16>(p0, p1);
+                const float2 x = f2_unpack(e[h]);
+                if constexpr (OWNP) mx2[h & 1] = fmaxf(mx2[h & 1], fmaxf(x.x, x.y));
+                const float p0 = exp2f(x.x), p1 = exp2f(x.y);
+                ls[h & 1] = f2_add(ls[h & 1], f2_pack(p0, p1));
+                w[h] = pack2<BF16>(p0, p1);
               }
-              tmem_st8(s_tm + 8 * i, ra);
-              if (i + 1 < ng) {
-                tmem_wait_ld();
-                if (i + 2 < ng) tmem_ld16(s_tm + 16 * (i + 2), ra);
-#pragma unroll
-                for (int h = 0; h < 8; ++h) {
-                  const float p0 = exp2f(fmaf(__uint_as_float(rb[2 * h]), c2, -mc));
-                  const float p1 = exp2f(fmaf(__uint_as_float(rb[2 * h + 1]), c2, -mc));
-                  ls4[h & 3] += p0 + p1;
-                  rb[h] = pack2<BF16>(p0, p1);
-                }
-                tmem_st8(s_tm + 8 * (i + 1), rb);
-              }
+              tmem_st8(s_tm + p_off + 8 * i, w);
             }
-            l += (ls4[0] + ls4[1]) + (ls4[2] + ls4[3]);
+            const float2 l2 = f2_unpack(f2_add(ls[0], ls[1]));
+            bl = l2.x + l2.y;
+            if (exact) break;
+            // rows whose maximum passes the threshold (or that had none yet) are done again with the true one
+            const float emx = fmaxf(mx2[0], mx2[1]);
+            const bool again = m_used == -INFINITY ? emx > none_thresh * c2 : emx > kRescaleThreshold;
+            if (!__any_sync(0xffffffffu, again)) break;
+            mx = again ? (emx + mc) / c2 : m_used;
+            exact = true;
+            tmem_ld16(s_tm, r);
+          }
+          l += bl;
+          const uint32_t Q = q0 + qi;
+          const int qp = (int)(Q >> 2) & 1;
+          if (q_hi - j < 2) {                     // its last one: hand maximum and sum to the epilogue warp
+            if (Q >= 8) wait_spin(&sh->ml_empty[qp][quarter], ((Q >> 3) - 1) & 1);
+            sh->ml[qp][quarter][g][0][lane] = m_used;
+            sh->ml[qp][quarter][g][1][lane] = l;
           }
           tmem_wait_st();
           tc_fence_before();
-          mbar_arrive(p_bar);
+          __syncwarp();
+          if (ok && q_hi - j < 2 && lane == 0) mbar_arrive(&sh->ml_full[qp][quarter][g]);
         }
+        if (ok && lane == 0) mbar_arrive(p_bar);
         trace_ev(p, 2 + g, tn, m == 0 && it >= p.trace_it, 2 * 16 + (j & 15));
       }
-      // hand this group's running maximum and sum of the item to the epilogue warps
-      if (it >= 2) wait_spin(&sh->ml_empty[it & 1], ((it >> 1) - 1) & 1);
-      if (ok) {
-        sh->ml[it & 1][g][0][m] = m_used;
-        sh->ml[it & 1][g][1][m] = l;
-        mbar_arrive(&sh->ml_full[it & 1]);
-      }
-      gbase += tp.nblk;
+      gbase += si.nblk;
+      q0 += si.nq;
     }
   } else if (warp < 4) {
-    setmaxnreg_dec<80>();
+    setmaxnreg_dec<104>();
     if (warp == 0) {
       // ------------------------------------------------------------------ TMA producer
-      if (elect_one()) {
-        prefetch_tmap(&tm_q);
-        prefetch_tmap(&tm_k);
-        prefetch_tmap(&tm_v);
-      }
-      __syncwarp();
-      int stage = 0, stage_par = 1;        // parity of the "empty" phase a refill of this stage waits for
-      bool ring_full = false;              // all stages have been filled once
-#pragma unroll 1
-      for (int it = 0, item = blockIdx.x; item < n_items; ++it, item += gridDim.x) {
-        const int bh = item / tiles_per_head, bi = bh / p.H, hi = bh - bi * p.H;
-        const TilePos tp = tile_pos(p, item - bh * tiles_per_head);
-        const int qb = it & 1;
-        if (it >= 2) wait_park(&sh->q_empty[qb], ((it >> 1) - 1) & 1);
-        if (ok && elect_one()) {
-          mbar_arrive_expect_tx(&sh->q_full[qb], q_bytes);
-#pragma unroll 1
-          for (int c = 0; c < p.qch; ++c)
-            tma_load_5d(q_smem + qb * q_bytes + c * 16384, &tm_q, &sh->q_full[qb], c * 64, tp.x0, tp.r0, hi, bi);
-        }
-        __syncwarp();
-#pragma unroll 1
-        for (int j = 0; j < tp.nblk; ++j) {
-          if (ring_full) wait_park(&sh->kv_empty[stage], stage_par);
-          if (ok && elect_one()) {
-            mbar_arrive_expect_tx(&sh->kv_full[stage], k_stage + v_stage);
-            int band, cblk;
-            block_pos(pl, j, band, cblk);
-            const int row = tp.hr_first + band * pl.KR, col = tp.hx0 + cblk * pl.KW;
-#pragma unroll 1
-            for (int c = 0; c < p.qch; ++c)
-              tma_load_5d(k_smem + stage * k_stage + c * blk_bytes, &tm_k, &sh->kv_full[stage], c * 64, col, row, hi, bi);
-#pragma unroll 1
-            for (int c = 0; c < p.vch; ++c)
-              tma_load_5d(v_smem + stage * v_stage + c * blk_bytes, &tm_v, &sh->kv_full[stage], c * 64, col, row, hi, bi);
-          }
-          __syncwarp();
-          if (++stage == pl.stages) { stage = 0; stage_par ^= 1; ring_full = true; }
-        }
-      }
+      const LoadArgs f{q_smem, q_bytes, q_bytes, k_smem, v_smem, k_stage, v_stage, blk_bytes, sh->q_full, sh->q_empty,
+                       sh->kv_full, sh->kv_empty, &sh->start, &tm_q, nullptr, &tm_k, &tm_v};
+      load_warp(p, f, ok);
     } else if (warp == 1) {
       // ------------------------------------------------------------------ score issuer
       const uint32_t fmt = BF16 ? 1u : 0u;
       const uint32_t idesc_s = instr_desc(fmt, 128, N, 0, 0);
-      const uint32_t hi_sw = smem_desc_hi(1024, true), hi_ns = smem_desc_hi(kXSbo, false);
+      const uint32_t hi_sw = smem_desc_hi(1024, true), hi_ns = smem_desc_hi(kUnitSbo, false);
       const uint64_t q_desc0 = smem_desc_from(smem_u32(q_smem), 16, hi_sw), k_desc0 = smem_desc_from(smem_u32(k_smem), 16, hi_sw),
-                     qx_desc0 = smem_desc_from(smem_u32(qx_smem), kXLbo, hi_ns), kx_desc0 = smem_desc_from(smem_u32(kx_smem), kXLbo, hi_ns);
-      const uint32_t k_stage16 = k_stage >> 4, kx_stage16 = kx_stage >> 4, blk16 = blk_bytes >> 4;
-      int s_it = 0, s_j = 0, s_nblk = 1, s_stage = 0, s_stage_par = 0, s_buf = 0;
-      uint32_t s_use = 0;                            // how often the ring of score buffers has wrapped
+                     qx_desc0 = smem_desc_from(smem_u32(qx_smem), 2048, hi_ns);
+      const uint32_t k_stage16 = k_stage >> 4, blk16 = blk_bytes >> 4;
+      const uint32_t kr0 = smem_u32(kr_smem), kc0 = smem_u32(kc_smem), kz0 = smem_u32(kz_smem);
+      int stage = 0, stage_par = 0, buf = 0, xb = 1, x_par = 1;   // query buffer in use; parity of its "full" phase
+      int mslot = 0, m_par = 0;
+      uint32_t use = 0;                              // how often the ring of score buffers has wrapped
       int tn = 0;
       const bool tl = (threadIdx.x & 31) == 0;
-      if (blockIdx.x < n_items) s_nblk = item_blocks(p, blockIdx.x, tiles_per_head);
+      ItemWalk w(sh->start);
 #pragma unroll 1
-      for (int s_item = blockIdx.x; s_item < n_items;) {
-        const int qb = s_it & 1;
-        trace_ev(p, 1, tn, tl && s_it >= p.trace_it, 2 * 16 + (s_j & 15));
-        if (s_j == 0) wait_spin(&sh->q_full[qb], (s_it >> 1) & 1);
-        wait_spin(&sh->kv_full[s_stage], s_stage_par);    // the block has landed ...
-        wait_spin(&sh->k_ready[s_stage], s_stage_par);    // ... and its window-mask rows are written
-        // the buffer is free once the PV MMA of the block that used it last has completed
-        if (s_use >= 1) wait_spin(&sh->s_free[s_buf], (s_use - 1) & 1);
-        if (ok) {
-          tc_fence_after();
-          if (elect_one()) {
-            const uint32_t sd = tmem + s_buf * s_stride;
-            uint64_t qd = q_desc0 + (uint64_t)(qb * (q_bytes >> 4)), kd = k_desc0 + (uint64_t)(s_stage * k_stage16);
-            uint32_t acc = 0u;
+      for (int it = 0; it < n_mine; ++it, w.next(p)) {
+        const StripItem si = strip_item(p, w);
+        int hi = min(4, si.nq);                        // the first four quarters enter with the item
+        int next_first = hi < si.nq ? quarter_first(p, si, hi) : si.nblk;
 #pragma unroll 1
-            for (int c = 0; c < p.qch; ++c, qd += 1024 - 8, kd += blk16 - 8) {
-#pragma unroll
-              for (int k = 0; k < 4; ++k, qd += 2, kd += 2, acc = 1u) umma_ss(sd, qd, kd, idesc_s, acc);
-            }
-            const uint64_t kxd = kx_desc0 + (uint64_t)(s_stage * kx_stage16);
-#pragma unroll
-            for (int k = 0; k < 2; ++k)  // + indicator x penalty: the window mask
-              umma_ss(sd, qx_desc0 + (uint64_t)(k * (kXStepBytes >> 4)), kxd + (uint64_t)(k * (kXStepBytes >> 4)), idesc_s, 1u);
-            umma_commit(&sh->s_full[s_buf]);
-            umma_commit(&sh->kx_free[s_stage]);                      // the mask rows of this stage may be overwritten
-            if (s_j == s_nblk - 1) umma_commit(&sh->q_empty[qb]);   // last read of this query buffer
+        for (int j = 0; j < si.nblk; ++j) {
+          trace_ev(p, 1, tn, tl && it >= p.trace_it, 2 * 16 + (j & 15));
+          bool enters = j == 0;                        // a quarter enters: the next version of the query rows
+#pragma unroll 1
+          while (next_first <= j) {
+            enters = true;
+            ++hi;
+            next_first = hi < si.nq ? quarter_first(p, si, hi) : si.nblk;
           }
-          __syncwarp();
-        }
-        trace_ev(p, 1, tn, tl && s_it >= p.trace_it, 3 * 16 + (s_j & 15));
-        if (++s_stage == pl.stages) { s_stage = 0; s_stage_par ^= 1; }
-        if (++s_buf == nsb) { s_buf = 0; ++s_use; }
-        if (++s_j == s_nblk) {
-          s_j = 0;
-          ++s_it;
-          s_item += gridDim.x;
-          if (s_item < n_items) s_nblk = item_blocks(p, s_item, tiles_per_head);
+          if (enters) {
+            xb ^= 1;
+            if (xb == 0) x_par ^= 1;
+            wait_spin(&sh->q_full[xb], x_par);
+          }
+          wait_spin(&sh->kv_full[stage], stage_par);    // the block has landed ...
+          wait_spin(&sh->k_ready[mslot], m_par);        // ... and its window-mask units are written
+          // the buffer is free once the PV MMA of the block that used it last has completed
+          if (use >= 1) wait_spin(&sh->s_free[buf], (use - 1) & 1);
+          if (ok) {
+            tc_fence_after();
+            if (elect_one()) {
+              const uint32_t sd = tmem + buf * s_stride;
+              uint64_t qd = q_desc0 + (uint64_t)(xb * (q_bytes >> 4)), kd = k_desc0 + (uint64_t)(stage * k_stage16);
+              uint32_t acc = 0u;
+#pragma unroll 1
+              for (int c = 0; c < qch; ++c, qd += 1024 - 8, kd += blk16 - 8) {
+#pragma unroll
+                for (int k = 0; k < 4; ++k, qd += 2, kd += 2, acc = 1u) umma_ss(sd, qd, kd, idesc_s, acc);
+              }
+              // + indicator x penalty, the window mask: row units, column units, the unused unit
+              const uint32_t yc = kc0 + mslot * (ub * (pl.TW >> 3));
+              const uint32_t u0 = kr0 + mslot * (ub * (pl.TH >> 3)), u1 = pl.TW == 8 ? u0 + ub : yc, u2 = pl.TW == 8 ? yc : yc + ub;
+              umma_ss(sd, qx_desc0, smem_desc_from(u0, u1 - u0, hi_ns), idesc_s, 1u);
+              umma_ss(sd, qx_desc0 + 256, smem_desc_from(u2, kz0 - u2, hi_ns), idesc_s, 1u);
+              umma_commit(&sh->s_full[buf]);
+              umma_commit(&sh->kx_free[mslot]);                        // its mask units may be overwritten
+              if (next_first == j + 1 || j == si.nblk - 1) umma_commit(&sh->q_empty[xb]);   // last read of this version
+            }
+            __syncwarp();
+          }
+          trace_ev(p, 1, tn, tl && it >= p.trace_it, 3 * 16 + (j & 15));
+          if (++stage == pl.stages) { stage = 0; stage_par ^= 1; }
+          if (++mslot == kMaskRing) { mslot = 0; m_par ^= 1; }
+          if (++buf == nsb) { buf = 0; ++use; }
         }
       }
     } else if (warp == 2) {
@@ -362,187 +352,185 @@ fwd2_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CU
       const uint64_t v_desc0 = smem_desc_from(smem_u32(v_smem), blk_bytes, hi_sw);
       const uint32_t v_stage16 = v_stage >> 4;
       const int nks = N >> 4;
-      int p_it = 0, p_j = 0, p_nblk = 1, p_stage = 0, p_buf = 0, p_buf_par = 0, p_grp = 0;
+      int stage = 0, buf = 0, buf_par = 0, grp = 0;
+      uint32_t q0 = 0;
       int tn = 0;
       const bool tl = (threadIdx.x & 31) == 0;
-      if (blockIdx.x < n_items) p_nblk = item_blocks(p, blockIdx.x, tiles_per_head);
+      ItemWalk w(sh->start);
 #pragma unroll 1
-      for (int p_item = blockIdx.x; p_item < n_items;) {
-        const bool first = p_j < 2;                       // first block of this item for group p_grp: O_g starts over
-        trace_ev(p, 6, tn, tl && p_it >= p.trace_it, 0 * 16 + (p_j & 15));
-        wait_spin(&sh->p_full[p_buf], p_buf_par);
-        if (first && p_it >= 1) wait_spin(&sh->o_free, (p_it - 1) & 1);   // the previous item's O_g has been read
-        trace_ev(p, 6, tn, tl && p_it >= p.trace_it, 4 * 16 + (p_j & 15));
-        if (ok) {
-          tc_fence_after();
-          if (elect_one()) {
-            const uint32_t pa = tmem + p_buf * s_stride, od = tmem + o_base + p_grp * o_cols;
-            uint64_t vd = v_desc0 + (uint64_t)(p_stage * v_stage16);
-            uint32_t acc = first ? 0u : 1u;
+      for (int it = 0; it < n_mine; ++it, w.next(p)) {
+        const StripItem si = strip_item(p, w);
+        QuarterCursor qc;
+        qc.begin(p, si);
+        uint32_t before = 0;                               // slots whose quarters entered with the previous block
 #pragma unroll 1
-            for (int ks = 0; ks < nks; ++ks, vd += 128, acc = 1u) umma_ts(od, pa + ks * 8, vd, idesc_pv, acc);
-            umma_commit(&sh->s_free[p_buf]);
-            umma_commit(&sh->kv_empty[p_stage]);
-            umma_commit(&sh->pv_done[p_grp]);
-            if (p_j == p_nblk - 1) umma_commit(&sh->o_full);
+        for (int j = 0; j < si.nblk; ++j) {
+          trace_ev(p, 6, tn, tl && it >= p.trace_it, 0 * 16 + (j & 15));
+          uint32_t entered = 0;                            // slots whose quarter starts with this block
+#pragma unroll 1
+          while (qc.hi < si.nq && qc.next_first <= j) {
+            const uint32_t Q = q0 + qc.hi;
+            if (Q >= 4) wait_spin(&sh->o_free[Q & 3], ((Q >> 2) - 1) & 1);   // its accumulators' last quarter has been read
+            entered |= 1u << (Q & 3);
+            qc.next_first = quarter_first(p, si, ++qc.hi);
           }
-          __syncwarp();
+          qc.act |= entered;
+          wait_spin(&sh->p_full[buf], buf_par);
+          trace_ev(p, 6, tn, tl && it >= p.trace_it, 4 * 16 + (j & 15));
+          const uint32_t act = qc.act, fresh = act & (entered | before);   // first block of these quarters for this group's O_g
+          before = entered;
+          uint32_t ends = 0;                               // slots whose quarter is complete with this block
+#pragma unroll 1
+          while (qc.lo < qc.hi && qc.lo_last <= j) {
+            ends |= 1u << ((q0 + qc.lo) & 3);
+            ++qc.lo;
+            qc.lo_last = quarter_last(p, si, qc.lo);
+          }
+          qc.act &= ~ends;
+          if (ok) {
+            tc_fence_after();
+            if (elect_one()) {
+              if (act)
+                accumulate_block(tmem + o_base + grp * o_cols, tmem + buf * s_stride + p_off, v_desc0 + (uint64_t)(stage * v_stage16), idesc_pv, nks,
+                                 nks, 0, act, fresh);
+              umma_commit(&sh->s_free[buf]);
+              umma_commit(&sh->kv_empty[stage]);
+              umma_commit(&sh->pv_done[grp]);
+#pragma unroll
+              for (int e = 0; e < 4; ++e)
+                if (ends & (1u << e)) umma_commit(&sh->o_full[e]);
+            }
+            __syncwarp();
+          }
+          trace_ev(p, 6, tn, tl && it >= p.trace_it, 1 * 16 + (j & 15));
+          grp ^= 1;
+          if (++stage == pl.stages) stage = 0;
+          if (++buf == nsb) { buf = 0; buf_par ^= 1; }
         }
-        trace_ev(p, 6, tn, tl && p_it >= p.trace_it, 1 * 16 + (p_j & 15));
-        p_grp ^= 1;
-        if (++p_stage == pl.stages) p_stage = 0;
-        if (++p_buf == nsb) { p_buf = 0; p_buf_par ^= 1; }
-        if (++p_j == p_nblk) {
-          p_j = 0;
-          ++p_it;
-          p_item += gridDim.x;
-          if (p_item < n_items) p_nblk = item_blocks(p, p_item, tiles_per_head);
-        }
+        q0 += si.nq;
       }
+    } else {
+      // ------------------------------------------------------------------ window mask
+      const MaskArgs f{kr_smem, kc_smem, sh->kx_free, sh->k_ready, nullptr, 0, nullptr, nullptr, nullptr, row_parts, &sh->start};
+      mask_warp<BF16, false>(p, f, ok, wait_park);
     }
   } else {
-    // ------------------------------------------------------------------ query rotation, mask rows, epilogue (warps 12-15)
-    const int t = (int)threadIdx.x - 384;          // 0..127: row of the query tile / of a streamed block
-    const int quarter = warp & 3;
-    const uint32_t lane_base = tmem + ((uint32_t)(quarter * 32) << 16);
-    using T = typename std::conditional<BF16, __nv_bfloat16, __half>::type;
+    setmaxnreg_inc<168>();
+    // ------------------------------------------------------------------ epilogue, one warp per slot, one thread per row
+    const int slot = warp & 3, lane = threadIdx.x & 31;
+    const uint32_t lane_base = tmem + ((uint32_t)(slot * 32) << 16);
     const float c2 = p.scale_log2;
+    const int own_r = lane >> pl.tw_log, own_c = lane & (pl.TW - 1);
+    uint8_t* const stg = stg_smem + slot * pl.stg * kStageChunk;
+    const uint32_t row0 = smem_u32(stg) + lane * 128, swz_x = (uint32_t)(lane & 7) << 4;
     int tn = 0;
-    write_indicator_row<BF16>(qx_smem, t, 0, 1, p);               // the same for every item
-    const bool row_on = t < N;
-    const int jr = t / pl.KW, jc = t % pl.KW;                     // this thread's row inside every streamed block
-    // Epilogue of one item: merge the two groups' partial results of this thread's row and store it.
-    // `gb` = stream position of the item's block 0, `nblk` = its blocks.
-    auto epilogue = [&](int item, int it, uint32_t gb, int nblk) {
-      const int bh = item / tiles_per_head, bi = bh / p.H, hi = bh - bi * p.H;
-      const TilePos tp = tile_pos(p, item - bh * tiles_per_head);
-      const int qr = tp.r0 + t / pl.TW, qx = tp.x0 + t % pl.TW;
-      const bool q_in = qr < p.t_h && qx < p.Wtok;
-      const int64_t tok = (int64_t)qr * p.Wtok + qx;
-      const int par = it & 1;
-      // the group that took the even blocks of the item, and how many blocks each parity had
-      const int g_even = (int)(gb & 1u);
-      const int cnt_e = (nblk + 1) >> 1, cnt_d = nblk >> 1;
-      trace_ev(p, 5, tn, t == 0 && it >= p.trace_it, 0 * 16 + (it & 15));
-      wait_spin(&sh->ml_full[par], (it >> 1) & 1);
-      const float m_e = sh->ml[par][g_even][0][t], l_e = sh->ml[par][g_even][1][t];
-      const float m_d = sh->ml[par][g_even ^ 1][0][t], l_d = sh->ml[par][g_even ^ 1][1][t];
-      if (ok) mbar_arrive(&sh->ml_empty[par]);
-      // Merge in an order fixed by the blocks' positions in the item (even ones first), not by which group
-      // happened to get them: the result of a tile must not depend on the work that preceded it.
-      const float mm = fmaxf(m_e, m_d);
-      const float w_e = (m_e == -INFINITY) ? 0.f : exp2f((m_e - mm) * c2);
-      const float w_d = (m_d == -INFINITY) ? 0.f : exp2f((m_d - mm) * c2);
-      const float lt = fmaf(l_d, w_d, l_e * w_e);
-      const float inv = 1.f / lt;
-      const float f_e = w_e * inv, f_d = w_d * inv;
-      const uint32_t o_even = lane_base + o_base + g_even * o_cols, o_odd = lane_base + o_base + (g_even ^ 1) * o_cols;
-      T* orow = (T*)o.ptr + bi * o.s0 + hi * o.s1 + tok * o.s2;
-      wait_spin(&sh->o_full, it & 1);
-      trace_ev(p, 5, tn, t == 0 && it >= p.trace_it, 1 * 16 + (it & 15));
-      if (ok) {
-        tc_fence_after();
+    int o_par = 0, ml_par = 0;                      // barrier parities (ml: bit per quarter parity and group)
+    uint32_t gb = 0, q0 = 0;
+    ItemWalk w(sh->start);
 #pragma unroll 1
-        for (int c0 = 0; c0 < p.dv; c0 += 32) {          // the real columns of O only
+    for (int it = 0; it < n_mine; ++it, w.next(p)) {
+      const StripItem si = strip_item(p, w);
+      // Blocks are even or odd by their position in the grid.  The two parities' partial results are merged in that order, not
+      // by which group happened to take them: the result of a row must not depend on the work that preceded it.
+      const int a0 = (int)((uint32_t)(si.h0 + p.wr) / (uint32_t)pl.KR) * pl.ncb;     // grid position of the item's block 0
+      const int g_even = (int)((gb + (uint32_t)a0) & 1u);   // the group that took the even blocks
+#pragma unroll 1
+      for (int i = (slot - (int)q0) & 3; i < si.nq; i += 4) {
+        const int qr = si.r0 + i * pl.R4;
+        const int b_lo = a0 + quarter_first(p, si, i), b_hi = a0 + quarter_last(p, si, i);
+        const bool has_e = b_hi > b_lo || !(b_lo & 1), has_d = b_hi > b_lo || (b_lo & 1);
+        const int qp = (int)((q0 + i) >> 2) & 1;
+        float m_e = -INFINITY, l_e = 0.f, m_d = -INFINITY, l_d = 0.f;
+        trace_ev(p, 5, tn, slot == 0 && lane == 0 && it >= p.trace_it, 0 * 16 + (i & 15));
+        if (has_e) {
+          wait_park(&sh->ml_full[qp][slot][g_even], (ml_par >> (2 * qp + g_even)) & 1);
+          ml_par ^= 1 << (2 * qp + g_even);
+          m_e = sh->ml[qp][slot][g_even][0][lane];
+          l_e = sh->ml[qp][slot][g_even][1][lane];
+        }
+        if (has_d) {
+          wait_park(&sh->ml_full[qp][slot][g_even ^ 1], (ml_par >> (2 * qp + (g_even ^ 1))) & 1);
+          ml_par ^= 1 << (2 * qp + (g_even ^ 1));
+          m_d = sh->ml[qp][slot][g_even ^ 1][0][lane];
+          l_d = sh->ml[qp][slot][g_even ^ 1][1][lane];
+        }
+        __syncwarp();
+        if (ok && lane == 0) mbar_arrive(&sh->ml_empty[qp][slot]);
+        const float mm = fmaxf(m_e, m_d);
+        const float w_e = (m_e == -INFINITY) ? 0.f : exp2f((m_e - mm) * c2);
+        const float w_d = (m_d == -INFINITY) ? 0.f : exp2f((m_d - mm) * c2);
+        const float lt = fmaf(l_d, w_d, l_e * w_e);
+        const float inv = 1.f / lt;
+        const float f_e = w_e * inv, f_d = w_d * inv;
+        // (a parity without blocks has weight 0 and an accumulator that may hold anything: the other one is read twice)
+        const uint32_t o_even = lane_base + o_base + (has_e ? g_even : g_even ^ 1) * o_cols;
+        const uint32_t o_odd = lane_base + o_base + (has_d ? g_even ^ 1 : g_even) * o_cols;
+        wait_park(&sh->o_full[slot], o_par);
+        o_par ^= 1;
+        trace_ev(p, 5, tn, slot == 0 && lane == 0 && it >= p.trace_it, 1 * 16 + (i & 15));
+        if (!ok) continue;
+        tc_fence_after();
+        // Heads of at most 64 leave through the staging by TMA; wider ones, which need the shared memory for larger blocks, are
+        // stored by the threads that hold the rows.
+        const int tr = qr + own_r, tx = si.x0 + own_c;
+        const bool t_in = tr < p.t_h && tx < p.Wtok;
+        const int64_t tok = (int64_t)tr * p.Wtok + tx;
+        using T = typename std::conditional<BF16, __nv_bfloat16, __half>::type;
+        [[maybe_unused]] T* const orow = (T*)o.ptr + w.bi * o.s0 + w.hi * o.s1 + tok * o.s2;
+        if (ONE && lane == 0) tma_store_wait_read();     // the previous quarter's rows have left the staging
+        __syncwarp();
+        const int halves = 2 * vch;
+#pragma unroll 1
+        for (int m = 0; m < halves; ++m) {               // 32 columns
           uint32_t a[32], b[32];
-          if (cnt_e > 0) tmem_ld32(o_even + c0, a);
-          if (cnt_d > 0) tmem_ld32(o_odd + c0, b);
+          tmem_ld32(o_even + 32 * m, a);
+          tmem_ld32(o_odd + 32 * m, b);
           tmem_wait_ld();
-          if (c0 + 32 >= p.dv) {                       // everything has been read: the next item may accumulate
+          if (m == halves - 1) {                         // the last column has been read
             tc_fence_before();
-            mbar_arrive(&sh->o_free);
-            trace_ev(p, 5, tn, t == 0 && it >= p.trace_it, 2 * 16 + (it & 15));
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&sh->o_free[slot]);
+            trace_ev(p, 5, tn, slot == 0 && lane == 0 && it >= p.trace_it, 2 * 16 + (i & 15));
           }
-          if (q_in) {
-            uint4* dst = reinterpret_cast<uint4*>(orow + c0);
+          [[maybe_unused]] const uint32_t row = row0;
 #pragma unroll
-            for (int uu = 0; uu < 4; ++uu) {
-              uint32_t w[4];
+          for (int u = 0; u < 4; ++u) {
+            uint32_t wd[4];
 #pragma unroll
-              for (int h = 0; h < 4; ++h) {
-                const int i0 = uu * 8 + 2 * h;
-                float v0 = 0.f, v1 = 0.f;
-                if (cnt_e > 0) { v0 = __uint_as_float(a[i0]) * f_e; v1 = __uint_as_float(a[i0 + 1]) * f_e; }
-                if (cnt_d > 0) { v0 = fmaf(__uint_as_float(b[i0]), f_d, v0); v1 = fmaf(__uint_as_float(b[i0 + 1]), f_d, v1); }
-                w[h] = pack2<BF16>(v0, v1);
-              }
-              dst[uu] = make_uint4(w[0], w[1], w[2], w[3]);
+            for (int h = 0; h < 4; ++h) {
+              const int e = 8 * u + 2 * h;
+              wd[h] = pack2<BF16>(fmaf(__uint_as_float(b[e]), f_d, __uint_as_float(a[e]) * f_e),
+                                  fmaf(__uint_as_float(b[e + 1]), f_d, __uint_as_float(a[e + 1]) * f_e));
+            }
+            if constexpr (ONE) {
+              sts128(row + (((uint32_t)(4 * m + u) << 4) ^ swz_x), wd[0], wd[1], wd[2], wd[3]);
+            } else if (t_in && 32 * m + 8 * u < p.dv) {
+              *reinterpret_cast<uint4*>(orow + 32 * m + 8 * u) = make_uint4(wd[0], wd[1], wd[2], wd[3]);
             }
           }
         }
-        if (q_in) lse[(int64_t)bh * p.t_h * p.Wtok + tok] = mm * c2 + log2f(lt);
-      }
-      trace_ev(p, 5, tn, t == 0 && it >= p.trace_it, 3 * 16 + (it & 15));
-    };
-
-    int stage = 0, stage_par = 1;                    // parity of the "free" phase a rewrite of this stage's rows waits for
-    bool ring_full = false;
-    uint64_t pen_sig = ~0ull;                        // geometry the penalty tables in shared memory were built for
-    uint32_t G = 0;                                  // stream position of the next block to prepare
-    bool pend = false;                               // an item whose epilogue has not run yet
-    int pend_item = 0, pend_it = 0, pend_nblk = 0;
-    uint32_t pend_gb = 0, pend_G = 0;                // its first stream position; the position before which it runs
-#pragma unroll 1
-    for (int it = 0, item = blockIdx.x;; ++it, item += gridDim.x) {   // one extra round flushes the last epilogue
-      const bool have = item < n_items;
-      const int bh = have ? item / tiles_per_head : 0;
-      TilePos tp;
-      tp.r0 = tp.x0 = tp.hx0 = tp.hr_first = tp.hr_last = 0;
-      tp.nblk = 0;
-      if (have) tp = tile_pos(p, item - bh * tiles_per_head);
-      const uint32_t gb = G;
-      if (have) {
-        // the tables depend only on how the halo is clipped by the grid: interior tiles share them
-        const uint64_t sig = penalty_signature(p, tp);
-        if (sig != pen_sig) {
-          pen_sig = sig;
-          named_bar_sync(5, 128);           // nobody still reads the previous tables
-          build_penalty_view<BF16>(pen, t, p, tp, 128);
-          named_bar_sync(5, 128);
-        }
-      }
-#pragma unroll 1
-      for (int j = 0;; ++j, ++G) {
-        // These warps run ahead of the score MMAs by up to `stages` blocks (a stage's mask rows are free as soon as
-        // the score MMA that read them has completed; the K / V data need not have landed).  The block at stream
-        // position (last block of an item + score buffers + stages) is the first one they would have to wait for
-        // until that item's last PV MMA has completed: the item's epilogue runs right before it (or at the end of
-        // a later item that ends earlier, or after the last item), hidden behind that lead.
-        const bool at_end = j >= tp.nblk;
-        if (pend && (at_end || G >= pend_G)) {
-          epilogue(pend_item, pend_it, pend_gb, pend_nblk);
-          pend = false;
-        }
-        if (at_end) break;
-        trace_ev(p, 4, tn, t == 0 && it >= p.trace_it, 0 * 16 + (j & 15));
-        if (ring_full) wait_park(&sh->kx_free[stage], (uint32_t)stage_par);
-        trace_ev(p, 4, tn, t == 0 && it >= p.trace_it, 1 * 16 + (j & 15));
-        if (ok) {
-          if (row_on) {
-            int band, cblk;
-            block_pos(pl, j, band, cblk);
-            write_penalty_row_v(kx_smem + stage * kx_stage, t, pen, band * pl.KR + jr, cblk * pl.KW + jc, pl.TH >> 3, pl.TW >> 3);
-          }
+        if constexpr (ONE) {
           fence_proxy_async_smem();
-          mbar_arrive(&sh->k_ready[stage]);
+          __syncwarp();
+          if (lane == 0) {
+            tma_store_5d(&tm_o, stg, 0, si.x0, qr, w.hi, w.bi);
+            tma_store_commit();
+          }
         }
-        trace_ev(p, 4, tn, t == 0 && it >= p.trace_it, 2 * 16 + (j & 15));
-        if (++stage == pl.stages) { stage = 0; stage_par ^= 1; ring_full = true; }
+        if (t_in) lse[(int64_t)(w.bi * p.H + w.hi) * p.t_h * p.Wtok + tok] = mm * c2 + log2f(lt);
+        trace_ev(p, 5, tn, slot == 0 && lane == 0 && it >= p.trace_it, 3 * 16 + (i & 15));
       }
-      if (!have) break;
-      pend = true;
-      pend_item = item;
-      pend_it = it;
-      pend_gb = gb;
-      pend_nblk = tp.nblk;
-      pend_G = G - 1 + (uint32_t)(pl.stages + nsb);
+      gb += si.nblk;
+      q0 += si.nq;
     }
+    if (lane == 0) tma_store_wait_all();
   }
 
   // ------------------------------------------------------------------ teardown
+  if (!ok) sh->abort_flag = 1;
   tc_fence_before();
   __syncthreads();
-  if (*abort_flag) {
+  if (*(volatile int*)&sh->abort_flag) {
     // let whatever is still in flight (TMA, MMA) land before shared memory and TMEM are released
 #pragma unroll 1
     for (int i = 0; i < 64; ++i) __nanosleep(1000);

@@ -54,6 +54,33 @@ __device__ __forceinline__ void setmaxnreg_inc() { asm volatile("setmaxnreg.inc.
 template <uint32_t REGS>
 __device__ __forceinline__ void setmaxnreg_dec() { asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(REGS)); }
 
+// ---- two fp32 values per instruction (sm_100's packed fma / add / mul), IEEE rounding as the scalar ones ----------
+__device__ __forceinline__ uint64_t f2_pack(float a, float b) {
+  uint64_t r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+  return r;
+}
+__device__ __forceinline__ float2 f2_unpack(uint64_t v) {
+  float2 r;
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
+  return r;
+}
+__device__ __forceinline__ uint64_t f2_fma(uint64_t a, uint64_t b, uint64_t c) {
+  uint64_t r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+  return r;
+}
+__device__ __forceinline__ uint64_t f2_add(uint64_t a, uint64_t b) {
+  uint64_t r;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+__device__ __forceinline__ uint64_t f2_mul(uint64_t a, uint64_t b) {
+  uint64_t r;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+
 // ---- mbarrier ----------------------------------------------------------------------------------
 __device__ __forceinline__ void mbar_init(uint64_t* bar, uint32_t count) {
   asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(bar)), "r"(count) : "memory");
@@ -76,19 +103,6 @@ __device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, uint32_t parity) {
   return ok != 0;
 }
 
-// Non-blocking test of the phase: never suspends the thread, so a polling loop reacts within a few cycles.
-__device__ __forceinline__ bool mbar_test_wait(uint64_t* bar, uint32_t parity) {
-  uint32_t ok;
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-      "selp.u32 %0, 1, 0, p;\n\t}"
-      : "=r"(ok)
-      : "r"(smem_u32(bar)), "r"(parity)
-      : "memory");
-  return ok != 0;
-}
-
 // try_wait that lets the hardware park the thread for up to `hint_ns` before it reports failure.
 __device__ __forceinline__ bool mbar_try_wait_hint(uint64_t* bar, uint32_t parity, uint32_t hint_ns) {
   uint32_t ok;
@@ -102,8 +116,6 @@ __device__ __forceinline__ bool mbar_try_wait_hint(uint64_t* bar, uint32_t parit
   return ok != 0;
 }
 
-constexpr uint32_t kWaitMaxPolls = 1u << 22;  // polls (spinning) resp. sleeps before a wait gives up: about half a second
-
 // Wait for the phase with the given parity to complete.  Returns false when the
 // CTA-wide abort flag is (or becomes) set or the poll budget runs out; in the
 // latter case it sets the flag so that every other role of the CTA leaves too.
@@ -111,44 +123,71 @@ constexpr uint32_t kWaitMaxPolls = 1u << 22;  // polls (spinning) resp. sleeps b
 // PARK_NS == 0: spin on try_wait (warps on the critical path).  PARK_NS > 0: each poll lets the
 // hardware park the thread for up to PARK_NS nanoseconds and wake it when the phase completes, so
 // a waiting warp takes (almost) no issue slots from the working warps of its sub-partition.
-// PARK_NS == kPollNoSuspend: spin on the non-blocking test_wait.
 //
-// Only the first probe is inlined at the call site; the polling loop is one shared out-of-line
-// function per mode.  The kernels are instruction-fetch bound in their rarely executed scalar
-// parts, so every call site has to stay small.
-constexpr uint32_t kPollNoSuspend = 0xffffffffu;
-// A wait gives up after one second of wall time: far beyond any legitimate wait of these kernels (a whole launch
-// takes milliseconds), yet short enough to leave a mis-synchronised kernel quickly; long enough that a context
-// that is time-sliced with another process does not trip it.
-constexpr unsigned long long kWaitBudgetNs = 1000ull * 1000 * 1000;
-__device__ __forceinline__ unsigned long long global_ns() {
-  unsigned long long t;
-  asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t));
-  return t;
-}
-template <uint32_t PARK_NS>
-__device__ __forceinline__ bool mbar_wait_slow(uint64_t* bar, uint32_t parity, volatile int* abort_flag) {
-  const unsigned long long t0 = global_ns();
-  for (uint32_t it = 0; it < kWaitMaxPolls; ++it) {
-    if constexpr (PARK_NS == kPollNoSuspend) {
-      if (mbar_test_wait(bar, parity)) return true;
-    } else if constexpr (PARK_NS == 0) {
-      if (mbar_try_wait(bar, parity)) return true;
-    } else {
-      if (mbar_try_wait_hint(bar, parity, PARK_NS)) return true;
-    }
-    if ((it & 15u) == 15u) {
-      if (*abort_flag) return false;
-      if (global_ns() - t0 > kWaitBudgetNs) break;
-    }
-  }
-  *abort_flag = 1;
-  return false;
-}
+// The loop is a dozen instructions: the kernels have two dozen waits, all of them inlined, and every role's code is
+// fetched anew once per block (a polling loop with a wall clock in it made up a third of the kernels' 60 to 90 KB).
+// The budget is polls that did not succeed: at 50 ns or more each, 1 << 24 of them are about a second, far beyond any
+// legitimate wait (a whole launch takes milliseconds); a context that is time-sliced with another process does not
+// use it up while it does not run.
+constexpr uint32_t kWaitMaxPolls = 1u << 24;
 template <uint32_t PARK_NS = 0>
 __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, volatile int* abort_flag) {
-  if (PARK_NS == kPollNoSuspend ? mbar_test_wait(bar, parity) : mbar_try_wait(bar, parity)) return true;
-  return mbar_wait_slow<PARK_NS>(bar, parity, abort_flag);
+  uint32_t polls = 0;
+#pragma unroll 1
+  while (!(PARK_NS == 0 ? mbar_try_wait(bar, parity) : mbar_try_wait_hint(bar, parity, PARK_NS))) {
+    if (*abort_flag) return false;
+    if (++polls == kWaitMaxPolls) {
+      *abort_flag = 1;
+      return false;
+    }
+  }
+  return true;
+}
+
+// The strip kernels' wait (swa_tc_strip.cuh): six instructions, because they have two dozen of them in code that is fetched
+// again for every block.  False once the poll budget is used up (about half a second); the caller then skips every
+// later wait, and the kernel's end tells the host.
+template <uint32_t PARK_NS>
+__device__ __forceinline__ bool mbar_wait_polls(uint32_t bar, uint32_t parity) {
+  uint32_t ok;
+  if constexpr (PARK_NS == 0)
+    asm volatile(
+        "{\n\t.reg .pred p, q;\n\t.reg .u32 n;\n\t"
+        "mov.u32 n, %3;\n"
+        "SWA_WAIT:\n\t"
+        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+        "@p bra SWA_DONE;\n\t"
+        "sub.u32 n, n, 1;\n\t"
+        "setp.ne.u32 q, n, 0;\n\t"
+        "@q bra SWA_WAIT;\n"
+        "SWA_DONE:\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t}"
+        : "=r"(ok) : "r"(bar), "r"(parity), "n"(1 << 22) : "memory");
+  else
+    asm volatile(
+        "{\n\t.reg .pred p, q;\n\t.reg .u32 n;\n\t"
+        "mov.u32 n, %3;\n"
+        "SWA_WAIT:\n\t"
+        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %4;\n\t"
+        "@p bra SWA_DONE;\n\t"
+        "sub.u32 n, n, 1;\n\t"
+        "setp.ne.u32 q, n, 0;\n\t"
+        "@q bra SWA_WAIT;\n"
+        "SWA_DONE:\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t}"
+        : "=r"(ok) : "r"(bar), "r"(parity), "n"(1 << 22), "n"(PARK_NS) : "memory");
+  return ok != 0;
+}
+
+// Whether the phase with the given parity has completed; never suspends.
+__device__ __forceinline__ bool mbar_test(uint32_t bar, uint32_t parity) {
+  uint32_t ok;
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+      "selp.u32 %0, 1, 0, p;\n\t}"
+      : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
+  return ok != 0;
 }
 
 __device__ __forceinline__ void fence_barrier_init() { asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory"); }
@@ -169,6 +208,22 @@ __device__ __forceinline__ void tma_load_5d(void* smem_dst, const CUtensorMap* m
       "r"(c3), "r"(c4)
       : "memory");
 }
+
+__device__ __forceinline__ void tma_prefetch_5d(const CUtensorMap* m, int c0, int c1, int c2, int c3, int c4) {
+  asm volatile("cp.async.bulk.prefetch.tensor.5d.L2.global [%0, {%1, %2, %3, %4, %5}];" ::"l"(reinterpret_cast<uint64_t>(m)), "r"(c0),
+               "r"(c1), "r"(c2), "r"(c3), "r"(c4)
+               : "memory");
+}
+// 5-D tiled store shared memory -> global (bounds clipped by the map); reads of shared memory are complete after
+// tma_store_wait_read of the issuing thread.
+__device__ __forceinline__ void tma_store_5d(const CUtensorMap* m, const void* smem_src, int c0, int c1, int c2, int c3, int c4) {
+  asm volatile("cp.async.bulk.tensor.5d.global.shared::cta.bulk_group [%0, {%2, %3, %4, %5, %6}], [%1];" ::"l"(
+                   reinterpret_cast<uint64_t>(m)), "r"(smem_u32(smem_src)), "r"(c0), "r"(c1), "r"(c2), "r"(c3), "r"(c4)
+               : "memory");
+}
+__device__ __forceinline__ void tma_store_commit() { asm volatile("cp.async.bulk.commit_group;" ::: "memory"); }
+__device__ __forceinline__ void tma_store_wait_read() { asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory"); }
+__device__ __forceinline__ void tma_store_wait_all() { asm volatile("cp.async.bulk.wait_group 0;" ::: "memory"); }
 
 // ---- tcgen05: TMEM allocation ---------------------------------------------------------------
 // Whole-warp instructions.  `cols` is a power of two in [32, 512].
@@ -239,6 +294,24 @@ __device__ __forceinline__ void umma_ts(uint32_t d_tmem, uint32_t a_tmem, uint64
       "setp.ne.b32 p, %4, 0;\n\t"
       "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}"
       ::"r"(d_tmem), "r"(a_tmem), "l"(b_desc), "r"(idesc), "r"(accumulate)
+      : "memory");
+}
+// The same with the accumulator rows limited: lanes 32 s .. 32 s + 31 of D are written only if bit s of `slots` is set
+// (the instruction's disable-output-lane operand), the other rows keep their values.
+struct SlotMask {
+  uint32_t off[4];
+  __device__ __forceinline__ explicit SlotMask(uint32_t slots) {
+#pragma unroll
+    for (int s = 0; s < 4; ++s) off[s] = (slots >> s & 1u) - 1u;
+  }
+};
+__device__ __forceinline__ void umma_ts_slots(uint32_t d_tmem, uint32_t a_tmem, uint64_t b_desc, uint32_t idesc, uint32_t accumulate,
+                                              const SlotMask& m) {
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "setp.ne.b32 p, %4, 0;\n\t"
+      "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, {%5, %6, %7, %8}, p;\n\t}"
+      ::"r"(d_tmem), "r"(a_tmem), "l"(b_desc), "r"(idesc), "r"(accumulate), "r"(m.off[0]), "r"(m.off[1]), "r"(m.off[2]), "r"(m.off[3])
       : "memory");
 }
 // Arrive on `bar` once every MMA issued so far by this thread has completed.

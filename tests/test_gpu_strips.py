@@ -1,0 +1,43 @@
+"""Strip kernels (no streamed rotation) at the sizes where their walk can go wrong: quarters of a strip that meet a
+single block, grids lower than a quarter or a block, heights and widths that leave remainders, strips cut into chunks,
+windows at which quarters just slide or just do not, several column blocks per band, many items per CTA."""
+import pytest
+import torch
+
+from oracle import swa_oracle as orc
+
+import dl_templates_b200 as swa
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda:0"
+
+
+@pytest.mark.parametrize("th,tw,b,wr,wc,dqk,dv,R,BH", [
+    (64, 64, 1, 0, 0, 64, 64, 0, 40), (63, 33, 1, 1, 1, 64, 64, 16, 64), (130, 9, 1, 1, 2, 32, 32, 8, 300),
+    (1, 200, 1, 0, 3, 64, 64, 16, 7), (3, 17, 1, 2, 2, 64, 64, 8, 5), (300, 7, 1, 2, 1, 64, 64, 16, 9),
+    (41, 24, 1, 5, 5, 64, 64, 16, 30), (41, 24, 1, 6, 6, 64, 64, 16, 30), (41, 24, 1, 7, 7, 64, 64, 8, 30),
+    (200, 16, 1, 3, 3, 64, 64, 16, 160), (37, 19, 1, 4, 2, 128, 128, 32, 20), (26, 40, 1, 12, 3, 96, 64, 16, 6),
+    (9, 6, 16, 1, 3, 32, 64, 0, 12), (12, 10, 2, 1, 2, 64, 128, 0, 33)])
+def test_strips_against_simt(th, tw, b, wr, wc, dqk, dv, R, BH):
+    N = th * tw * b
+    g = torch.Generator(device=DEV).manual_seed(th * 1000 + tw)
+    q, k = (torch.randn(1, BH, N, dqk, device=DEV, generator=g).to(torch.bfloat16) for _ in range(2))
+    v, do = (torch.randn(1, BH, N, dv, device=DEV, generator=g).to(torch.bfloat16) for _ in range(2))
+    win, sc = (b, th, tw, wr, wc), dqk ** -0.5
+    if R:
+        rope = tuple(t.to(DEV) for t in (orc.encode_idx(th, tw * b), orc.make_cs_table(R, max(th, 2)), orc.make_cs_table(R, max(tw * b, 2))))
+        o, lse, qr, kr = swa.swa_forward_rot(q, k, v, rope, *win, sc, impl="tc")
+        got = (o, *swa.swa_backward_rot(qr, kr, v, o, lse, do, rope, *win, sc, impl="tc"))
+        o1, l1, qs, ks = swa.swa_forward_rot(q, k, v, rope, *win, sc, impl="simt")
+        want = (o1, *swa.swa_backward_rot(qs, ks, v, o1, l1, do, rope, *win, sc, impl="simt"))
+    else:
+        o, lse = swa.swa_forward(q, k, v, None, *win, sc, impl="tc")
+        got = (o, *swa.swa_backward(q, k, v, o, lse, do, None, *win, sc, impl="tc"))
+        o1, l1 = swa.swa_forward(q, k, v, None, *win, sc, impl="simt")
+        want = (o1, *swa.swa_backward(q, k, v, o1, l1, do, None, *win, sc, impl="simt"))
+    swa.check_status()
+    assert (lse - l1).abs().max().item() < 1e-3
+    for a, c, n in zip(got, want, ("o", "dq", "dk", "dv")):
+        assert torch.isfinite(a.float()).all(), n
+        err = (a.float() - c.float()).norm() / max(c.float().norm(), 0.1 * c.numel() ** 0.5)     # (a 1 x 1 window has dq = dk = 0)
+        assert err < 1e-2, f"{n}: relative error {float(err):.2e}"
