@@ -1,4 +1,5 @@
 // C ABI (include/swa2d.h): argument validation, kernel-family selection, launches.
+#include <algorithm>
 #include <atomic>
 #include <cstdarg>
 #include <cstdio>
@@ -8,6 +9,7 @@
 #include "common.cuh"
 #include "stream_kernels.cuh"
 #include "swa_simt.cuh"
+#include "swa_simt_tile.cuh"
 #include "swa_tc.cuh"
 
 namespace {
@@ -83,6 +85,55 @@ int resolve_impl(const swa_geom_t* g, const swa_rope_t* rope, const swa_tensor_t
   return SWA_IMPL_SIMT;
 }
 
+// fp32 problems the tiled kernels take (swa_simt_tile.cuh): true when the launch was made (*err: its return code).  `rope`
+// only rotates dQ / dK back; streamed rows are never rotated here.  The band of halo rows that is staged at a time is
+// what fits 100 KB beside the resident rows, so that two blocks share an SM; a single row that does not fit takes up to the
+// 227 KB there are, and a wider one is left to the one-warp-per-token kernels.
+bool launch_simt_tile(int kind, const swa_geom_t* g, const swa_rope_t* rope, const swa_tensor_t* x1, const swa_tensor_t* x2,
+                      const swa_tensor_t* y1, const swa_tensor_t* y2, const swa_tensor_t* o1, const swa_tensor_t* o2, float* lse_out,
+                      const float* lse, const float* delta, cudaStream_t st, int* err) {
+  if (g->dtype != SWA_F32 || g->d_qk % 4 || g->d_v % 4 || g->d_qk > 128 || g->d_v > 128) return false;
+  for (const swa_tensor_t* t : {x1, x2, y1, y2, o1, o2})
+    if (t && (t->stride[3] != 1 || (uintptr_t)t->ptr % 16 || t->stride[0] % 4 || t->stride[1] % 4 || t->stride[2] % 4)) return false;
+  const swa_tensor_t none{nullptr, {0, 0, 0, 0}};
+  const int Wtok = g->t_width * g->b_size;
+  swa::TileArgs a;
+  a.g = swa::make_geom(g);
+  a.rope = swa::make_rope(rope);
+  a.x1 = swa::make_view(x1); a.x2 = swa::make_view(x2 ? x2 : &none);
+  a.y1 = swa::make_view(y1); a.y2 = swa::make_view(y2);
+  a.o1 = swa::make_view(o1); a.o2 = swa::make_view(o2 ? o2 : &none);
+  a.lse_out = lse_out;
+  a.lse = lse;
+  a.delta = delta;
+  const int cols = std::min(Wtok, swa::tile_halo_cols(g->b_size, g->col_size));
+  const int rows = std::min(g->t_height, swa::kTileRows + 2 * g->row_size);
+  auto bytes = [&](int rb) { return 4 * swa::tile_smem_floats(kind, g->d_qk, g->d_v, rb * cols); };
+  int rb = 1;
+  if (bytes(1) > 227 * 1024 || cols > 4000) return false;
+  while (rb < rows && bytes(rb + 1) <= 100 * 1024 && (rb + 1) * cols <= 4000) ++rb;
+  const int bands = (rows + rb - 1) / rb;
+  a.rb = (rows + bands - 1) / bands;
+  a.max_keys = a.rb * cols;
+  a.n_tiles_x = (Wtok + swa::kTileCols - 1) / swa::kTileCols;
+  const int64_t tiles = (int64_t)a.n_tiles_x * ((g->t_height + swa::kTileRows - 1) / swa::kTileRows);
+  const dim3 grid((unsigned)tiles, (unsigned)(g->B * g->H));
+  using Kernel = void (*)(const swa::TileArgs);
+  static const Kernel table[3][2][2] = {   // [kind][d_qk > 64][d_v > 64]
+      {{swa::simt_tile_kernel<0, 2, 2>, swa::simt_tile_kernel<0, 2, 4>}, {swa::simt_tile_kernel<0, 2, 2>, swa::simt_tile_kernel<0, 2, 4>}},
+      {{swa::simt_tile_kernel<1, 2, 2>, swa::simt_tile_kernel<1, 2, 2>}, {swa::simt_tile_kernel<1, 4, 2>, swa::simt_tile_kernel<1, 4, 2>}},
+      {{swa::simt_tile_kernel<2, 2, 2>, swa::simt_tile_kernel<2, 2, 4>}, {swa::simt_tile_kernel<2, 4, 2>, swa::simt_tile_kernel<2, 4, 4>}}};
+  const Kernel kern = table[kind][g->d_qk > 64 ? 1 : 0][g->d_v > 64 ? 1 : 0];
+  const int smem = (int)bytes(a.rb);
+  if (cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem); e != cudaSuccess) {
+    *err = fail(E_LAUNCH, "cudaFuncSetAttribute(%d bytes): %s", smem, cudaGetErrorString(e));
+    return true;
+  }
+  kern<<<grid, 256, smem, st>>>(a);
+  *err = launch_ok("simt tile");
+  return true;
+}
+
 }  // namespace
 
 extern "C" {
@@ -126,6 +177,9 @@ int swa_fwd(const swa_geom_t* g, const swa_rope_t* rope, const swa_tensor_t* q, 
     if (e) return fail(E_LAUNCH, "tcgen05 forward: %s", swa::tc::last_error());
     return launch_ok("tcgen05 forward");
   }
+  const bool plain = !rope || !rope->idx;
+  int err = 0;
+  if (plain && launch_simt_tile(0, g, nullptr, q, nullptr, k, v, o, nullptr, lse, nullptr, nullptr, st, &err)) return err;
   const swa::Geom gg = swa::make_geom(g);
   const swa::RopeDev rp = swa::make_rope(rope);
   const int N = g->t_height * g->t_width * g->b_size;
@@ -211,6 +265,8 @@ int swa_bwd_dq(const swa_geom_t* g, const swa_rope_t* rope, const swa_tensor_t* 
     if (e) return fail(E_LAUNCH, "tcgen05 dq: %s", swa::tc::last_error());
     return launch_ok("tcgen05 dq");
   }
+  int err = 0;
+  if ((!rope || !rope->idx) && launch_simt_tile(1, g, nullptr, q, d_o, k, v, dq, nullptr, nullptr, lse, delta, st, &err)) return err;
   const swa::Geom gg = swa::make_geom(g);
   const swa::RopeDev rp = swa::make_rope(rope);
   const int N = g->t_height * g->t_width * g->b_size;
@@ -242,6 +298,8 @@ int swa_bwd_dkdv(const swa_geom_t* g, const swa_rope_t* rope, const swa_tensor_t
     if (e) return fail(E_LAUNCH, "tcgen05 dkdv: %s", swa::tc::last_error());
     return launch_ok("tcgen05 dkdv");
   }
+  int err = 0;
+  if ((!rope || !rope->idx) && launch_simt_tile(2, g, nullptr, k, v, q, d_o, dk, dv, nullptr, lse, delta, st, &err)) return err;
   const swa::Geom gg = swa::make_geom(g);
   const swa::RopeDev rp = swa::make_rope(rope);
   const int N = g->t_height * g->t_width * g->b_size;
@@ -318,6 +376,8 @@ int swa_fwd_rot(const swa_geom_t* g, const swa_rope_t* rope, const swa_tensor_t*
     if (e) return fail(E_LAUNCH, "tcgen05 forward: %s", swa::tc::last_error());
     return launch_ok("tcgen05 forward (rotation handed on)");
   }
+  int err = 0;
+  if (launch_simt_tile(0, g, nullptr, q_rot, nullptr, k_rot, v, o, nullptr, lse, nullptr, nullptr, st, &err)) return err;
   const swa::Geom gg = swa::make_geom(g);
   const swa::RopeDev none = swa::make_rope(nullptr);
   const int N = g->t_height * g->t_width * g->b_size;
@@ -349,6 +409,8 @@ int swa_bwd_dq_rot(const swa_geom_t* g, const swa_rope_t* rope, const swa_tensor
     if (e) return fail(E_LAUNCH, "tcgen05 dq: %s", swa::tc::last_error());
     return launch_ok("tcgen05 dq (inputs rotated)");
   }
+  int err = 0;
+  if (launch_simt_tile(1, g, rope, q_rot, d_o, k_rot, v, dq, nullptr, nullptr, lse, delta, st, &err)) return err;
   const swa::Geom gg = swa::make_geom(g);
   const swa::RopeDev none = swa::make_rope(nullptr);
   const int N = g->t_height * g->t_width * g->b_size;
@@ -382,6 +444,8 @@ int swa_bwd_dkdv_rot(const swa_geom_t* g, const swa_rope_t* rope, const swa_tens
     if (e) return fail(E_LAUNCH, "tcgen05 dkdv: %s", swa::tc::last_error());
     return launch_ok("tcgen05 dkdv (inputs rotated)");
   }
+  int err = 0;
+  if (launch_simt_tile(2, g, rope, k_rot, v, q_rot, d_o, dk, dv, nullptr, lse, delta, st, &err)) return err;
   const swa::Geom gg = swa::make_geom(g);
   const swa::RopeDev none = swa::make_rope(nullptr);
   const int N = g->t_height * g->t_width * g->b_size;

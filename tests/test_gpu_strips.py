@@ -41,3 +41,23 @@ def test_strips_against_simt(th, tw, b, wr, wc, dqk, dv, R, BH):
         assert torch.isfinite(a.float()).all(), n
         err = (a.float() - c.float()).norm() / max(c.float().norm(), 0.1 * c.numel() ** 0.5)     # (a 1 x 1 window has dq = dk = 0)
         assert err < 1e-2, f"{n}: relative error {float(err):.2e}"
+
+
+@pytest.mark.parametrize("th,tw,b,wr,wc,dqk,dv,R,BH", [
+    (16, 16, 1, 3, 3, 32, 32, 8, 2), (9, 13, 1, 0, 0, 64, 64, 0, 3), (1, 5, 1, 2, 2, 4, 8, 1, 2), (33, 17, 1, 4, 6, 64, 64, 16, 5),
+    (20, 9, 2, 2, 1, 80, 48, 16, 3), (6, 5, 16, 1, 2, 96, 128, 8, 2), (40, 21, 1, 12, 12, 128, 128, 32, 2), (11, 30, 1, 1, 14, 128, 64, 0, 2)])
+def test_fp32_tiles_against_oracle(th, tw, b, wr, wc, dqk, dv, R, BH):
+    """fp32 (tiled CUDA-core kernels): tiles cut at the grid's edge, halos in one and several bands, head dims that leave
+    lanes idle, both rotation paths' common kernels."""
+    N = th * tw * b
+    q, k, v, do = orc.seeded_inputs(1, BH, N, dqk, dv, torch.float32, th)
+    rope_cpu = (orc.encode_idx(th, tw * b), orc.make_cs_table(R, max(th, 2)), orc.make_cs_table(R, max(tw * b, 2))) if R else (None,) * 3
+    win, sc = (b, th, tw, wr, wc), dqk ** -0.5
+    want = orc.fused_ref(q.double(), k.double(), v.double(), do.double(), *(t if t is None or t.dtype == torch.int32 else t.double() for t in rope_cpu),
+                         *win, sc)
+    qd, kd, vd = (t.to(DEV).requires_grad_(True) for t in (q, k, v))
+    o = swa.TiledSwaRope2D.apply(qd, kd, vd, *(t if t is None else t.to(DEV) for t in rope_cpu), *win, sc)
+    got = (o.detach(), *torch.autograd.grad(o, (qd, kd, vd), do.to(DEV)))
+    for a, c, n in zip(got, want, ("o", "dq", "dk", "dv")):
+        err = (a.cpu().double() - c).norm() / max(c.norm(), 0.1 * c.numel() ** 0.5)
+        assert err < 2e-6, f"{n}: relative error {float(err):.2e}"
