@@ -8,30 +8,29 @@
 namespace swa {
 
 // ---- delta ------------------------------------------------------------------------------------
-// Vector path (16-bit types, d_v % 8 == 0, unit last stride, 16-byte aligned rows):
-// a group of d_v/8 consecutive threads owns one token, each thread reads 8 elements
-// of o and of do, the group reduces with shuffles.  Groups never straddle a warp
-// because d_v/8 is a power of two <= 32 on this path.
+// Vector path (unit last stride, 16-byte aligned rows of whole 16-byte units): a group of lanes -- the power of two
+// that holds the row's units -- owns one token, each lane reads one unit of o and of do, the group reduces with
+// shuffles.  Groups never straddle a warp.
 template <typename T>
 __global__ void __launch_bounds__(256) delta_vec_kernel(View4 o, View4 d_o, float* __restrict__ delta, int H,
-                                                        int64_t N, int dv, int64_t total_rows) {
-  const int tpr = dv >> 3;  // threads per row
+                                                        int64_t N, int units, int group, int64_t total_rows) {
+  constexpr int E = 16 / sizeof(T);
   const int64_t gid = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  const int64_t row = gid / tpr;
-  const int part = (int)(gid - row * tpr);
+  const int64_t row = gid / group;
+  const int part = (int)(gid - row * group);
   float acc = 0.f;
-  if (row < total_rows) {
+  if (row < total_rows && part < units) {
     const int64_t bh = row / N, n = row - bh * N;
     const int64_t bi = bh / H, hi = bh - bi * H;
-    const uint4 a = *reinterpret_cast<const uint4*>((const T*)o.ptr + bi * o.s0 + hi * o.s1 + n * o.s2 + part * 8);
+    const uint4 a = *reinterpret_cast<const uint4*>((const T*)o.ptr + bi * o.s0 + hi * o.s1 + n * o.s2 + part * E);
     const uint4 b =
-        *reinterpret_cast<const uint4*>((const T*)d_o.ptr + bi * d_o.s0 + hi * d_o.s1 + n * d_o.s2 + part * 8);
+        *reinterpret_cast<const uint4*>((const T*)d_o.ptr + bi * d_o.s0 + hi * d_o.s1 + n * d_o.s2 + part * E);
     const T* pa = reinterpret_cast<const T*>(&a);
     const T* pb = reinterpret_cast<const T*>(&b);
 #pragma unroll
-    for (int i = 0; i < 8; ++i) acc += to_f(pa[i]) * to_f(pb[i]);
+    for (int i = 0; i < E; ++i) acc += to_f(pa[i]) * to_f(pb[i]);
   }
-  for (int off = tpr >> 1; off > 0; off >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, off);
+  for (int off = group >> 1; off > 0; off >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, off);
   if (row < total_rows && part == 0) delta[row] = acc;
 }
 

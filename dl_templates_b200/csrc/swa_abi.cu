@@ -77,8 +77,8 @@ int launch_ok(const char* what) {
 
 // Resolve AUTO / reject TC requests the tensor-core kernels cannot serve.
 int resolve_impl(const swa_geom_t* g, const swa_rope_t* rope, const swa_tensor_t* const* tensors, int n_tensors,
-                 int which, bool prerotated = false) {
-  const char* why = swa::tc::unsupported_reason(g, rope, tensors, n_tensors, which, prerotated);
+                 int which, bool prerotated = false, bool any8 = false) {
+  const char* why = swa::tc::unsupported_reason(g, rope, tensors, n_tensors, which, prerotated, any8);
   if (g->impl == SWA_IMPL_SIMT) return SWA_IMPL_SIMT;
   if (why == nullptr) return SWA_IMPL_TC;
   if (g->impl == SWA_IMPL_TC) return fail(E_IMPL, "tensor-core path unavailable: %s", why);
@@ -159,8 +159,7 @@ int swa_describe_plan(const swa_geom_t* g, const swa_rope_t* rope, int32_t which
   return 0;
 }
 
-int swa_fwd(const swa_geom_t* g, const swa_rope_t* rope, const swa_tensor_t* q, const swa_tensor_t* k,
-            const swa_tensor_t* v, const swa_tensor_t* o, float* lse, int32_t* status, void* stream) {
+static int fwd_call(bool any8, const swa_geom_t* g, const swa_rope_t* rope, const swa_tensor_t* q, const swa_tensor_t* k, const swa_tensor_t* v, const swa_tensor_t* o, float* lse, int32_t* status, void* stream) {
   if (int e = check_geom(g)) return e;
   if (int e = check_rope(g, rope)) return e;
   if (int e = check_tensor(q, "q")) return e;
@@ -169,7 +168,7 @@ int swa_fwd(const swa_geom_t* g, const swa_rope_t* rope, const swa_tensor_t* q, 
   if (int e = check_tensor(o, "o")) return e;
   if (!lse) return fail(E_NULL, "lse is NULL");
   const swa_tensor_t* ts[] = {q, k, v, o};
-  const int impl = resolve_impl(g, rope, ts, 4, 0);
+  const int impl = resolve_impl(g, rope, ts, 4, 0, false, any8);
   if (impl < 0) return impl;
   cudaStream_t st = (cudaStream_t)stream;
   if (impl == SWA_IMPL_TC) {
@@ -189,6 +188,10 @@ int swa_fwd(const swa_geom_t* g, const swa_rope_t* rope, const swa_tensor_t* q, 
                                    swa::make_view(o), lse));
   return launch_ok("simt forward");
 }
+int swa_fwd(const swa_geom_t* g, const swa_rope_t* rope, const swa_tensor_t* q, const swa_tensor_t* k,
+            const swa_tensor_t* v, const swa_tensor_t* o, float* lse, int32_t* status, void* stream) {
+  return fwd_call(false, g, rope, q, k, v, o, lse, status, stream);
+}
 
 int swa_bwd_delta(const swa_geom_t* g, const swa_tensor_t* o, const swa_tensor_t* d_o, float* delta, void* stream) {
   if (int e = check_geom(g)) return e;
@@ -204,39 +207,26 @@ int swa_bwd_delta(const swa_geom_t* g, const swa_tensor_t* o, const swa_tensor_t
     return t->stride[3] == 1 && ((uintptr_t)t->ptr % 16) == 0 && (t->stride[0] * esz) % 16 == 0 &&
            (t->stride[1] * esz) % 16 == 0 && (t->stride[2] * esz) % 16 == 0;
   };
-  const bool pow2 = (dv & (dv - 1)) == 0;
-  if (esz == 2 && pow2 && dv >= 8 && dv <= 256 && vec_ok(o) && vec_ok(d_o)) {
-    const int64_t threads = rows * (dv / 8);
-    const unsigned blocks = (unsigned)((threads + 255) / 256);
+  const int units = dv * esz / 16;                       // 16-byte units of a row, one per lane of its group
+  if (dv * esz % 16 == 0 && units <= 32 && vec_ok(o) && vec_ok(d_o)) {
+    int group = 1;                                       // lanes of a row's group: the power of two that holds its units
+    while (group < units) group *= 2;
+    const unsigned blocks = (unsigned)((rows * group + 255) / 256);
     auto flat = [&](const swa_tensor_t* t) {
       return t->stride[2] == dv && t->stride[1] == N * dv && (g->B == 1 || t->stride[0] == (int64_t)g->H * N * dv);
     };
-    if (flat(o) && flat(d_o)) {
-      if (g->dtype == SWA_F16)
-        swa::delta_flat_kernel<__half><<<blocks, 256, 0, st>>>((const __half*)o->ptr, (const __half*)d_o->ptr, delta, dv, rows);
-      else
-        swa::delta_flat_kernel<__nv_bfloat16><<<blocks, 256, 0, st>>>((const __nv_bfloat16*)o->ptr,
-                                                                      (const __nv_bfloat16*)d_o->ptr, delta, dv, rows);
-      return launch_ok("delta");
-    }
     auto token_major = [&](const swa_tensor_t* t) {   // [B,N,H,d_v] row-major seen as [B,H,N,d_v]
       return t->stride[1] == dv && t->stride[2] == (int64_t)g->H * dv && (g->B == 1 || t->stride[0] == (int64_t)g->H * N * dv);
     };
-    if (token_major(o) && token_major(d_o)) {
-      if (g->dtype == SWA_F16)
-        swa::delta_flat_kernel<__half, true><<<blocks, 256, 0, st>>>((const __half*)o->ptr, (const __half*)d_o->ptr, delta, dv,
-                                                                     rows, g->H, N);
-      else
-        swa::delta_flat_kernel<__nv_bfloat16, true><<<blocks, 256, 0, st>>>(
-            (const __nv_bfloat16*)o->ptr, (const __nv_bfloat16*)d_o->ptr, delta, dv, rows, g->H, N);
-      return launch_ok("delta");
+    if (esz == 2 && group == units && flat(o) && flat(d_o)) {
+      SWA_DISPATCH_DTYPE(g->dtype, swa::delta_flat_kernel<T><<<blocks, 256, 0, st>>>((const T*)o->ptr, (const T*)d_o->ptr, delta, dv, rows));
+    } else if (esz == 2 && group == units && token_major(o) && token_major(d_o)) {
+      SWA_DISPATCH_DTYPE(g->dtype, swa::delta_flat_kernel<T, true><<<blocks, 256, 0, st>>>((const T*)o->ptr, (const T*)d_o->ptr, delta, dv,
+                                                                                        rows, g->H, N));
+    } else {
+      SWA_DISPATCH_DTYPE(g->dtype, swa::delta_vec_kernel<T><<<blocks, 256, 0, st>>>(swa::make_view(o), swa::make_view(d_o), delta, g->H, N,
+                                                                                 units, group, rows));
     }
-    if (g->dtype == SWA_F16)
-      swa::delta_vec_kernel<__half><<<blocks, 256, 0, st>>>(swa::make_view(o), swa::make_view(d_o), delta, g->H, N,
-                                                            dv, rows);
-    else
-      swa::delta_vec_kernel<__nv_bfloat16><<<blocks, 256, 0, st>>>(swa::make_view(o), swa::make_view(d_o), delta,
-                                                                   g->H, N, dv, rows);
     return launch_ok("delta");
   }
   const unsigned blocks = (unsigned)((rows + 7) / 8);
@@ -245,9 +235,7 @@ int swa_bwd_delta(const swa_geom_t* g, const swa_tensor_t* o, const swa_tensor_t
   return launch_ok("delta");
 }
 
-int swa_bwd_dq(const swa_geom_t* g, const swa_rope_t* rope, const swa_tensor_t* q, const swa_tensor_t* k,
-               const swa_tensor_t* v, const swa_tensor_t* d_o, const float* lse, const float* delta,
-               const swa_tensor_t* dq, int32_t* status, void* stream) {
+static int dq_call(bool any8, const swa_geom_t* g, const swa_rope_t* rope, const swa_tensor_t* q, const swa_tensor_t* k, const swa_tensor_t* v, const swa_tensor_t* d_o, const float* lse, const float* delta, const swa_tensor_t* dq, int32_t* status, void* stream) {
   if (int e = check_geom(g)) return e;
   if (int e = check_rope(g, rope)) return e;
   if (int e = check_tensor(q, "q")) return e;
@@ -257,7 +245,7 @@ int swa_bwd_dq(const swa_geom_t* g, const swa_rope_t* rope, const swa_tensor_t* 
   if (int e = check_tensor(dq, "dq")) return e;
   if (!lse || !delta) return fail(E_NULL, "lse/delta is NULL");
   const swa_tensor_t* ts[] = {q, k, v, d_o, dq};
-  const int impl = resolve_impl(g, rope, ts, 5, 1);
+  const int impl = resolve_impl(g, rope, ts, 5, 1, false, any8);
   if (impl < 0) return impl;
   cudaStream_t st = (cudaStream_t)stream;
   if (impl == SWA_IMPL_TC) {
@@ -276,10 +264,13 @@ int swa_bwd_dq(const swa_geom_t* g, const swa_rope_t* rope, const swa_tensor_t* 
                                    swa::make_view(d_o), lse, delta, swa::make_view(dq)));
   return launch_ok("simt dq");
 }
+int swa_bwd_dq(const swa_geom_t* g, const swa_rope_t* rope, const swa_tensor_t* q, const swa_tensor_t* k,
+               const swa_tensor_t* v, const swa_tensor_t* d_o, const float* lse, const float* delta,
+               const swa_tensor_t* dq, int32_t* status, void* stream) {
+  return dq_call(false, g, rope, q, k, v, d_o, lse, delta, dq, status, stream);
+}
 
-int swa_bwd_dkdv(const swa_geom_t* g, const swa_rope_t* rope, const swa_tensor_t* q, const swa_tensor_t* k,
-                 const swa_tensor_t* v, const swa_tensor_t* d_o, const float* lse, const float* delta,
-                 const swa_tensor_t* dk, const swa_tensor_t* dv, int32_t* status, void* stream) {
+static int dkdv_call(bool any8, const swa_geom_t* g, const swa_rope_t* rope, const swa_tensor_t* q, const swa_tensor_t* k, const swa_tensor_t* v, const swa_tensor_t* d_o, const float* lse, const float* delta, const swa_tensor_t* dk, const swa_tensor_t* dv, int32_t* status, void* stream) {
   if (int e = check_geom(g)) return e;
   if (int e = check_rope(g, rope)) return e;
   if (int e = check_tensor(q, "q")) return e;
@@ -290,7 +281,7 @@ int swa_bwd_dkdv(const swa_geom_t* g, const swa_rope_t* rope, const swa_tensor_t
   if (int e = check_tensor(dv, "dv")) return e;
   if (!lse || !delta) return fail(E_NULL, "lse/delta is NULL");
   const swa_tensor_t* ts[] = {q, k, v, d_o, dk, dv};
-  const int impl = resolve_impl(g, rope, ts, 6, 2);
+  const int impl = resolve_impl(g, rope, ts, 6, 2, false, any8);
   if (impl < 0) return impl;
   cudaStream_t st = (cudaStream_t)stream;
   if (impl == SWA_IMPL_TC) {
@@ -308,6 +299,11 @@ int swa_bwd_dkdv(const swa_geom_t* g, const swa_rope_t* rope, const swa_tensor_t
                                    gg, rp, swa::make_view(q), swa::make_view(k), swa::make_view(v),
                                    swa::make_view(d_o), lse, delta, swa::make_view(dk), swa::make_view(dv)));
   return launch_ok("simt dkdv");
+}
+int swa_bwd_dkdv(const swa_geom_t* g, const swa_rope_t* rope, const swa_tensor_t* q, const swa_tensor_t* k,
+                 const swa_tensor_t* v, const swa_tensor_t* d_o, const float* lse, const float* delta,
+                 const swa_tensor_t* dk, const swa_tensor_t* dv, int32_t* status, void* stream) {
+  return dkdv_call(false, g, rope, q, k, v, d_o, lse, delta, dk, dv, status, stream);
 }
 
 // ---- rotation handed on between the kernels ---------------------------------------------------
@@ -350,9 +346,7 @@ int require_rope(const swa_rope_t* rope, const char* who) {
 
 }  // namespace
 
-int swa_fwd_rot(const swa_geom_t* g, const swa_rope_t* rope, const swa_tensor_t* q, const swa_tensor_t* k,
-                const swa_tensor_t* v, const swa_tensor_t* o, float* lse, const swa_tensor_t* q_rot,
-                const swa_tensor_t* k_rot, int32_t* status, void* stream) {
+static int fwd_rot_call(bool any8, const swa_geom_t* g, const swa_rope_t* rope, const swa_tensor_t* q, const swa_tensor_t* k, const swa_tensor_t* v, const swa_tensor_t* o, float* lse, const swa_tensor_t* q_rot, const swa_tensor_t* k_rot, int32_t* status, void* stream) {
   if (int e = check_geom(g)) return e;
   if (int e = require_rope(rope, "swa_fwd_rot")) return e;
   if (int e = check_rope(g, rope)) return e;
@@ -365,7 +359,7 @@ int swa_fwd_rot(const swa_geom_t* g, const swa_rope_t* rope, const swa_tensor_t*
   if (!lse) return fail(E_NULL, "lse is NULL");
   if (q_rot->ptr == q->ptr || k_rot->ptr == k->ptr) return fail(E_SHAPE, "q_rot / k_rot must not alias q / k");
   const swa_tensor_t* ts[] = {q, k, v, o, q_rot, k_rot};
-  const int impl = resolve_impl(g, rope, ts, 6, 0, true);
+  const int impl = resolve_impl(g, rope, ts, 6, 0, true, any8);
   if (impl < 0) return impl;
   cudaStream_t st = (cudaStream_t)stream;
   // every q and k row is rotated exactly once, by a streaming pass; the attention kernels read the rotated rows
@@ -387,10 +381,13 @@ int swa_fwd_rot(const swa_geom_t* g, const swa_rope_t* rope, const swa_tensor_t*
                                    swa::make_view(o), lse));
   return launch_ok("simt forward");
 }
+int swa_fwd_rot(const swa_geom_t* g, const swa_rope_t* rope, const swa_tensor_t* q, const swa_tensor_t* k,
+                const swa_tensor_t* v, const swa_tensor_t* o, float* lse, const swa_tensor_t* q_rot,
+                const swa_tensor_t* k_rot, int32_t* status, void* stream) {
+  return fwd_rot_call(false, g, rope, q, k, v, o, lse, q_rot, k_rot, status, stream);
+}
 
-int swa_bwd_dq_rot(const swa_geom_t* g, const swa_rope_t* rope, const swa_tensor_t* q_rot, const swa_tensor_t* k_rot,
-                   const swa_tensor_t* v, const swa_tensor_t* d_o, const float* lse, const float* delta,
-                   const swa_tensor_t* dq, int32_t* status, void* stream) {
+static int dq_rot_call(bool any8, const swa_geom_t* g, const swa_rope_t* rope, const swa_tensor_t* q_rot, const swa_tensor_t* k_rot, const swa_tensor_t* v, const swa_tensor_t* d_o, const float* lse, const float* delta, const swa_tensor_t* dq, int32_t* status, void* stream) {
   if (int e = check_geom(g)) return e;
   if (int e = require_rope(rope, "swa_bwd_dq_rot")) return e;
   if (int e = check_rope(g, rope)) return e;
@@ -401,7 +398,7 @@ int swa_bwd_dq_rot(const swa_geom_t* g, const swa_rope_t* rope, const swa_tensor
   if (int e = check_tensor(dq, "dq")) return e;
   if (!lse || !delta) return fail(E_NULL, "lse/delta is NULL");
   const swa_tensor_t* ts[] = {q_rot, k_rot, v, d_o, dq};
-  const int impl = resolve_impl(g, rope, ts, 5, 1, true);
+  const int impl = resolve_impl(g, rope, ts, 5, 1, true, any8);
   if (impl < 0) return impl;
   cudaStream_t st = (cudaStream_t)stream;
   if (impl == SWA_IMPL_TC) {
@@ -421,10 +418,13 @@ int swa_bwd_dq_rot(const swa_geom_t* g, const swa_rope_t* rope, const swa_tensor
   if (int e = launch_ok("simt dq")) return e;
   return launch_rope4(g, rope, dq, dq, true, st);
 }
+int swa_bwd_dq_rot(const swa_geom_t* g, const swa_rope_t* rope, const swa_tensor_t* q_rot, const swa_tensor_t* k_rot,
+                   const swa_tensor_t* v, const swa_tensor_t* d_o, const float* lse, const float* delta,
+                   const swa_tensor_t* dq, int32_t* status, void* stream) {
+  return dq_rot_call(false, g, rope, q_rot, k_rot, v, d_o, lse, delta, dq, status, stream);
+}
 
-int swa_bwd_dkdv_rot(const swa_geom_t* g, const swa_rope_t* rope, const swa_tensor_t* q_rot, const swa_tensor_t* k_rot,
-                     const swa_tensor_t* v, const swa_tensor_t* d_o, const float* lse, const float* delta,
-                     const swa_tensor_t* dk, const swa_tensor_t* dv, int32_t* status, void* stream) {
+static int dkdv_rot_call(bool any8, const swa_geom_t* g, const swa_rope_t* rope, const swa_tensor_t* q_rot, const swa_tensor_t* k_rot, const swa_tensor_t* v, const swa_tensor_t* d_o, const float* lse, const float* delta, const swa_tensor_t* dk, const swa_tensor_t* dv, int32_t* status, void* stream) {
   if (int e = check_geom(g)) return e;
   if (int e = require_rope(rope, "swa_bwd_dkdv_rot")) return e;
   if (int e = check_rope(g, rope)) return e;
@@ -436,7 +436,7 @@ int swa_bwd_dkdv_rot(const swa_geom_t* g, const swa_rope_t* rope, const swa_tens
   if (int e = check_tensor(dv, "dv")) return e;
   if (!lse || !delta) return fail(E_NULL, "lse/delta is NULL");
   const swa_tensor_t* ts[] = {q_rot, k_rot, v, d_o, dk, dv};
-  const int impl = resolve_impl(g, rope, ts, 6, 2, true);
+  const int impl = resolve_impl(g, rope, ts, 6, 2, true, any8);
   if (impl < 0) return impl;
   cudaStream_t st = (cudaStream_t)stream;
   if (impl == SWA_IMPL_TC) {
@@ -455,6 +455,39 @@ int swa_bwd_dkdv_rot(const swa_geom_t* g, const swa_rope_t* rope, const swa_tens
                                    swa::make_view(d_o), lse, delta, swa::make_view(dk), swa::make_view(dv)));
   if (int e = launch_ok("simt dkdv")) return e;
   return launch_rope4(g, rope, dk, dk, true, st);
+}
+int swa_bwd_dkdv_rot(const swa_geom_t* g, const swa_rope_t* rope, const swa_tensor_t* q_rot, const swa_tensor_t* k_rot,
+                     const swa_tensor_t* v, const swa_tensor_t* d_o, const float* lse, const float* delta,
+                     const swa_tensor_t* dk, const swa_tensor_t* dv, int32_t* status, void* stream) {
+  return dkdv_rot_call(false, g, rope, q_rot, k_rot, v, d_o, lse, delta, dk, dv, status, stream);
+}
+
+// ---- one call per direction -------------------------------------------------------------------
+int swa_step_select(const swa_geom_t* g, const swa_rope_t* rope) {
+  if (int e = check_geom(g)) return e;
+  if (int e = check_rope(g, rope)) return e;
+  const bool rot = rope && rope->idx;
+  for (int which = 0; which < 3; ++which)
+    if (resolve_impl(g, rope, nullptr, 0, which, rot, true) != SWA_IMPL_TC) return SWA_IMPL_SIMT;
+  return SWA_IMPL_TC;
+}
+
+int swa_step_fwd(const swa_geom_t* g, const swa_rope_t* rope, const swa_tensor_t* q, const swa_tensor_t* k, const swa_tensor_t* v,
+                 const swa_tensor_t* o, float* lse, const swa_tensor_t* q_rot, const swa_tensor_t* k_rot, int32_t* status, void* stream) {
+  if (rope && rope->idx) return fwd_rot_call(true, g, rope, q, k, v, o, lse, q_rot, k_rot, status, stream);
+  return fwd_call(true, g, nullptr, q, k, v, o, lse, status, stream);
+}
+
+int swa_step_bwd(const swa_geom_t* g, const swa_rope_t* rope, const swa_tensor_t* q, const swa_tensor_t* k, const swa_tensor_t* v,
+                 const swa_tensor_t* o, const swa_tensor_t* d_o, const float* lse, float* delta, const swa_tensor_t* dq,
+                 const swa_tensor_t* dk, const swa_tensor_t* dv, int32_t* status, void* stream) {
+  if (int e = swa_bwd_delta(g, o, d_o, delta, stream)) return e;
+  if (rope && rope->idx) {
+    if (int e = dq_rot_call(true, g, rope, q, k, v, d_o, lse, delta, dq, status, stream)) return e;
+    return dkdv_rot_call(true, g, rope, q, k, v, d_o, lse, delta, dk, dv, status, stream);
+  }
+  if (int e = dq_call(true, g, nullptr, q, k, v, d_o, lse, delta, dq, status, stream)) return e;
+  return dkdv_call(true, g, nullptr, q, k, v, d_o, lse, delta, dk, dv, status, stream);
 }
 
 // ---- backward without allocation ------------------------------------------------------------

@@ -546,7 +546,7 @@ void refresh_env() {
 }
 
 const char* unsupported_reason(const swa_geom_t* g, const swa_rope_t* rope, const swa_tensor_t* const* tensors,
-                               int n_tensors, int which, bool prerotated) {
+                               int n_tensors, int which, bool prerotated, bool any8) {
   if (knobs().disable) return "disabled by SWA_TC_DISABLE";
   if (g->dtype != SWA_F16 && g->dtype != SWA_BF16) return "fp32 runs on the SIMT kernels";
   // The kernels work on 64-element chunks of a row.  Those without streamed rotation also take head dims of 32 and
@@ -555,7 +555,7 @@ const char* unsupported_reason(const swa_geom_t* g, const swa_rope_t* rope, cons
   // never stored), which costs MMA work on zeros but no HBM traffic and no padded copies.
   {
     const bool v2_dims = prerotated || !(rope && rope->idx);
-    auto dim_ok = [&](int d) { return v2_dims ? (d >= 32 && d <= 128 && d % 32 == 0) : (d == 64 || d == 128); };
+    auto dim_ok = [&](int d) { return v2_dims && any8 ? (d >= 8 && d <= 128 && d % 8 == 0) : v2_dims ? (d >= 32 && d <= 128 && d % 32 == 0) : (d == 64 || d == 128); };
     if (!dim_ok(g->d_qk) || !dim_ok(g->d_v))
       return v2_dims ? "head dims must be 32, 64, 96 or 128" : "head dims must be 64 or 128 for the kernels that rotate streamed rows";
   }

@@ -9,9 +9,10 @@ namespace tc {
 // nullptr when the tensor-core kernels cover this call, else the reason they do not.
 // `which`: 0 forward, 1 dQ, 2 dK/dV.  `tensors` may be null (shape-only query).
 // `prerotated`: the call hands rotated copies of q / k between the kernels (swa_fwd_rot and the *_rot backward
-// entries), so no kernel rotates streamed rows and the plan is the one without RoPE.
+// entries), so no kernel rotates streamed rows and the plan is the one without RoPE.  `any8`: head dims of any multiple
+// of 8 (the swa_step_* entries) instead of 32, 64, 96 and 128.
 const char* unsupported_reason(const swa_geom_t* g, const swa_rope_t* rope, const swa_tensor_t* const* tensors,
-                               int n_tensors, int which, bool prerotated = false);
+                               int n_tensors, int which, bool prerotated = false, bool any8 = false);
 const char* last_error();
 
 // Re-read the SWA_TC_* experiment knobs from the environment and drop the cached plans (both are otherwise read /

@@ -190,6 +190,17 @@ std::array<int64_t, 2> padded_dims(const Tensor& q, int64_t d_v, const Rope* rop
   return {p_qk, p_v};
 }
 
+// Whether the kernels without streamed rotation take the head dims as they are (or fp32, which is never padded).
+bool native_dims(const Tensor& q, int64_t d_v, const Rope* rope, const Win& w, int32_t impl) {
+  if (impl != SWA_IMPL_AUTO || q.scalar_type() == at::kFloat) return true;
+  if (q.dim() != 4) return false;
+  swa_rope_t r;
+  const swa_rope_t* rp = nullptr;
+  if (rope && rope->on()) { r = rope_view(*rope); rp = &r; }
+  const swa_geom_t g = geom(q, q.size(3), d_v, w, forced_impl(SWA_IMPL_AUTO));
+  return swa_step_select(&g, rp) == SWA_IMPL_TC;
+}
+
 Tensor pad_last(const Tensor& t, int64_t d) {
   return t.size(3) == d ? t : at::constant_pad_nd(t, {0, d - t.size(3)});
 }
@@ -211,7 +222,8 @@ struct Grads {
 Fwd forward(Tensor q, Tensor k, Tensor v, const Rope& rope, const Win& w, int32_t impl, Tensor out) {
   check_inputs(q, k, v, w);
   q = materialise(q); k = materialise(k); v = materialise(v);
-  const auto pad = padded_dims(q, v.size(3), &rope, w, impl);
+  const auto pad = !rope.on() && native_dims(q, v.size(3), nullptr, w, impl) ? std::array<int64_t, 2>{0, 0}
+                                                                          : padded_dims(q, v.size(3), &rope, w, impl);
   if (pad[0]) {
     Fwd f = forward(pad_last(q, pad[0]), pad_last(k, pad[0]), pad_last(v, pad[1]), rope, w, impl, Tensor());
     const Tensor o_v = f.o.narrow(3, 0, v.size(3));
@@ -234,8 +246,11 @@ Fwd forward(Tensor q, Tensor k, Tensor v, const Rope& rope, const Win& w, int32_
   swa_rope_t r;
   if (rope.on()) r = rope_view(rope);
   const swa_tensor_t tq = view4(q), tk = view4(k), tv = view4(v), to = view4(f.o);
-  check(swa_fwd(&g, rope.on() ? &r : nullptr, &tq, &tk, &tv, &to, f.lse.data_ptr<float>(), status_ptr(q.get_device()),
-                stream_of(q)), "swa_fwd");
+  if (rope.on())
+    check(swa_fwd(&g, &r, &tq, &tk, &tv, &to, f.lse.data_ptr<float>(), status_ptr(q.get_device()), stream_of(q)), "swa_fwd");
+  else
+    check(swa_step_fwd(&g, nullptr, &tq, &tk, &tv, &to, f.lse.data_ptr<float>(), nullptr, nullptr, status_ptr(q.get_device()),
+                       stream_of(q)), "swa_step_fwd");
   debug_sync();
   return f;
 }
@@ -254,8 +269,8 @@ Fwd forward_rot(Tensor q, Tensor k, Tensor v, const Rope& rope, const Win& w, in
   const swa_geom_t g = geom(q, q.size(3), v.size(3), w, forced_impl(impl));
   const swa_rope_t r = rope_view(rope);
   const swa_tensor_t tq = view4(q), tk = view4(k), tv = view4(v), to = view4(f.o), tqr = view4(f.q_rot), tkr = view4(f.k_rot);
-  check(swa_fwd_rot(&g, &r, &tq, &tk, &tv, &to, f.lse.data_ptr<float>(), &tqr, &tkr, status_ptr(q.get_device()), stream_of(q)),
-        "swa_fwd_rot");
+  check(swa_step_fwd(&g, &r, &tq, &tk, &tv, &to, f.lse.data_ptr<float>(), &tqr, &tkr, status_ptr(q.get_device()), stream_of(q)),
+        "swa_step_fwd");
   debug_sync();
   return f;
 }
@@ -266,7 +281,7 @@ Grads backward(Tensor q, Tensor k, Tensor v, Tensor o, const Tensor& lse, Tensor
   poll_status();
   q = materialise(q); k = materialise(k); v = materialise(v); o = materialise(o); d_o = materialise(d_o);
   const bool given = out.dq.defined();
-  if (!rotated) {
+  if (!rotated && !(!rope.on() && native_dims(q, v.size(3), nullptr, w, impl))) {
     const auto pad = padded_dims(q, v.size(3), &rope, w, impl);
     if (pad[0]) {
       Grads g = backward(pad_last(q, pad[0]), pad_last(k, pad[0]), pad_last(v, pad[1]), pad_last(o, pad[1]), lse,
@@ -303,13 +318,12 @@ Grads backward(Tensor q, Tensor k, Tensor v, Tensor o, const Tensor& lse, Tensor
   int32_t* status = status_ptr(q.get_device());
   const float* l = lse.data_ptr<float>();
   float* de = delta.data_ptr<float>();
-  check(swa_bwd_delta(&g, &to, &tdo, de, st), "swa_bwd_delta");
-  if (rotated) {
-    check(swa_bwd_dq_rot(&g, rp, &tq, &tk, &tv, &tdo, l, de, &tdq, status, st), "swa_bwd_dq_rot");
-    check(swa_bwd_dkdv_rot(&g, rp, &tq, &tk, &tv, &tdo, l, de, &tdk, &tdv, status, st), "swa_bwd_dkdv_rot");
-  } else {
+  if (rope.on() && !rotated) {                       // the kernels that rotate streamed rows
+    check(swa_bwd_delta(&g, &to, &tdo, de, st), "swa_bwd_delta");
     check(swa_bwd_dq(&g, rp, &tq, &tk, &tv, &tdo, l, de, &tdq, status, st), "swa_bwd_dq");
     check(swa_bwd_dkdv(&g, rp, &tq, &tk, &tv, &tdo, l, de, &tdk, &tdv, status, st), "swa_bwd_dkdv");
+  } else {
+    check(swa_step_bwd(&g, rp, &tq, &tk, &tv, &to, &tdo, l, de, &tdq, &tdk, &tdv, status, st), "swa_step_bwd");
   }
   debug_sync();
   return r;
@@ -356,7 +370,7 @@ Tensor flat3(const Tensor& t) { return t.reshape({-1, t.size(2), t.size(3)}); }
 int mode_for(const Tensor& q, int64_t d_v, const Rope& rope, const Win& w) {
   if (!rope.on()) return kNone;
   const int m = g_rope_mode.load(std::memory_order_relaxed);
-  if (m == kHandoff && padded_dims(q, d_v, &rope, w, SWA_IMPL_AUTO)[0]) return kFused;
+  if (m == kHandoff && !native_dims(q, d_v, &rope, w, SWA_IMPL_AUTO) && padded_dims(q, d_v, &rope, w, SWA_IMPL_AUTO)[0]) return kFused;
   return m;
 }
 

@@ -185,8 +185,11 @@ def _mode_for(q, v, rope, win) -> str:
     zero padding take the fused path (the padding wrapper lives there)."""
     if rope is None:
         return "none"
-    if _rope_mode == "handoff" and padded_head_dims(q, v, rope, *win) is not None:
-        return "fused"
+    if _rope_mode == "handoff":
+        g = _geom(q, v, *win, "auto")
+        native = q.dtype == torch.float32 or _lib.lib.swa_step_select(C.byref(g), _ref(_lib.make_rope(*rope))) == _lib.IMPL_TC
+        if not native and padded_head_dims(q, v, rope, *win) is not None:
+            return "fused"
     return _rope_mode
 
 

@@ -119,6 +119,20 @@ int swa_bwd_dkdv_rot(const swa_geom_t* g, const swa_rope_t* rope, const swa_tens
                      const swa_tensor_t* v, const swa_tensor_t* d_o, const float* lse, const float* delta,
                      const swa_tensor_t* dk, const swa_tensor_t* dv, int32_t* status, void* stream);
 
+/* One call per direction, what the Python surface uses: swa_step_fwd is swa_fwd_rot with RoPE and swa_fwd without
+ * (q_rot / k_rot unused then); swa_step_bwd is swa_bwd_delta, then swa_bwd_dq_rot and swa_bwd_dkdv_rot (q, k = the rotated
+ * copies) or swa_bwd_dq and swa_bwd_dkdv, with `delta` as scratch.  Beyond the single entries they take 16-bit head dims of
+ * any multiple of 8 up to 128 on the tensor-core kernels as they are (the tensor maps carry the real head dim, TMA fills and
+ * clips).  swa_step_select: the kernel family they run for a geometry.  Replace the same launches of the reference as
+ * the entries they stand for. */
+int swa_step_select(const swa_geom_t* g, const swa_rope_t* rope);
+int swa_step_fwd(const swa_geom_t* g, const swa_rope_t* rope, const swa_tensor_t* q, const swa_tensor_t* k,
+                 const swa_tensor_t* v, const swa_tensor_t* o, float* lse, const swa_tensor_t* q_rot,
+                 const swa_tensor_t* k_rot, int32_t* status, void* stream);
+int swa_step_bwd(const swa_geom_t* g, const swa_rope_t* rope, const swa_tensor_t* q, const swa_tensor_t* k,
+                 const swa_tensor_t* v, const swa_tensor_t* o, const swa_tensor_t* d_o, const float* lse, float* delta,
+                 const swa_tensor_t* dq, const swa_tensor_t* dk, const swa_tensor_t* dv, int32_t* status, void* stream);
+
 /* Stand-alone in-place RoPE-2D on x [batch, N, C] (element strides xs[3]).
  * inverse = 0 replaces rope2d_fwd_kernel (src/fused_rope2d.py:24-72), inverse = 1
  * replaces rope2d_bwd_kernel (src/fused_rope2d.py:74-122).  A negative index half

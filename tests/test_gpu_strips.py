@@ -61,3 +61,24 @@ def test_fp32_tiles_against_oracle(th, tw, b, wr, wc, dqk, dv, R, BH):
     for a, c, n in zip(got, want, ("o", "dq", "dk", "dv")):
         err = (a.cpu().double() - c).norm() / max(c.norm(), 0.1 * c.numel() ** 0.5)
         assert err < 2e-6, f"{n}: relative error {float(err):.2e}"
+
+
+@pytest.mark.parametrize("dqk,dv,R", [(80, 80, 16), (48, 48, 8), (8, 24, 0), (72, 104, 8), (120, 40, 16), (32, 32, 8), (96, 96, 16)])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+def test_head_dims_of_any_multiple_of_8_as_they_are(dqk, dv, R, dtype):
+    """The autograd surface hands such head dims to the tensor-core kernels without padded copies: no launch but its own,
+    results against the oracle."""
+    th, tw, win, sc = 21, 26, (1, 21, 26, 3, 2), dqk ** -0.5
+    q, k, v, do = orc.seeded_inputs(1, 2, th * tw, dqk, dv, dtype, dqk)
+    rope = (orc.encode_idx(th, tw), orc.make_cs_table(R, th), orc.make_cs_table(R, tw)) if R else (None,) * 3
+    want = orc.fused_ref(q.float(), k.float(), v.float(), do.float(), *rope, *win, sc)
+    qd, kd, vd = (t.to(DEV).requires_grad_(True) for t in (q, k, v))
+    rd = tuple(None if t is None else t.to(DEV) for t in rope)
+    before = swa._lib.launch_count()
+    o = swa.TiledSwaRope2D.apply(qd, kd, vd, *rd, *win, sc)
+    got = (o.detach(), *torch.autograd.grad(o, (qd, kd, vd), do.to(DEV)))
+    swa.check_status()
+    assert swa._lib.launch_count() - before <= (6 if R else 4)
+    assert swa.tiled_swa._mode_for(qd, vd, rd if R else None, (*win, sc)) == ("handoff" if R else "none")
+    for a, c, n in zip(got, want, ("o", "dq", "dk", "dv")):
+        assert orc.max_abs(a.float().cpu(), c) < 2e-2 and orc.mean_rel(a.float().cpu(), c) < 5e-3, n
