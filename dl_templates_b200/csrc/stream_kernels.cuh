@@ -14,6 +14,8 @@ namespace swa {
 template <typename T>
 __global__ void __launch_bounds__(256) delta_vec_kernel(View4 o, View4 d_o, float* __restrict__ delta, int H,
                                                         int64_t N, int units, int group, int64_t total_rows) {
+  pdl_enter();
+  pdl_wait();
   constexpr int E = 16 / sizeof(T);
   const int64_t gid = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   const int64_t row = gid / group;
@@ -40,7 +42,9 @@ __global__ void __launch_bounds__(256) delta_vec_kernel(View4 o, View4 d_o, floa
 template <typename T, bool TOKEN_MAJOR = false>
 __global__ void __launch_bounds__(256) delta_flat_kernel(const T* __restrict__ o, const T* __restrict__ d_o,
                                                          float* __restrict__ delta, int dv, int64_t total_rows,
-                                                         int H = 1, int64_t N = 1) {
+                                                         int H, int64_t N) {
+  pdl_enter();
+  pdl_wait();
   const int tpr = dv >> 3;  // threads per row
   const int64_t gid = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   const int64_t row = gid / tpr;
@@ -178,52 +182,70 @@ __global__ void __launch_bounds__(256) rope2d_copy_kernel(const T* __restrict__ 
   *reinterpret_cast<uint4*>(y + bi * ys0 + tok * ys1 + u * 8) = own;
 }
 
-// One-pass clone + rotate for a strided [B, H, N, C] 16-bit tensor (both tensors described by four element
-// strides, so packed projection outputs need no flattening copy).  One thread per "slot" of a token row: a slot of
-// the rotated dims is a 16-byte unit together with its partner unit R elements further (both halves of eight
-// pairs: two 16-byte loads, one set of cos/sin values, two 16-byte stores, nothing read twice); a slot of the dims
-// beyond 4R is two consecutive units that are copied.  grid = (slots of one (batch, head) slice / 256, B * H).
+// One-pass clone + rotate of q and of k, strided [B, H, N, C] (each described by four element strides, so packed
+// projection outputs need no flattening copy).  One thread per "slot" of a token row of both: a slot of the rotated dims is
+// a 16-byte unit together with its partner unit R elements further (all pairs of the unit: two 16-byte loads and stores per
+// tensor, nothing read twice, one set of cos/sin values for both tensors); a slot of the dims beyond 4R is two consecutive
+// units that are copied.  grid = (slots of one (batch, head) slice / 256, B * H).
 template <typename T>
-__global__ void __launch_bounds__(256) rope2d_copy4_kernel(View4 x, View4 y, int H, int N, int C, RopeDev rp, float sign) {
-  const uint32_t rot_slots = (uint32_t)rp.R >> 2;                       // 4R / 8 units, two per slot
-  const uint32_t spr = rot_slots + ((((uint32_t)C >> 3) - 2 * rot_slots + 1) >> 1);   // slots per row
+__global__ void __launch_bounds__(256) rope2d_copy4_kernel(View4 x, View4 y, View4 x2, View4 y2, int H, int N, int C, RopeDev rp,
+                                                           float sign) {
+  pdl_enter();
+  pdl_wait();
+  constexpr uint32_t E = 16 / sizeof(T);
+  const uint32_t per_half = (uint32_t)rp.R / E, rot_slots = 2 * per_half;
+  const uint32_t spr = rot_slots + (((uint32_t)C / E - 2 * rot_slots + 1) >> 1);      // slots per row
   const uint32_t gid = blockIdx.x * blockDim.x + threadIdx.x;
   const uint32_t tok = gid / spr;
   if (tok >= (uint32_t)N) return;
   const uint32_t sl = gid - tok * spr;
   const uint32_t bh = blockIdx.y;
   const int64_t b = bh / (uint32_t)H, h = bh - (uint32_t)b * (uint32_t)H;
-  const T* src = (const T*)x.ptr + b * x.s0 + h * x.s1 + (int64_t)tok * x.s2;
-  T* dst = (T*)y.ptr + b * y.s0 + h * y.s1 + (int64_t)tok * y.s2;
+  auto row = [&](const View4& v) { return (T*)v.ptr + b * v.s0 + h * v.s1 + (int64_t)tok * v.s2; };
+  const T *src = row(x), *src2 = row(x2);
+  T *dst = row(y), *dst2 = row(y2);
+  auto ld = [](const T* p) { return *reinterpret_cast<const uint4*>(p); };
   if (sl < rot_slots) {
-    const uint32_t per_half = (uint32_t)rp.R >> 3;                      // slots of the row-angle half
-    const uint32_t half = sl / per_half, i0 = (sl - half * per_half) * 8;
+    const uint32_t half = sl / per_half, i0 = (sl - half * per_half) * E;
     const uint32_t e0 = half * 2 * rp.R + i0, e1 = e0 + rp.R;
-    uint4 va = *reinterpret_cast<const uint4*>(src + e0), vb = *reinterpret_cast<const uint4*>(src + e1);
+    uint4 v[4] = {ld(src + e0), ld(src + e1), ld(src2 + e0), ld(src2 + e1)};
     int irow, icol;
     decode_idx(__ldg(rp.idx + tok), rp.max_h, rp.max_w, irow, icol);
     const int pos = half ? icol : irow;
     if (pos >= 0) {
       const float4* tab = reinterpret_cast<const float4*>((half ? rp.col_cs : rp.row_cs) + ((int64_t)pos * rp.R + i0) * 2);
-      T* ea = reinterpret_cast<T*>(&va);
-      T* eb = reinterpret_cast<T*>(&vb);
 #pragma unroll
-      for (int j = 0; j < 8; j += 2) {
+      for (int j = 0; j < (int)E; j += 2) {
         const float4 cs = __ldg(tab + (j >> 1));                        // (cos, sin) of pairs j and j + 1
-        const float a0 = to_f(ea[j]), b0 = to_f(eb[j]), a1 = to_f(ea[j + 1]), b1 = to_f(eb[j + 1]);
         const float s0 = cs.y * sign, s1 = cs.w * sign;
-        ea[j] = from_f<T>(a0 * cs.x - b0 * s0);
-        eb[j] = from_f<T>(a0 * s0 + b0 * cs.x);
-        ea[j + 1] = from_f<T>(a1 * cs.z - b1 * s1);
-        eb[j + 1] = from_f<T>(a1 * s1 + b1 * cs.z);
+#pragma unroll
+        for (int t = 0; t < 4; t += 2) {
+          T* ea = reinterpret_cast<T*>(&v[t]);
+          T* eb = reinterpret_cast<T*>(&v[t + 1]);
+          const float a0 = to_f(ea[j]), b0 = to_f(eb[j]), a1 = to_f(ea[j + 1]), b1 = to_f(eb[j + 1]);
+          ea[j] = from_f<T>(a0 * cs.x - b0 * s0);
+          eb[j] = from_f<T>(a0 * s0 + b0 * cs.x);
+          ea[j + 1] = from_f<T>(a1 * cs.z - b1 * s1);
+          eb[j + 1] = from_f<T>(a1 * s1 + b1 * cs.z);
+        }
       }
     }
-    *reinterpret_cast<uint4*>(dst + e0) = va;
-    *reinterpret_cast<uint4*>(dst + e1) = vb;
+    *reinterpret_cast<uint4*>(dst + e0) = v[0];
+    *reinterpret_cast<uint4*>(dst + e1) = v[1];
+    *reinterpret_cast<uint4*>(dst2 + e0) = v[2];
+    *reinterpret_cast<uint4*>(dst2 + e1) = v[3];
   } else {
-    const uint32_t e0 = 4 * rp.R + (sl - rot_slots) * 16;
-    *reinterpret_cast<uint4*>(dst + e0) = *reinterpret_cast<const uint4*>(src + e0);
-    if (e0 + 8 < (uint32_t)C) *reinterpret_cast<uint4*>(dst + e0 + 8) = *reinterpret_cast<const uint4*>(src + e0 + 8);
+    const uint32_t e0 = 4 * rp.R + (sl - rot_slots) * 2 * E;
+    const bool two = e0 + E < (uint32_t)C;
+    const uint4 a = ld(src + e0), c = ld(src2 + e0);
+    uint4 a1 = a, c1 = c;
+    if (two) { a1 = ld(src + e0 + E); c1 = ld(src2 + e0 + E); }
+    *reinterpret_cast<uint4*>(dst + e0) = a;
+    *reinterpret_cast<uint4*>(dst2 + e0) = c;
+    if (two) {
+      *reinterpret_cast<uint4*>(dst + e0 + E) = a1;
+      *reinterpret_cast<uint4*>(dst2 + e0 + E) = c1;
+    }
   }
 }
 

@@ -125,11 +125,12 @@ bool launch_simt_tile(int kind, const swa_geom_t* g, const swa_rope_t* rope, con
       {{swa::simt_tile_kernel<2, 2, 2>, swa::simt_tile_kernel<2, 2, 4>}, {swa::simt_tile_kernel<2, 4, 2>, swa::simt_tile_kernel<2, 4, 4>}}};
   const Kernel kern = table[kind][g->d_qk > 64 ? 1 : 0][g->d_v > 64 ? 1 : 0];
   const int smem = (int)bytes(a.rb);
-  if (cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem); e != cudaSuccess) {
-    *err = fail(E_LAUNCH, "cudaFuncSetAttribute(%d bytes): %s", smem, cudaGetErrorString(e));
+  cudaError_t e = swa::allow_smem((const void*)kern);
+  if (e == cudaSuccess) e = swa::launch_pdl(kern, grid, 256, smem, st, a);
+  if (e != cudaSuccess) {
+    *err = fail(E_LAUNCH, "simt tile (%d bytes): %s", smem, cudaGetErrorString(e));
     return true;
   }
-  kern<<<grid, 256, smem, st>>>(a);
   *err = launch_ok("simt tile");
   return true;
 }
@@ -219,13 +220,14 @@ int swa_bwd_delta(const swa_geom_t* g, const swa_tensor_t* o, const swa_tensor_t
       return t->stride[1] == dv && t->stride[2] == (int64_t)g->H * dv && (g->B == 1 || t->stride[0] == (int64_t)g->H * N * dv);
     };
     if (esz == 2 && group == units && flat(o) && flat(d_o)) {
-      SWA_DISPATCH_DTYPE(g->dtype, swa::delta_flat_kernel<T><<<blocks, 256, 0, st>>>((const T*)o->ptr, (const T*)d_o->ptr, delta, dv, rows));
+      SWA_DISPATCH_DTYPE(g->dtype, swa::launch_stream(swa::delta_flat_kernel<T, false>, blocks, 256, st, (const T*)o->ptr,
+                                                   (const T*)d_o->ptr, delta, dv, rows, 1, (int64_t)1));
     } else if (esz == 2 && group == units && token_major(o) && token_major(d_o)) {
-      SWA_DISPATCH_DTYPE(g->dtype, swa::delta_flat_kernel<T, true><<<blocks, 256, 0, st>>>((const T*)o->ptr, (const T*)d_o->ptr, delta, dv,
-                                                                                        rows, g->H, N));
+      SWA_DISPATCH_DTYPE(g->dtype, swa::launch_stream(swa::delta_flat_kernel<T, true>, blocks, 256, st, (const T*)o->ptr,
+                                                   (const T*)d_o->ptr, delta, dv, rows, g->H, N));
     } else {
-      SWA_DISPATCH_DTYPE(g->dtype, swa::delta_vec_kernel<T><<<blocks, 256, 0, st>>>(swa::make_view(o), swa::make_view(d_o), delta, g->H, N,
-                                                                                 units, group, rows));
+      SWA_DISPATCH_DTYPE(g->dtype, swa::launch_stream(swa::delta_vec_kernel<T>, blocks, 256, st, swa::make_view(o), swa::make_view(d_o),
+                                                   delta, g->H, N, units, group, rows));
     }
     return launch_ok("delta");
   }
@@ -309,34 +311,33 @@ int swa_bwd_dkdv(const swa_geom_t* g, const swa_rope_t* rope, const swa_tensor_t
 // ---- rotation handed on between the kernels ---------------------------------------------------
 namespace {
 
-// y = rope(x) (inverse: the transposed rotation) for a strided [B, H, N, C] tensor; x == y rotates in place.
-int launch_rope4(const swa_geom_t* g, const swa_rope_t* rope, const swa_tensor_t* x, const swa_tensor_t* y, bool inverse,
-                 cudaStream_t st) {
+// y = rope(x) (inverse: the transposed rotation) for strided [B, H, N, C] tensors, and y2 = rope(x2) beside it where given;
+// x == y rotates in place.
+int launch_rope4(const swa_geom_t* g, const swa_rope_t* rope, const swa_tensor_t* x, const swa_tensor_t* y, const swa_tensor_t* x2,
+                 const swa_tensor_t* y2, bool inverse, cudaStream_t st) {
   const swa::RopeDev rp = swa::make_rope(rope);
   const int64_t N = (int64_t)g->t_height * g->t_width * g->b_size;
   const int64_t rows = N * g->B * g->H;
-  const int C = g->d_qk;
+  const int C = g->d_qk, E = g->dtype == SWA_F32 ? 4 : 8;        // elements of a 16-byte unit
   const float sign = inverse ? -1.f : 1.f;
-  auto rows16 = [](const swa_tensor_t* t) {
-    return t->stride[3] == 1 && ((uintptr_t)t->ptr % 16) == 0 && t->stride[0] % 8 == 0 && t->stride[1] % 8 == 0 &&
-           t->stride[2] % 8 == 0;
+  auto rows16 = [E](const swa_tensor_t* t) {
+    return t->stride[3] == 1 && ((uintptr_t)t->ptr % 16) == 0 && t->stride[0] % E == 0 && t->stride[1] % E == 0 && t->stride[2] % E == 0;
   };
-  const bool vec = g->dtype != SWA_F32 && x->ptr != y->ptr && rp.R % 8 == 0 && C % 8 == 0 && rows16(x) && rows16(y) &&
+  const bool vec = x2 && x->ptr != y->ptr && rp.R % E == 0 && C % E == 0 && rows16(x) && rows16(y) && rows16(x2) && rows16(y2) &&
                    ((uintptr_t)rp.row_cs % 16) == 0 && ((uintptr_t)rp.col_cs % 16) == 0;
   if (vec) {
-    const int64_t slots = rp.R / 4 + ((C / 8 - rp.R / 2) + 1) / 2;   // per token row (see the kernel)
+    const int64_t units = C / E, rot = 2 * rp.R / E, slots = rot + (units - 2 * rot + 1) / 2;   // per token row (see the kernel)
     dim3 grid((unsigned)((N * slots + 255) / 256), (unsigned)(g->B * g->H));
-    if (g->dtype == SWA_F16)
-      swa::rope2d_copy4_kernel<__half><<<grid, 256, 0, st>>>(swa::make_view(x), swa::make_view(y), g->H, (int)N, C, rp, sign);
-    else
-      swa::rope2d_copy4_kernel<__nv_bfloat16><<<grid, 256, 0, st>>>(swa::make_view(x), swa::make_view(y), g->H, (int)N, C, rp, sign);
-  } else {
-    const int64_t threads = rows * 2 * rp.R;
-    const unsigned blocks = (unsigned)((threads + 255) / 256);
-    SWA_DISPATCH_DTYPE(g->dtype, swa::rope2d_generic4_kernel<T><<<blocks, 256, 0, st>>>(swa::make_view(x), swa::make_view(y),
-                                                                                      rows, g->H, N, C, rp, sign));
+    SWA_DISPATCH_DTYPE(g->dtype, swa::launch_stream(swa::rope2d_copy4_kernel<T>, grid, 256, st, swa::make_view(x), swa::make_view(y),
+                                                 swa::make_view(x2), swa::make_view(y2), g->H, (int)N, C, rp, sign));
+    return launch_ok("rope2d (4-D)");
   }
-  return launch_ok("rope2d (4-D)");
+  const int64_t threads = rows * 2 * rp.R;
+  const unsigned blocks = (unsigned)((threads + 255) / 256);
+  SWA_DISPATCH_DTYPE(g->dtype, swa::rope2d_generic4_kernel<T><<<blocks, 256, 0, st>>>(swa::make_view(x), swa::make_view(y), rows, g->H, N,
+                                                                                    C, rp, sign));
+  if (int e = launch_ok("rope2d (4-D)")) return e;
+  return x2 ? launch_rope4(g, rope, x2, y2, nullptr, nullptr, inverse, st) : 0;
 }
 
 int require_rope(const swa_rope_t* rope, const char* who) {
@@ -363,8 +364,7 @@ static int fwd_rot_call(bool any8, const swa_geom_t* g, const swa_rope_t* rope, 
   if (impl < 0) return impl;
   cudaStream_t st = (cudaStream_t)stream;
   // every q and k row is rotated exactly once, by a streaming pass; the attention kernels read the rotated rows
-  if (int e = launch_rope4(g, rope, q, q_rot, false, st)) return e;
-  if (int e = launch_rope4(g, rope, k, k_rot, false, st)) return e;
+  if (int e = launch_rope4(g, rope, q, q_rot, k, k_rot, false, st)) return e;
   if (impl == SWA_IMPL_TC) {
     int e = swa::tc::launch_fwd2(g, q_rot, k_rot, v, o, lse, status, st);
     if (e) return fail(E_LAUNCH, "tcgen05 forward: %s", swa::tc::last_error());
@@ -416,7 +416,7 @@ static int dq_rot_call(bool any8, const swa_geom_t* g, const swa_rope_t* rope, c
                                    gg, none, swa::make_view(q_rot), swa::make_view(k_rot), swa::make_view(v),
                                    swa::make_view(d_o), lse, delta, swa::make_view(dq)));
   if (int e = launch_ok("simt dq")) return e;
-  return launch_rope4(g, rope, dq, dq, true, st);
+  return launch_rope4(g, rope, dq, dq, nullptr, nullptr, true, st);
 }
 int swa_bwd_dq_rot(const swa_geom_t* g, const swa_rope_t* rope, const swa_tensor_t* q_rot, const swa_tensor_t* k_rot,
                    const swa_tensor_t* v, const swa_tensor_t* d_o, const float* lse, const float* delta,
@@ -454,7 +454,7 @@ static int dkdv_rot_call(bool any8, const swa_geom_t* g, const swa_rope_t* rope,
                                    gg, none, swa::make_view(q_rot), swa::make_view(k_rot), swa::make_view(v),
                                    swa::make_view(d_o), lse, delta, swa::make_view(dk), swa::make_view(dv)));
   if (int e = launch_ok("simt dkdv")) return e;
-  return launch_rope4(g, rope, dk, dk, true, st);
+  return launch_rope4(g, rope, dk, dk, nullptr, nullptr, true, st);
 }
 int swa_bwd_dkdv_rot(const swa_geom_t* g, const swa_rope_t* rope, const swa_tensor_t* q_rot, const swa_tensor_t* k_rot,
                      const swa_tensor_t* v, const swa_tensor_t* d_o, const float* lse, const float* delta,

@@ -115,6 +115,8 @@ __global__ void __launch_bounds__(256) simt_tile_kernel(const __grid_constant__ 
   const int ty = blockIdx.x / t.n_tiles_x, r0 = ty * kTileRows, c0 = (blockIdx.x - ty * t.n_tiles_x) * kTileCols;
   auto slice = [&](const View4& v) { return (float*)v.ptr + bi * v.s0 + hi * v.s1; };
 
+  pdl_enter();
+  pdl_wait();
   // resident rows (zeros beyond the grid)
   auto load_resident = [&](float* dst, const View4& v, int d) {
     const float* src = slice(v);

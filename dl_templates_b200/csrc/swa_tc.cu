@@ -3,6 +3,7 @@
 #include <cudaTypedefs.h>
 
 #include <algorithm>
+#include <atomic>
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
@@ -85,9 +86,8 @@ struct Knobs {
   int nmax, nxb, kr, kw, stages, nsb, th_all, th[3], trace_it;
   bool no_tabs, disable, verbose, trace;
 };
-std::mutex g_plan_mu;                 // guards the knobs and the plan cache
-bool g_knobs_read = false;
-Knobs g_knobs;
+std::mutex g_plan_mu;                 // guards the plan cache and the reading of the knobs
+std::atomic<const Knobs*> g_knobs{nullptr};      // (a snapshot is never freed: refresh_env is a diagnostic)
 
 int env_raw(const char* name, int dflt) {
   const char* v = getenv(name);
@@ -110,13 +110,14 @@ void read_knobs_locked() {
   k.disable = getenv("SWA_TC_DISABLE") != nullptr;
   k.verbose = getenv("SWA_TC_VERBOSE") != nullptr;
   k.trace = getenv("SWA_TC_TRACE") != nullptr;
-  g_knobs = k;
-  g_knobs_read = true;
+  g_knobs.store(new Knobs(k), std::memory_order_release);
 }
-Knobs knobs() {
+const Knobs& knobs() {
+  const Knobs* k = g_knobs.load(std::memory_order_acquire);
+  if (k) return *k;
   std::lock_guard<std::mutex> lock(g_plan_mu);
-  if (!g_knobs_read) read_knobs_locked();
-  return g_knobs;
+  if (!g_knobs.load()) read_knobs_locked();
+  return *g_knobs.load();
 }
 
 // Widest halo, in token columns, over all resident-tile columns.
@@ -481,12 +482,23 @@ bool mask_constants(float sm_scale, float* a, float* b) {
 
 // Plan of the kernels that rotate no streamed row (rotation handed on between the kernels, or no RoPE).
 bool make_plan_prerot(const swa_geom_t* g, int which, Plan* out) {
+  // a step asks for the same three plans a dozen times: the last one of each kind, per thread, needs no lock
+  struct Last { PlanKey key; bool ok; Plan pl; const Knobs* epoch; };
+  static thread_local Last last[3] = {};
+  const Knobs* epoch = &knobs();
   const PlanKey key = plan_key(g, nullptr, which, true);
+  Last& l = last[which];
+  if (l.epoch == epoch && l.key == key) {
+    if (l.ok) *out = l.pl;
+    return l.ok;
+  }
   bool ok = false;
-  if (cache_lookup(key, &ok, out)) return ok;
   Plan pl{};
-  ok = make_strip_plan(g, which, &pl);
-  cache_store(key, ok, pl);
+  if (!cache_lookup(key, &ok, &pl)) {
+    ok = make_strip_plan(g, which, &pl);
+    cache_store(key, ok, pl);
+  }
+  l = Last{key, ok, pl, epoch};
   if (ok) *out = pl;
   return ok;
 }
@@ -637,7 +649,7 @@ int launch_fwd(const swa_geom_t* g, const swa_rope_t* rope, const swa_tensor_t* 
     snprintf(g_tc_err, sizeof(g_tc_err), "n_rdim %d has no tensor-core kernel", rope ? rope->n_rdim : 0);
     return -1;
   }
-  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)pl.smem_bytes);
+  cudaError_t e = allow_smem((const void*)kern);
   if (e != cudaSuccess) {
     snprintf(g_tc_err, sizeof(g_tc_err), "cudaFuncSetAttribute(%u bytes): %s", pl.smem_bytes, cudaGetErrorString(e));
     return -1;
@@ -669,7 +681,7 @@ int launch_fwd2(const swa_geom_t* g, const swa_tensor_t* q, const swa_tensor_t* 
       {{fwd2_kernel<false, false, false>, fwd2_kernel<false, false, true>}, {fwd2_kernel<false, true, false>, fwd2_kernel<false, true, true>}},
       {{fwd2_kernel<true, false, false>, fwd2_kernel<true, false, true>}, {fwd2_kernel<true, true, false>, fwd2_kernel<true, true, true>}}};
   const FwdKernel kern = table[g->dtype == SWA_BF16 ? 1 : 0][one ? 1 : 0][pl.p_off ? 1 : 0];
-  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)pl.smem_bytes);
+  cudaError_t e = allow_smem((const void*)kern);
   if (e != cudaSuccess) {
     snprintf(g_tc_err, sizeof(g_tc_err), "cudaFuncSetAttribute(%u bytes): %s", pl.smem_bytes, cudaGetErrorString(e));
     return -1;
@@ -677,8 +689,9 @@ int launch_fwd2(const swa_geom_t* g, const swa_tensor_t* q, const swa_tensor_t* 
   if (knobs().verbose)
     fprintf(stderr, "[swa2d] fwd2 plan: tile %dx%d, block %dx%d (N=%d), stages %d, score buffers %d, %d quarters per chunk, smem %u, %d items on %u CTAs\n",
             pl.TH, pl.TW, pl.KR, pl.KW, pl.N, pl.stages, pl.nsb, pl.nq, pl.smem_bytes, p.n_items, grid.x);
-  kern<<<grid, block, pl.smem_bytes, st>>>(tq, tk, tv, to, p, make_view(o), lse);
-  return 0;
+  e = launch_pdl(kern, grid, block.x, pl.smem_bytes, st, tq, tk, tv, to, p, make_view(o), lse);
+  if (e != cudaSuccess) snprintf(g_tc_err, sizeof(g_tc_err), "launch: %s", cudaGetErrorString(e));
+  return e == cudaSuccess ? 0 : -1;
 }
 
 namespace {
@@ -736,7 +749,7 @@ int launch_bwd(const swa_geom_t* g, const swa_rope_t* rope, bool prerotated, con
     mov = moqk;
     if (DKDV && !make_map(&mov, out_v, g, g->d_v, pl.TW, pl.R4)) return -1;
   }
-  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)pl.smem_bytes);
+  cudaError_t e = allow_smem((const void*)kern);
   if (e != cudaSuccess) {
     snprintf(g_tc_err, sizeof(g_tc_err), "cudaFuncSetAttribute(%u bytes): %s", pl.smem_bytes, cudaGetErrorString(e));
     return -1;
@@ -744,11 +757,13 @@ int launch_bwd(const swa_geom_t* g, const swa_rope_t* rope, bool prerotated, con
   if (knobs().verbose)
     fprintf(stderr, "[swa2d] %s plan: tile %dx%d, block %dx%d (N=%d), stages %d, nsb %d, nxb %d, %d quarters per chunk, tables %u, smem %u, %d items on %u CTAs\n",
             DKDV ? "dkdv" : "dq", pl.TH, pl.TW, pl.KR, pl.KW, pl.N, pl.stages, pl.nsb, pl.nxb, pl.nq, pl.tab_bytes, pl.smem_bytes, p.n_items, grid.x);
-  if (v2)
-    kern2<<<grid, block, pl.smem_bytes, st>>>(mxqk, mxv, myqk, myv, moqk, mov, p, lse, delta);
-  else
-    kern1<<<grid, block, pl.smem_bytes, st>>>(mxqk, mxv, myqk, myv, p, lse, delta, make_view(out_qk),
-                                              out_v ? make_view(out_v) : View4{nullptr, 0, 0, 0, 0});
+  if (v2) {
+    e = launch_pdl(kern2, grid, block.x, pl.smem_bytes, st, mxqk, mxv, myqk, myv, moqk, mov, p, lse, delta);
+    if (e != cudaSuccess) snprintf(g_tc_err, sizeof(g_tc_err), "launch: %s", cudaGetErrorString(e));
+    return e == cudaSuccess ? 0 : -1;
+  }
+  kern1<<<grid, block, pl.smem_bytes, st>>>(mxqk, mxv, myqk, myv, p, lse, delta, make_view(out_qk),
+                                            out_v ? make_view(out_v) : View4{nullptr, 0, 0, 0, 0});
   return 0;
 }
 

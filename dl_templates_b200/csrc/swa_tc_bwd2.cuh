@@ -95,6 +95,8 @@ bwd2_kernel(const __grid_constant__ CUtensorMap tm_xqk, const __grid_constant__ 
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
+  pdl_enter();                                                   // not before the allocation: a successor on this SM must not be first
+  pdl_wait();                                                    // from here on: global memory
   const uint32_t tmem = sh->tmem_base;
 
   bool ok = true;   // warp-uniform: a failed wait does not leave the loops, but nothing is waited for or touched any more
