@@ -87,7 +87,7 @@ int resolve_impl(const swa_geom_t* g, const swa_rope_t* rope, const swa_tensor_t
 
 // fp32 problems the tiled kernels take (swa_simt_tile.cuh): true when the launch was made (*err: its return code).  `rope`
 // only rotates dQ / dK back; streamed rows are never rotated here.  The band of halo rows that is staged at a time is
-// what fits 100 KB beside the resident rows, so that two blocks share an SM; a single row that does not fit takes up to the
+// what fits 74 KB beside the resident rows, so that three blocks share an SM; a single row that does not fit takes up to the
 // 227 KB there are, and a wider one is left to the one-warp-per-token kernels.
 bool launch_simt_tile(int kind, const swa_geom_t* g, const swa_rope_t* rope, const swa_tensor_t* x1, const swa_tensor_t* x2,
                       const swa_tensor_t* y1, const swa_tensor_t* y2, const swa_tensor_t* o1, const swa_tensor_t* o2, float* lse_out,
@@ -111,7 +111,7 @@ bool launch_simt_tile(int kind, const swa_geom_t* g, const swa_rope_t* rope, con
   auto bytes = [&](int rb) { return 4 * swa::tile_smem_floats(kind, g->d_qk, g->d_v, rb * cols); };
   int rb = 1;
   if (bytes(1) > 227 * 1024 || cols > 4000) return false;
-  while (rb < rows && bytes(rb + 1) <= 100 * 1024 && (rb + 1) * cols <= 4000) ++rb;
+  while (rb < rows && bytes(rb + 1) <= 74 * 1024 && (rb + 1) * cols <= 4000) ++rb;
   const int bands = (rows + rb - 1) / rb;
   a.rb = (rows + bands - 1) / bands;
   a.max_keys = a.rb * cols;
@@ -126,7 +126,7 @@ bool launch_simt_tile(int kind, const swa_geom_t* g, const swa_rope_t* rope, con
   const Kernel kern = table[kind][g->d_qk > 64 ? 1 : 0][g->d_v > 64 ? 1 : 0];
   const int smem = (int)bytes(a.rb);
   cudaError_t e = swa::allow_smem((const void*)kern);
-  if (e == cudaSuccess) e = swa::launch_pdl(kern, grid, 256, smem, st, a);
+  if (e == cudaSuccess) e = swa::launch_pdl(kern, grid, swa::kTileWarps * 32, smem, st, a);
   if (e != cudaSuccess) {
     *err = fail(E_LAUNCH, "simt tile (%d bytes): %s", smem, cudaGetErrorString(e));
     return true;
