@@ -85,10 +85,41 @@ int resolve_impl(const swa_geom_t* g, const swa_rope_t* rope, const swa_tensor_t
   return SWA_IMPL_SIMT;
 }
 
+// Halo rows staged at a time.  Small bands let more blocks share an SM, large ones cost fewer barriers and leave fewer warps
+// waiting for the one whose window has most of the band: counted in steps of 32 streamed tokens of the slowest warp, one more
+// for a band's load, times the waves of blocks, times what a step costs beside its neighbours (3 blocks an SM against 2: 1.34;
+// a lone block, whose loads nothing hides: 1.1; measured at 40 x 40, window 9, d = 64, 32 slices).  48 x 48, window 5, d = 128: three blocks 229 us a training step, two
+// 158; 40 x 40, window 9, d = 64, 8 slices: 132 against 174.
+template <typename Bytes>
+int tile_band_rows(const swa_geom_t* g, int rows, int cols, int64_t blocks, Bytes&& bytes) {
+  static const struct { int per_sm, kb; double step; } kinds[3] = {{3, 74, 1.34}, {2, 112, 1.}, {1, 227, 1.1}};
+  const int wcols = std::min(g->t_width * g->b_size, swa::tile_halo_cols(4, g->b_size, g->col_size)), span = 2 * g->row_size + 2;
+  double best = -1.;
+  int best_rb = 1;
+  for (const auto& c : kinds) {
+    int most = 0;
+    while (most < rows && bytes(most + 1) <= (size_t)c.kb * 1024 && (most + 1) * cols <= 4000) ++most;
+    if (!most) continue;
+    const int bands = (rows + most - 1) / most, rb = (rows + bands - 1) / bands;
+    int steps = 0;
+    for (int b0 = 0; b0 < rows; b0 += rb) {
+      const int b1 = std::min(b0 + rb, rows);              // rows 0 .. span - 1 are the upper warps' window, 2 .. span + 1 the lower ones'
+      const int upper = std::min(b1, span) - b0, lower = b1 - std::max(b0, 2);
+      steps += (std::max(upper, lower) * wcols + 31) / 32 + 1;
+    }
+    const int64_t slots = (int64_t)c.per_sm * 148;
+    const double cost = (double)((blocks + slots - 1) / slots) * steps * c.step;
+    if (best < 0. || cost < best) {
+      best = cost;
+      best_rb = rb;
+    }
+  }
+  return best_rb;
+}
+
 // fp32 problems the tiled kernels take (swa_simt_tile.cuh): true when the launch was made (*err: its return code).  `rope`
-// only rotates dQ / dK back; streamed rows are never rotated here.  The band of halo rows that is staged at a time is
-// what fits 74 KB beside the resident rows, so that three blocks share an SM; a single row that does not fit takes up to the
-// 227 KB there are, and a wider one is left to the one-warp-per-token kernels.
+// only rotates dQ / dK back; streamed rows are never rotated here.  A halo row that
+// does not fit shared memory is left to the one-warp-per-token kernels.
 bool launch_simt_tile(int kind, const swa_geom_t* g, const swa_rope_t* rope, const swa_tensor_t* x1, const swa_tensor_t* x2,
                       const swa_tensor_t* y1, const swa_tensor_t* y2, const swa_tensor_t* o1, const swa_tensor_t* o2, float* lse_out,
                       const float* lse, const float* delta, cudaStream_t st, int* err) {
@@ -106,27 +137,26 @@ bool launch_simt_tile(int kind, const swa_geom_t* g, const swa_rope_t* rope, con
   a.lse_out = lse_out;
   a.lse = lse;
   a.delta = delta;
-  const int cols = std::min(Wtok, swa::tile_halo_cols(g->b_size, g->col_size));
+  const int cols = std::min(Wtok, swa::tile_halo_cols(swa::kTileCols, g->b_size, g->col_size));
   const int rows = std::min(g->t_height, swa::kTileRows + 2 * g->row_size);
   auto bytes = [&](int rb) { return 4 * swa::tile_smem_floats(kind, g->d_qk, g->d_v, rb * cols); };
-  int rb = 1;
   if (bytes(1) > 227 * 1024 || cols > 4000) return false;
-  while (rb < rows && bytes(rb + 1) <= 74 * 1024 && (rb + 1) * cols <= 4000) ++rb;
-  const int bands = (rows + rb - 1) / rb;
-  a.rb = (rows + bands - 1) / bands;
-  a.max_keys = a.rb * cols;
   a.n_tiles_x = (Wtok + swa::kTileCols - 1) / swa::kTileCols;
   const int64_t tiles = (int64_t)a.n_tiles_x * ((g->t_height + swa::kTileRows - 1) / swa::kTileRows);
+  a.rb = tile_band_rows(g, rows, cols, tiles * g->B * g->H, bytes);
+  a.max_keys = a.rb * cols;
   const dim3 grid((unsigned)tiles, (unsigned)(g->B * g->H));
   using Kernel = void (*)(const swa::TileArgs);
-  static const Kernel table[3][2][2] = {   // [kind][d_qk > 64][d_v > 64]
-      {{swa::simt_tile_kernel<0, 2, 2>, swa::simt_tile_kernel<0, 2, 4>}, {swa::simt_tile_kernel<0, 2, 2>, swa::simt_tile_kernel<0, 2, 4>}},
-      {{swa::simt_tile_kernel<1, 2, 2>, swa::simt_tile_kernel<1, 2, 2>}, {swa::simt_tile_kernel<1, 4, 2>, swa::simt_tile_kernel<1, 4, 2>}},
-      {{swa::simt_tile_kernel<2, 2, 2>, swa::simt_tile_kernel<2, 2, 4>}, {swa::simt_tile_kernel<2, 4, 2>, swa::simt_tile_kernel<2, 4, 4>}}};
-  const Kernel kern = table[kind][g->d_qk > 64 ? 1 : 0][g->d_v > 64 ? 1 : 0];
+  const int g1 = (g->d_qk + 31) / 32 - 1, g2 = (g->d_v + 31) / 32 - 1;
+#define SWA_TILE_ROW(i) {swa::simt_tile_kernel<2, i, 1>, swa::simt_tile_kernel<2, i, 2>, swa::simt_tile_kernel<2, i, 3>, swa::simt_tile_kernel<2, i, 4>}
+  static const Kernel fwd[4] = {swa::simt_tile_kernel<0, 1, 1>, swa::simt_tile_kernel<0, 1, 2>, swa::simt_tile_kernel<0, 1, 3>, swa::simt_tile_kernel<0, 1, 4>};
+  static const Kernel dq[4] = {swa::simt_tile_kernel<1, 1, 1>, swa::simt_tile_kernel<1, 2, 1>, swa::simt_tile_kernel<1, 3, 1>, swa::simt_tile_kernel<1, 4, 1>};
+  static const Kernel dkdv[4][4] = {SWA_TILE_ROW(1), SWA_TILE_ROW(2), SWA_TILE_ROW(3), SWA_TILE_ROW(4)};
+#undef SWA_TILE_ROW
+  const Kernel kern = kind == 0 ? fwd[g2] : kind == 1 ? dq[g1] : dkdv[g1][g2];
   const int smem = (int)bytes(a.rb);
   cudaError_t e = swa::allow_smem((const void*)kern);
-  if (e == cudaSuccess) e = swa::launch_pdl(kern, grid, swa::kTileWarps * 32, smem, st, a);
+  if (e == cudaSuccess) e = swa::launch_pdl(kern, grid, swa::kTileThreads, smem, st, a);
   if (e != cudaSuccess) {
     *err = fail(E_LAUNCH, "simt tile (%d bytes): %s", smem, cudaGetErrorString(e));
     return true;

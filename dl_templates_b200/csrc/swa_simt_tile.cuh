@@ -1,15 +1,17 @@
 // fp32 attention on CUDA cores, tiled: forward, dQ and dK/dV for fp32 tensors with unit last stride, 16-byte aligned
 // rows and head dims that are multiples of 4 up to 128 (anything else runs on swa_simt.cuh's one-warp-per-token kernels).
 //
-// A block of eight warps owns 4 grid rows x 8 token columns, a warp 4 columns of a row; the rows of the halo are staged in
-// shared memory band by band (asynchronous copies) and shared by the warps.  A warp takes the streamed tokens of its own
-// window 32 at a time:
-//   scores       lane = streamed token, 4 resident rows read as broadcasts: one 16-byte load of the token's row and
-//                four broadcasts per 8 packed multiply-adds
-//   accumulation lane = 2 or 4 head dims, the 32 x 4 weights passed through shared memory: one broadcast and one
-//                8- or 16-byte load per 4 or 8 packed multiply-adds
-// Multiply-adds and shared-memory wavefronts (about as many cycles each) bound it once there are warps enough: three
-// blocks share an SM.  Only the columns of the warp's halo are scored in vain, (4 + 2 wc) / (2 wc + 1).
+// A block of four warps owns 4 grid rows x 8 token columns, a warp 2 x 4 of them; the rows of the halo are staged in shared
+// memory band by band (asynchronous copies) and shared by the warps.  A warp takes the streamed tokens of its own window 32
+// at a time; lane (a, b), a < 4, b < 8, owns two resident rows, 2a and 2a + 1, throughout:
+//   scores       of its two rows with the streamed tokens b, b + 8, ...: six 16-byte loads for 16 packed multiply-adds
+//   accumulation of its two rows' head dims 4b .. 4b + 3 (and 32 further on): a 16-byte load per 4 head dims and token for
+//                four packed multiply-adds, the 8 x 32 weights passed through shared memory, four tokens a load
+// Latency bounds it -- 8 to 12 warps an SM, half of the issue slots and two thirds of the shared-memory wavefronts used --
+// and what the bands cost: their barriers, and warps that wait for the one whose window has most of the band
+// (tile_band_rows in swa_abi.cu).  In vain are scored the columns of the warp's halo beyond a row's own window,
+// (4 + 2 wc) / (2 wc + 1), and one row in 2 wr + 2.  Training steps: 64 x 64, window 21, d = 64, 4 slices 641 -> 500 us, 32 x 32,
+// window 31, d = 128 1091 -> 523 us against one streamed token per lane and four resident rows per warp.
 #pragma once
 
 #include "swa_simt.cuh"
@@ -17,8 +19,9 @@
 
 namespace swa {
 
-constexpr int kTileRows = 4, kTileCols = 8, kTileQ = 4, kTileWarps = 8;
-constexpr int kTileTokens = kTileRows * kTileCols;
+constexpr int kTileRows = 4, kTileCols = 8, kTileWarps = 4, kTileThreads = kTileWarps * 32;
+constexpr int kTileQ = 8;                          // resident rows of a warp: 2 grid rows x 4 columns
+constexpr int kTileW = 36;                         // floats from one row of weights to the next
 
 // Tensors of one launch; `kind` 0: forward (x1 = q; y1 = k, y2 = v; o1 = o), 1: dQ (x1 = q, x2 = dO; y1 = k, y2 = v; o1 = dq),
 // 2: dK/dV (x1 = k, x2 = v; y1 = q, y2 = dO; o1 = dk, o2 = dv).
@@ -31,80 +34,97 @@ struct TileArgs {
   int rb, n_tiles_x, max_keys;   // halo rows per band, tiles per row of tiles, streamed tokens of the largest band
 };
 
-__host__ __device__ __forceinline__ int tile_halo_cols(int b, int wc) { return ((kTileCols + b - 2) / b + 1 + 2 * wc) * b; }
+__host__ __device__ __forceinline__ int tile_halo_cols(int cols, int b, int wc) { return ((cols + b - 2) / b + 1 + 2 * wc) * b; }
 
-// Floats of shared memory of a launch with `keys` staged tokens.
+// Floats of shared memory of a launch with `keys` staged tokens.  All rows lie 4 floats further apart than they are long:
+// rows at distance 1 (streamed) or 2 (resident) start in banks of their own.
 __host__ __device__ __forceinline__ size_t tile_smem_floats(int kind, int d1, int d2, int keys) {
-  const size_t resident = kTileTokens * (size_t)(kind == 0 ? d1 : d1 + d2);
-  const size_t weights = (size_t)kTileWarps * 32 * (kTileQ * (kind == 2 ? 2 : 1) + 1);
+  const size_t resident = kTileWarps * kTileQ * (size_t)(kind == 0 ? d1 + 4 : d1 + 4 + d2 + 4);
+  const size_t weights = (size_t)kTileWarps * (kTileQ * kTileW * (kind == 2 ? 2 : 1) + 32);
   return resident + weights + (size_t)keys * (d1 + 4 + d2 + 4) + (kind == 2 ? 2 * (size_t)keys : 0);
 }
 
-// out[j] = x_j . y for the warp's resident rows x (stride d) and this lane's streamed row y.
-__device__ __forceinline__ void tile_dot(const float* x, const float* y, int d, float* out) {
+// out[e][i] = x_e . y_i for two resident rows (stride d + 4) and four streamed rows that lie off[i] floats into y.
+__device__ __forceinline__ void tile_dot(const float* x, const float* y, const int (&off)[4], int d, float (&out)[2][4]) {
   using namespace ptx;
-  uint64_t acc[kTileQ];
+  uint64_t acc[2][4];
 #pragma unroll
-  for (int j = 0; j < kTileQ; ++j) acc[j] = 0ull;
+  for (int i = 0; i < 4; ++i) acc[0][i] = acc[1][i] = 0ull;
+  const float *x1 = x + d + 4, *y0 = y + off[0], *y1 = y + off[1], *y2 = y + off[2], *y3 = y + off[3];
 #pragma unroll 4
   for (int c = 0; c < d; c += 4) {
-    const ulonglong2 b = *reinterpret_cast<const ulonglong2*>(y + c);
+    const ulonglong2 a0 = *reinterpret_cast<const ulonglong2*>(x + c), a1 = *reinterpret_cast<const ulonglong2*>(x1 + c);
+    const ulonglong2 b[4] = {*reinterpret_cast<const ulonglong2*>(y0 + c), *reinterpret_cast<const ulonglong2*>(y1 + c),
+                             *reinterpret_cast<const ulonglong2*>(y2 + c), *reinterpret_cast<const ulonglong2*>(y3 + c)};
 #pragma unroll
-    for (int j = 0; j < kTileQ; ++j) {
-      const ulonglong2 a = *reinterpret_cast<const ulonglong2*>(x + j * d + c);
-      acc[j] = f2_fma(a.x, b.x, acc[j]);
-      acc[j] = f2_fma(a.y, b.y, acc[j]);
+    for (int i = 0; i < 4; ++i) {
+      acc[0][i] = f2_fma(a0.x, b[i].x, acc[0][i]);
+      acc[1][i] = f2_fma(a1.x, b[i].x, acc[1][i]);
+    }
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      acc[0][i] = f2_fma(a0.y, b[i].y, acc[0][i]);
+      acc[1][i] = f2_fma(a1.y, b[i].y, acc[1][i]);
     }
   }
 #pragma unroll
-  for (int j = 0; j < kTileQ; ++j) {
-    const float2 v = f2_unpack(acc[j]);
-    out[j] = v.x + v.y;
-  }
+  for (int e = 0; e < 2; ++e)
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const float2 v = f2_unpack(acc[e][i]);
+      out[e][i] = v.x + v.y;
+    }
 }
 
-// acc[dd][jp] += w[k][2 jp, 2 jp + 1] * y[at[k]][dd] over n staged tokens (at: their positions; rows `stride` floats apart).
-template <int P>
-__device__ __forceinline__ void tile_accumulate(uint64_t (&acc)[P][2], const float* w, const int* at, const float* y, int stride, int n) {
+// Accumulators of a lane: [its resident row][32-dim group][pair of head dims].
+template <int G>
+using TileAcc = uint64_t[2][G][2];
+
+// acc[e] += w[e][k] * y[at[k]] over n staged tokens (rows `stride` floats apart); goff: the lane's head dims in
+// each group.
+template <int G>
+__device__ __forceinline__ void tile_accumulate(TileAcc<G>& acc, const float* w, const int* at, const float* y, int stride,
+                                                const int (&goff)[G], int n) {
   using namespace ptx;
-  auto one = [&](int k, int pos) {
-    const ulonglong2 a = *reinterpret_cast<const ulonglong2*>(w + kTileQ * k);
-    const float* row = y + pos * stride;
-    float v[P];
-    if constexpr (P == 2) {
-      const float2 t = *reinterpret_cast<const float2*>(row);
-      v[0] = t.x; v[1] = t.y;
-    } else {
-      const float4 t = *reinterpret_cast<const float4*>(row);
-      v[0] = t.x; v[1] = t.y; v[2] = t.z; v[3] = t.w;
-    }
-#pragma unroll
-    for (int dd = 0; dd < P; ++dd) {
-      const uint64_t vv = f2_pack(v[dd], v[dd]);
-      acc[dd][0] = f2_fma(a.x, vv, acc[dd][0]);
-      acc[dd][1] = f2_fma(a.y, vv, acc[dd][1]);
-    }
-  };
 #pragma unroll 2
   for (int k = 0; k < n; k += 4) {                               // (tokens beyond the last: weight 0, a valid position)
-    const int4 pos = *reinterpret_cast<const int4*>(at + k);
-    one(k, pos.x);
-    one(k + 1, pos.y);
-    one(k + 2, pos.z);
-    one(k + 3, pos.w);
+    const int4 at4 = *reinterpret_cast<const int4*>(at + k);
+    const float4 u = *reinterpret_cast<const float4*>(w + k), v = *reinterpret_cast<const float4*>(w + kTileW + k);
+    const int pos[4] = {at4.x, at4.y, at4.z, at4.w};
+    const float wu[4] = {u.x, u.y, u.z, u.w}, wv[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const float* row = y + pos[i] * stride;
+      const uint64_t w0 = f2_pack(wu[i], wu[i]), w1 = f2_pack(wv[i], wv[i]);
+#pragma unroll
+      for (int h = 0; h < G; ++h) {
+        const ulonglong2 r = *reinterpret_cast<const ulonglong2*>(row + goff[h]);
+        acc[0][h][0] = f2_fma(w0, r.x, acc[0][h][0]);
+        acc[0][h][1] = f2_fma(w0, r.y, acc[0][h][1]);
+        acc[1][h][0] = f2_fma(w1, r.x, acc[1][h][0]);
+        acc[1][h][1] = f2_fma(w1, r.y, acc[1][h][1]);
+      }
+    }
   }
 }
 
-template <int P>
-__device__ __forceinline__ void tile_clear(uint64_t (&acc)[P][2]) {
+template <int G>
+__device__ __forceinline__ void tile_scale(TileAcc<G>& acc, int e, float f) {
+  const uint64_t ff = ptx::f2_pack(f, f);
 #pragma unroll
-  for (int dd = 0; dd < P; ++dd) acc[dd][0] = acc[dd][1] = 0ull;
+  for (int h = 0; h < G; ++h) {
+    acc[e][h][0] = ptx::f2_mul(acc[e][h][0], ff);
+    acc[e][h][1] = ptx::f2_mul(acc[e][h][1], ff);
+  }
 }
-// Element j of a lane's accumulators of head dim dd.
-template <int P>
-__device__ __forceinline__ float tile_get(const uint64_t (&acc)[P][2], int dd, int j) {
-  const float2 v = ptx::f2_unpack(acc[dd][j >> 1]);
-  return j & 1 ? v.y : v.x;
+// Row e of the lane's accumulators, times f, to `dst` (the row's first element, 16-byte aligned).
+template <int G>
+__device__ __forceinline__ void tile_store(const TileAcc<G>& acc, int e, float f, float* dst, int b4, int d) {
+#pragma unroll
+  for (int h = 0; h < G; ++h) {
+    const float2 x = ptx::f2_unpack(acc[e][h][0]), y = ptx::f2_unpack(acc[e][h][1]);
+    if (b4 + 32 * h < d) *reinterpret_cast<float4*>(dst + b4 + 32 * h) = make_float4(x.x * f, x.y * f, y.x * f, y.y * f);
+  }
 }
 
 __device__ __forceinline__ void tile_copy16(float* dst, const float* src) {
@@ -112,79 +132,88 @@ __device__ __forceinline__ void tile_copy16(float* dst, const float* src) {
 }
 __device__ __forceinline__ void tile_copy_wait() { asm volatile("cp.async.wait_all;" ::: "memory"); }
 
-// KIND as in TileArgs; P1 / P2: head dims of the q-k / v tensors per lane (2: up to 64, 4: up to 128).
-template <int KIND, int P1, int P2>
-__global__ void __launch_bounds__(kTileWarps * 32, 3) simt_tile_kernel(const __grid_constant__ TileArgs t) {
-  using namespace ptx;
+// KIND as in TileArgs; G1 / G2: 32-dim groups of the q-k / v tensors (dQ: only G1 is used, forward: only G2).
+template <int KIND, int G1, int G2>
+__global__ void __launch_bounds__(kTileThreads, 3) simt_tile_kernel(const __grid_constant__ TileArgs t) {
   extern __shared__ __align__(16) float tile_smem[];
-  constexpr int Q = kTileQ, WSETS = KIND == 2 ? 2 : 1;
+  constexpr int WSETS = KIND == 2 ? 2 : 1;
   const Geom& g = t.g;
   const int d1 = g.dqk, d2 = g.dv, s1 = d1 + 4, s2 = d2 + 4, Wtok = g.tw * g.b;
-  float* x1 = tile_smem;                                         // resident rows [32][d]
-  float* x2 = x1 + kTileTokens * d1;
-  float* wbuf = KIND == 0 ? x2 : x2 + kTileTokens * d2;          // weights [warp][1 or 2][32][4]
-  int* at_all = reinterpret_cast<int*>(wbuf + kTileWarps * 32 * Q * WSETS);   // positions of a warp's 32 tokens in the band
-  float* y1 = reinterpret_cast<float*>(at_all + kTileWarps * 32);             // staged tokens
+  float* x1 = tile_smem;                                         // resident rows [warp][8][d + 4]
+  float* x2 = x1 + kTileWarps * kTileQ * s1;
+  float* wbuf = KIND == 0 ? x2 : x2 + kTileWarps * kTileQ * s2;  // weights [warp][1 or 2][8][36]
+  int* at_all = reinterpret_cast<int*>(wbuf + kTileWarps * kTileQ * kTileW * WSETS);   // positions of a warp's 32 tokens in the band
+  float* y1 = reinterpret_cast<float*>(at_all + kTileWarps * 32);                      // staged tokens
   float* y2 = y1 + t.max_keys * s1;
   float* vec = y2 + t.max_keys * s2;                             // dK/dV: their lse, delta
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, a = lane >> 3, b = lane & 7, b4 = 4 * b;
   const int bh = blockIdx.y, bi = bh / g.H, hi = bh - bi * g.H;
   const int ty = blockIdx.x / t.n_tiles_x, r0 = ty * kTileRows, c0 = (blockIdx.x - ty * t.n_tiles_x) * kTileCols;
   auto slice = [&](const View4& v) { return (float*)v.ptr + bi * v.s0 + hi * v.s1; };
 
-  const int my_r = r0 + (warp >> 1), my_c = c0 + (warp & 1) * Q;
-  const bool on = my_r < g.th && my_c < Wtok;
-  float* const mx1 = x1 + warp * Q * d1;
-  float* const mx2 = x2 + warp * Q * d2;
-  float* const w1 = wbuf + warp * 32 * Q * WSETS;
-  float* const w2 = w1 + 32 * Q;
+  // the warp's corner; the lane's rows: columns my_c and my_c + 1 of grid row my_r
+  const int wr0 = r0 + (warp >> 1) * 2, wc0 = c0 + (warp & 1) * 4, my_r = wr0 + (a >> 1), my_c = wc0 + (a & 1) * 2;
+  const bool on = wr0 < g.th && wc0 < Wtok;
+  const int n_out = my_r < g.th ? min(2, max(0, Wtok - my_c)) : 0;           // rows of this lane inside the grid
+  float* const mx1 = x1 + (warp * kTileQ + 2 * a) * s1;
+  float* const mx2 = x2 + (warp * kTileQ + 2 * a) * s2;
+  float* const w1 = wbuf + (warp * kTileQ * WSETS + 2 * a) * kTileW;
+  float* const w2 = w1 + kTileQ * kTileW;
   int* const at = at_all + warp * 32;
   const int64_t row_base = (int64_t)bh * g.th * Wtok + (int64_t)my_r * Wtok + my_c;
 
   // halo of the block and of the warp, clipped to the grid
   const int x_lo = max(0, (c0 / g.b - g.wc) * g.b), x_hi = min(Wtok, ((min(c0 + kTileCols, Wtok) - 1) / g.b + g.wc + 1) * g.b);
   const int h_lo = max(0, r0 - g.wr), h_hi = min(g.th - 1, min(r0 + kTileRows, g.th) - 1 + g.wr), nc = x_hi - x_lo;
-  const int wx_lo = max(0, (my_c / g.b - g.wc) * g.b), wx_hi = min(Wtok, ((min(my_c + Q, Wtok) - 1) / g.b + g.wc + 1) * g.b);
+  const int wx_lo = max(0, (wc0 / g.b - g.wc) * g.b), wx_hi = min(Wtok, ((min(wc0 + 4, Wtok) - 1) / g.b + g.wc + 1) * g.b);
   const int wnc = max(1, wx_hi - wx_lo);
   const uint32_t nc_inv = (0x1000000u + nc - 1) / nc, wnc_inv = (0x1000000u + wnc - 1) / wnc;   // n / nc == (n * nc_inv) >> 24 for n < 4096
 
-  // rows are copied by groups of 8, 16 or 32 lanes, a 16-byte unit each
-  auto lanes_log = [](int d) { return d <= 32 ? 3 : d <= 64 ? 4 : 5; };
   pdl_enter();
   pdl_wait();
+  // rows are copied by groups of 8, 16 or 32 lanes, a 16-byte unit each
+  auto lanes_log = [](int d) { return d <= 32 ? 3 : d <= 64 ? 4 : 5; };
   auto load_resident = [&](float* dst, const View4& v, int d) {
     const float* src = slice(v);
     const int lg = lanes_log(d), c = (tid & ((1 << lg) - 1)) * 4;
     if (c >= d) return;
-    for (int row = tid >> lg; row < kTileTokens; row += kTileWarps * 32 >> lg) {      // row: warp * 4 + column in the warp
-      const int rr = r0 + (row >> 3), cc = c0 + (row & 7);
-      if (rr < g.th && cc < Wtok) tile_copy16(dst + row * d + c, src + ((int64_t)rr * Wtok + cc) * v.s2 + c);
-      else *reinterpret_cast<float4*>(dst + row * d + c) = make_float4(0.f, 0.f, 0.f, 0.f);
+    for (int row = tid >> lg; row < kTileWarps * kTileQ; row += kTileThreads >> lg) {      // row: warp * 8 + (grid row, column) in the warp
+      const int rr = r0 + (row >> 4) * 2 + ((row >> 2) & 1), cc = c0 + ((row >> 3) & 1) * 4 + (row & 3);
+      float* to = dst + row * (d + 4) + c;
+      if (rr < g.th && cc < Wtok) tile_copy16(to, src + ((int64_t)rr * Wtok + cc) * v.s2 + c);
+      else *reinterpret_cast<float4*>(to) = make_float4(0.f, 0.f, 0.f, 0.f);
     }
   };
   load_resident(x1, t.x1, d1);
   if constexpr (KIND != 0) load_resident(x2, t.x2, d2);
 
-  float m[Q], l[Q];                  // forward: running maximum (the same in all lanes), this lane's part of the sum; dQ: lse, delta
+  float m[2], l[2];                  // forward: running maximum (the same in all lanes of a row), this lane's part of the sum; dQ: lse, delta
 #pragma unroll
-  for (int j = 0; j < Q; ++j) {
-    m[j] = -INFINITY;
-    l[j] = 0.f;
+  for (int e = 0; e < 2; ++e) {
+    m[e] = KIND == 1 ? 0.f : -INFINITY;
+    l[e] = 0.f;
     if constexpr (KIND == 1) {
-      m[j] = 0.f;
-      if (on && my_c + j < Wtok) {
-        m[j] = t.lse[row_base + j];
-        l[j] = t.delta[row_base + j];
+      if (e < n_out) {
+        m[e] = t.lse[row_base + e];
+        l[e] = t.delta[row_base + e];
       }
     }
   }
-  constexpr int PA = KIND == 0 ? P2 : P1;
-  uint64_t acc[PA][2];
-  [[maybe_unused]] uint64_t acc2[P2][2];
-  tile_clear(acc);
-  if constexpr (KIND == 2) tile_clear(acc2);
-  const int ca = lane * PA < (KIND == 0 ? d2 : d1) ? lane * PA : 0;          // this lane's head dims (lanes beyond them: idle copies)
-  [[maybe_unused]] const int ca2 = lane * P2 < d2 ? lane * P2 : 0;
+  constexpr int GA = KIND == 0 ? G2 : G1, GB = KIND == 2 ? G2 : 1;
+  TileAcc<GA> acc;
+  [[maybe_unused]] TileAcc<GB> acc2;
+  int goff[GA];
+  [[maybe_unused]] int goff2[GB];
+#pragma unroll
+  for (int h = 0; h < GA; ++h) {                                 // head dims beyond the row: some that exist, sums unused
+    acc[0][h][0] = acc[0][h][1] = acc[1][h][0] = acc[1][h][1] = 0ull;
+    goff[h] = b4 + 32 * h < (KIND == 0 ? d2 : d1) ? b4 + 32 * h : 0;
+  }
+#pragma unroll
+  for (int h = 0; h < GB; ++h) {
+    acc2[0][h][0] = acc2[0][h][1] = acc2[1][h][0] = acc2[1][h][1] = 0ull;
+    goff2[h] = b4 + 32 * h < d2 ? b4 + 32 * h : 0;
+  }
 
   for (int b0 = h_lo; b0 <= h_hi; b0 += t.rb) {
     const int b1 = min(b0 + t.rb - 1, h_hi), n_band = (b1 - b0 + 1) * nc;
@@ -193,8 +222,8 @@ __global__ void __launch_bounds__(kTileWarps * 32, 3) simt_tile_kernel(const __g
       const float* src = slice(v) + ((int64_t)b0 * Wtok + x_lo) * v.s2;
       const int lg = lanes_log(d), c = (tid & ((1 << lg) - 1)) * 4;
       if (c >= d) return;
-#pragma unroll 2
-      for (int n = tid >> lg; n < n_band; n += kTileWarps * 32 >> lg) {
+#pragma unroll 4
+      for (int n = tid >> lg; n < n_band; n += kTileThreads >> lg) {
         const int rr = (int)(((uint64_t)(uint32_t)n * nc_inv) >> 24);
         tile_copy16(dst + n * s + c, src + (int64_t)(rr * (Wtok - nc) + n) * v.s2 + c);
       }
@@ -202,7 +231,7 @@ __global__ void __launch_bounds__(kTileWarps * 32, 3) simt_tile_kernel(const __g
     load_band(y1, t.y1, d1, s1);
     load_band(y2, t.y2, d2, s2);
     if constexpr (KIND == 2) {
-      for (int i = tid; i < n_band; i += kTileWarps * 32) {
+      for (int i = tid; i < n_band; i += kTileThreads) {
         const int rr = (int)(((uint64_t)(uint32_t)i * nc_inv) >> 24);
         const int64_t src = (int64_t)bh * g.th * Wtok + (int64_t)(b0 + rr) * Wtok + x_lo + i - rr * nc;
         vec[i] = t.lse[src];
@@ -211,71 +240,84 @@ __global__ void __launch_bounds__(kTileWarps * 32, 3) simt_tile_kernel(const __g
     }
     tile_copy_wait();
     __syncthreads();
-    const int f0 = max(b0, my_r - g.wr), f1 = min(b1, my_r + g.wr);          // this warp's rows of the band
+    const int f0 = max(b0, wr0 - g.wr), f1 = min(b1, wr0 + 1 + g.wr);        // this warp's rows of the band
     if (!on || f0 > f1) continue;
     const int n0 = (f0 - b0) * nc + wx_lo - x_lo, n_all = (f1 - f0 + 1) * wnc;
 #pragma unroll 1
     for (int k0 = 0; k0 < n_all; k0 += 32) {
-      const int cnt = min(32, n_all - k0), k = min(k0 + lane, n_all - 1);
-      const int kr = (int)(((uint64_t)(uint32_t)k * wnc_inv) >> 24), yx = wx_lo + k - kr * wnc, n = n0 + kr * (nc - wnc) + k;
-      const int yc = g.b == 1 ? yx : yx / g.b;
-      int lo = (yc - g.wc) * g.b - my_c, hi_ = (yc + g.wc + 1) * g.b - 1 - my_c;   // resident columns this token may interact with
-      if (lane >= cnt) hi_ = -1;
-      at[lane] = n;
-      float s[Q];
-      tile_dot(mx1, y1 + n * s1, d1, s);
-      if constexpr (KIND == 0) {
-        bool grow = false;
+      const int cnt = min(32, n_all - k0);
+      int n[4], off[4];
+      uint32_t see = 0;                                          // bit 4 e + i: row e of the lane and token i see each other
 #pragma unroll
-        for (int j = 0; j < Q; ++j) {
-          s[j] = j >= lo && j <= hi_ ? s[j] * g.scale_log2 : -INFINITY;
-          grow = grow || s[j] > m[j] + 16.f || (m[j] == -INFINITY && s[j] > -INFINITY);
-        }
-        // the maximum is renewed only when a score passes it by more than 2^16: fp32 has the range to spare
-        if (__any_sync(0xffffffffu, grow)) {
-          float a[Q];
-#pragma unroll
-          for (int j = 0; j < Q; ++j) {
-            float v = s[j];
-#pragma unroll
-            for (int o = 16; o > 0; o >>= 1) v = fmaxf(v, __shfl_xor_sync(0xffffffffu, v, o));
-            const float mn = fmaxf(m[j], v);
-            a[j] = m[j] == -INFINITY ? 0.f : exp2f(m[j] - mn);
-            m[j] = mn;
-            l[j] *= a[j];
-          }
-          const uint64_t fa = f2_pack(a[0], a[1]), fb = f2_pack(a[2], a[3]);
-#pragma unroll
-          for (int dd = 0; dd < PA; ++dd) {
-            acc[dd][0] = f2_mul(acc[dd][0], fa);
-            acc[dd][1] = f2_mul(acc[dd][1], fb);
-          }
-        }
-#pragma unroll
-        for (int j = 0; j < Q; ++j) {
-          s[j] = s[j] == -INFINITY ? 0.f : exp2f(s[j] - m[j]);
-          l[j] += s[j];
-        }
-      } else {
-        float dp[Q];
-        tile_dot(mx2, y2 + n * s2, d2, dp);
-        const float ls = KIND == 2 ? vec[n] : 0.f, de = KIND == 2 ? vec[t.max_keys + n] : 0.f;
-#pragma unroll
-        for (int j = 0; j < Q; ++j) {
-          const bool see = j >= lo && j <= hi_;
-          const float p = see ? exp2f(fmaf(s[j], g.scale_log2, -(KIND == 1 ? m[j] : ls))) : 0.f;
-          s[j] = p * (dp[j] - (KIND == 1 ? l[j] : de));
-          dp[j] = p;
-        }
-        if constexpr (KIND == 2) *reinterpret_cast<float4*>(w2 + lane * Q) = make_float4(dp[0], dp[1], dp[2], dp[3]);
+      for (int i = 0; i < 4; ++i) {
+        const int k = min(k0 + b + 8 * i, n_all - 1);
+        const int kr = (int)(((uint64_t)(uint32_t)k * wnc_inv) >> 24), yx = wx_lo + k - kr * wnc, yc = g.b == 1 ? yx : yx / g.b;
+        n[i] = n0 + kr * (nc - wnc) + k;
+        off[i] = n[i] * s1;
+        const int lo = (yc - g.wc) * g.b - my_c, last = (yc + g.wc + 1) * g.b - 1 - my_c;  // columns the token may interact with
+        const bool row = (uint32_t)(f0 + kr - my_r + g.wr) <= (uint32_t)(2 * g.wr) && b + 8 * i < cnt;
+        if (row && lo <= 0 && last >= 0) see |= 1u << i;
+        if (row && lo <= 1 && last >= 1) see |= 16u << i;
+        if (a == 0) at[b + 8 * i] = n[i];
       }
-      *reinterpret_cast<float4*>(w1 + lane * Q) = make_float4(s[0], s[1], s[2], s[3]);
+      float s[2][4];
+      tile_dot(mx1, y1, off, d1, s);
+      if constexpr (KIND == 0) {
+        float mx[2] = {-INFINITY, -INFINITY};
+#pragma unroll
+        for (int e = 0; e < 2; ++e)
+#pragma unroll
+          for (int i = 0; i < 4; ++i) {
+            s[e][i] = see >> (4 * e + i) & 1 ? s[e][i] * g.scale_log2 : -INFINITY;
+            mx[e] = fmaxf(mx[e], s[e][i]);
+          }
+        // the maximum is renewed only when a score passes it by more than 2^16: fp32 has the range to spare
+        const bool grow = mx[0] > m[0] + 16.f || mx[1] > m[1] + 16.f;        // (no maximum yet: -INFINITY + 16 is that still)
+        if (__any_sync(0xffffffffu, grow)) {
+#pragma unroll
+          for (int e = 0; e < 2; ++e) {
+            float v = mx[e];
+#pragma unroll
+            for (int o = 4; o > 0; o >>= 1) v = fmaxf(v, __shfl_xor_sync(0xffffffffu, v, o));
+            const float mn = fmaxf(m[e], v), f = m[e] == -INFINITY ? 0.f : exp2f(m[e] - mn);
+            m[e] = mn;
+            l[e] *= f;
+            tile_scale<GA>(acc, e, f);
+          }
+        }
+#pragma unroll
+        for (int e = 0; e < 2; ++e)
+#pragma unroll
+          for (int i = 0; i < 4; ++i) {
+            s[e][i] = s[e][i] == -INFINITY ? 0.f : exp2f(s[e][i] - m[e]);
+            l[e] += s[e][i];
+          }
+      } else {
+        float dp[2][4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) off[i] = n[i] * s2;
+        tile_dot(mx2, y2, off, d2, dp);
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          const float ls = KIND == 2 ? vec[n[i]] : 0.f, de = KIND == 2 ? vec[t.max_keys + n[i]] : 0.f;
+#pragma unroll
+          for (int e = 0; e < 2; ++e) {
+            const float p = see >> (4 * e + i) & 1 ? exp2f(fmaf(s[e][i], g.scale_log2, -(KIND == 1 ? m[e] : ls))) : 0.f;
+            s[e][i] = p * (dp[e][i] - (KIND == 1 ? l[e] : de));
+            if constexpr (KIND == 2) w2[e * kTileW + b + 8 * i] = p;
+          }
+        }
+      }
+#pragma unroll
+      for (int e = 0; e < 2; ++e)
+#pragma unroll
+        for (int i = 0; i < 4; ++i) w1[e * kTileW + b + 8 * i] = s[e][i];
       __syncwarp();
       if constexpr (KIND == 0) {
-        tile_accumulate<PA>(acc, w1, at, y2 + ca, s2, cnt);
+        tile_accumulate<GA>(acc, w1, at, y2, s2, goff, cnt);
       } else {
-        tile_accumulate<PA>(acc, w1, at, y1 + ca, s1, cnt);
-        if constexpr (KIND == 2) tile_accumulate<P2>(acc2, w2, at, y2 + ca2, s2, cnt);
+        tile_accumulate<GA>(acc, w1, at, y1, s1, goff, cnt);
+        if constexpr (KIND == 2) tile_accumulate<GB>(acc2, w2, at, y2, s2, goff2, cnt);
       }
       __syncwarp();
     }
@@ -286,39 +328,34 @@ __global__ void __launch_bounds__(kTileWarps * 32, 3) simt_tile_kernel(const __g
   if constexpr (KIND == 0) {
     float* dst = slice(t.o1) + ((int64_t)my_r * Wtok + my_c) * t.o1.s2;
 #pragma unroll
-    for (int j = 0; j < Q; ++j) {
-      const float lt = warp_sum(l[j]), inv = 1.f / lt;
-      if (my_c + j >= Wtok) continue;
+    for (int e = 0; e < 2; ++e) {
+      float lt = l[e];
 #pragma unroll
-      for (int dd = 0; dd < PA; ++dd)
-        if (lane * PA + dd < d2) dst[j * t.o1.s2 + lane * PA + dd] = tile_get(acc, dd, j) * inv;
-      if (lane == 0) t.lse_out[row_base + j] = m[j] + log2f(lt);
+      for (int o = 4; o > 0; o >>= 1) lt += __shfl_xor_sync(0xffffffffu, lt, o);
+      if (e >= n_out) continue;
+      tile_store<GA>(acc, e, 1.f / lt, dst + e * t.o1.s2, b4, d2);
+      if (b == 0) t.lse_out[row_base + e] = m[e] + log2f(lt);
     }
   } else {
-    float* dst = slice(t.o1) + ((int64_t)my_r * Wtok + my_c) * t.o1.s2;
     __syncwarp();
 #pragma unroll
-    for (int j = 0; j < Q; ++j)                                  // the resident rows are done with: they take the result
-#pragma unroll
-      for (int dd = 0; dd < PA; ++dd)
-        if (lane * PA + dd < d1) mx1[j * d1 + lane * PA + dd] = tile_get(acc, dd, j) * g.sm_scale;
+    for (int e = 0; e < 2; ++e) tile_store<GA>(acc, e, g.sm_scale, mx1 + e * s1, b4, d1);   // the resident rows are done with: they take the result
     __syncwarp();
+    float* dst = slice(t.o1);
 #pragma unroll 1
-    for (int j = 0; j < Q; ++j) {
-      if (my_c + j >= Wtok) break;
+    for (int j = 0; j < kTileQ; ++j) {
+      const int rr = wr0 + (j >> 2), cc = wc0 + (j & 3);
+      if (rr >= g.th || cc >= Wtok) continue;
       int irow = -1, icol = -1;
-      if (t.rope.idx) decode_idx(t.rope.idx[my_r * Wtok + my_c + j], t.rope.max_h, t.rope.max_w, irow, icol);
-      for (int d = lane; d < d1; d += 32) dst[j * t.o1.s2 + d] = load_rot<float>(mx1 + j * d1, 1, d, t.rope, irow, icol, -1.f);
+      if (t.rope.idx) decode_idx(t.rope.idx[rr * Wtok + cc], t.rope.max_h, t.rope.max_w, irow, icol);
+      for (int d = lane; d < d1; d += 32)
+        dst[((int64_t)rr * Wtok + cc) * t.o1.s2 + d] = load_rot<float>(x1 + (warp * kTileQ + j) * s1, 1, d, t.rope, irow, icol, -1.f);
     }
     if constexpr (KIND == 2) {
       float* dst2 = slice(t.o2) + ((int64_t)my_r * Wtok + my_c) * t.o2.s2;
 #pragma unroll
-      for (int j = 0; j < Q; ++j) {
-        if (my_c + j >= Wtok) continue;
-#pragma unroll
-        for (int dd = 0; dd < P2; ++dd)
-          if (lane * P2 + dd < d2) dst2[j * t.o2.s2 + lane * P2 + dd] = tile_get(acc2, dd, j);
-      }
+      for (int e = 0; e < 2; ++e)
+        if (e < n_out) tile_store<GB>(acc2, e, 1.f, dst2 + e * t.o2.s2, b4, d2);
     }
   }
 }

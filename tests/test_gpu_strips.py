@@ -44,7 +44,7 @@ def test_strips_against_simt(th, tw, b, wr, wc, dqk, dv, R, BH):
 
 
 @pytest.mark.parametrize("th,tw,b,wr,wc,dqk,dv,R,BH", [
-    (16, 16, 1, 3, 3, 32, 32, 8, 2), (9, 13, 1, 0, 0, 64, 64, 0, 3), (1, 5, 1, 2, 2, 4, 8, 1, 2), (33, 17, 1, 4, 6, 64, 64, 16, 5),
+    (16, 16, 1, 3, 3, 32, 32, 8, 2), (9, 13, 1, 0, 0, 64, 64, 0, 3), (1, 5, 1, 2, 2, 4, 8, 1, 2), (33, 17, 1, 4, 6, 64, 64, 16, 5), (7, 10, 1, 2, 2, 100, 36, 8, 1),
     (20, 9, 2, 2, 1, 80, 48, 16, 3), (6, 5, 16, 1, 2, 96, 128, 8, 2), (40, 21, 1, 12, 12, 128, 128, 32, 2), (11, 30, 1, 1, 14, 128, 64, 0, 2)])
 def test_fp32_tiles_against_oracle(th, tw, b, wr, wc, dqk, dv, R, BH):
     """fp32 (tiled CUDA-core kernels): tiles cut at the grid's edge, halos in one and several bands, head dims that leave
