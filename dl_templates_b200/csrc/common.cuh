@@ -97,18 +97,8 @@ inline cudaError_t launch_pdl(void (*kern)(P...), dim3 grid, unsigned threads, s
   return cudaLaunchKernelEx(&cfg, kern, static_cast<P>(args)...);
 }
 
-// Streaming kernels (no shared memory, loads in flight wherever L1 has room) follow their predecessor early only while their
-// blocks are resident all at once: started on an SM that the attention kernels have split for shared memory, they keep the
-// 28 KB of L1 that it leaves -- 480 instead of 310 us for the 2.1 GB that q and k of 256 slices of 128 x 128 x 64 move.
-template <typename... P, typename... A>
-inline cudaError_t launch_stream(void (*kern)(P...), dim3 grid, unsigned threads, cudaStream_t st, A&&... args) {
-  if ((uint64_t)grid.x * grid.y <= 148u * 8u) return launch_pdl(kern, grid, threads, 0, st, static_cast<A&&>(args)...);
-  kern<<<grid, threads, 0, st>>>(static_cast<P>(args)...);
-  return cudaGetLastError();
-}
-
-// Opt a kernel in to all the dynamic shared memory there is, once per kernel and device (the call costs a microsecond).
-inline cudaError_t allow_smem(const void* kern) {
+// Set an attribute of a kernel once per kernel and device (the call costs a microsecond).
+inline cudaError_t set_once(const void* kern, cudaFuncAttribute attr, int value) {
   struct Entry { const void* kern; int dev; };
   static Entry table[512];
   static std::atomic<int> n{0};
@@ -118,13 +108,26 @@ inline cudaError_t allow_smem(const void* kern) {
   for (int i = 0, have = n.load(std::memory_order_acquire); i < have; ++i)
     if (table[i].kern == kern && table[i].dev == dev) return cudaSuccess;
   std::lock_guard<std::mutex> lock(mu);
-  if (cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024); e != cudaSuccess) return e;
+  if (cudaError_t e = cudaFuncSetAttribute(kern, attr, value); e != cudaSuccess) return e;
   const int now = n.load();
   if (now < 512) {
     table[now] = Entry{kern, dev};
     n.store(now + 1, std::memory_order_release);
   }
   return cudaSuccess;
+}
+
+// All the dynamic shared memory there is.
+inline cudaError_t allow_smem(const void* kern) { return set_once(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024); }
+
+// Streaming kernels (no shared memory, loads in flight wherever L1 has room) ask for all of L1: started early on an SM that the
+// attention kernels have split for shared memory, they would keep the 28 KB of L1 that it leaves -- 480 instead of 310 us for
+// the 2.1 GB that q and k of 256 slices of 128 x 128 x 64 move.
+template <typename... P, typename... A>
+inline cudaError_t launch_stream(void (*kern)(P...), dim3 grid, unsigned threads, cudaStream_t st, A&&... args) {
+  if (cudaError_t e = set_once((const void*)kern, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxL1); e != cudaSuccess)
+    return e;
+  return launch_pdl(kern, grid, threads, 0, st, static_cast<A&&>(args)...);
 }
 
 }  // namespace swa

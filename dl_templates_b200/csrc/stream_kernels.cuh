@@ -101,6 +101,8 @@ __global__ void __launch_bounds__(256) delta_generic_kernel(View4 o, View4 d_o, 
 template <typename T, int VEC>
 __global__ void __launch_bounds__(256) rope2d_kernel(T* __restrict__ x, int64_t batch, int64_t N, int64_t xs0,
                                                      int64_t xs1, int64_t xs2, RopeDev rp, float sign) {
+  pdl_enter();
+  pdl_wait();
   const int per_tok = 2 * (rp.R / VEC);  // work items per token: halves x chunks
   const int64_t gid = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   const int64_t tok = gid / per_tok;

@@ -601,18 +601,13 @@ int rope2d_apply(int32_t dtype, void* x, int64_t batch, int64_t n_tokens, int32_
                       (xs[1] * esz) % 16 == 0 && ((uintptr_t)rp.row_cs % 16) == 0 && ((uintptr_t)rp.col_cs % 16) == 0;
   const int per_tok = 2 * (vec_ok ? rp.R / vec : rp.R);
   const int64_t items = n_tokens * per_tok;
-  dim3 grid((unsigned)((items + 255) / 256), (unsigned)batch), block(256);
+  dim3 grid((unsigned)((items + 255) / 256), (unsigned)batch);
   if (vec_ok) {
-    if (dtype == SWA_F32)
-      swa::rope2d_kernel<float, 4><<<grid, block, 0, st>>>((float*)x, batch, n_tokens, xs[0], xs[1], xs[2], rp, sign);
-    else if (dtype == SWA_F16)
-      swa::rope2d_kernel<__half, 8><<<grid, block, 0, st>>>((__half*)x, batch, n_tokens, xs[0], xs[1], xs[2], rp, sign);
-    else
-      swa::rope2d_kernel<__nv_bfloat16, 8><<<grid, block, 0, st>>>((__nv_bfloat16*)x, batch, n_tokens, xs[0], xs[1],
-                                                                   xs[2], rp, sign);
+    SWA_DISPATCH_DTYPE(dtype, swa::launch_stream(swa::rope2d_kernel<T, 16 / (int)sizeof(T)>, grid, 256, st, (T*)x, batch, n_tokens, xs[0],
+                                                 xs[1], xs[2], rp, sign));
   } else {
-    SWA_DISPATCH_DTYPE(dtype, swa::rope2d_kernel<T, 1><<<grid, block, 0, st>>>((T*)x, batch, n_tokens, xs[0], xs[1],
-                                                                              xs[2], rp, sign));
+    SWA_DISPATCH_DTYPE(dtype, swa::launch_stream(swa::rope2d_kernel<T, 1>, grid, 256, st, (T*)x, batch, n_tokens, xs[0], xs[1], xs[2], rp,
+                                                 sign));
   }
   return launch_ok("rope2d");
 }
