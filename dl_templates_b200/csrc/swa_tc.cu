@@ -284,7 +284,7 @@ void choose_chunk(const swa_geom_t* g, Plan* pl) {
 
 // Plan of the kernels without streamed rotation for strips TW token columns wide (swa_tc_strip.cuh).  Halos wider than any
 // block are walked in `ncb` column blocks per row band.
-bool make_strip_shape(const swa_geom_t* g, int which, int TW, Plan* out, long* cost_out) {
+bool make_strip_shape(const swa_geom_t* g, int which, int TW, Plan* out) {
   Plan pl{};
   pl.TW = TW;
   pl.TH = 128 / TW;
@@ -363,7 +363,6 @@ bool make_strip_shape(const swa_geom_t* g, int which, int TW, Plan* out, long* c
     pl.s_stride = per <= 128 && pl.nsb * 128 <= room ? 128 : per;
   }
   *out = pl;
-  *cost_out = best_cost;
   // tensor-memory columns of the final plan (the environment overrides above included): a plan beyond the
   // 512-column allocation is refused here, never launched
   const uint32_t tmem_cols = (uint32_t)(which == 0 ? pl.nsb * pl.s_stride : 4 * pl.N) + (uint32_t)acc_cols;
@@ -371,15 +370,29 @@ bool make_strip_shape(const swa_geom_t* g, int which, int TW, Plan* out, long* c
          pl.stages <= kMaxStages && pl.nsb >= 2 && pl.nsb <= 4 && tmem_cols <= 512u;
 }
 
-// Strip width by block cost.
+// Strip width by the time of a whole image (the choice, and with it the order of every sum, must not depend on the batch): its
+// blocks, each its columns and what it costs beside them (as in make_strip_shape), and per item the load of its resident rows
+// where one buffer holds them, here at half of what it weighs against a second buffer there: the next item's first blocks
+// hide the rest.  At 250 columns, 131 x 24, window 11, d = 96 took strips of 8 backward (1165 us a training step of 128 slices
+// against 949 with strips of 16), 128 x 128, window 15, d_v = 128 strips of 16 in dQ (151 against 135 us for 16 slices).
 bool make_strip_plan(const swa_geom_t* g, int which, Plan* out) {
   const Knobs kn = knobs();
   const int th = kn.th[which] ? kn.th[which] : kn.th_all;
-  Plan a, b;
-  long ca = 0, cb = 0;
-  const bool oa = th != 8 && make_strip_shape(g, which, 8, &a, &ca), ob = th != 16 && make_strip_shape(g, which, 16, &b, &cb);
-  if (!oa && !ob) return false;
-  *out = oa && (!ob || ca <= cb) ? a : b;
+  const double beside = which == 0 ? 40. : 100.;
+  double best = -1.;
+  for (int TW : {8, 16}) {
+    Plan pl;
+    if ((th && th != 128 / TW) || !make_strip_shape(g, which, TW, &pl)) continue;
+    const int quarters = (g->t_height + pl.R4 - 1) / pl.R4, step = strip_slides(g, pl.R4, pl.KR) ? quarters : 4;
+    double cost = 0.;
+    for (int q = 0; q < quarters; q += step) cost += strip_blocks(g, pl, q * pl.R4, step) * (pl.N + beside) + (pl.nxb == 1 ? 125. : 0.);
+    cost *= pl.n_tiles_x;
+    if (best < 0. || cost < best) {
+      best = cost;
+      *out = pl;
+    }
+  }
+  if (best < 0.) return false;
   choose_chunk(g, out);
   return true;
 }
