@@ -118,13 +118,14 @@ int tile_band_rows(const swa_geom_t* g, int rows, int cols, int64_t blocks, Byte
 }
 
 // fp32 problems the tiled kernels take (swa_simt_tile.cuh): true when the launch was made (*err: its return code).  `rope`
-// only rotates dQ / dK back; streamed rows are never rotated here.  A halo row that
+// only rotates dQ / dK back; streamed rows are never rotated here; with `delta_out` the dQ launch makes delta from `o` itself.  A halo row that
 // does not fit shared memory is left to the one-warp-per-token kernels.
 bool launch_simt_tile(int kind, const swa_geom_t* g, const swa_rope_t* rope, const swa_tensor_t* x1, const swa_tensor_t* x2,
                       const swa_tensor_t* y1, const swa_tensor_t* y2, const swa_tensor_t* o1, const swa_tensor_t* o2, float* lse_out,
-                      const float* lse, const float* delta, cudaStream_t st, int* err) {
+                      const float* lse, const float* delta, cudaStream_t st, int* err, const swa_tensor_t* o = nullptr,
+                      float* delta_out = nullptr) {
   if (g->dtype != SWA_F32 || g->d_qk % 4 || g->d_v % 4 || g->d_qk > 128 || g->d_v > 128) return false;
-  for (const swa_tensor_t* t : {x1, x2, y1, y2, o1, o2})
+  for (const swa_tensor_t* t : {x1, x2, y1, y2, o1, o2, o})
     if (t && (t->stride[3] != 1 || (uintptr_t)t->ptr % 16 || t->stride[0] % 4 || t->stride[1] % 4 || t->stride[2] % 4)) return false;
   const swa_tensor_t none{nullptr, {0, 0, 0, 0}};
   const int Wtok = g->t_width * g->b_size;
@@ -137,6 +138,8 @@ bool launch_simt_tile(int kind, const swa_geom_t* g, const swa_rope_t* rope, con
   a.lse_out = lse_out;
   a.lse = lse;
   a.delta = delta;
+  a.o = swa::make_view(o ? o : &none);
+  a.delta_out = delta_out;
   const int cols = std::min(Wtok, swa::tile_halo_cols(swa::kTileCols, g->b_size, g->col_size));
   const int rows = std::min(g->t_height, swa::kTileRows + 2 * g->row_size);
   auto bytes = [&](int rb) { return 4 * swa::tile_smem_floats(kind, g->d_qk, g->d_v, rb * cols); };
@@ -267,7 +270,8 @@ int swa_bwd_delta(const swa_geom_t* g, const swa_tensor_t* o, const swa_tensor_t
   return launch_ok("delta");
 }
 
-static int dq_call(bool any8, const swa_geom_t* g, const swa_rope_t* rope, const swa_tensor_t* q, const swa_tensor_t* k, const swa_tensor_t* v, const swa_tensor_t* d_o, const float* lse, const float* delta, const swa_tensor_t* dq, int32_t* status, void* stream) {
+static int dq_call(bool any8, const swa_geom_t* g, const swa_rope_t* rope, const swa_tensor_t* q, const swa_tensor_t* k, const swa_tensor_t* v, const swa_tensor_t* d_o, const float* lse, const float* delta, const swa_tensor_t* dq, int32_t* status, void* stream,
+                   const swa_tensor_t* o = nullptr, float* delta_out = nullptr) {
   if (int e = check_geom(g)) return e;
   if (int e = check_rope(g, rope)) return e;
   if (int e = check_tensor(q, "q")) return e;
@@ -281,12 +285,16 @@ static int dq_call(bool any8, const swa_geom_t* g, const swa_rope_t* rope, const
   if (impl < 0) return impl;
   cudaStream_t st = (cudaStream_t)stream;
   if (impl == SWA_IMPL_TC) {
+    if (delta_out)
+      if (int e = swa_bwd_delta(g, o, d_o, delta_out, stream)) return e;
     int e = swa::tc::launch_dq(g, rope, q, k, v, d_o, lse, delta, dq, status, st);
     if (e) return fail(E_LAUNCH, "tcgen05 dq: %s", swa::tc::last_error());
     return launch_ok("tcgen05 dq");
   }
   int err = 0;
-  if ((!rope || !rope->idx) && launch_simt_tile(1, g, nullptr, q, d_o, k, v, dq, nullptr, nullptr, lse, delta, st, &err)) return err;
+  if ((!rope || !rope->idx) && launch_simt_tile(1, g, nullptr, q, d_o, k, v, dq, nullptr, nullptr, lse, delta, st, &err, o, delta_out)) return err;
+  if (delta_out)
+    if (int e = swa_bwd_delta(g, o, d_o, delta_out, stream)) return e;
   const swa::Geom gg = swa::make_geom(g);
   const swa::RopeDev rp = swa::make_rope(rope);
   const int N = g->t_height * g->t_width * g->b_size;
@@ -417,7 +425,8 @@ int swa_fwd_rot(const swa_geom_t* g, const swa_rope_t* rope, const swa_tensor_t*
   return fwd_rot_call(false, g, rope, q, k, v, o, lse, q_rot, k_rot, status, stream);
 }
 
-static int dq_rot_call(bool any8, const swa_geom_t* g, const swa_rope_t* rope, const swa_tensor_t* q_rot, const swa_tensor_t* k_rot, const swa_tensor_t* v, const swa_tensor_t* d_o, const float* lse, const float* delta, const swa_tensor_t* dq, int32_t* status, void* stream) {
+static int dq_rot_call(bool any8, const swa_geom_t* g, const swa_rope_t* rope, const swa_tensor_t* q_rot, const swa_tensor_t* k_rot, const swa_tensor_t* v, const swa_tensor_t* d_o, const float* lse, const float* delta, const swa_tensor_t* dq, int32_t* status, void* stream,
+                   const swa_tensor_t* o = nullptr, float* delta_out = nullptr) {
   if (int e = check_geom(g)) return e;
   if (int e = require_rope(rope, "swa_bwd_dq_rot")) return e;
   if (int e = check_rope(g, rope)) return e;
@@ -432,12 +441,16 @@ static int dq_rot_call(bool any8, const swa_geom_t* g, const swa_rope_t* rope, c
   if (impl < 0) return impl;
   cudaStream_t st = (cudaStream_t)stream;
   if (impl == SWA_IMPL_TC) {
+    if (delta_out)
+      if (int e = swa_bwd_delta(g, o, d_o, delta_out, stream)) return e;
     int e = swa::tc::launch_dq(g, rope, q_rot, k_rot, v, d_o, lse, delta, dq, status, st, true);
     if (e) return fail(E_LAUNCH, "tcgen05 dq: %s", swa::tc::last_error());
     return launch_ok("tcgen05 dq (inputs rotated)");
   }
   int err = 0;
-  if (launch_simt_tile(1, g, rope, q_rot, d_o, k_rot, v, dq, nullptr, nullptr, lse, delta, st, &err)) return err;
+  if (launch_simt_tile(1, g, rope, q_rot, d_o, k_rot, v, dq, nullptr, nullptr, lse, delta, st, &err, o, delta_out)) return err;
+  if (delta_out)
+    if (int e = swa_bwd_delta(g, o, d_o, delta_out, stream)) return e;
   const swa::Geom gg = swa::make_geom(g);
   const swa::RopeDev none = swa::make_rope(nullptr);
   const int N = g->t_height * g->t_width * g->b_size;
@@ -511,12 +524,12 @@ int swa_step_fwd(const swa_geom_t* g, const swa_rope_t* rope, const swa_tensor_t
 int swa_step_bwd(const swa_geom_t* g, const swa_rope_t* rope, const swa_tensor_t* q, const swa_tensor_t* k, const swa_tensor_t* v,
                  const swa_tensor_t* o, const swa_tensor_t* d_o, const float* lse, float* delta, const swa_tensor_t* dq,
                  const swa_tensor_t* dk, const swa_tensor_t* dv, int32_t* status, void* stream) {
-  if (int e = swa_bwd_delta(g, o, d_o, delta, stream)) return e;
-  if (rope && rope->idx) {
-    if (int e = dq_rot_call(true, g, rope, q, k, v, d_o, lse, delta, dq, status, stream)) return e;
+  if (int e = check_tensor(o, "o")) return e;
+  if (rope && rope->idx) {                                       // (delta comes with dQ)
+    if (int e = dq_rot_call(true, g, rope, q, k, v, d_o, lse, delta, dq, status, stream, o, delta)) return e;
     return dkdv_rot_call(true, g, rope, q, k, v, d_o, lse, delta, dk, dv, status, stream);
   }
-  if (int e = dq_call(true, g, nullptr, q, k, v, d_o, lse, delta, dq, status, stream)) return e;
+  if (int e = dq_call(true, g, nullptr, q, k, v, d_o, lse, delta, dq, status, stream, o, delta)) return e;
   return dkdv_call(true, g, nullptr, q, k, v, d_o, lse, delta, dk, dv, status, stream);
 }
 

@@ -31,6 +31,8 @@ struct TileArgs {
   View4 x1, x2, y1, y2, o1, o2;
   float* lse_out;        // forward
   const float *lse, *delta;
+  View4 o;               // dQ with delta_out: the forward result; delta = rowsum(o * dO) of the block's own rows is made here
+  float* delta_out;
   int rb, n_tiles_x, max_keys;   // halo rows per band, tiles per row of tiles, streamed tokens of the largest band
 };
 
@@ -195,7 +197,7 @@ __global__ void __launch_bounds__(kTileThreads, 3) simt_tile_kernel(const __grid
     if constexpr (KIND == 1) {
       if (e < n_out) {
         m[e] = t.lse[row_base + e];
-        l[e] = t.delta[row_base + e];
+        if (!t.delta_out) l[e] = t.delta[row_base + e];
       }
     }
   }
@@ -236,6 +238,24 @@ __global__ void __launch_bounds__(kTileThreads, 3) simt_tile_kernel(const __grid
         const int64_t src = (int64_t)bh * g.th * Wtok + (int64_t)(b0 + rr) * Wtok + x_lo + i - rr * nc;
         vec[i] = t.lse[src];
         vec[t.max_keys + i] = t.delta[src];
+      }
+    }
+    if constexpr (KIND == 1) {
+      if (t.delta_out && b0 == h_lo) {                           // (while the first band is on its way)
+        const int64_t row = (int64_t)my_r * Wtok + my_c;
+#pragma unroll
+        for (int e = 0; e < 2; ++e) {
+          const float *po = slice(t.o) + (row + e) * t.o.s2, *pd = slice(t.x2) + (row + e) * t.x2.s2;
+          float sum = 0.f;
+          for (int c = b4; e < n_out && c < d2; c += 32) {
+            const float4 x = *reinterpret_cast<const float4*>(po + c), y = *reinterpret_cast<const float4*>(pd + c);
+            sum += x.x * y.x + x.y * y.y + x.z * y.z + x.w * y.w;
+          }
+#pragma unroll
+          for (int o = 4; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+          l[e] = sum;
+          if (b == 0 && e < n_out) t.delta_out[row_base + e] = sum;
+        }
       }
     }
     tile_copy_wait();

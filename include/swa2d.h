@@ -120,7 +120,7 @@ int swa_bwd_dkdv_rot(const swa_geom_t* g, const swa_rope_t* rope, const swa_tens
                      const swa_tensor_t* dk, const swa_tensor_t* dv, int32_t* status, void* stream);
 
 /* One call per direction, what the Python surface uses: swa_step_fwd is swa_fwd_rot with RoPE and swa_fwd without
- * (q_rot / k_rot unused then); swa_step_bwd is swa_bwd_delta, then swa_bwd_dq_rot and swa_bwd_dkdv_rot (q, k = the rotated
+ * (q_rot / k_rot unused then); swa_step_bwd is swa_bwd_delta (fp32: made by the dQ launch), then swa_bwd_dq_rot and swa_bwd_dkdv_rot (q, k = the rotated
  * copies) or swa_bwd_dq and swa_bwd_dkdv, with `delta` as scratch.  Beyond the single entries they take 16-bit head dims of
  * any multiple of 8 up to 128 on the tensor-core kernels as they are (the tensor maps carry the real head dim, TMA fills and
  * clips).  swa_step_select: the kernel family they run for a geometry.  Replace the same launches of the reference as
