@@ -79,6 +79,10 @@ inline Geom make_geom(const swa_geom_t* g) {
 // half of a small step's GPU time.  Every kernel lets its successor start at once (launch_dependents), does what needs no
 // global memory, and then waits until its predecessor has finished and its writes are visible.  A kernel that allocates tensor
 // memory calls pdl_enter only once it has it: a successor resident on the same SM would otherwise hold what it waits for.
+//
+// Such a kernel is resident while its predecessor still writes what it will read.  So nothing it reads goes through the
+// read-only path (__ldg, or `const __restrict__`, which the compiler may turn into it): that path is for data nobody writes while
+// the kernel lives, and `__restrict__` would also allow a load to move above pdl_wait, whose memory clobber orders plain loads only.
 __device__ __forceinline__ void pdl_enter() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 

@@ -12,7 +12,7 @@ namespace swa {
 // that holds the row's units -- owns one token, each lane reads one unit of o and of do, the group reduces with
 // shuffles.  Groups never straddle a warp.
 template <typename T>
-__global__ void __launch_bounds__(256) delta_vec_kernel(View4 o, View4 d_o, float* __restrict__ delta, int H,
+__global__ void __launch_bounds__(256) delta_vec_kernel(View4 o, View4 d_o, float* delta, int H,
                                                         int64_t N, int units, int group, int64_t total_rows) {
   pdl_enter();
   pdl_wait();
@@ -40,9 +40,8 @@ __global__ void __launch_bounds__(256) delta_vec_kernel(View4 o, View4 d_o, floa
 // ([B,H,N,d_v] row-major) writes delta[row]; TOKEN_MAJOR memory ([B,N,H,d_v] row-major, the layout next to an
 // output projection) is walked in memory order and row (b, n, h) writes delta[(b*H + h)*N + n].
 template <typename T, bool TOKEN_MAJOR = false>
-__global__ void __launch_bounds__(256) delta_flat_kernel(const T* __restrict__ o, const T* __restrict__ d_o,
-                                                         float* __restrict__ delta, int dv, int64_t total_rows,
-                                                         int H, int64_t N) {
+__global__ void __launch_bounds__(256) delta_flat_kernel(const T* o, const T* d_o, float* delta, int dv,
+                                                         int64_t total_rows, int H, int64_t N) {
   pdl_enter();
   pdl_wait();
   const int tpr = dv >> 3;  // threads per row
@@ -50,8 +49,8 @@ __global__ void __launch_bounds__(256) delta_flat_kernel(const T* __restrict__ o
   const int64_t row = gid / tpr;
   float acc = 0.f;
   if (row < total_rows) {
-    const uint4 a = __ldg(reinterpret_cast<const uint4*>(o) + gid);
-    const uint4 b = __ldg(reinterpret_cast<const uint4*>(d_o) + gid);
+    const uint4 a = reinterpret_cast<const uint4*>(o)[gid];
+    const uint4 b = reinterpret_cast<const uint4*>(d_o)[gid];
     const T* pa = reinterpret_cast<const T*>(&a);
     const T* pb = reinterpret_cast<const T*>(&b);
 #pragma unroll
@@ -99,7 +98,7 @@ __global__ void __launch_bounds__(256) delta_generic_kernel(View4 o, View4 d_o, 
 // batch entry; tokens whose half has a negative index are skipped without
 // touching memory.  blockIdx.y is the batch entry.
 template <typename T, int VEC>
-__global__ void __launch_bounds__(256) rope2d_kernel(T* __restrict__ x, int64_t batch, int64_t N, int64_t xs0,
+__global__ void __launch_bounds__(256) rope2d_kernel(T* x, int64_t batch, int64_t N, int64_t xs0,
                                                      int64_t xs1, int64_t xs2, RopeDev rp, float sign) {
   pdl_enter();
   pdl_wait();
@@ -212,13 +211,13 @@ __global__ void __launch_bounds__(256) rope2d_copy4_kernel(View4 x, View4 y, Vie
     const uint32_t e0 = half * 2 * rp.R + i0, e1 = e0 + rp.R;
     uint4 v[4] = {ld(src + e0), ld(src + e1), ld(src2 + e0), ld(src2 + e1)};
     int irow, icol;
-    decode_idx(__ldg(rp.idx + tok), rp.max_h, rp.max_w, irow, icol);
+    decode_idx(rp.idx[tok], rp.max_h, rp.max_w, irow, icol);
     const int pos = half ? icol : irow;
     if (pos >= 0) {
       const float4* tab = reinterpret_cast<const float4*>((half ? rp.col_cs : rp.row_cs) + ((int64_t)pos * rp.R + i0) * 2);
 #pragma unroll
       for (int j = 0; j < (int)E; j += 2) {
-        const float4 cs = __ldg(tab + (j >> 1));                        // (cos, sin) of pairs j and j + 1
+        const float4 cs = tab[j >> 1];                        // (cos, sin) of pairs j and j + 1
         const float s0 = cs.y * sign, s1 = cs.w * sign;
 #pragma unroll
         for (int t = 0; t < 4; t += 2) {

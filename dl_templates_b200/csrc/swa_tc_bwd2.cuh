@@ -44,7 +44,7 @@ __global__ void __launch_bounds__(kBwdThreads, 1)
 bwd2_kernel(const __grid_constant__ CUtensorMap tm_xqk, const __grid_constant__ CUtensorMap tm_xv,
             const __grid_constant__ CUtensorMap tm_yqk, const __grid_constant__ CUtensorMap tm_yv,
             const __grid_constant__ CUtensorMap tm_oqk, const __grid_constant__ CUtensorMap tm_ov, const __grid_constant__ KParams p,
-            const float* __restrict__ lse, const float* __restrict__ delta) {
+            const float* lse, const float* delta) {
   using namespace ptx;
   constexpr int R = NE > 0 ? 8 * NE : 8;
   extern __shared__ uint8_t smem_raw[];
@@ -140,8 +140,8 @@ bwd2_kernel(const __grid_constant__ CUtensorMap tm_xqk, const __grid_constant__ 
           const int tr = si.r0 + i * pl.R4 + own_r, tx = si.x0 + own_c;
           if (i < si.nq && tr < p.t_h && tx < p.Wtok) {
             const int64_t at = ((int64_t)(w.bi * p.H + w.hi) * p.t_h + tr) * p.Wtok + tx;
-            a = -__ldg(lse + at);
-            b = __ldg(delta + at);
+            a = -lse[at];
+            b = delta[at];
           }
         }
       };
@@ -423,7 +423,7 @@ bwd2_kernel(const __grid_constant__ CUtensorMap tm_xqk, const __grid_constant__ 
           const bool colk = NE == 4 ? c != 0 : NE == 2 ? m != 0 : e >= 4;
           cs[e] = make_float4(1.f, 0.f, 1.f, 0.f);
           if (pos >= 0) {
-            cs[e] = __ldg(reinterpret_cast<const float4*>((colk ? p.rope.col_cs : p.rope.row_cs) + ((int64_t)pos * R + pair) * 2));
+            cs[e] = *reinterpret_cast<const float4*>((colk ? p.rope.col_cs : p.rope.row_cs) + ((int64_t)pos * R + pair) * 2);
           }
         }
       }
@@ -468,7 +468,7 @@ bwd2_kernel(const __grid_constant__ CUtensorMap tm_xqk, const __grid_constant__ 
         int irow = -1, icol = -1;
         if constexpr (NE > 0) {
           const int tr = qr + own_r, tx = si.x0 + own_c;
-          if (rope_on && tr < p.t_h && tx < p.Wtok) decode_idx(__ldg(p.rope.idx + (int64_t)tr * p.Wtok + tx), p.rope.max_h, p.rope.max_w, irow, icol);
+          if (rope_on && tr < p.t_h && tx < p.Wtok) decode_idx(p.rope.idx[(int64_t)tr * p.Wtok + tx], p.rope.max_h, p.rope.max_w, irow, icol);
         }
         trace_ev(p, 5, tn, slot == 0 && lane == 0 && it >= p.trace_it, 0 * 16 + (i & 15));
         wait_park(&sh->acc_full[slot], acc_par);

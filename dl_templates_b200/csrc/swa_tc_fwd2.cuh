@@ -50,7 +50,7 @@ template <bool BF16, bool ONE, bool OWNP>
 __global__ void __launch_bounds__(kFwdThreads, 1)
 fwd2_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
             const __grid_constant__ CUtensorMap tm_v, const __grid_constant__ CUtensorMap tm_o,
-            const __grid_constant__ KParams p, const __grid_constant__ View4 o, float* __restrict__ lse) {
+            const __grid_constant__ KParams p, const __grid_constant__ View4 o, float* lse) {
   using namespace ptx;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);   // an offset: the compiler keeps seeing shared memory

@@ -334,8 +334,8 @@ __device__ __forceinline__ void mask_warp(const KParams& p, const MaskArgs& f, b
           dl[e] = 0.f;
           if ((uint32_t)y < (uint32_t)p.t_h && (uint32_t)c < (uint32_t)p.Wtok) {
             const int64_t at = slice + y * p.Wtok + c;
-            nl[e] = __ldg(f.lse + at);
-            dl[e] = __ldg(f.delta + at);
+            nl[e] = f.lse[at];
+            dl[e] = f.delta[at];
           }
         }
       }

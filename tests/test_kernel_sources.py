@@ -1,0 +1,47 @@
+"""What the kernels' sources have to keep to and no run can show: rules whose violation is a race or a hang that a machine
+may never exhibit.  Read as text; no GPU."""
+import os
+import re
+
+from conftest import ROOT
+
+CSRC = os.path.join(ROOT, "dl_templates_b200", "csrc")
+
+
+def source(name):
+    text = open(os.path.join(CSRC, name)).read()
+    text = re.sub(r"/\*.*?\*/", "", text, flags=re.S)
+    return re.sub(r"//[^\n]*", "", text)
+
+
+def body_at(text, start):
+    """The brace-balanced block that opens at or after `start`."""
+    i = text.index("{", start)
+    depth = 0
+    for j in range(i, len(text)):
+        depth += {"{": 1, "}": -1}.get(text[j], 0)
+        if depth == 0:
+            return text[start:j + 1]
+    raise AssertionError("unbalanced braces")
+
+
+def kernels():
+    """(name, signature and body) of every __global__ function."""
+    for f in sorted(os.listdir(CSRC)):
+        if f.endswith((".cuh", ".cu")):
+            text = source(f)
+            for m in re.finditer(r"__global__\s+void", text):
+                block = body_at(text, m.start())
+                yield re.search(r"(\w+)\s*\((?!\s*\w+\s*[,)]\s*\w+\s*\()", block[block.index("__launch_bounds__") + 18:]).group(1), block
+
+
+def test_early_started_kernels_read_nothing_through_the_read_only_path():
+    """A kernel that is started before its predecessor has finished (pdl_wait) is resident while its inputs are still being
+    written: no __ldg (the read-only path wants data that nobody writes while the kernel lives) and no __restrict__ (which the
+    compiler may turn into that path, or take as leave to move a load above the wait)."""
+    early = [(n, b) for n, b in kernels() if "pdl_wait" in b]
+    assert len(early) >= 7
+    for name, block in early:
+        assert "__ldg" not in block and "__restrict__" not in block and "ld.global.nc" not in block, name
+    for helper in ("swa_tc_strip.cuh", "swa_simt_tile.cuh"):          # what those kernels are made of
+        assert "__ldg" not in source(helper) and "__restrict__" not in source(helper), helper
