@@ -176,6 +176,8 @@ __device__ __forceinline__ void accumulate_block(uint32_t d, uint32_t a, uint64_
 // ("versions") and a buffer is brought up to date -- the slots whose quarter has changed since it was last loaded -- as soon as
 // the score MMAs of its previous version are done.  With two buffers a quarter crosses L2 twice (it is fetched into L2 one
 // quarter ahead), and its load has one whole block's time to arrive.
+// Whether a barrier's phase has completed is voted on: two lanes that test it while it completes may see different answers, and
+// the walk's state and elect_one must not part ways.
 struct LoadArgs {
   uint8_t* x_smem;              // nxb buffers of qk chunks, then v chunks (128 rows of 128 bytes each)
   uint32_t x_bytes, xqk_bytes;
@@ -200,7 +202,7 @@ __device__ __forceinline__ void load_warp(const KParams& p, const LoadArgs& f, b
 #pragma unroll 1
   while (ok && (ity < count || itx < count)) {
     bool idle = true;
-    if (ity < count && (!ring_full || mbar_test(smem_u32(f.y_empty + stage), stage_par))) {
+    if (ity < count && (!ring_full || __all_sync(0xffffffffu, mbar_test(smem_u32(f.y_empty + stage), stage_par)))) {
       idle = false;
       if (elect_one()) {
         uint64_t* bar = f.y_full + stage;
@@ -223,7 +225,7 @@ __device__ __forceinline__ void load_warp(const KParams& p, const LoadArgs& f, b
         ++ity;
       }
     }
-    if (itx < count && (!x_ring_full || mbar_test(smem_u32(f.x_empty + xb), x_par))) {
+    if (itx < count && (!x_ring_full || __all_sync(0xffffffffu, mbar_test(smem_u32(f.x_empty + xb), x_par)))) {
       idle = false;
       if (jx == 0) stale0 = stale1 = 0;
       // the quarters that enter: the first four with the item, the others with the first block that needs them

@@ -45,3 +45,15 @@ def test_early_started_kernels_read_nothing_through_the_read_only_path():
         assert "__ldg" not in block and "__restrict__" not in block and "ld.global.nc" not in block, name
     for helper in ("swa_tc_strip.cuh", "swa_simt_tile.cuh"):          # what those kernels are made of
         assert "__ldg" not in source(helper) and "__restrict__" not in source(helper), helper
+
+
+def test_a_warp_never_branches_on_one_lanes_view_of_a_barrier():
+    """Lanes that test a barrier while its phase completes may see different answers.  A warp that walks a ring together votes on
+    the answer: every test or wait in the strip kernels stands inside a warp vote."""
+    seen = 0
+    for f in ("swa_tc_strip.cuh", "swa_tc_fwd2.cuh", "swa_tc_bwd2.cuh"):
+        text = re.sub(r"\s+", " ", source(f))
+        for m in re.finditer(r"\b(mbar_test|mbar_wait_polls|mbar_try_wait\w*|mbar_wait)\b", text):
+            assert text[:m.start()].rstrip().endswith("__all_sync(0xffffffffu,"), (f, text[m.start() - 80:m.end() + 40])
+            seen += 1
+    assert seen >= 6
