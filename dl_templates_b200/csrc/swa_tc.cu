@@ -120,16 +120,18 @@ const Knobs& knobs() {
   return *g_knobs.load();
 }
 
-// Widest halo, in token columns, over all resident-tile columns.
+// Widest halo, in token columns, over all resident-tile columns; at most kHaloMost, more than any plan takes (a half-size may be
+// any 32-bit number: in 32 bits the width of a huge one wrapped round to a narrow halo, and to a plan for that).
+constexpr int kHaloMost = 1 << 20;
 int halo_width(const swa_geom_t* g, int TW) {
-  const int Wtok = g->t_width * g->b_size, b = g->b_size;
-  int best = 0;
-  for (int x0 = 0; x0 < Wtok; x0 += TW) {
-    const int lo = (x0 / b - g->col_size) * b;
-    const int hi = ((x0 + TW - 1) / b + g->col_size + 1) * b;
+  const int64_t Wtok = (int64_t)g->t_width * g->b_size, b = g->b_size, wc = g->col_size;
+  int64_t best = 0;
+  for (int64_t x0 = 0; x0 < Wtok; x0 += TW) {
+    const int64_t lo = (x0 / b - wc) * b;
+    const int64_t hi = ((x0 + TW - 1) / b + wc + 1) * b;
     best = hi - lo > best ? hi - lo : best;
   }
-  return best;
+  return (int)std::min<int64_t>(best, kHaloMost);
 }
 
 // Choose the resident tile, the streamed-block shape and the pipeline depths.  Tile shapes tried: 16 x 8 first -- a warp's 32 rows then span

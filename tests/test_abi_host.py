@@ -149,6 +149,15 @@ def test_every_tile_plan_fits_shared_and_tensor_memory():
     assert n_plans > 500
 
 
+def test_windows_too_wide_for_32_bits_get_no_plan():
+    """(2 wc + 1) * b beyond 32 bits must not wrap round to a plan for a narrow halo: no plan, the SIMT kernels take it."""
+    for b, wc in ((16, 2 ** 27), (16, 2 ** 27 + 3), (1, 2 ** 30), (1, 2 ** 31 - 1), (4, 2 ** 29), (16, 2 ** 31 - 1), (16, 5000)):
+        g = _geom(b_size=b, t_height=8, t_width=8, col_size=wc)
+        for which in (0, 1, 2):
+            assert _lib.lib.swa_select_impl(C.byref(g), None, which) == _lib.IMPL_SIMT, (b, wc)
+            assert _plan(g, None, which)[0] < 0
+
+
 def test_head_dims_the_tensor_core_kernels_take():
     """32, 64, 96, 128 where no streamed row is rotated (no RoPE, or the entries that take rotated copies); 64 and
     128 only for the kernels that rotate what they stream; anything else runs on the SIMT kernels."""
