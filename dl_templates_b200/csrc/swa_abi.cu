@@ -91,9 +91,9 @@ int resolve_impl(const swa_geom_t* g, const swa_rope_t* rope, const swa_tensor_t
 // a lone block, whose loads nothing hides: 1.1; measured at 40 x 40, window 9, d = 64, 32 slices).  48 x 48, window 5, d = 128: three blocks 229 us a training step, two
 // 158; 40 x 40, window 9, d = 64, 8 slices: 132 against 174.
 template <typename Bytes>
-int tile_band_rows(const swa_geom_t* g, int rows, int cols, int64_t blocks, Bytes&& bytes) {
+int tile_band_rows(const swa::Geom& g, int rows, int cols, int64_t blocks, Bytes&& bytes) {
   static const struct { int per_sm, kb; double step; } kinds[3] = {{3, 74, 1.34}, {2, 112, 1.}, {1, 227, 1.1}};
-  const int wcols = std::min(g->t_width * g->b_size, swa::tile_halo_cols(4, g->b_size, g->col_size)), span = 2 * g->row_size + 2;
+  const int wcols = (int)std::min((int64_t)g.tw * g.b, swa::tile_halo_cols(4, g.b, g.wc)), span = (int)std::min((int64_t)rows, 2 * (int64_t)g.wr + 2);
   double best = -1.;
   int best_rb = 1;
   for (const auto& c : kinds) {
@@ -140,13 +140,13 @@ bool launch_simt_tile(int kind, const swa_geom_t* g, const swa_rope_t* rope, con
   a.delta = delta;
   a.o = swa::make_view(o ? o : &none);
   a.delta_out = delta_out;
-  const int cols = std::min(Wtok, swa::tile_halo_cols(swa::kTileCols, g->b_size, g->col_size));
-  const int rows = std::min(g->t_height, swa::kTileRows + 2 * g->row_size);
+  const int cols = (int)std::min((int64_t)Wtok, swa::tile_halo_cols(swa::kTileCols, g->b_size, a.g.wc));
+  const int rows = (int)std::min((int64_t)g->t_height, swa::kTileRows + 2 * (int64_t)a.g.wr);
   auto bytes = [&](int rb) { return 4 * swa::tile_smem_floats(kind, g->d_qk, g->d_v, rb * cols); };
   if (bytes(1) > 227 * 1024 || cols > 4000) return false;
   a.n_tiles_x = (Wtok + swa::kTileCols - 1) / swa::kTileCols;
   const int64_t tiles = (int64_t)a.n_tiles_x * ((g->t_height + swa::kTileRows - 1) / swa::kTileRows);
-  a.rb = tile_band_rows(g, rows, cols, tiles * g->B * g->H, bytes);
+  a.rb = tile_band_rows(a.g, rows, cols, tiles * g->B * g->H, bytes);
   a.max_keys = a.rb * cols;
   const dim3 grid((unsigned)tiles, (unsigned)(g->B * g->H));
   using Kernel = void (*)(const swa::TileArgs);

@@ -36,7 +36,8 @@ struct TileArgs {
   int rb, n_tiles_x, max_keys;   // halo rows per band, tiles per row of tiles, streamed tokens of the largest band
 };
 
-__host__ __device__ __forceinline__ int tile_halo_cols(int cols, int b, int wc) { return ((cols + b - 2) / b + 1 + 2 * wc) * b; }
+// Token columns of the halo of `cols` columns, not clipped to the grid.
+inline int64_t tile_halo_cols(int cols, int64_t b, int64_t wc) { return ((cols + b - 2) / b + 1 + 2 * wc) * b; }
 
 // Floats of shared memory of a launch with `keys` staged tokens.  All rows lie 4 floats further apart than they are long:
 // rows at distance 1 (streamed) or 2 (resident) start in banks of their own.

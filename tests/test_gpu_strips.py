@@ -82,3 +82,19 @@ def test_head_dims_of_any_multiple_of_8_as_they_are(dqk, dv, R, dtype):
     assert swa.tiled_swa._mode_for(qd, vd, rd if R else None, (*win, sc)) == ("handoff" if R else "none")
     for a, c, n in zip(got, want, ("o", "dq", "dk", "dv")):
         assert orc.max_abs(a.float().cpu(), c) < 2e-2 and orc.mean_rel(a.float().cpu(), c) < 5e-3, n
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("wr,wc", [(2 ** 31 - 1, 2 ** 31 - 1), (3, 2 ** 27), (2 ** 30, 2 ** 27 + 3), (2 ** 30 - 1, 1)])
+def test_windows_of_any_size_beyond_the_grid(wr, wc, dtype):
+    """A half-size that reaches past the grid is the whole grid, also where (2 wc + 1) * b or r + wr does not fit 32 bits."""
+    b, th, tw = 16, 6, 5
+    q, k, v, do = (t.to(DEV) for t in orc.seeded_inputs(1, 2, th * tw * b, 64, 64, dtype, 5))
+    got, want = [], []
+    for res, win in ((got, (b, th, tw, wr, wc)), (want, (b, th, tw, min(wr, th), min(wc, tw)))):
+        t = [x.clone().requires_grad_(True) for x in (q, k, v)]
+        o = swa.TiledSwa.apply(*t, *win, 0.125)
+        res += [o.detach(), *torch.autograd.grad(o, t, do)]
+    swa.check_status()
+    for a, c in zip(got, want):
+        assert orc.max_abs(a.float(), c.float()) < (2e-6 if dtype == torch.float32 else 2e-2)
