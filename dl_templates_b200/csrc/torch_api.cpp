@@ -116,7 +116,8 @@ swa_tensor_t view4(const Tensor& t) {
   return r;
 }
 
-swa_rope_t rope_view(const Rope& r) {
+// What the planner needs of a rotation; nothing of it is read on the device.
+swa_rope_t rope_shape(const Rope& r) {
   require(r.idx.scalar_type() == at::kInt && r.idx.is_contiguous(), "idx must be contiguous int32");
   require(r.row.scalar_type() == at::kFloat && r.col.scalar_type() == at::kFloat, "cos/sin tables must be float32");
   require(r.row.is_contiguous() && r.col.is_contiguous(), "cos/sin tables must be contiguous");
@@ -124,6 +125,16 @@ swa_rope_t rope_view(const Rope& r) {
           "cos/sin tables must be [max, n_rdim, 2] with the same n_rdim");
   return swa_rope_t{r.idx.data_ptr<int32_t>(), r.row.data_ptr<float>(), r.col.data_ptr<float>(), (int32_t)r.row.size(1),
                     (int32_t)r.row.size(0), (int32_t)r.col.size(0)};
+}
+
+// ... and for a launch: the kernels read one index per token, and all three tensors as pointers of q's device.
+swa_rope_t rope_view(const Rope& r, int64_t n_tokens, const Tensor& q) {
+  const swa_rope_t v = rope_shape(r);
+  require(r.idx.numel() >= n_tokens, "one index per token expected");
+  TORCH_CHECK(r.idx.device() == q.device() && r.row.device() == q.device() && r.col.device() == q.device(),
+              "idx and the cos/sin tables must be on the tensors' device: ", r.idx.device(), ", ", r.row.device(), ", ", r.col.device(),
+              " beside ", q.device());
+  return v;
 }
 
 int32_t forced_impl(int32_t impl) {
@@ -144,6 +155,7 @@ void check_inputs(const Tensor& q, const Tensor& k, const Tensor& v, const Win& 
   poll_status();
   TORCH_CHECK(q.is_cuda() && k.is_cuda() && v.is_cuda(),
               "dl_templates_b200 runs on CUDA tensors only (sm_100a); there is no CPU path");
+  TORCH_CHECK(k.device() == q.device() && v.device() == q.device(), "q, k, v must be on one device");
   TORCH_CHECK_VALUE(q.dim() == 4 && v.dim() == 4 && k.sizes() == q.sizes() && v.sizes().slice(0, 3) == q.sizes().slice(0, 3),
                     "expected q,k [B,H,N,d_qk] and v [B,H,N,d_v]");
   TORCH_CHECK_TYPE(q.scalar_type() == k.scalar_type() && q.scalar_type() == v.scalar_type(), "q, k, v must share a dtype");
@@ -179,7 +191,7 @@ std::array<int64_t, 2> padded_dims(const Tensor& q, int64_t d_v, const Rope* rop
   if (off && *off) return none;
   swa_rope_t r;
   const swa_rope_t* rp = nullptr;
-  if (rope && rope->on()) { r = rope_view(*rope); rp = &r; }
+  if (rope && rope->on()) { r = rope_shape(*rope); rp = &r; }
   auto all_tc = [&](int64_t a, int64_t b) {
     const swa_geom_t g = geom(q, a, b, w, forced_impl(SWA_IMPL_AUTO));
     for (int which = 0; which < 3; ++which)
@@ -196,7 +208,7 @@ bool native_dims(const Tensor& q, int64_t d_v, const Rope* rope, const Win& w, i
   if (q.dim() != 4) return false;
   swa_rope_t r;
   const swa_rope_t* rp = nullptr;
-  if (rope && rope->on()) { r = rope_view(*rope); rp = &r; }
+  if (rope && rope->on()) { r = rope_shape(*rope); rp = &r; }
   const swa_geom_t g = geom(q, q.size(3), d_v, w, forced_impl(SWA_IMPL_AUTO));
   return swa_step_select(&g, rp) == SWA_IMPL_TC;
 }
@@ -244,7 +256,7 @@ Fwd forward(Tensor q, Tensor k, Tensor v, const Rope& rope, const Win& w, int32_
   f.lse = new_lse(q);
   const swa_geom_t g = geom(q, q.size(3), v.size(3), w, forced_impl(impl));
   swa_rope_t r;
-  if (rope.on()) r = rope_view(rope);
+  if (rope.on()) r = rope_view(rope, q.size(2), q);
   const swa_tensor_t tq = view4(q), tk = view4(k), tv = view4(v), to = view4(f.o);
   if (rope.on())
     check(swa_fwd(&g, &r, &tq, &tk, &tv, &to, f.lse.data_ptr<float>(), status_ptr(q.get_device()), stream_of(q)), "swa_fwd");
@@ -267,7 +279,7 @@ Fwd forward_rot(Tensor q, Tensor k, Tensor v, const Rope& rope, const Win& w, in
   f.q_rot = at::empty(q.sizes(), q.options());
   f.k_rot = at::empty(q.sizes(), q.options());
   const swa_geom_t g = geom(q, q.size(3), v.size(3), w, forced_impl(impl));
-  const swa_rope_t r = rope_view(rope);
+  const swa_rope_t r = rope_view(rope, q.size(2), q);
   const swa_tensor_t tq = view4(q), tk = view4(k), tv = view4(v), to = view4(f.o), tqr = view4(f.q_rot), tkr = view4(f.k_rot);
   check(swa_step_fwd(&g, &r, &tq, &tk, &tv, &to, f.lse.data_ptr<float>(), &tqr, &tkr, status_ptr(q.get_device()), stream_of(q)),
         "swa_step_fwd");
@@ -275,10 +287,24 @@ Fwd forward_rot(Tensor q, Tensor k, Tensor v, const Rope& rope, const Win& w, in
   return f;
 }
 
+// What backward reads beside the inputs: the forward's result and its gradient, the softmax statistic.
+void check_saved(const Tensor& q, const Tensor& v, const Tensor& o, const Tensor& lse, const Tensor& d_o) {
+  for (const Tensor* t : {&o, &d_o}) {
+    TORCH_CHECK(t->device() == q.device(), "o and do must be on the device of q");
+    TORCH_CHECK_VALUE(t->sizes() == v.sizes(), "expected o, do [B,H,N,d_v]");
+    TORCH_CHECK_TYPE(t->scalar_type() == q.scalar_type(), "o and do must have the dtype of q");
+  }
+  TORCH_CHECK(lse.device() == q.device(), "lse must be on the device of q");
+  TORCH_CHECK_TYPE(lse.scalar_type() == at::kFloat, "lse must be float32");
+  TORCH_CHECK_VALUE(lse.numel() == q.size(0) * q.size(1) * q.size(2), "expected lse [B,H,N]");
+}
+
 // `rotated`: q and k are the rotated copies forward_rot left behind (swa_bwd_*_rot).
-Grads backward(Tensor q, Tensor k, Tensor v, Tensor o, const Tensor& lse, Tensor d_o, const Rope& rope, bool rotated, const Win& w,
+Grads backward(Tensor q, Tensor k, Tensor v, Tensor o, Tensor lse, Tensor d_o, const Rope& rope, bool rotated, const Win& w,
                int32_t impl, Grads out) {
-  poll_status();
+  check_inputs(q, k, v, w);
+  check_saved(q, v, o, lse, d_o);
+  lse = lse.contiguous();
   q = materialise(q); k = materialise(k); v = materialise(v); o = materialise(o); d_o = materialise(d_o);
   const bool given = out.dq.defined();
   if (!rotated && !(!rope.on() && native_dims(q, v.size(3), nullptr, w, impl))) {
@@ -310,7 +336,7 @@ Grads backward(Tensor q, Tensor k, Tensor v, Tensor o, const Tensor& lse, Tensor
   const Tensor delta = new_lse(q);
   const swa_geom_t g = geom(q, q.size(3), v.size(3), w, forced_impl(impl));
   swa_rope_t rv;
-  if (rope.on()) rv = rope_view(rope);
+  if (rope.on()) rv = rope_view(rope, q.size(2), q);
   const swa_rope_t* rp = rope.on() ? &rv : nullptr;
   const swa_tensor_t tq = view4(q), tk = view4(k), tv = view4(v), to = view4(o), tdo = view4(d_o), tdq = view4(r.dq),
                      tdk = view4(r.dk), tdv = view4(r.dv);
@@ -336,7 +362,7 @@ void rope_inplace(const Tensor& x, const Rope& rope, bool inverse) {
   require(rope.row.size(1) == rope.col.size(1), "row and column tables differ in width");
   require(rope.idx.size(0) == x.size(1), "one index per token expected");
   const c10::cuda::OptionalCUDAGuard guard(x.device());
-  const swa_rope_t r = rope_view(rope);
+  const swa_rope_t r = rope_view(rope, x.size(1), x);
   const int64_t xs[3] = {x.stride(0), x.stride(1), x.stride(2)};
   check(rope2d_apply(dtype_code(x.scalar_type()), x.data_ptr(), x.size(0), x.size(1), (int32_t)x.size(2), xs, &r, inverse ? 1 : 0,
                      stream_of(x)), "rope2d_apply");
@@ -351,7 +377,7 @@ Tensor rope_to(const Tensor& x, const Rope& rope, bool inverse) {
                       x.stride(1) % 8 == 0;
   if ((x.scalar_type() == at::kHalf || x.scalar_type() == at::kBFloat16) && rope.row.size(1) % 8 == 0 && x.size(2) % 8 == 0 && rows16) {
     const c10::cuda::OptionalCUDAGuard guard(x.device());
-    const swa_rope_t r = rope_view(rope);
+    const swa_rope_t r = rope_view(rope, x.size(1), x);
     const int64_t xs[3] = {x.stride(0), x.stride(1), x.stride(2)}, ys[3] = {y.stride(0), y.stride(1), y.stride(2)};
     check(rope2d_apply_to(dtype_code(x.scalar_type()), x.data_ptr(), y.data_ptr(), x.size(0), x.size(1), (int32_t)x.size(2), xs, ys,
                           &r, inverse ? 1 : 0, stream_of(x)), "rope2d_apply_to");
@@ -676,6 +702,20 @@ PyObject* py_backward(PyObject*, PyObject* const* args, Py_ssize_t n) {
     return pack({g.dq, g.dk, g.dv});
   });
 }
+// check_backward(q, k, v, o, lse, do, idx, row_cs, col_cs, window..., sm_scale): raises what backward would raise, launches nothing
+PyObject* py_check_backward(PyObject*, PyObject* const* args, Py_ssize_t n) {
+  return guarded([&]() -> PyObject* {
+    Args a{args, n};
+    const Tensor &q = a.tensor(), &k = a.tensor(), &v = a.tensor(), &o = a.tensor(), &lse = a.tensor(), &d_o = a.tensor();
+    const Rope r = a.rope();
+    const Win w = a.win();
+    a.done();
+    check_inputs(q, k, v, w);
+    check_saved(q, v, o, lse, d_o);
+    if (r.on()) rope_view(r, q.size(2), q);
+    Py_RETURN_NONE;
+  });
+}
 // rope2d_(x [batch,N,C], idx, row_cs, col_cs, inverse) -> x, rotated in place
 PyObject* py_rope2d_inplace(PyObject*, PyObject* const* args, Py_ssize_t n) {
   return guarded([&]() -> PyObject* {
@@ -780,6 +820,7 @@ PyMethodDef g_methods[] = {SWA_DEF("tiled_swa", py_tiled_swa),
                            SWA_DEF("forward", py_forward),
                            SWA_DEF("forward_rot", py_forward_rot),
                            SWA_DEF("backward", py_backward),
+                           SWA_DEF("check_backward", py_check_backward),
                            SWA_DEF("rope2d_", py_rope2d_inplace),
                            SWA_DEF("rope2d_to", py_rope2d_to),
                            SWA_DEF("rope2d_heads_", py_rope2d_heads_inplace),

@@ -116,7 +116,12 @@ def swa_backward_noalloc(q, k, v, o, lse, do, rope, b_size, t_height, t_width, r
     Calls on one device share that array, so do not let two of them overlap on the GPU; the
     first call on a device does a one-time address lookup and should come before any stream
     capture.  Returns ``(dq, dk, dv)``."""
-    B, H, N, _ = q.shape
+    _native.check_backward(q, k, v, o, lse, do, *(rope or _NO_ROPE), b_size, t_height, t_width, row_size, col_size, sm_scale)
+    if not lse.is_contiguous():
+        raise ValueError("lse must be contiguous")
+    for t, like, what in ((dq, q, "dq"), (dk, k, "dk"), (dv, v, "dv")):
+        if t.shape != like.shape or t.dtype != like.dtype or t.device != like.device:
+            raise ValueError(f"{what}: expected shape {tuple(like.shape)}, dtype {like.dtype} on {like.device}")
     g = _geom(q, v, b_size, t_height, t_width, row_size, col_size, sm_scale, impl)
     r = _lib.make_rope(*rope) if rope is not None else None
     tq, tk, tv, to, tdo, tdq, tdk, tdv = (_lib.tensor4(t) for t in (q, k, v, o, do, dq, dk, dv))
