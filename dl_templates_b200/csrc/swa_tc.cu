@@ -591,6 +591,8 @@ const char* unsupported_reason(const swa_geom_t* g, const swa_rope_t* rope, cons
   if (!mask_constants(g->sm_scale, &ma, &mb)) return "sm_scale too small for the MMA-side window mask";
   if (rope && rope->idx && rope->n_rdim != 8 && rope->n_rdim != 16 && rope->n_rdim != 32)
     return "n_rdim must be 8, 16 or 32 (RoPE on 32, 64 or 128 dims)";
+  if (rope && rope->idx && !(prerotated && which == 0) && (((uintptr_t)rope->row_cs | (uintptr_t)rope->col_cs) & 15))
+    return "cos/sin tables must be 16-byte aligned";      // (the forward kernel of rotated copies reads none)
   if (g->row_size > 64) return "row window too tall for the penalty tables";
   if ((int64_t)g->t_height * g->t_width * g->b_size > (1 << 30)) return "grid too large";
   Plan pl;

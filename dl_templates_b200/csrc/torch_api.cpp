@@ -137,6 +137,13 @@ swa_rope_t rope_view(const Rope& r, int64_t n_tokens, const Tensor& q) {
   return v;
 }
 
+// The tensor-core kernels read the tables by 16 bytes: tables that start elsewhere are copied, like tensors (materialise).
+Rope aligned_tables(Rope r) {
+  for (Tensor* t : {&r.row, &r.col})
+    if (r.on() && t->is_cuda() && reinterpret_cast<uintptr_t>(t->data_ptr()) % 16) *t = t->clone();
+  return r;
+}
+
 int32_t forced_impl(int32_t impl) {
   const char* e = std::getenv("SWA_FORCE_IMPL");
   if (!e) return impl;
@@ -231,8 +238,9 @@ struct Grads {
   Tensor dq, dk, dv;
 };
 
-Fwd forward(Tensor q, Tensor k, Tensor v, const Rope& rope, const Win& w, int32_t impl, Tensor out) {
+Fwd forward(Tensor q, Tensor k, Tensor v, const Rope& rope_, const Win& w, int32_t impl, Tensor out) {
   check_inputs(q, k, v, w);
+  const Rope rope = aligned_tables(rope_);
   q = materialise(q); k = materialise(k); v = materialise(v);
   const auto pad = !rope.on() && native_dims(q, v.size(3), nullptr, w, impl) ? std::array<int64_t, 2>{0, 0}
                                                                           : padded_dims(q, v.size(3), &rope, w, impl);
@@ -267,8 +275,9 @@ Fwd forward(Tensor q, Tensor k, Tensor v, const Rope& rope, const Win& w, int32_
   return f;
 }
 
-Fwd forward_rot(Tensor q, Tensor k, Tensor v, const Rope& rope, const Win& w, int32_t impl, Tensor out) {
+Fwd forward_rot(Tensor q, Tensor k, Tensor v, const Rope& rope_, const Win& w, int32_t impl, Tensor out) {
   check_inputs(q, k, v, w);
+  const Rope rope = aligned_tables(rope_);
   q = materialise(q); k = materialise(k); v = materialise(v);
   const c10::cuda::OptionalCUDAGuard guard(q.device());
   Fwd f;
@@ -300,10 +309,11 @@ void check_saved(const Tensor& q, const Tensor& v, const Tensor& o, const Tensor
 }
 
 // `rotated`: q and k are the rotated copies forward_rot left behind (swa_bwd_*_rot).
-Grads backward(Tensor q, Tensor k, Tensor v, Tensor o, Tensor lse, Tensor d_o, const Rope& rope, bool rotated, const Win& w,
+Grads backward(Tensor q, Tensor k, Tensor v, Tensor o, Tensor lse, Tensor d_o, const Rope& rope_, bool rotated, const Win& w,
                int32_t impl, Grads out) {
   check_inputs(q, k, v, w);
   check_saved(q, v, o, lse, d_o);
+  const Rope rope = aligned_tables(rope_);
   lse = lse.contiguous();
   q = materialise(q); k = materialise(k); v = materialise(v); o = materialise(o); d_o = materialise(d_o);
   const bool given = out.dq.defined();

@@ -158,6 +158,17 @@ def test_windows_too_wide_for_32_bits_get_no_plan():
             assert _plan(g, None, which)[0] < 0
 
 
+def test_misaligned_tables_keep_off_the_tensor_core_kernels():
+    """Those read the cos/sin tables by 16 bytes; tables that start elsewhere are the SIMT kernels' (the forward kernel of
+    rotated copies reads none)."""
+    g = _geom(t_height=16, t_width=16)
+    for row, col, plain in ((2048, 4096, True), (2052, 4096, False), (2048, 4104, False)):
+        r = _lib.Rope(1024, row, col, 16, 16, 16)
+        for which in (0, 1, 2):
+            assert (_lib.lib.swa_select_impl(C.byref(g), C.byref(r), which) == _lib.IMPL_TC) == plain
+        assert (_plan(g, r, 3)[0] == 0) and (_plan(g, r, 4)[0] == 0) == plain and (_plan(g, r, 5)[0] == 0) == plain
+
+
 def test_head_dims_the_tensor_core_kernels_take():
     """32, 64, 96, 128 where no streamed row is rotated (no RoPE, or the entries that take rotated copies); 64 and
     128 only for the kernels that rotate what they stream; anything else runs on the SIMT kernels."""

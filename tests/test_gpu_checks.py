@@ -67,3 +67,25 @@ def test_refused_before_any_launch(dtype):
     assert all(torch.equal(a, b) for a, b in zip(got, want))
     longer = (torch.cat([idx, idx]), row, col)
     assert torch.equal(swa.swa_forward(q, k, v, longer, *WIN, 0.125)[0], swa.swa_forward(q, k, v, rope, *WIN, 0.125)[0])
+
+
+@pytest.mark.parametrize("mode", ["handoff", "fused"])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+def test_tables_that_start_off_a_16_byte_boundary(dtype, mode):
+    q, k, v, do, rope = case(dtype)
+    off = [rope[0]]
+    for t in rope[1:]:
+        buf = torch.empty(t.numel() + 1, device=DEV)
+        buf[1:] = t.flatten()
+        off.append(buf[1:].view(t.shape))
+        assert off[-1].data_ptr() % 16 and off[-1].is_contiguous()
+    prev = swa.set_rope_mode(mode)
+    try:
+        res = []
+        for r in (rope, off):
+            t = [x.clone().requires_grad_(True) for x in (q, k, v)]
+            out = swa.TiledSwaRope2D.apply(*t, *r, *WIN, 0.125)
+            res.append((out.detach(), *torch.autograd.grad(out, t, do)))
+    finally:
+        swa.set_rope_mode(prev)
+    assert all(torch.equal(a, b) for a, b in zip(*res))
