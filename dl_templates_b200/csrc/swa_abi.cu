@@ -180,6 +180,7 @@ int64_t swa_launch_count(void) { return g_launches.load(); }
 int swa_select_impl(const swa_geom_t* g, const swa_rope_t* rope, int32_t which) {
   if (int e = check_geom(g)) return e;
   if (int e = check_rope(g, rope)) return e;
+  if (which < 0 || which > 2) return fail(E_IMPL, "kernel %d: 0 forward, 1 dQ, 2 dK/dV", which);   // (an index into the plans kept)
   return resolve_impl(g, rope, nullptr, 0, which);
 }
 

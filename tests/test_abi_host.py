@@ -169,6 +169,13 @@ def test_misaligned_tables_keep_off_the_tensor_core_kernels():
         assert (_plan(g, r, 3)[0] == 0) and (_plan(g, r, 4)[0] == 0) == plain and (_plan(g, r, 5)[0] == 0) == plain
 
 
+def test_select_impl_refuses_kernels_that_do_not_exist():
+    g = _geom(t_height=16, t_width=16)
+    for which in (-1, 3, 5, 1000):
+        assert _lib.lib.swa_select_impl(C.byref(g), None, which) < 0
+        assert b"kernel" in _lib.lib.swa_last_error()
+
+
 def test_head_dims_the_tensor_core_kernels_take():
     """32, 64, 96, 128 where no streamed row is rotated (no RoPE, or the entries that take rotated copies); 64 and
     128 only for the kernels that rotate what they stream; anything else runs on the SIMT kernels."""
