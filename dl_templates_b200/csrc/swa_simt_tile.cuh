@@ -135,6 +135,62 @@ __device__ __forceinline__ void tile_copy16(float* dst, const float* src) {
 }
 __device__ __forceinline__ void tile_copy_wait() { asm volatile("cp.async.wait_all;" ::: "memory"); }
 
+// Whether any of a row's sums is an infinity or a NaN.
+template <int G>
+__device__ __forceinline__ bool tile_not_finite(const TileAcc<G>& acc, int e) {
+  uint64_t z = 0ull;
+#pragma unroll
+  for (int h = 0; h < G; ++h) z = ptx::f2_fma(acc[e][h][0], 0ull, ptx::f2_fma(acc[e][h][1], 0ull, z));
+  const float2 v = ptx::f2_unpack(z);
+  return !(v.x + v.y == 0.f);
+}
+
+// One row again, over the tokens of its own window only and straight from global memory.  A warp's 32 tokens hold some that a row
+// does not see; their weight is 0, which is nothing to a sum until such a token holds an infinity or a NaN (0 * inf).  A row
+// whose sums are not finite is therefore done anew, so that what it does not see cannot reach it, and what it does see
+// still does.  x1, x2: the resident row; m, l: as in the kernel (forward: l the whole sum).  Results: forward to `dst`; else
+// to x1 in shared memory (scaled, not yet rotated back), dV to `dst`.
+template <int KIND>
+__device__ __noinline__ void tile_row_again(const TileArgs& t, float* x1, const float* x2, float* dst, int rr, int cc, float m, float l) {
+  const Geom& g = t.g;
+  const int lane = threadIdx.x & 31, bh = blockIdx.y, bi = bh / g.H, hi = bh - bi * g.H, Wtok = g.tw * g.b, cell = cc / g.b;
+  const float *y1 = (const float*)t.y1.ptr + bi * t.y1.s0 + hi * t.y1.s1, *y2 = (const float*)t.y2.ptr + bi * t.y2.s0 + hi * t.y2.s1;
+  float acc[4] = {}, acc2[4] = {};
+  for (int r = max(0, rr - g.wr); r <= min(g.th - 1, rr + g.wr); ++r)
+    for (int c = max(0, cell - g.wc) * g.b; c < (min(g.tw - 1, cell + g.wc) + 1) * g.b; ++c) {
+      const int64_t n = (int64_t)r * Wtok + c;
+      const float *row1 = y1 + n * t.y1.s2, *row2 = y2 + n * t.y2.s2;
+      float s = 0.f, dp = 0.f;
+      for (int d = lane; d < g.dqk; d += 32) s = fmaf(x1[d], row1[d], s);
+      s = warp_sum(s);
+      float p, w;
+      if constexpr (KIND == 0) {
+        s *= g.scale_log2;
+        w = p = s == -INFINITY ? 0.f : exp2f(s - m);
+      } else {
+        for (int d = lane; d < g.dv; d += 32) dp = fmaf(x2[d], row2[d], dp);
+        dp = warp_sum(dp);
+        const float ls = KIND == 1 ? m : t.lse[(int64_t)bh * g.th * Wtok + n], de = KIND == 1 ? l : t.delta[(int64_t)bh * g.th * Wtok + n];
+        p = exp2f(fmaf(s, g.scale_log2, -ls));
+        w = p * (dp - de);
+      }
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const int d = lane + 32 * i;
+        if (d < (KIND == 0 ? g.dv : g.dqk)) acc[i] = fmaf(w, KIND == 0 ? row2[d] : row1[d], acc[i]);
+        if (KIND == 2 && d < g.dv) acc2[i] = fmaf(p, row2[d], acc2[i]);
+      }
+    }
+  __syncwarp();
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const int d = lane + 32 * i;
+    if (KIND == 0 && d < g.dv) dst[d] = acc[i] * (1.f / l);
+    if (KIND != 0 && d < g.dqk) x1[d] = acc[i] * g.sm_scale;
+    if (KIND == 2 && d < g.dv) dst[d] = acc2[i];
+  }
+}
+
 // KIND as in TileArgs; G1 / G2: 32-dim groups of the q-k / v tensors (dQ: only G1 is used, forward: only G2).
 template <int KIND, int G1, int G2>
 __global__ void __launch_bounds__(kTileThreads, 3) simt_tile_kernel(const __grid_constant__ TileArgs t) {
@@ -345,22 +401,45 @@ __global__ void __launch_bounds__(kTileThreads, 3) simt_tile_kernel(const __grid
   }
   if (!on) return;
 
+  // rows of this warp whose sums are not finite (bit e of the lanes' byte): done again (tile_row_again)
+  uint32_t again[2];
+#pragma unroll
+  for (int e = 0; e < 2; ++e) {
+    bool bad = tile_not_finite<GA>(acc, e);
+    if constexpr (KIND == 2) bad |= tile_not_finite<GB>(acc2, e);
+    again[e] = __ballot_sync(0xffffffffu, bad && e < n_out);
+    if constexpr (KIND == 0) {
+#pragma unroll
+      for (int o = 4; o > 0; o >>= 1) l[e] += __shfl_xor_sync(0xffffffffu, l[e], o);
+    }
+  }
+  auto redo = [&](int e) { return (again[e] >> (8 * a) & 255u) != 0; };
+  if (again[0] | again[1]) {
+#pragma unroll 1
+    for (int j = 0; j < kTileQ; ++j) {
+      const float mj = __shfl_sync(0xffffffffu, j & 1 ? m[1] : m[0], 4 * (j & 6)), lj = __shfl_sync(0xffffffffu, j & 1 ? l[1] : l[0], 4 * (j & 6));
+      if (!((j & 1 ? again[1] : again[0]) >> (4 * (j & 6)) & 255u)) continue;
+      const int rr = wr0 + (j >> 2), cc = wc0 + (j & 3), row = warp * kTileQ + j;
+      const View4& o = KIND == 0 ? t.o1 : t.o2;
+      tile_row_again<KIND>(t, x1 + row * s1, x2 + row * s2, KIND == 1 ? nullptr : slice(o) + ((int64_t)rr * Wtok + cc) * o.s2, rr, cc, mj, lj);
+    }
+    __syncwarp();
+  }
+
   // out: accumulators scaled, rotated back where asked, rows of this warp
   if constexpr (KIND == 0) {
     float* dst = slice(t.o1) + ((int64_t)my_r * Wtok + my_c) * t.o1.s2;
 #pragma unroll
     for (int e = 0; e < 2; ++e) {
-      float lt = l[e];
-#pragma unroll
-      for (int o = 4; o > 0; o >>= 1) lt += __shfl_xor_sync(0xffffffffu, lt, o);
       if (e >= n_out) continue;
-      tile_store<GA>(acc, e, 1.f / lt, dst + e * t.o1.s2, b4, d2);
-      if (b == 0) t.lse_out[row_base + e] = m[e] + log2f(lt);
+      if (!redo(e)) tile_store<GA>(acc, e, 1.f / l[e], dst + e * t.o1.s2, b4, d2);
+      if (b == 0) t.lse_out[row_base + e] = m[e] + log2f(l[e]);
     }
   } else {
     __syncwarp();
 #pragma unroll
-    for (int e = 0; e < 2; ++e) tile_store<GA>(acc, e, g.sm_scale, mx1 + e * s1, b4, d1);   // the resident rows are done with: they take the result
+    for (int e = 0; e < 2; ++e)
+      if (!redo(e)) tile_store<GA>(acc, e, g.sm_scale, mx1 + e * s1, b4, d1);   // the resident rows are done with: they take the result
     __syncwarp();
     float* dst = slice(t.o1);
 #pragma unroll 1
@@ -376,7 +455,7 @@ __global__ void __launch_bounds__(kTileThreads, 3) simt_tile_kernel(const __grid
       float* dst2 = slice(t.o2) + ((int64_t)my_r * Wtok + my_c) * t.o2.s2;
 #pragma unroll
       for (int e = 0; e < 2; ++e)
-        if (e < n_out) tile_store<GB>(acc2, e, 1.f, dst2 + e * t.o2.s2, b4, d2);
+        if (e < n_out && !redo(e)) tile_store<GB>(acc2, e, 1.f, dst2 + e * t.o2.s2, b4, d2);
     }
   }
 }

@@ -98,3 +98,35 @@ def test_windows_of_any_size_beyond_the_grid(wr, wc, dtype):
     swa.check_status()
     for a, c in zip(got, want):
         assert orc.max_abs(a.float(), c.float()) < (2e-6 if dtype == torch.float32 else 2e-2)
+
+
+@pytest.mark.parametrize("what", ["q", "k", "v", "do"])
+@pytest.mark.parametrize("bad", [float("inf"), float("nan")])
+@pytest.mark.parametrize("th,tw,b,wr,wc,dqk,dv,R", [(9, 11, 1, 2, 1, 64, 64, 8), (6, 5, 4, 1, 1, 32, 96, 0), (14, 30, 1, 3, 3, 100, 36, 16)])
+def test_fp32_rows_are_not_touched_by_what_they_do_not_see(th, tw, b, wr, wc, dqk, dv, R, bad, what):
+    """One token with an infinity or a NaN: the tiled kernels spoil exactly the rows that the one-warp-per-token kernels, which look at
+    nothing but a row's own window, spoil; all others keep their values.  (A last stride of 2 takes those kernels.)"""
+    N = th * tw * b
+    q, k, v, do = (t.to(DEV) for t in orc.seeded_inputs(1, 2, N, dqk, dv, torch.float32, th))
+    {"q": q, "k": k, "v": v, "do": do}[what][0, 1, (th // 2 * tw + tw // 2) * b, 5] = bad
+    rope = tuple(t.to(DEV) for t in (orc.encode_idx(th, tw * b), orc.make_cs_table(R, th), orc.make_cs_table(R, tw * b))) if R else None
+    win, sc = (b, th, tw, wr, wc), dqk ** -0.5
+    wide = lambda t: torch.empty(*t.shape[:3], 2 * t.shape[3], device=DEV)[..., ::2].copy_(t)
+    res = []
+    for f in (lambda t: t, wide):
+        if R:
+            o, lse, qr, kr = swa.swa_forward_rot(f(q), k, f(v), rope, *win, sc)
+            res.append((o, lse, *swa.swa_backward_rot(f(qr), kr, f(v), o, lse, do, rope, *win, sc)))
+        else:
+            o, lse = swa.swa_forward(f(q), k, f(v), None, *win, sc)
+            res.append((o, lse, *swa.swa_backward(f(q), k, f(v), o, lse, do, None, *win, sc)))
+    spoiled = 0
+    for a, c, n in zip(*res, ("o", "lse", "dq", "dk", "dv")):
+        ok, ref = torch.isfinite(a), torch.isfinite(c)
+        # (a score of -inf has weight 0 here; where it is the first of a window, the running maximum of the one-warp kernels is -inf too
+        # and makes the row a NaN: they may then spoil more)
+        assert torch.equal(ok | ref, ok) if bad == float("inf") and what in "qk" else torch.equal(ok, ref), n
+        spoiled += int((~ok).any(-1).sum())
+        ok = ok & ref
+        assert (a[ok] - c[ok]).abs().max().item() < 1e-5, n
+    assert spoiled > 0
