@@ -8,6 +8,7 @@
 #include <Python.h>
 
 #include <ATen/ATen.h>
+#include <ATen/TracerMode.h>
 #include <ATen/cuda/CUDAContext.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <torch/csrc/Exceptions.h>
@@ -468,6 +469,21 @@ bool wants_grad(std::initializer_list<const Tensor*> ts) {
   return false;
 }
 
+// Whether the native node records all there is to record.  Forward-mode tangents, functorch's transforms, jit tracing, tensors
+// with a Python dispatch of their own and tables that ask for gradients are for the autograd.Function of the same name, which
+// refuses or handles them as torch does for every such function; the entry points below then answer None.
+bool plain_call(std::initializer_list<const Tensor*> inputs, const Rope& rope) {
+  if (c10::impl::tls_is_dispatch_key_included(c10::DispatchKey::FuncTorchDynamicLayerFrontMode) || at::tracer::impl::is_dispatch_enabled())
+    return false;
+  auto plain = [](const Tensor& t) { return !t._fw_grad(0).defined() && !t.key_set().has(c10::DispatchKey::Python); };
+  for (const Tensor* t : inputs)
+    if (!plain(*t)) return false;
+  if (rope.on())
+    for (const Tensor* t : {&rope.row, &rope.col})
+      if (!plain(*t) || wants_grad({t})) return false;
+  return true;
+}
+
 std::shared_ptr<SwaNode> new_node(const Rope& rope, const Win& w, int mode) {
   std::shared_ptr<SwaNode> n(new SwaNode(), torch::autograd::deleteNode);
   n->win = w;
@@ -635,13 +651,14 @@ PyObject* pack(std::initializer_list<Tensor> ts) {
   return t;
 }
 
-// apply(q, k, v, b_size, t_height, t_width, row_size, col_size, sm_scale)
+// apply(q, k, v, b_size, t_height, t_width, row_size, col_size, sm_scale); None: not a plain_call
 PyObject* py_tiled_swa(PyObject*, PyObject* const* args, Py_ssize_t n) {
   return guarded([&]() -> PyObject* {
     Args a{args, n};
     const Tensor &q = a.tensor(), &k = a.tensor(), &v = a.tensor();
     const Win w = a.win();
     a.done();
+    if (!plain_call({&q, &k, &v}, Rope())) Py_RETURN_NONE;
     return THPVariable_Wrap(apply_swa(q, k, v, Rope(), w));
   });
 }
@@ -653,6 +670,7 @@ PyObject* py_tiled_swa_rope2d(PyObject*, PyObject* const* args, Py_ssize_t n) {
     const Rope r = a.rope();
     const Win w = a.win();
     a.done();
+    if (!plain_call({&q, &k, &v}, r)) Py_RETURN_NONE;
     return THPVariable_Wrap(apply_swa(q, k, v, r, w));
   });
 }
@@ -664,6 +682,7 @@ PyObject* py_tiled_swa_packed(PyObject*, PyObject* const* args, Py_ssize_t n) {
     const Rope r = a.rope();
     const Win w = a.win();
     a.done();
+    if (!plain_call({&qkv}, r)) Py_RETURN_NONE;
     return THPVariable_Wrap(apply_packed(qkv, r, w));
   });
 }
@@ -759,7 +778,7 @@ PyObject* py_rope2d_heads_inplace(PyObject*, PyObject* const* args, Py_ssize_t n
     const Tensor& x = a.tensor();
     const Rope r = a.rope();
     a.done();
-    if (x.dim() != 4 || wants_grad({&x})) Py_RETURN_NONE;
+    if (x.dim() != 4 || wants_grad({&x}) || !plain_call({&x}, r)) Py_RETURN_NONE;
     const Tensor flat = flat3(x);
     rope_inplace(flat, r, false);
     flat.unsafeGetTensorImpl()->bump_version();
@@ -779,6 +798,18 @@ PyObject* py_padded_dims(PyObject*, PyObject* const* args, Py_ssize_t n) {
     const auto p = padded_dims(q, d_v, &r, w, impl);
     if (!p[0]) Py_RETURN_NONE;
     return Py_BuildValue("(LL)", (long long)p[0], (long long)p[1]);
+  });
+}
+// rope_mode(q, d_v, idx, row_cs, col_cs, window..., sm_scale) -> code of the mode a call runs in
+PyObject* py_rope_mode(PyObject*, PyObject* const* args, Py_ssize_t n) {
+  return guarded([&]() -> PyObject* {
+    Args a{args, n};
+    const Tensor& q = a.tensor();
+    const int32_t d_v = a.i32();
+    const Rope r = a.rope();
+    const Win w = a.win();
+    a.done();
+    return PyLong_FromLong(mode_for(q, d_v, r, w));
   });
 }
 PyObject* py_set_rope_mode(PyObject*, PyObject* const* args, Py_ssize_t n) {
@@ -835,6 +866,7 @@ PyMethodDef g_methods[] = {SWA_DEF("tiled_swa", py_tiled_swa),
                            SWA_DEF("rope2d_to", py_rope2d_to),
                            SWA_DEF("rope2d_heads_", py_rope2d_heads_inplace),
                            SWA_DEF("padded_dims", py_padded_dims),
+                           SWA_DEF("rope_mode", py_rope_mode),
                            SWA_DEF("set_rope_mode", py_set_rope_mode),
                            SWA_DEF("status_words", py_status_words),
                            SWA_DEF("check_status", py_check_status),

@@ -32,6 +32,7 @@ import torch
 
 from . import _lib
 from ._lib import native as _native
+from .fused_rope2d import rope2d_apply_, rope2d_apply_to
 
 
 def _status(device: torch.device) -> torch.Tensor:
@@ -149,11 +150,34 @@ def tiled_swa_fwd(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, b_size: int
     return swa_forward(q, k, v, None, b_size, t_height, t_width, row_size, col_size, sm_scale)[0]
 
 
-class TiledSwa:
-    """``TiledSwa.apply(q, k, v, b_size, t_height, t_width, row_size, col_size, sm_scale)``
-    -- src/tiled_swa.py:602-689.  Differentiable in q, k and v (a native autograd node)."""
+class _NativeFunction(torch.autograd.Function):
+    """An autograd.Function whose ``apply`` runs natively (argument checks, launches and the autograd node in C++).  ``forward`` and
+    ``backward`` below are the general path: what carries forward-mode tangents, runs under functorch's transforms, is
+    being traced or has a Python dispatch of its own, where the native entry answers ``None``."""
 
-    apply = staticmethod(_native.tiled_swa)
+    @classmethod
+    def apply(cls, *args):
+        o = cls._native(*args)
+        return super().apply(*args) if o is None else o
+
+
+class TiledSwa(_NativeFunction):
+    """``TiledSwa.apply(q, k, v, b_size, t_height, t_width, row_size, col_size, sm_scale)``
+    -- src/tiled_swa.py:602-689."""
+
+    _native = _native.tiled_swa
+
+    @staticmethod
+    def forward(ctx, q, k, v, *win):
+        o, lse = swa_forward(q, k, v, None, *win)
+        ctx.save_for_backward(q, k, v, lse, o)
+        ctx.win = win
+        return o
+
+    @staticmethod
+    def backward(ctx, do):
+        q, k, v, lse, o = ctx.saved_tensors
+        return (*swa_backward(q, k, v, o, lse, do, None, *ctx.win), *(None,) * 6)
 
 
 _rope_mode = "handoff"
@@ -187,18 +211,11 @@ set_rope_mode(os.environ.get("SWA_ROPE_MODE", "handoff"))
 
 def _mode_for(q, v, rope, win) -> str:
     """The mode a call runs in: 'none' without RoPE; head dims that only reach the tensor-core kernels through
-    zero padding take the fused path (the padding wrapper lives there)."""
-    if rope is None:
-        return "none"
-    if _rope_mode == "handoff":
-        g = _geom(q, v, *win, "auto")
-        native = q.dtype == torch.float32 or _lib.lib.swa_step_select(C.byref(g), _ref(_lib.make_rope(*rope))) == _lib.IMPL_TC
-        if not native and padded_head_dims(q, v, rope, *win) is not None:
-            return "fused"
-    return _rope_mode
+    zero padding take the fused path (the padding lives there)."""
+    return _ROPE_MODES[_native.rope_mode(q, v.shape[-1], *(rope or _NO_ROPE), *win)]
 
 
-class TiledSwaRope2D:
+class TiledSwaRope2D(_NativeFunction):
     """RoPE-2D and the attention as one differentiable function:
     ``TiledSwaRope2D.apply(q, k, v, idx, row_cs_buffer, col_cs_buffer, b_size, t_height, t_width, row_size, col_size,
     sm_scale)``.
@@ -210,10 +227,41 @@ class TiledSwaRope2D:
     ``idx`` may be ``None`` (no rotation).
     """
 
-    apply = staticmethod(_native.tiled_swa_rope2d)
+    _native = _native.tiled_swa_rope2d
+
+    @staticmethod
+    def forward(ctx, q, k, v, idx, row_cs_buffer, col_cs_buffer, *win):
+        rope = None if idx is None else (idx, row_cs_buffer, col_cs_buffer)
+        if rope is not None:
+            assert idx.shape[0] == q.shape[2] and row_cs_buffer.shape[1] == col_cs_buffer.shape[1]
+        ctx.mode, ctx.win = _mode_for(q, v, rope, win), win
+        if ctx.mode == "handoff":            # q, k are the rotated copies from here on: they are what backward needs
+            o, lse, q, k = swa_forward_rot(q, k, v, rope, *win)
+        elif ctx.mode == "prerotate":
+            q, k = (rope2d_apply_to(t.reshape(-1, *t.shape[2:]), *rope).view(t.shape) for t in (q, k))
+            o, lse = swa_forward(q, k, v, None, *win)
+        else:
+            o, lse = swa_forward(q, k, v, rope, *win)
+        ctx.save_for_backward(q, k, v, lse, o, *(rope or ()))
+        return o
+
+    @staticmethod
+    def backward(ctx, do):
+        q, k, v, lse, o, *rope = ctx.saved_tensors
+        if ctx.mode == "handoff":
+            grads = swa_backward_rot(q, k, v, o, lse, do, rope, *ctx.win)
+        elif ctx.mode == "prerotate":
+            dq, dk, dv = swa_backward(q, k, v, o, lse, do, None, *ctx.win)
+            dq, dk = dq.contiguous(), dk.contiguous()
+            for t in (dq, dk):
+                rope2d_apply_(t.view(-1, *t.shape[2:]), *rope, inverse=True)
+            grads = dq, dk, dv
+        else:
+            grads = swa_backward(q, k, v, o, lse, do, tuple(rope) or None, *ctx.win)
+        return (*grads, *(None,) * 9)
 
 
-class TiledSwaPackedQKV:
+class TiledSwaPackedQKV(_NativeFunction):
     """The op between a packed QKV projection and the output projection, without the
     permute / contiguous copies either side of it.
 
@@ -227,4 +275,33 @@ class TiledSwaPackedQKV:
     Same mathematics as ``TiledSwaRope2D`` on the permuted views.
     """
 
-    apply = staticmethod(_native.tiled_swa_packed)
+    _native = _native.tiled_swa_packed
+
+    @staticmethod
+    def forward(ctx, qkv, idx, row_cs_buffer, col_cs_buffer, *win):
+        if qkv.dim() != 5 or qkv.shape[2] != 3:
+            raise ValueError("expected qkv [B, N, 3, H, d]")
+        B, N, _, H, d = qkv.shape
+        q, k, v = (qkv[:, :, i].permute(0, 2, 1, 3) for i in range(3))
+        rope = None if idx is None else (idx, row_cs_buffer, col_cs_buffer)
+        ctx.handoff, ctx.win = _mode_for(q, v, rope, win) == "handoff", win
+        o = torch.empty((B, N, H, d), dtype=qkv.dtype, device=qkv.device)
+        _, lse, *rotated = (swa_forward_rot if ctx.handoff else swa_forward)(q, k, v, rope, *win, out=o.permute(0, 2, 1, 3))
+        ctx.save_for_backward(qkv, lse, o, *(rope or ()), *rotated)      # (v is read from the packed tensor again)
+        return o.view(B, N, H * d)
+
+    @staticmethod
+    def backward(ctx, do):
+        qkv, lse, o, *rest = ctx.saved_tensors
+        B, N, _, H, d = qkv.shape
+        if do.stride(-1) != 1 or do.stride(1) % 8 or do.stride(0) % 8 or do.data_ptr() % 16:
+            do = do.contiguous()
+        q, k, v = (qkv[:, :, i].permute(0, 2, 1, 3) for i in range(3))
+        dqkv = torch.empty((B, N, 3, H, d), dtype=qkv.dtype, device=qkv.device)
+        outs = tuple(dqkv[:, :, i].permute(0, 2, 1, 3) for i in range(3))
+        saved = (o.permute(0, 2, 1, 3), lse, do.view(B, N, H, d).permute(0, 2, 1, 3))
+        if ctx.handoff:
+            swa_backward_rot(*rest[3:], v, *saved, rest[:3], *ctx.win, out=outs)
+        else:
+            swa_backward(q, k, v, *saved, tuple(rest) or None, *ctx.win, out=outs)
+        return (dqkv, *(None,) * 9)
