@@ -570,7 +570,7 @@ struct Args {
     }
     return a[at++];
   }
-  const Tensor& tensor() {
+  Tensor tensor() {
     PyObject* o = next();
     if (!THPVariable_Check(o)) {
       PyErr_Format(PyExc_TypeError, "argument %zd must be a tensor, not %s", at, Py_TYPE(o)->tp_name);
@@ -642,6 +642,14 @@ struct NoGil {
   PyThreadState* s = PyEval_SaveThread();
   ~NoGil() { PyEval_RestoreThread(s); }
 };
+// Allocations and launches run without the interpreter's lock: a launch waits for room when the stream's queue is full, and
+// other Python threads -- one of which the GPU may be waiting for -- have to run meanwhile.  The tensors a call works on are held by
+// copies of its own (Args::tensor), whatever another thread does to its arguments.
+template <typename F>
+auto without_gil(F&& f) {
+  const NoGil nogil;
+  return f();
+}
 
 PyObject* pack(std::initializer_list<Tensor> ts) {
   PyObject* t = PyTuple_New((Py_ssize_t)ts.size());
@@ -655,49 +663,49 @@ PyObject* pack(std::initializer_list<Tensor> ts) {
 PyObject* py_tiled_swa(PyObject*, PyObject* const* args, Py_ssize_t n) {
   return guarded([&]() -> PyObject* {
     Args a{args, n};
-    const Tensor &q = a.tensor(), &k = a.tensor(), &v = a.tensor();
+    const Tensor q = a.tensor(), k = a.tensor(), v = a.tensor();
     const Win w = a.win();
     a.done();
     if (!plain_call({&q, &k, &v}, Rope())) Py_RETURN_NONE;
-    return THPVariable_Wrap(apply_swa(q, k, v, Rope(), w));
+    return THPVariable_Wrap(without_gil([&] { return apply_swa(q, k, v, Rope(), w); }));
   });
 }
 // apply(q, k, v, idx, row_cs, col_cs, b_size, t_height, t_width, row_size, col_size, sm_scale)
 PyObject* py_tiled_swa_rope2d(PyObject*, PyObject* const* args, Py_ssize_t n) {
   return guarded([&]() -> PyObject* {
     Args a{args, n};
-    const Tensor &q = a.tensor(), &k = a.tensor(), &v = a.tensor();
+    const Tensor q = a.tensor(), k = a.tensor(), v = a.tensor();
     const Rope r = a.rope();
     const Win w = a.win();
     a.done();
     if (!plain_call({&q, &k, &v}, r)) Py_RETURN_NONE;
-    return THPVariable_Wrap(apply_swa(q, k, v, r, w));
+    return THPVariable_Wrap(without_gil([&] { return apply_swa(q, k, v, r, w); }));
   });
 }
 // apply(qkv, idx, row_cs, col_cs, b_size, t_height, t_width, row_size, col_size, sm_scale)
 PyObject* py_tiled_swa_packed(PyObject*, PyObject* const* args, Py_ssize_t n) {
   return guarded([&]() -> PyObject* {
     Args a{args, n};
-    const Tensor& qkv = a.tensor();
+    const Tensor qkv = a.tensor();
     const Rope r = a.rope();
     const Win w = a.win();
     a.done();
     if (!plain_call({&qkv}, r)) Py_RETURN_NONE;
-    return THPVariable_Wrap(apply_packed(qkv, r, w));
+    return THPVariable_Wrap(without_gil([&] { return apply_packed(qkv, r, w); }));
   });
 }
 // forward(q, k, v, idx, row_cs, col_cs, window..., sm_scale, impl, out) -> (o, lse)
 PyObject* py_forward(PyObject*, PyObject* const* args, Py_ssize_t n) {
   return guarded([&]() -> PyObject* {
     Args a{args, n};
-    const Tensor &q = a.tensor(), &k = a.tensor(), &v = a.tensor();
+    const Tensor q = a.tensor(), k = a.tensor(), v = a.tensor();
     const Rope r = a.rope();
     const Win w = a.win();
     const int32_t impl = a.i32();
     const Tensor out = a.maybe_tensor();
     a.done();
     const at::AutoGradMode no_grad(false);
-    const Fwd f = forward(q, k, v, r, w, impl, out);
+    const Fwd f = without_gil([&] { return forward(q, k, v, r, w, impl, out); });
     return pack({f.o, f.lse});
   });
 }
@@ -705,14 +713,14 @@ PyObject* py_forward(PyObject*, PyObject* const* args, Py_ssize_t n) {
 PyObject* py_forward_rot(PyObject*, PyObject* const* args, Py_ssize_t n) {
   return guarded([&]() -> PyObject* {
     Args a{args, n};
-    const Tensor &q = a.tensor(), &k = a.tensor(), &v = a.tensor();
+    const Tensor q = a.tensor(), k = a.tensor(), v = a.tensor();
     const Rope r = a.rope();
     const Win w = a.win();
     const int32_t impl = a.i32();
     const Tensor out = a.maybe_tensor();
     a.done();
     const at::AutoGradMode no_grad(false);
-    const Fwd f = forward_rot(q, k, v, r, w, impl, out);
+    const Fwd f = without_gil([&] { return forward_rot(q, k, v, r, w, impl, out); });
     return pack({f.o, f.lse, f.q_rot, f.k_rot});
   });
 }
@@ -720,14 +728,14 @@ PyObject* py_forward_rot(PyObject*, PyObject* const* args, Py_ssize_t n) {
 PyObject* py_backward(PyObject*, PyObject* const* args, Py_ssize_t n) {
   return guarded([&]() -> PyObject* {
     Args a{args, n};
-    const Tensor &q = a.tensor(), &k = a.tensor(), &v = a.tensor(), &o = a.tensor(), &lse = a.tensor(), &d_o = a.tensor();
+    const Tensor q = a.tensor(), k = a.tensor(), v = a.tensor(), o = a.tensor(), lse = a.tensor(), d_o = a.tensor();
     const Rope r = a.rope();
     const Win w = a.win();
     const int32_t impl = a.i32(), rotated = a.i32();
     const Grads out{a.maybe_tensor(), a.maybe_tensor(), a.maybe_tensor()};
     a.done();
     const at::AutoGradMode no_grad(false);
-    const Grads g = backward(q, k, v, o, lse, d_o, r, rotated != 0, w, impl, out);
+    const Grads g = without_gil([&] { return backward(q, k, v, o, lse, d_o, r, rotated != 0, w, impl, out); });
     return pack({g.dq, g.dk, g.dv});
   });
 }
@@ -735,7 +743,7 @@ PyObject* py_backward(PyObject*, PyObject* const* args, Py_ssize_t n) {
 PyObject* py_check_backward(PyObject*, PyObject* const* args, Py_ssize_t n) {
   return guarded([&]() -> PyObject* {
     Args a{args, n};
-    const Tensor &q = a.tensor(), &k = a.tensor(), &v = a.tensor(), &o = a.tensor(), &lse = a.tensor(), &d_o = a.tensor();
+    const Tensor q = a.tensor(), k = a.tensor(), v = a.tensor(), o = a.tensor(), lse = a.tensor(), d_o = a.tensor();
     const Rope r = a.rope();
     const Win w = a.win();
     a.done();
@@ -749,11 +757,11 @@ PyObject* py_check_backward(PyObject*, PyObject* const* args, Py_ssize_t n) {
 PyObject* py_rope2d_inplace(PyObject*, PyObject* const* args, Py_ssize_t n) {
   return guarded([&]() -> PyObject* {
     Args a{args, n};
-    const Tensor& x = a.tensor();
+    const Tensor x = a.tensor();
     const Rope r = a.rope();
     const bool inverse = a.i32() != 0;
     a.done();
-    rope_inplace(x, r, inverse);
+    without_gil([&] { rope_inplace(x, r, inverse); });
     Py_INCREF(args[0]);
     return args[0];
   });
@@ -762,12 +770,12 @@ PyObject* py_rope2d_inplace(PyObject*, PyObject* const* args, Py_ssize_t n) {
 PyObject* py_rope2d_to(PyObject*, PyObject* const* args, Py_ssize_t n) {
   return guarded([&]() -> PyObject* {
     Args a{args, n};
-    const Tensor& x = a.tensor();
+    const Tensor x = a.tensor();
     const Rope r = a.rope();
     const bool inverse = a.i32() != 0;
     a.done();
     const at::AutoGradMode no_grad(false);
-    return THPVariable_Wrap(rope_to(x, r, inverse));
+    return THPVariable_Wrap(without_gil([&] { return rope_to(x, r, inverse); }));
   });
 }
 // rope2d_heads_(x [B,H,N,C], idx, row_cs, col_cs) -> view of x (of a copy when x cannot be flattened), rotated in place.
@@ -775,21 +783,23 @@ PyObject* py_rope2d_to(PyObject*, PyObject* const* args, Py_ssize_t n) {
 PyObject* py_rope2d_heads_inplace(PyObject*, PyObject* const* args, Py_ssize_t n) {
   return guarded([&]() -> PyObject* {
     Args a{args, n};
-    const Tensor& x = a.tensor();
+    const Tensor x = a.tensor();
     const Rope r = a.rope();
     a.done();
     if (x.dim() != 4 || wants_grad({&x}) || !plain_call({&x}, r)) Py_RETURN_NONE;
-    const Tensor flat = flat3(x);
-    rope_inplace(flat, r, false);
-    flat.unsafeGetTensorImpl()->bump_version();
-    return THPVariable_Wrap(flat.view(x.sizes()));
+    return THPVariable_Wrap(without_gil([&] {
+      const Tensor flat = flat3(x);
+      rope_inplace(flat, r, false);
+      flat.unsafeGetTensorImpl()->bump_version();
+      return flat.view(x.sizes());
+    }));
   });
 }
 // padded_dims(q, d_v, idx, row_cs, col_cs, window..., sm_scale, impl) -> (d_qk', d_v') or None
 PyObject* py_padded_dims(PyObject*, PyObject* const* args, Py_ssize_t n) {
   return guarded([&]() -> PyObject* {
     Args a{args, n};
-    const Tensor& q = a.tensor();
+    const Tensor q = a.tensor();
     const int32_t d_v = a.i32();
     const Rope r = a.rope();
     const Win w = a.win();
@@ -804,7 +814,7 @@ PyObject* py_padded_dims(PyObject*, PyObject* const* args, Py_ssize_t n) {
 PyObject* py_rope_mode(PyObject*, PyObject* const* args, Py_ssize_t n) {
   return guarded([&]() -> PyObject* {
     Args a{args, n};
-    const Tensor& q = a.tensor();
+    const Tensor q = a.tensor();
     const int32_t d_v = a.i32();
     const Rope r = a.rope();
     const Win w = a.win();
