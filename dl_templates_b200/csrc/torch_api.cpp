@@ -93,8 +93,8 @@ void poll_status() {
 }
 
 void debug_sync() {
-  static const bool on = [] { const char* e = std::getenv("SWA_DEBUG_SYNC"); return e && *e; }();
-  if (!on) return;
+  const char* on = std::getenv("SWA_DEBUG_SYNC");      // read on every call: a debugger's switch is set when it is wanted
+  if (!on || !*on) return;
   c10::cuda::device_synchronize();
   poll_status();
 }
