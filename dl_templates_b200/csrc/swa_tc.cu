@@ -245,39 +245,84 @@ bool strip_slides(const swa_geom_t* g, int R4, int KR) {
 }
 
 // Chunk height in quarters.  Sliding strips: the tallest chunk has the fewest blocks per row (2 wr rows of halo are met
-// once per chunk), short ones spread a small problem over all SMs; the slowest SM's blocks decide.  The height is a
-// multiple of the block height, so that no row's blocks depend on it.
+// once per chunk), short ones spread a small problem over all SMs; the slowest SM's blocks decide, the taller of two equals.  The
+// height is a multiple of the block height, so that no row's blocks depend on it.
+// A call of a batch size not met before pays for this (1 to 60 us for three plans up to 512 x 512; walking every height's items
+// took 14 ms on a grid 4096 rows high): heights are taken in the order of a bound -- their mean load, their largest item -- and
+// the load of every CTA is put together only for those whose bound is not beyond the best load found.
 void choose_chunk(const swa_geom_t* g, Plan* pl) {
   const int quarters = (g->t_height + pl->R4 - 1) / pl->R4;
   const int64_t strips = (int64_t)pl->n_tiles_x * g->B * g->H;
   if (!strip_slides(g, pl->R4, pl->KR)) {
     pl->nq = 4;
   } else {
+    struct Height {
+      double bound;
+      int nq, lo, hi;                                        // chunks [lo, hi) meet their whole halo inside the grid: the same blocks
+      int64_t mid;
+      bool exact;
+      bool operator<(const Height& o) const { return bound < o.bound || (bound == o.bound && nq > o.nq); }
+    };
     const int sms = sm_count();
     int unit = 1;
     while (unit * pl->R4 % pl->KR) ++unit;
     const int most = std::max(1, 2048 / pl->R4);            // chunk rows the kernels' div_kr covers
-    double best = -1.;
+    auto cost = [&](int nq, int c) { return (int64_t)strip_blocks(g, *pl, c * nq * pl->R4, nq) + 2; };
+    std::vector<Height> heights;
     for (int nq = unit; ; nq += unit) {
       const bool whole = nq >= quarters;
-      if (nq > most && !(whole && quarters <= most)) break;
-      const int chunks = (quarters + nq - 1) / nq;
+      if (nq > most && !(whole && quarters <= most) && nq > unit) break;
+      const int chunks = (quarters + nq - 1) / nq, rows = nq * pl->R4;
+      Height h;
+      h.nq = nq;
+      h.lo = std::min(chunks, (g->row_size + rows - 1) / rows);
+      h.hi = std::max(h.lo, (g->t_height - g->row_size) / rows);
+      h.mid = h.hi > h.lo ? cost(nq, h.lo) : 0;
+      int64_t total = (h.hi - h.lo) * h.mid, largest = h.mid;
+      for (int c = 0; c < chunks; ++c) {
+        if (c == h.lo) c = h.hi;
+        if (c >= chunks) break;
+        const int64_t x = cost(nq, c);
+        total += x;
+        largest = std::max(largest, x);
+      }
       const int64_t items = strips * chunks;
-      double load;
-      if (items <= 8 * sms) {                                // the items as the CTAs walk them
-        std::vector<long> cta(sms, 0);
-        for (int64_t i = 0; i < items; ++i) cta[i % sms] += strip_blocks(g, *pl, (int)(i / pl->n_tiles_x % chunks) * nq * pl->R4, nq) + 2;
-        load = (double)*std::max_element(cta.begin(), cta.end());
-      } else {
-        double total = 0.;
-        for (int c = 0; c < chunks; ++c) total += strip_blocks(g, *pl, c * nq * pl->R4, nq) + 2;
-        load = total * strips / sms + 0.5 * strip_blocks(g, *pl, 0, nq);
-      }
-      if (best < 0. || load <= best) {
-        best = load;
-        pl->nq = nq;
-      }
+      h.exact = items <= sms || items > 8 * sms;
+      h.bound = items > 8 * sms ? (double)total * strips / sms + 0.5 * strip_blocks(g, *pl, 0, nq)
+                                : (double)std::max(largest, items <= sms ? 0 : (total * strips + sms - 1) / sms);
+      heights.push_back(h);
       if (whole) break;
+    }
+    std::sort(heights.begin(), heights.end());
+    double best = -1.;
+    std::vector<int64_t> cta(sms);
+    for (const Height& h : heights) {
+      if (best >= 0. && (h.bound > best || (h.bound == best && h.nq < pl->nq))) {
+        if (h.bound > best) break;
+        continue;
+      }
+      double load = h.bound;
+      if (!h.exact) {
+        const int chunks = (quarters + h.nq - 1) / h.nq, items = (int)(strips * chunks), each = items / sms, more = items % sms;
+        for (int i = 0; i < sms; ++i) cta[i] = (each + (i < more ? 1 : 0)) * h.mid;
+        for (int c = 0; c < chunks; ++c) {                     // what the chunks at the edges have less
+          if (c == h.lo) c = h.hi;
+          if (c >= chunks) break;
+          const int64_t x = cost(h.nq, c) - h.mid;
+          for (int i = c * pl->n_tiles_x; i < items; i += chunks * pl->n_tiles_x) {
+            int at = i % sms;
+            for (int tx = 0; tx < pl->n_tiles_x; ++tx) {
+              cta[at] += x;
+              if (++at == sms) at = 0;
+            }
+          }
+        }
+        load = (double)*std::max_element(cta.begin(), cta.end());
+      }
+      if (best < 0. || load < best || (load == best && h.nq > pl->nq)) {
+        best = load;
+        pl->nq = h.nq;
+      }
     }
   }
   pl->n_tiles_y = (quarters + pl->nq - 1) / pl->nq;
@@ -394,9 +439,7 @@ bool make_strip_plan(const swa_geom_t* g, int which, Plan* out) {
       *out = pl;
     }
   }
-  if (best < 0.) return false;
-  choose_chunk(g, out);
-  return true;
+  return best >= 0.;
 }
 
 // Bytes of the cos/sin tables when they are small enough to be staged in shared memory, else 0.
@@ -441,10 +484,11 @@ static bool make_plan_tab(const swa_geom_t* g, const swa_rope_t* rope, int which
 using PlanKey = std::tuple<int, int, int, int, int, int, int, int, int, int, int, int, int>;
 std::map<PlanKey, std::pair<bool, Plan>> g_plan_cache;
 
-PlanKey plan_key(const swa_geom_t* g, const swa_rope_t* rope, int which, bool v2) {
+// `items`: batch x heads, which only the strips' chunk height depends on (0: everything else of a plan).
+PlanKey plan_key(const swa_geom_t* g, const swa_rope_t* rope, int which, bool v2, int items = 0) {
   const bool has = rope && rope->idx;
   return PlanKey(which + (v2 ? 3 : 0), g->t_height, g->t_width, g->b_size, g->row_size, g->col_size, g->d_qk, g->d_v,
-                 has ? rope->n_rdim : 0, has ? rope->max_h : 0, has ? rope->max_w : 0, g->dtype == SWA_BF16 ? 1 : 0, v2 ? g->B * g->H : 0);
+                 has ? rope->n_rdim : 0, has ? rope->max_h : 0, has ? rope->max_w : 0, g->dtype == SWA_BF16 ? 1 : 0, items);
 }
 bool cache_lookup(const PlanKey& k, bool* ok, Plan* out) {
   std::lock_guard<std::mutex> lock(g_plan_mu);
@@ -501,7 +545,7 @@ bool make_plan_prerot(const swa_geom_t* g, int which, Plan* out) {
   struct Last { PlanKey key; bool ok; Plan pl; const Knobs* epoch; };
   static thread_local Last last[3] = {};
   const Knobs* epoch = &knobs();
-  const PlanKey key = plan_key(g, nullptr, which, true);
+  const PlanKey key = plan_key(g, nullptr, which, true, g->B * g->H);
   Last& l = last[which];
   if (l.epoch == epoch && l.key == key) {
     if (l.ok) *out = l.pl;
@@ -510,7 +554,12 @@ bool make_plan_prerot(const swa_geom_t* g, int which, Plan* out) {
   bool ok = false;
   Plan pl{};
   if (!cache_lookup(key, &ok, &pl)) {
-    ok = make_strip_plan(g, which, &pl);
+    const PlanKey shape = plan_key(g, nullptr, which, true);
+    if (!cache_lookup(shape, &ok, &pl)) {
+      ok = make_strip_plan(g, which, &pl);
+      cache_store(shape, ok, pl);
+    }
+    if (ok) choose_chunk(g, &pl);
     cache_store(key, ok, pl);
   }
   l = Last{key, ok, pl, epoch};

@@ -249,6 +249,21 @@ def test_plans_are_cached_and_cheap():
     assert (t2 - t1) / 200 < 20e-6
 
 
+def test_a_new_batch_size_of_a_known_grid_is_planned_cheaply():
+    """Of a plan only the chunk height depends on the batch: another batch size of a grid met before does not repeat the search for
+    block shapes, nor walk every item of every height (host-only timing, generous bounds: 24 and 470 us measured)."""
+    import time
+    for grid, bound in (((128, 128), 300e-6), ((4096, 64), 3e-3)):
+        g = _geom(t_height=grid[0], t_width=grid[1], row_size=6, col_size=6, B=100)
+        _lib.lib.swa_refresh_env()
+        assert _lib.lib.swa_step_select(C.byref(g), None) == _lib.IMPL_TC
+        t0 = time.perf_counter()
+        for B in range(1, 41):
+            g.B = B
+            assert _lib.lib.swa_step_select(C.byref(g), None) == _lib.IMPL_TC
+        assert (time.perf_counter() - t0) / 40 < bound, grid
+
+
 def test_broadcast_strides_fall_back_to_simt():
     """A 16-bit tensor broadcast over batch or heads (stride 0) cannot be described by a tensor map: AUTO demotes the
     call to the SIMT kernels instead of failing in the map encoder; a forced tensor-core request is rejected."""
