@@ -36,8 +36,8 @@ class Rope(C.Structure):
 
 
 EXPORTS = ("swa_fwd", "swa_bwd_delta", "swa_bwd_dq", "swa_bwd_dkdv", "swa_fwd_rot", "swa_bwd_dq_rot", "swa_bwd_dkdv_rot",
-           "swa_bwd_noalloc", "swa_step_select", "swa_step_fwd", "swa_step_bwd", "rope2d_apply",
-           "rope2d_apply_to", "swa_select_impl", "swa_describe_plan", "swa_refresh_env", "swa_launch_count", "swa_last_error", "swa_version")
+           "swa_bwd_noalloc", "swa_step_select", "swa_step_select_impl", "swa_step_describe_plan", "swa_step_fwd", "swa_step_bwd",
+           "rope2d_apply", "rope2d_apply_to", "swa_select_impl", "swa_describe_plan", "swa_refresh_env", "swa_launch_count", "swa_last_error", "swa_version")
 
 
 def _load() -> C.CDLL:
@@ -65,6 +65,8 @@ def _load() -> C.CDLL:
     lib.rope2d_apply_to.argtypes = [C.c_int32, C.c_void_p, C.c_void_p, C.c_int64, C.c_int64, C.c_int32, P(C.c_int64),
                                     P(C.c_int64), P(Rope), C.c_int32, C.c_void_p]
     lib.swa_step_select.argtypes = [P(Geom), P(Rope)]
+    lib.swa_step_select_impl.argtypes = [P(Geom), P(Rope), C.c_int32]
+    lib.swa_step_describe_plan.argtypes = [P(Geom), P(Rope), C.c_int32, P(C.c_int32)]
     lib.swa_step_fwd.argtypes = [P(Geom), P(Rope), P(Tensor4), P(Tensor4), P(Tensor4), P(Tensor4), C.c_void_p, P(Tensor4),
                                  P(Tensor4), C.c_void_p, C.c_void_p]
     lib.swa_step_bwd.argtypes = [P(Geom), P(Rope), P(Tensor4), P(Tensor4), P(Tensor4), P(Tensor4), P(Tensor4), C.c_void_p,
@@ -72,7 +74,8 @@ def _load() -> C.CDLL:
     lib.swa_select_impl.argtypes = [P(Geom), P(Rope), C.c_int32]
     lib.swa_describe_plan.argtypes = [P(Geom), P(Rope), C.c_int32, P(C.c_int32)]
     for name in ("swa_fwd", "swa_bwd_delta", "swa_bwd_dq", "swa_bwd_dkdv", "swa_fwd_rot", "swa_bwd_dq_rot",
-                 "swa_bwd_dkdv_rot", "swa_bwd_noalloc", "swa_step_select", "swa_step_fwd", "swa_step_bwd", "rope2d_apply",
+                 "swa_bwd_dkdv_rot", "swa_bwd_noalloc", "swa_step_select", "swa_step_select_impl", "swa_step_describe_plan", "swa_step_fwd",
+                 "swa_step_bwd", "rope2d_apply",
                  "rope2d_apply_to", "swa_select_impl", "swa_describe_plan", "swa_version"):
         getattr(lib, name).restype = C.c_int
     lib.swa_refresh_env.restype = None

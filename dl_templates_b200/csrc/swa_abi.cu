@@ -507,13 +507,29 @@ int swa_bwd_dkdv_rot(const swa_geom_t* g, const swa_rope_t* rope, const swa_tens
 }
 
 // ---- one call per direction -------------------------------------------------------------------
+int swa_step_select_impl(const swa_geom_t* g, const swa_rope_t* rope, int32_t which) {
+  if (int e = check_geom(g)) return e;
+  if (int e = check_rope(g, rope)) return e;
+  if (which < 0 || which > 2) return fail(E_IMPL, "kernel %d: 0 forward, 1 dQ, 2 dK/dV", which);
+  return resolve_impl(g, rope, nullptr, 0, which, rope && rope->idx, true);
+}
+
 int swa_step_select(const swa_geom_t* g, const swa_rope_t* rope) {
   if (int e = check_geom(g)) return e;
   if (int e = check_rope(g, rope)) return e;
-  const bool rot = rope && rope->idx;
   for (int which = 0; which < 3; ++which)
-    if (resolve_impl(g, rope, nullptr, 0, which, rot, true) != SWA_IMPL_TC) return SWA_IMPL_SIMT;
+    if (swa_step_select_impl(g, rope, which) != SWA_IMPL_TC) return SWA_IMPL_SIMT;
   return SWA_IMPL_TC;
+}
+
+int swa_step_describe_plan(const swa_geom_t* g, const swa_rope_t* rope, int32_t which, int32_t* out) {
+  if (int e = check_geom(g)) return e;
+  if (int e = check_rope(g, rope)) return e;
+  if (!out || which < 0 || which > 2) return fail(E_NULL, "swa_step_describe_plan: out is NULL or `which` not in 0..2");
+  const bool rot = rope && rope->idx;
+  if (swa::tc::unsupported_reason(g, rope, nullptr, 0, which, rot, true) != nullptr || !swa::tc::describe_plan(g, rope, which + (rot ? 3 : 0), out))
+    return fail(E_SHAPE, "the tensor-core kernels do not take this shape");
+  return 0;
 }
 
 int swa_step_fwd(const swa_geom_t* g, const swa_rope_t* rope, const swa_tensor_t* q, const swa_tensor_t* k, const swa_tensor_t* v,

@@ -626,14 +626,15 @@ const char* unsupported_reason(const swa_geom_t* g, const swa_rope_t* rope, cons
   if (knobs().disable) return "disabled by SWA_TC_DISABLE";
   if (g->dtype != SWA_F16 && g->dtype != SWA_BF16) return "fp32 runs on the SIMT kernels";
   // The kernels work on 64-element chunks of a row.  Those without streamed rotation also take head dims of 32 and
-  // 96: the tensor map's innermost extent is the real head dim, so TMA zero-fills the missing half of the last chunk
+  // 96, and with any8 any multiple of 8 (a tensor map's rows and strides are counted in 16 bytes): the tensor map's innermost
+  // extent is the real head dim, so TMA zero-fills the missing part of the last chunk
   // (zero columns of q, k leave every score unchanged, zero columns of v and dO give zero columns of O, dV that are
   // never stored), which costs MMA work on zeros but no HBM traffic and no padded copies.
   {
     const bool v2_dims = prerotated || !(rope && rope->idx);
     auto dim_ok = [&](int d) { return v2_dims && any8 ? (d >= 8 && d <= 128 && d % 8 == 0) : v2_dims ? (d >= 32 && d <= 128 && d % 32 == 0) : (d == 64 || d == 128); };
     if (!dim_ok(g->d_qk) || !dim_ok(g->d_v))
-      return v2_dims ? "head dims must be 32, 64, 96 or 128" : "head dims must be 64 or 128 for the kernels that rotate streamed rows";
+      return v2_dims && any8 ? "head dims must be multiples of 8 up to 128" : v2_dims ? "head dims must be 32, 64, 96 or 128" : "head dims must be 64 or 128 for the kernels that rotate streamed rows";
   }
   if (!(g->sm_scale > 0.f)) return "sm_scale must be positive";
   float ma, mb;

@@ -187,7 +187,7 @@ void check_out(const Tensor& t, at::IntArrayRef shape, const Tensor& like, const
 }
 
 // (d_qk', d_v') if zero-padding the head dims to 64 or 128 moves this problem from the SIMT kernels to the tensor-core
-// kernels, else (0, 0).  `prerotated`: the entries that rotate no streamed row.
+// kernels, else (0, 0).  With RoPE: to the kernels that rotate what they stream.
 std::array<int64_t, 2> padded_dims(const Tensor& q, int64_t d_v, const Rope* rope, const Win& w, int32_t impl) {
   const std::array<int64_t, 2> none{0, 0};
   if (impl != SWA_IMPL_AUTO || q.scalar_type() == at::kFloat) return none;
@@ -202,6 +202,7 @@ std::array<int64_t, 2> padded_dims(const Tensor& q, int64_t d_v, const Rope* rop
   if (rope && rope->on()) { r = rope_shape(*rope); rp = &r; }
   auto all_tc = [&](int64_t a, int64_t b) {
     const swa_geom_t g = geom(q, a, b, w, forced_impl(SWA_IMPL_AUTO));
+    if (!rp) return swa_step_select(&g, nullptr) == SWA_IMPL_TC;
     for (int which = 0; which < 3; ++which)
       if (swa_select_impl(&g, rp, which) != SWA_IMPL_TC) return false;
     return true;
@@ -243,8 +244,7 @@ Fwd forward(Tensor q, Tensor k, Tensor v, const Rope& rope_, const Win& w, int32
   check_inputs(q, k, v, w);
   const Rope rope = aligned_tables(rope_);
   q = materialise(q); k = materialise(k); v = materialise(v);
-  const auto pad = !rope.on() && native_dims(q, v.size(3), nullptr, w, impl) ? std::array<int64_t, 2>{0, 0}
-                                                                          : padded_dims(q, v.size(3), &rope, w, impl);
+  const auto pad = padded_dims(q, v.size(3), &rope, w, impl);
   if (pad[0]) {
     Fwd f = forward(pad_last(q, pad[0]), pad_last(k, pad[0]), pad_last(v, pad[1]), rope, w, impl, Tensor());
     const Tensor o_v = f.o.narrow(3, 0, v.size(3));
@@ -318,7 +318,7 @@ Grads backward(Tensor q, Tensor k, Tensor v, Tensor o, Tensor lse, Tensor d_o, c
   lse = lse.contiguous();
   q = materialise(q); k = materialise(k); v = materialise(v); o = materialise(o); d_o = materialise(d_o);
   const bool given = out.dq.defined();
-  if (!rotated && !(!rope.on() && native_dims(q, v.size(3), nullptr, w, impl))) {
+  if (!rotated) {
     const auto pad = padded_dims(q, v.size(3), &rope, w, impl);
     if (pad[0]) {
       Grads g = backward(pad_last(q, pad[0]), pad_last(k, pad[0]), pad_last(v, pad[1]), pad_last(o, pad[1]), lse,

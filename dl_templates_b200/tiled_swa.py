@@ -60,8 +60,8 @@ def _ref(x):
 def padded_head_dims(q, v, rope, b_size, t_height, t_width, row_size, col_size, sm_scale=1.0, impl="auto"):
     """``(d_qk', d_v')`` if zero-padding the head dims to 64 or 128 moves this problem from the SIMT kernels to
     the tensor-core kernels, else ``None``.  Padding q and k with zero columns leaves every score unchanged,
-    padding v adds zero columns to O; the reference's own test shape (d = 32, b_size = 16,
-    src/tiled_swa.py:736-746) is the case this exists for."""
+    padding v adds zero columns to O.  Without ``rope`` the tensor-core kernels take any multiple of 8 as it is; with it the
+    answer is that of the kernels that rotate what they stream (``set_rope_mode("fused")``), which take 64 and 128."""
     return _native.padded_dims(q, v.shape[-1], *(rope or _NO_ROPE), b_size, t_height, t_width, row_size, col_size,
                                sm_scale, _lib.impl_code(impl))
 
@@ -135,10 +135,11 @@ def swa_backward_noalloc(q, k, v, o, lse, do, rope, b_size, t_height, t_width, r
 
 
 def selected_impl(q, v, rope, b_size, t_height, t_width, row_size, col_size, sm_scale=1.0, which=0, impl="auto"):
-    """'tc' or 'simt': the kernel family a call with these shapes would run."""
+    """'tc' or 'simt': the kernel family ``swa_forward`` / ``swa_backward`` (``which``: 0 forward, 1 dQ, 2 dK/dV) run for these
+    shapes as they are; where that is 'simt', ``padded_head_dims`` says whether the call is padded instead."""
     g = _geom(q, v, b_size, t_height, t_width, row_size, col_size, sm_scale, impl)
     r = _lib.make_rope(*rope) if rope is not None else None
-    code = _lib.lib.swa_select_impl(C.byref(g), _ref(r), which)
+    code = (_lib.lib.swa_step_select_impl if r is None else _lib.lib.swa_select_impl)(C.byref(g), _ref(r), which)
     if code < 0:
         _lib.check(code, "swa_select_impl")
     return {_lib.IMPL_SIMT: "simt", _lib.IMPL_TC: "tc"}[code]

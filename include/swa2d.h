@@ -120,12 +120,17 @@ int swa_bwd_dkdv_rot(const swa_geom_t* g, const swa_rope_t* rope, const swa_tens
                      const swa_tensor_t* dk, const swa_tensor_t* dv, int32_t* status, void* stream);
 
 /* One call per direction, what the Python surface uses: swa_step_fwd is swa_fwd_rot with RoPE and swa_fwd without
- * (q_rot / k_rot unused then); swa_step_bwd is swa_bwd_delta (fp32: made by the dQ launch), then swa_bwd_dq_rot and swa_bwd_dkdv_rot (q, k = the rotated
- * copies) or swa_bwd_dq and swa_bwd_dkdv, with `delta` as scratch.  Beyond the single entries they take 16-bit head dims of
+ * (q_rot / k_rot unused then); swa_step_bwd is swa_bwd_delta (fp32: made by the dQ launch), then swa_bwd_dq_rot and
+ * swa_bwd_dkdv_rot (q, k = the rotated copies) or swa_bwd_dq and swa_bwd_dkdv, with `delta` as scratch.  Beyond the single entries they take 16-bit head dims of
  * any multiple of 8 up to 128 on the tensor-core kernels as they are (the tensor maps carry the real head dim, TMA fills and
- * clips).  swa_step_select: the kernel family they run for a geometry.  Replace the same launches of the reference as
- * the entries they stand for. */
+ * clips); the single entries keep the head dims they have always named (32, 64, 96, 128), so that what swa_select_impl and
+ * swa_describe_plan say of them stays true for callers that plan by it.  Replace the same launches of the reference as the
+ * entries they stand for.
+ * swa_step_select_impl, swa_step_describe_plan: as swa_select_impl and swa_describe_plan, for the three kernels of these
+ * entries (`which`: 0 fwd, 1 dq, 2 dkdv).  swa_step_select: SWA_IMPL_TC if all three run on the tensor cores. */
 int swa_step_select(const swa_geom_t* g, const swa_rope_t* rope);
+int swa_step_select_impl(const swa_geom_t* g, const swa_rope_t* rope, int32_t which);
+int swa_step_describe_plan(const swa_geom_t* g, const swa_rope_t* rope, int32_t which, int32_t* out);
 int swa_step_fwd(const swa_geom_t* g, const swa_rope_t* rope, const swa_tensor_t* q, const swa_tensor_t* k,
                  const swa_tensor_t* v, const swa_tensor_t* o, float* lse, const swa_tensor_t* q_rot,
                  const swa_tensor_t* k_rot, int32_t* status, void* stream);

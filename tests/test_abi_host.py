@@ -176,6 +176,45 @@ def test_select_impl_refuses_kernels_that_do_not_exist():
         assert b"kernel" in _lib.lib.swa_last_error()
 
 
+def test_step_entries_plans_and_answers_for_any_multiple_of_8():
+    """The step entries' plans keep the same invariants at head dims that fill no 64-wide chunk, and what selected_impl and
+    padded_head_dims say is what the call surface does: such head dims run on the tensor cores without padding."""
+    idx = torch.zeros(16, dtype=torch.int32)
+    n_plans = 0
+    for d_qk, d_v in ((8, 8), (24, 48), (48, 48), (72, 104), (80, 80), (104, 16), (120, 120), (128, 8)):
+        for th, tw, bs, rs, cs in ((33, 47, 1, 5, 5), (16, 16, 4, 1, 1), (128, 128, 1, 6, 6), (24, 40, 1, 13, 13), (9, 7, 2, 20, 4), (40, 9, 16, 1, 2)):
+            for n_rdim in (0, 8, 16):
+                if 4 * n_rdim > d_qk:
+                    continue
+                tab = torch.zeros(64, max(n_rdim, 1), 2)
+                r = _lib.make_rope(idx, tab, tab) if n_rdim else None
+                g = _geom(t_height=th, t_width=tw, b_size=bs, row_size=rs, col_size=cs, d_qk=d_qk, d_v=d_v)
+                rr = None if r is None else C.byref(r)
+                for which in (0, 1, 2):
+                    out = (C.c_int32 * 12)()
+                    code = _lib.lib.swa_step_describe_plan(C.byref(g), rr, which, out)
+                    assert (code == 0) == (_lib.lib.swa_step_select_impl(C.byref(g), rr, which) == _lib.IMPL_TC)
+                    if code:
+                        continue
+                    th_, tw_, kr, kw, n, stages, nsb, nxb, tab_b, req, used, tmem = out
+                    what = (d_qk, d_v, th, tw, bs, rs, cs, n_rdim, which, list(out))
+                    assert th_ * tw_ == 128 and n == kr * kw and n % 16 == 0 and 16 <= n <= 128, what
+                    assert 2 <= stages <= 8 and 2 <= nsb <= 4 and 1 <= nxb <= 2 and tab_b == 0, what
+                    assert used <= req <= 227 * 1024 and tmem <= 512, what
+                    n_plans += 1
+            q, v = (torch.zeros(1, 1, th * tw * bs, d, dtype=torch.bfloat16) for d in (d_qk, d_v))
+            win = (bs, th, tw, rs, cs)
+            assert swa.selected_impl(q, v, None, *win) == "tc" and swa.padded_head_dims(q, v, None, *win) is None, win
+    assert n_plans > 250
+    g = _geom(d_qk=84, d_v=84, impl="tc")
+    assert _lib.lib.swa_step_select_impl(C.byref(g), None, 0) < 0 and b"multiples of 8" in _lib.lib.swa_last_error()
+    for which in (-1, 3):
+        assert _lib.lib.swa_step_select_impl(C.byref(_geom()), None, which) < 0
+        assert _lib.lib.swa_step_describe_plan(C.byref(_geom()), None, which, (C.c_int32 * 12)()) < 0
+    q = torch.zeros(1, 1, 64, 44, dtype=torch.bfloat16)                       # no multiple of 8: padded
+    assert swa.selected_impl(q, q, None, 1, 8, 8, 2, 2) == "simt" and swa.padded_head_dims(q, q, None, 1, 8, 8, 2, 2) == (64, 64)
+
+
 def test_head_dims_the_tensor_core_kernels_take():
     """32, 64, 96, 128 where no streamed row is rotated (no RoPE, or the entries that take rotated copies); 64 and
     128 only for the kernels that rotate what they stream; anything else runs on the SIMT kernels."""
