@@ -66,14 +66,12 @@ struct Geom {
   float sm_scale;
 };
 
-// A window that reaches beyond the grid is cut to the grid: the same pairs, and r + wr, (c + wc) * b stay far from overflow
-// whatever half-size the caller names.
+// (A window taller than the grid is cut to the grid: the same pairs, and r + wr stays far from overflow.)
 inline Geom make_geom(const swa_geom_t* g) {
   Geom r;
   r.B = g->B; r.H = g->H; r.b = g->b_size; r.th = g->t_height; r.tw = g->t_width;
   r.wr = g->row_size < g->t_height ? g->row_size : g->t_height - 1;
-  r.wc = g->col_size < g->t_width ? g->col_size : g->t_width - 1;
-  r.dqk = g->d_qk; r.dv = g->d_v;
+  r.wc = g->col_size; r.dqk = g->d_qk; r.dv = g->d_v;
   r.sm_scale = g->sm_scale; r.scale_log2 = g->sm_scale * kLog2e;
   return r;
 }

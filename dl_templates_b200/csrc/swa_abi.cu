@@ -44,6 +44,17 @@ int check_geom(const swa_geom_t* g) {
   return 0;
 }
 
+// The geometry every plan and kernel works with: a window wider than the grid is cut to the grid.  The same pairs; no columns
+// streamed that do not exist (one column of 14 cells of 64 tokens, 13 x 13 window: a halo of 64 instead of 832 columns, 494 -> 53 us
+// of a training step of 4 slices on the GPU; one of 120 cells of 16, 1 x 15 window, d = 128: 1343 -> 220), and (c + wc) * b stays far from
+// overflow whatever half-size the caller names.  Taller ones are left as they are: streamed rows are clipped to the grid anyway, and
+// blocks begin at -wr (mod KR), which the caller's wr may suit better (2 x 2427, wr = 20: 181 us, cut to 1 210).
+swa_geom_t cut_window(const swa_geom_t& g) {
+  swa_geom_t c = g;
+  c.col_size = std::min(c.col_size, c.t_width - 1);
+  return c;
+}
+
 int check_rope(const swa_geom_t* g, const swa_rope_t* r) {
   if (!r || !r->idx) return 0;
   if (!r->row_cs || !r->col_cs) return fail(E_ROPE, "rope tables are NULL");
@@ -177,15 +188,17 @@ void swa_refresh_env(void) { swa::tc::refresh_env(); }
 const char* swa_last_error(void) { return g_err; }
 int64_t swa_launch_count(void) { return g_launches.load(); }
 
-int swa_select_impl(const swa_geom_t* g, const swa_rope_t* rope, int32_t which) {
-  if (int e = check_geom(g)) return e;
+int swa_select_impl(const swa_geom_t* geom, const swa_rope_t* rope, int32_t which) {
+  if (int e = check_geom(geom)) return e;
+  const swa_geom_t cut = cut_window(*geom), *g = &cut;
   if (int e = check_rope(g, rope)) return e;
   if (which < 0 || which > 2) return fail(E_IMPL, "kernel %d: 0 forward, 1 dQ, 2 dK/dV", which);   // (an index into the plans kept)
   return resolve_impl(g, rope, nullptr, 0, which);
 }
 
-int swa_describe_plan(const swa_geom_t* g, const swa_rope_t* rope, int32_t which, int32_t* out) {
-  if (int e = check_geom(g)) return e;
+int swa_describe_plan(const swa_geom_t* geom, const swa_rope_t* rope, int32_t which, int32_t* out) {
+  if (int e = check_geom(geom)) return e;
+  const swa_geom_t cut = cut_window(*geom), *g = &cut;
   if (int e = check_rope(g, rope)) return e;
   if (!out || which < 0 || which > 5) return fail(E_NULL, "swa_describe_plan: out is NULL or `which` not in 0..5");
   if (which >= 3 && !(rope && rope->idx)) return fail(E_ROPE, "swa_describe_plan: kernels 3..5 are the RoPE hand-off entries");
@@ -194,8 +207,9 @@ int swa_describe_plan(const swa_geom_t* g, const swa_rope_t* rope, int32_t which
   return 0;
 }
 
-static int fwd_call(bool any8, const swa_geom_t* g, const swa_rope_t* rope, const swa_tensor_t* q, const swa_tensor_t* k, const swa_tensor_t* v, const swa_tensor_t* o, float* lse, int32_t* status, void* stream) {
-  if (int e = check_geom(g)) return e;
+static int fwd_call(bool any8, const swa_geom_t* geom, const swa_rope_t* rope, const swa_tensor_t* q, const swa_tensor_t* k, const swa_tensor_t* v, const swa_tensor_t* o, float* lse, int32_t* status, void* stream) {
+  if (int e = check_geom(geom)) return e;
+  const swa_geom_t cut = cut_window(*geom), *g = &cut;
   if (int e = check_rope(g, rope)) return e;
   if (int e = check_tensor(q, "q")) return e;
   if (int e = check_tensor(k, "k")) return e;
@@ -271,9 +285,10 @@ int swa_bwd_delta(const swa_geom_t* g, const swa_tensor_t* o, const swa_tensor_t
   return launch_ok("delta");
 }
 
-static int dq_call(bool any8, const swa_geom_t* g, const swa_rope_t* rope, const swa_tensor_t* q, const swa_tensor_t* k, const swa_tensor_t* v, const swa_tensor_t* d_o, const float* lse, const float* delta, const swa_tensor_t* dq, int32_t* status, void* stream,
+static int dq_call(bool any8, const swa_geom_t* geom, const swa_rope_t* rope, const swa_tensor_t* q, const swa_tensor_t* k, const swa_tensor_t* v, const swa_tensor_t* d_o, const float* lse, const float* delta, const swa_tensor_t* dq, int32_t* status, void* stream,
                    const swa_tensor_t* o = nullptr, float* delta_out = nullptr) {
-  if (int e = check_geom(g)) return e;
+  if (int e = check_geom(geom)) return e;
+  const swa_geom_t cut = cut_window(*geom), *g = &cut;
   if (int e = check_rope(g, rope)) return e;
   if (int e = check_tensor(q, "q")) return e;
   if (int e = check_tensor(k, "k")) return e;
@@ -311,8 +326,9 @@ int swa_bwd_dq(const swa_geom_t* g, const swa_rope_t* rope, const swa_tensor_t* 
   return dq_call(false, g, rope, q, k, v, d_o, lse, delta, dq, status, stream);
 }
 
-static int dkdv_call(bool any8, const swa_geom_t* g, const swa_rope_t* rope, const swa_tensor_t* q, const swa_tensor_t* k, const swa_tensor_t* v, const swa_tensor_t* d_o, const float* lse, const float* delta, const swa_tensor_t* dk, const swa_tensor_t* dv, int32_t* status, void* stream) {
-  if (int e = check_geom(g)) return e;
+static int dkdv_call(bool any8, const swa_geom_t* geom, const swa_rope_t* rope, const swa_tensor_t* q, const swa_tensor_t* k, const swa_tensor_t* v, const swa_tensor_t* d_o, const float* lse, const float* delta, const swa_tensor_t* dk, const swa_tensor_t* dv, int32_t* status, void* stream) {
+  if (int e = check_geom(geom)) return e;
+  const swa_geom_t cut = cut_window(*geom), *g = &cut;
   if (int e = check_rope(g, rope)) return e;
   if (int e = check_tensor(q, "q")) return e;
   if (int e = check_tensor(k, "k")) return e;
@@ -386,8 +402,9 @@ int require_rope(const swa_rope_t* rope, const char* who) {
 
 }  // namespace
 
-static int fwd_rot_call(bool any8, const swa_geom_t* g, const swa_rope_t* rope, const swa_tensor_t* q, const swa_tensor_t* k, const swa_tensor_t* v, const swa_tensor_t* o, float* lse, const swa_tensor_t* q_rot, const swa_tensor_t* k_rot, int32_t* status, void* stream) {
-  if (int e = check_geom(g)) return e;
+static int fwd_rot_call(bool any8, const swa_geom_t* geom, const swa_rope_t* rope, const swa_tensor_t* q, const swa_tensor_t* k, const swa_tensor_t* v, const swa_tensor_t* o, float* lse, const swa_tensor_t* q_rot, const swa_tensor_t* k_rot, int32_t* status, void* stream) {
+  if (int e = check_geom(geom)) return e;
+  const swa_geom_t cut = cut_window(*geom), *g = &cut;
   if (int e = require_rope(rope, "swa_fwd_rot")) return e;
   if (int e = check_rope(g, rope)) return e;
   if (int e = check_tensor(q, "q")) return e;
@@ -426,9 +443,10 @@ int swa_fwd_rot(const swa_geom_t* g, const swa_rope_t* rope, const swa_tensor_t*
   return fwd_rot_call(false, g, rope, q, k, v, o, lse, q_rot, k_rot, status, stream);
 }
 
-static int dq_rot_call(bool any8, const swa_geom_t* g, const swa_rope_t* rope, const swa_tensor_t* q_rot, const swa_tensor_t* k_rot, const swa_tensor_t* v, const swa_tensor_t* d_o, const float* lse, const float* delta, const swa_tensor_t* dq, int32_t* status, void* stream,
+static int dq_rot_call(bool any8, const swa_geom_t* geom, const swa_rope_t* rope, const swa_tensor_t* q_rot, const swa_tensor_t* k_rot, const swa_tensor_t* v, const swa_tensor_t* d_o, const float* lse, const float* delta, const swa_tensor_t* dq, int32_t* status, void* stream,
                    const swa_tensor_t* o = nullptr, float* delta_out = nullptr) {
-  if (int e = check_geom(g)) return e;
+  if (int e = check_geom(geom)) return e;
+  const swa_geom_t cut = cut_window(*geom), *g = &cut;
   if (int e = require_rope(rope, "swa_bwd_dq_rot")) return e;
   if (int e = check_rope(g, rope)) return e;
   if (int e = check_tensor(q_rot, "q_rot")) return e;
@@ -468,8 +486,9 @@ int swa_bwd_dq_rot(const swa_geom_t* g, const swa_rope_t* rope, const swa_tensor
   return dq_rot_call(false, g, rope, q_rot, k_rot, v, d_o, lse, delta, dq, status, stream);
 }
 
-static int dkdv_rot_call(bool any8, const swa_geom_t* g, const swa_rope_t* rope, const swa_tensor_t* q_rot, const swa_tensor_t* k_rot, const swa_tensor_t* v, const swa_tensor_t* d_o, const float* lse, const float* delta, const swa_tensor_t* dk, const swa_tensor_t* dv, int32_t* status, void* stream) {
-  if (int e = check_geom(g)) return e;
+static int dkdv_rot_call(bool any8, const swa_geom_t* geom, const swa_rope_t* rope, const swa_tensor_t* q_rot, const swa_tensor_t* k_rot, const swa_tensor_t* v, const swa_tensor_t* d_o, const float* lse, const float* delta, const swa_tensor_t* dk, const swa_tensor_t* dv, int32_t* status, void* stream) {
+  if (int e = check_geom(geom)) return e;
+  const swa_geom_t cut = cut_window(*geom), *g = &cut;
   if (int e = require_rope(rope, "swa_bwd_dkdv_rot")) return e;
   if (int e = check_rope(g, rope)) return e;
   if (int e = check_tensor(q_rot, "q_rot")) return e;
@@ -507,8 +526,9 @@ int swa_bwd_dkdv_rot(const swa_geom_t* g, const swa_rope_t* rope, const swa_tens
 }
 
 // ---- one call per direction -------------------------------------------------------------------
-int swa_step_select_impl(const swa_geom_t* g, const swa_rope_t* rope, int32_t which) {
-  if (int e = check_geom(g)) return e;
+int swa_step_select_impl(const swa_geom_t* geom, const swa_rope_t* rope, int32_t which) {
+  if (int e = check_geom(geom)) return e;
+  const swa_geom_t cut = cut_window(*geom), *g = &cut;
   if (int e = check_rope(g, rope)) return e;
   if (which < 0 || which > 2) return fail(E_IMPL, "kernel %d: 0 forward, 1 dQ, 2 dK/dV", which);
   return resolve_impl(g, rope, nullptr, 0, which, rope && rope->idx, true);
@@ -522,8 +542,9 @@ int swa_step_select(const swa_geom_t* g, const swa_rope_t* rope) {
   return SWA_IMPL_TC;
 }
 
-int swa_step_describe_plan(const swa_geom_t* g, const swa_rope_t* rope, int32_t which, int32_t* out) {
-  if (int e = check_geom(g)) return e;
+int swa_step_describe_plan(const swa_geom_t* geom, const swa_rope_t* rope, int32_t which, int32_t* out) {
+  if (int e = check_geom(geom)) return e;
+  const swa_geom_t cut = cut_window(*geom), *g = &cut;
   if (int e = check_rope(g, rope)) return e;
   if (!out || which < 0 || which > 2) return fail(E_NULL, "swa_step_describe_plan: out is NULL or `which` not in 0..2");
   const bool rot = rope && rope->idx;
@@ -579,11 +600,12 @@ int noalloc_scratch(float** out) {
 }
 }  // namespace
 
-int swa_bwd_noalloc(const swa_geom_t* g, const swa_rope_t* rope, const swa_tensor_t* q, const swa_tensor_t* k,
+int swa_bwd_noalloc(const swa_geom_t* geom, const swa_rope_t* rope, const swa_tensor_t* q, const swa_tensor_t* k,
                     const swa_tensor_t* v, const swa_tensor_t* o, const swa_tensor_t* d_o, const float* lse,
                     const swa_tensor_t* dq, const swa_tensor_t* dk, const swa_tensor_t* dv, int32_t* status,
                     void* stream) {
-  if (int e = check_geom(g)) return e;
+  if (int e = check_geom(geom)) return e;
+  const swa_geom_t cut = cut_window(*geom), *g = &cut;
   const int64_t rows = (int64_t)g->B * g->H * g->t_height * g->t_width * g->b_size;
   if (rows > (int64_t)SWA_NOALLOC_MAX_ROWS)
     return fail(E_SHAPE, "swa_bwd_noalloc: B*H*N = %lld exceeds the built-in scratch of %d rows; use swa_bwd_delta/"

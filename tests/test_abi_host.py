@@ -149,13 +149,15 @@ def test_every_tile_plan_fits_shared_and_tensor_memory():
     assert n_plans > 500
 
 
-def test_windows_too_wide_for_32_bits_get_no_plan():
-    """(2 wc + 1) * b beyond 32 bits must not wrap round to a plan for a narrow halo: no plan, the SIMT kernels take it."""
-    for b, wc in ((16, 2 ** 27), (16, 2 ** 27 + 3), (1, 2 ** 30), (1, 2 ** 31 - 1), (4, 2 ** 29), (16, 2 ** 31 - 1), (16, 5000)):
-        g = _geom(b_size=b, t_height=8, t_width=8, col_size=wc)
+def test_windows_wider_than_the_grid_are_planned_as_the_grid():
+    """A half-size that reaches past the grid's columns is the whole width, for the plans too: no columns that do not exist, and
+    no (2 wc + 1) * b that wraps round in 32 bits to a narrow halo."""
+    for b, wc in ((16, 2 ** 27), (16, 2 ** 27 + 3), (1, 2 ** 30), (1, 2 ** 31 - 1), (4, 2 ** 29), (16, 2 ** 31 - 1), (16, 5000), (1, 8)):
         for which in (0, 1, 2):
-            assert _lib.lib.swa_select_impl(C.byref(g), None, which) == _lib.IMPL_SIMT, (b, wc)
-            assert _plan(g, None, which)[0] < 0
+            got, want = (_plan(_geom(b_size=b, t_height=9, t_width=8, col_size=c), None, which) for c in (wc, 7))
+            assert got == want and got[0] == 0, (b, wc)
+    g = _geom(b_size=16, t_height=8, t_width=5000, col_size=4000)              # ... but a halo no plan takes gets none
+    assert _lib.lib.swa_select_impl(C.byref(g), None, 0) == _lib.IMPL_SIMT
 
 
 def test_misaligned_tables_keep_off_the_tensor_core_kernels():
