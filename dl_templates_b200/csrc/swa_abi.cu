@@ -118,7 +118,7 @@ int tile_band_rows(const swa::Geom& g, int rows, int cols, int64_t blocks, Bytes
       const int upper = std::min(b1, span) - b0, lower = b1 - std::max(b0, 2);
       steps += (std::max(upper, lower) * wcols + 31) / 32 + 1;
     }
-    const int64_t slots = (int64_t)c.per_sm * 148;
+    const int64_t slots = (int64_t)c.per_sm * swa::tc::sm_count();
     const double cost = (double)((blocks + slots - 1) / slots) * steps * c.step;
     if (best < 0. || cost < best) {
       best = cost;

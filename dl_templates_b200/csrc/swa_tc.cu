@@ -67,19 +67,6 @@ bool make_map(CUtensorMap* m, const swa_tensor_t* t, const swa_geom_t* g, int d,
   return true;
 }
 
-// SMs of the current device (cached per device ordinal).
-int sm_count() {
-  static int cached[64] = {};
-  int dev = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 148;
-  if (cached[dev] == 0) {
-    int n = 0;
-    if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n <= 0) n = 148;
-    cached[dev] = n;
-  }
-  return cached[dev];
-}
-
 // Experiment knobs (environment variables), read ONCE per process -- a launch must not pay for a dozen getenv
 // calls -- and again only when refresh_env() is called (tests that vary them do).  -1 / 0 = not set.
 struct Knobs {
@@ -615,6 +602,18 @@ bool tensor_ok(const swa_tensor_t* t, int B, int H) {
 
 const char* last_error() { return g_tc_err; }
 
+int sm_count() {
+  static std::atomic<int> cached[64] = {};
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 148;
+  int n = cached[dev].load(std::memory_order_relaxed);
+  if (n == 0) {
+    if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n <= 0) n = 148;
+    cached[dev].store(n, std::memory_order_relaxed);
+  }
+  return n;
+}
+
 void refresh_env() {
   std::lock_guard<std::mutex> lock(g_plan_mu);
   read_knobs_locked();
@@ -703,14 +702,14 @@ int launch_fwd(const swa_geom_t* g, const swa_rope_t* rope, const swa_tensor_t* 
   const int sms = sm_count();
   dim3 grid(n_items < sms ? n_items : sms), block(kFwdThreads);
   using FwdKernel = void (*)(const CUtensorMap, const CUtensorMap, const CUtensorMap, KParams, View4, float*);
-  // the RoPE table width is a template parameter of the kernel (index: n_rdim / 8, 0 = no rotation)
-  // ... and so is whether the cos/sin tables are staged in shared memory
+  // the RoPE table width is a template parameter of the kernel (index: n_rdim / 8; calls without rotation went to launch_fwd2),
+  // and so is whether the cos/sin tables are staged in shared memory
   static const FwdKernel fwd_table[2][2][5] = {
-      {{fwd_kernel<false, 0, false>, fwd_kernel<false, 1, false>, fwd_kernel<false, 2, false>, nullptr, fwd_kernel<false, 4, false>},
-       {fwd_kernel<false, 0, false>, fwd_kernel<false, 1, true>, fwd_kernel<false, 2, true>, nullptr, fwd_kernel<false, 4, true>}},
-      {{fwd_kernel<true, 0, false>, fwd_kernel<true, 1, false>, fwd_kernel<true, 2, false>, nullptr, fwd_kernel<true, 4, false>},
-       {fwd_kernel<true, 0, false>, fwd_kernel<true, 1, true>, fwd_kernel<true, 2, true>, nullptr, fwd_kernel<true, 4, true>}}};
-  const int ni = (rope && rope->idx) ? rope->n_rdim / 8 : 0;
+      {{nullptr, fwd_kernel<false, 1, false>, fwd_kernel<false, 2, false>, nullptr, fwd_kernel<false, 4, false>},
+       {nullptr, fwd_kernel<false, 1, true>, fwd_kernel<false, 2, true>, nullptr, fwd_kernel<false, 4, true>}},
+      {{nullptr, fwd_kernel<true, 1, false>, fwd_kernel<true, 2, false>, nullptr, fwd_kernel<true, 4, false>},
+       {nullptr, fwd_kernel<true, 1, true>, fwd_kernel<true, 2, true>, nullptr, fwd_kernel<true, 4, true>}}};
+  const int ni = rope->n_rdim / 8;
   FwdKernel kern = fwd_table[g->dtype == SWA_BF16 ? 1 : 0][pl.tab_bytes ? 1 : 0][ni];
   if (kern == nullptr) {
     snprintf(g_tc_err, sizeof(g_tc_err), "n_rdim %d has no tensor-core kernel", rope ? rope->n_rdim : 0);

@@ -15,6 +15,9 @@ const char* unsupported_reason(const swa_geom_t* g, const swa_rope_t* rope, cons
                                int n_tensors, int which, bool prerotated = false, bool any8 = false);
 const char* last_error();
 
+// SMs of the current device (148 where there is none to ask), kept per device.
+int sm_count();
+
 // Re-read the SWA_TC_* experiment knobs from the environment and drop the cached plans (both are otherwise read /
 // computed once per process).
 void refresh_env();
