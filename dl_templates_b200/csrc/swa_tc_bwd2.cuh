@@ -15,8 +15,9 @@
 // The order the single issuer gave for free ("the accumulating MMAs of the block that used this pair last were issued
 // before") is one more barrier, pair_free, that the accumulate issuer commits and the score issuer waits for.
 //
-// All waits are bounded; a timed-out wait raises a CTA-wide abort flag, every role runs its loops to the
-// end without touching anything, TMEM is freed and the status word records it.
+// All waits are bounded by polls, about a second each (umma.cuh).  A warp whose wait gave up runs its loops to the end without waiting
+// for or touching anything; the others run into their own limit, unless they have all they wait for.  At the end any of them
+// raises the CTA's flag: what is in flight is given time to land, TMEM is freed and the status word records it.
 #pragma once
 
 #include "swa_tc_bwd.cuh"

@@ -20,8 +20,9 @@
 // query tile in this kernel as well (about 400 dependent instructions per row on the critical path, 1.1 ms per launch
 // at the default workload, against 0.1 ms for a streaming pass over q).
 //
-// All waits are bounded; a timed-out wait raises a CTA-wide abort flag, every role runs its loops to the
-// end without touching anything, TMEM is freed and the status word records it.
+// All waits are bounded by polls, about a second each (umma.cuh).  A warp whose wait gave up runs its loops to the end without waiting
+// for or touching anything; the others run into their own limit, unless they have all they wait for.  At the end any of them
+// raises the CTA's flag: what is in flight is given time to land, TMEM is freed and the status word records it.
 #pragma once
 
 #include "swa_tc_fwd.cuh"

@@ -188,6 +188,8 @@ struct LoadArgs {
   const CUtensorMap *xqk, *xv, *yqk, *yv;   // xv: null in the forward kernel (no second resident tensor)
 };
 
+constexpr uint32_t kLoadPolls = 1u << 23;   // rounds that found no room in a row: 64 ns or more each, 0.5 s and up
+
 __device__ __forceinline__ void load_warp(const KParams& p, const LoadArgs& f, bool& ok) {
   using namespace ptx;
   const Plan& pl = p.pl;
@@ -279,7 +281,7 @@ __device__ __forceinline__ void load_warp(const KParams& p, const LoadArgs& f, b
     }
     polls = idle ? polls + 1 : 0;
     if (idle) __nanosleep(32);
-    if (polls == 1u << 24) ok = false;             // about a second
+    if (polls == kLoadPolls) ok = false;
   }
 }
 

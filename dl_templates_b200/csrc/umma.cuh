@@ -126,17 +126,18 @@ __device__ __forceinline__ bool mbar_try_wait_hint(uint64_t* bar, uint32_t parit
 //
 // The loop is a dozen instructions: the kernels have two dozen waits, all of them inlined, and every role's code is
 // fetched anew once per block (a polling loop with a wall clock in it made up a third of the kernels' 60 to 90 KB).
-// The budget is polls that did not succeed: at 50 ns or more each, 1 << 24 of them are about a second, far beyond any
+// The budget is polls that did not succeed.  try_wait suspends the warp for 1.98 us before it answers no, with a 100 ns hint for
+// 3.98 us (measured; arrivals that do not complete the phase change neither): 2^19 and 2^18 of them are 1.04 s, far beyond any
 // legitimate wait (a whole launch takes milliseconds); a context that is time-sliced with another process does not
 // use it up while it does not run.
-constexpr uint32_t kWaitMaxPolls = 1u << 24;
+constexpr uint32_t kSpinPolls = 1u << 19, kParkPolls = 1u << 18;
 template <uint32_t PARK_NS = 0>
 __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, volatile int* abort_flag) {
   uint32_t polls = 0;
 #pragma unroll 1
   while (!(PARK_NS == 0 ? mbar_try_wait(bar, parity) : mbar_try_wait_hint(bar, parity, PARK_NS))) {
     if (*abort_flag) return false;
-    if (++polls == kWaitMaxPolls) {
+    if (++polls == (PARK_NS == 0 ? kSpinPolls : kParkPolls)) {
       *abort_flag = 1;
       return false;
     }
@@ -145,8 +146,8 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, volati
 }
 
 // The strip kernels' wait (swa_tc_strip.cuh): six instructions, because they have two dozen of them in code that is fetched
-// again for every block.  False once the poll budget is used up (about half a second); the caller then skips every
-// later wait, and the kernel's end tells the host.
+// again for every block.  False once the poll budget is used up (a second, as above); the caller's warp then skips every
+// later wait, the others run into their own limit, and the kernel's end tells the host.
 template <uint32_t PARK_NS>
 __device__ __forceinline__ bool mbar_wait_polls(uint32_t bar, uint32_t parity) {
   uint32_t ok;
@@ -162,7 +163,7 @@ __device__ __forceinline__ bool mbar_wait_polls(uint32_t bar, uint32_t parity) {
         "@q bra SWA_WAIT;\n"
         "SWA_DONE:\n\t"
         "selp.u32 %0, 1, 0, p;\n\t}"
-        : "=r"(ok) : "r"(bar), "r"(parity), "n"(1 << 22) : "memory");
+        : "=r"(ok) : "r"(bar), "r"(parity), "n"(kSpinPolls) : "memory");
   else
     asm volatile(
         "{\n\t.reg .pred p, q;\n\t.reg .u32 n;\n\t"
@@ -175,7 +176,7 @@ __device__ __forceinline__ bool mbar_wait_polls(uint32_t bar, uint32_t parity) {
         "@q bra SWA_WAIT;\n"
         "SWA_DONE:\n\t"
         "selp.u32 %0, 1, 0, p;\n\t}"
-        : "=r"(ok) : "r"(bar), "r"(parity), "n"(1 << 22), "n"(PARK_NS) : "memory");
+        : "=r"(ok) : "r"(bar), "r"(parity), "n"(kParkPolls), "n"(PARK_NS) : "memory");
   return ok != 0;
 }
 

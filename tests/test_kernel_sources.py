@@ -57,3 +57,15 @@ def test_a_warp_never_branches_on_one_lanes_view_of_a_barrier():
             assert text[:m.start()].rstrip().endswith("__all_sync(0xffffffffu,"), (f, text[m.start() - 80:m.end() + 40])
             seen += 1
     assert seen >= 6
+
+
+def test_waits_give_up_after_about_a_second():
+    """Every bounded wait counts polls that failed.  A failed mbarrier.try_wait takes 1.98 us (3.98 us with a 100 ns hint; a
+    test_wait and a short sleep 64 ns), measured: the budgets come to half a second to a second and a half."""
+    text = source("umma.cuh") + source("swa_tc_strip.cuh")
+    polls = {n: 1 << int(e) for n, e in re.findall(r"\b(k(?:Spin|Park|Load)Polls) = 1u << (\d+)", text)}
+    assert set(polls) == {"kSpinPolls", "kParkPolls", "kLoadPolls"}
+    for name, ns in (("kSpinPolls", 1980), ("kParkPolls", 3980), ("kLoadPolls", 64)):
+        assert 0.5 <= polls[name] * ns * 1e-9 <= 1.5, name
+    for f in ("umma.cuh", "swa_tc_strip.cuh", "swa_tc_fwd2.cuh", "swa_tc_bwd2.cuh"):          # ... and no wait has a budget of its own
+        assert not re.search(r"(?<!Polls = )1u? << 2\d", source(f)), f
