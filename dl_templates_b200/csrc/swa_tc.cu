@@ -234,8 +234,8 @@ bool strip_slides(const swa_geom_t* g, int R4, int KR) {
 // Chunk height in quarters.  Sliding strips: the tallest chunk has the fewest blocks per row (2 wr rows of halo are met
 // once per chunk), short ones spread a small problem over all SMs; the slowest SM's blocks decide, the taller of two equals.  The
 // height is a multiple of the block height, so that no row's blocks depend on it.
-// A call of a batch size not met before pays for this (1 to 60 us for three plans up to 512 x 512; walking every height's items
-// took 14 ms on a grid 4096 rows high): heights are taken in the order of a bound -- their mean load, their largest item -- and
+// A call of a batch size not met before pays for this (three plans: 2 us at 24 x 24, 24 at 128 x 128 with one head, 470 at
+// 4096 x 64; walking every item of every height took 28, 750 and 11100): heights are taken in the order of a bound -- their mean load, their largest item -- and
 // the load of every CTA is put together only for those whose bound is not beyond the best load found.
 void choose_chunk(const swa_geom_t* g, Plan* pl) {
   const int quarters = (g->t_height + pl->R4 - 1) / pl->R4;
@@ -762,8 +762,8 @@ int launch_fwd2(const swa_geom_t* g, const swa_tensor_t* q, const swa_tensor_t* 
 
 namespace {
 
-// `prerotated`: q and k are rotated copies made by an earlier kernel (the forward kernel of swa_fwd_rot); the
-// kernels then run in their no-RoPE structure and only rotate dQ / dK back in the epilogue.
+// `prerotated`: q and k are the rotated copies the streaming pass of swa_fwd_rot made; the strip kernels rotate nothing
+// they stream and only rotate dQ / dK back in the epilogue.
 template <bool DKDV>
 int launch_bwd(const swa_geom_t* g, const swa_rope_t* rope, bool prerotated, const swa_tensor_t* xqk, const swa_tensor_t* xv,
                const swa_tensor_t* yqk, const swa_tensor_t* yv, const float* lse, const float* delta,

@@ -65,8 +65,8 @@ bwd2_kernel(const __grid_constant__ CUtensorMap tm_xqk, const __grid_constant__ 
   uint8_t* yr_smem = xx_smem + 8192;                            // ... row units of the mask ring,
   uint8_t* yc_smem = yr_smem + kMaskRing * ub * (pl.TH >> 3);   // ... column units,
   uint8_t* yz_smem = yc_smem + kMaskRing * ub * (pl.TW >> 3);  // ... the unused unit
-  // -lse / delta of the streamed queries (dK/dV): a ring of stages + 2 slots [slot][-lse | -delta][128], two deeper
-  // than the block ring because the feeder runs ahead of the compute warps
+  // -lse / delta of the streamed queries (dK/dV): a ring of kMaskRing + 2 slots [slot][-lse | -delta][128], two deeper
+  // than the ring of mask units because the warp that fills both runs ahead of the compute warps
   float* vec_smem = reinterpret_cast<float*>(yz_smem + ub);
   constexpr int vslots = kMaskRing + 2;
   Bwd2Shared* sh = reinterpret_cast<Bwd2Shared*>(reinterpret_cast<uint8_t*>(vec_smem) + (DKDV ? vslots * 1024 : 0));
