@@ -471,7 +471,7 @@ bool wants_grad(std::initializer_list<const Tensor*> ts) {
 
 // Whether the native node records all there is to record.  Forward-mode tangents, functorch's transforms, jit tracing, tensors
 // with a Python dispatch of their own and tables that ask for gradients are for the autograd.Function of the same name, which
-// refuses or handles them as torch does for every such function; the entry points below then answer None.
+// refuses or handles them as torch does for every such function (general, below).
 bool plain_call(std::initializer_list<const Tensor*> inputs, const Rope& rope) {
   if (c10::impl::tls_is_dispatch_key_included(c10::DispatchKey::FuncTorchDynamicLayerFrontMode) || at::tracer::impl::is_dispatch_enabled())
     return false;
@@ -659,14 +659,35 @@ PyObject* pack(std::initializer_list<Tensor> ts) {
   return t;
 }
 
-// apply(q, k, v, b_size, t_height, t_width, row_size, col_size, sm_scale); None: not a plain_call
+// The `apply` of torch.autograd.Function for TiledSwa, TiledSwaRope2D and TiledSwaPackedQKV: what is no plain_call goes there.
+// (Asked from here: a Python method around the native entry that looks at its answer costs every call 0.4 us.)
+PyObject* g_general[3] = {};
+PyObject* general(int i, PyObject* const* args, Py_ssize_t n) {
+  TORCH_CHECK(g_general[i], "set_general has not been called");
+  return PyObject_Vectorcall(g_general[i], args, (size_t)n, nullptr);
+}
+// set_general(three callables)
+PyObject* py_set_general(PyObject*, PyObject* const* args, Py_ssize_t n) {
+  return guarded([&]() -> PyObject* {
+    Args a{args, n};
+    for (PyObject*& g : g_general) {
+      PyObject* o = a.next();
+      Py_INCREF(o);
+      Py_XSETREF(g, o);
+    }
+    a.done();
+    Py_RETURN_NONE;
+  });
+}
+
+// apply(q, k, v, b_size, t_height, t_width, row_size, col_size, sm_scale)
 PyObject* py_tiled_swa(PyObject*, PyObject* const* args, Py_ssize_t n) {
   return guarded([&]() -> PyObject* {
     Args a{args, n};
     const Tensor q = a.tensor(), k = a.tensor(), v = a.tensor();
     const Win w = a.win();
     a.done();
-    if (!plain_call({&q, &k, &v}, Rope())) Py_RETURN_NONE;
+    if (!plain_call({&q, &k, &v}, Rope())) return general(0, args, n);
     return THPVariable_Wrap(without_gil([&] { return apply_swa(q, k, v, Rope(), w); }));
   });
 }
@@ -678,7 +699,7 @@ PyObject* py_tiled_swa_rope2d(PyObject*, PyObject* const* args, Py_ssize_t n) {
     const Rope r = a.rope();
     const Win w = a.win();
     a.done();
-    if (!plain_call({&q, &k, &v}, r)) Py_RETURN_NONE;
+    if (!plain_call({&q, &k, &v}, r)) return general(1, args, n);
     return THPVariable_Wrap(without_gil([&] { return apply_swa(q, k, v, r, w); }));
   });
 }
@@ -690,7 +711,7 @@ PyObject* py_tiled_swa_packed(PyObject*, PyObject* const* args, Py_ssize_t n) {
     const Rope r = a.rope();
     const Win w = a.win();
     a.done();
-    if (!plain_call({&qkv}, r)) Py_RETURN_NONE;
+    if (!plain_call({&qkv}, r)) return general(2, args, n);
     return THPVariable_Wrap(without_gil([&] { return apply_packed(qkv, r, w); }));
   });
 }
@@ -868,6 +889,7 @@ PyObject* py_poll_status(PyObject*, PyObject* const* args, Py_ssize_t n) {
 PyMethodDef g_methods[] = {SWA_DEF("tiled_swa", py_tiled_swa),
                            SWA_DEF("tiled_swa_rope2d", py_tiled_swa_rope2d),
                            SWA_DEF("tiled_swa_packed", py_tiled_swa_packed),
+                           SWA_DEF("set_general", py_set_general),
                            SWA_DEF("forward", py_forward),
                            SWA_DEF("forward_rot", py_forward_rot),
                            SWA_DEF("backward", py_backward),

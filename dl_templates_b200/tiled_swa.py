@@ -151,22 +151,15 @@ def tiled_swa_fwd(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, b_size: int
     return swa_forward(q, k, v, None, b_size, t_height, t_width, row_size, col_size, sm_scale)[0]
 
 
-class _NativeFunction(torch.autograd.Function):
-    """An autograd.Function whose ``apply`` runs natively (argument checks, launches and the autograd node in C++).  ``forward`` and
-    ``backward`` below are the general path: what carries forward-mode tangents, runs under functorch's transforms, is
-    being traced or has a Python dispatch of its own, where the native entry answers ``None``."""
-
-    @classmethod
-    def apply(cls, *args):
-        o = cls._native(*args)
-        return super().apply(*args) if o is None else o
-
-
-class TiledSwa(_NativeFunction):
+class TiledSwa(torch.autograd.Function):
     """``TiledSwa.apply(q, k, v, b_size, t_height, t_width, row_size, col_size, sm_scale)``
-    -- src/tiled_swa.py:602-689."""
+    -- src/tiled_swa.py:602-689.
 
-    _native = _native.tiled_swa
+    ``apply`` runs natively, here and in the two functions below (argument checks, launches and the autograd node in C++).
+    ``forward`` and ``backward`` are the general path: what carries forward-mode tangents, runs under functorch's transforms,
+    is being traced or has a Python dispatch of its own, which the native entry hands to ``Function.apply``."""
+
+    apply = staticmethod(_native.tiled_swa)
 
     @staticmethod
     def forward(ctx, q, k, v, *win):
@@ -216,7 +209,7 @@ def _mode_for(q, v, rope, win) -> str:
     return _ROPE_MODES[_native.rope_mode(q, v.shape[-1], *(rope or _NO_ROPE), *win)]
 
 
-class TiledSwaRope2D(_NativeFunction):
+class TiledSwaRope2D(torch.autograd.Function):
     """RoPE-2D and the attention as one differentiable function:
     ``TiledSwaRope2D.apply(q, k, v, idx, row_cs_buffer, col_cs_buffer, b_size, t_height, t_width, row_size, col_size,
     sm_scale)``.
@@ -228,7 +221,7 @@ class TiledSwaRope2D(_NativeFunction):
     ``idx`` may be ``None`` (no rotation).
     """
 
-    _native = _native.tiled_swa_rope2d
+    apply = staticmethod(_native.tiled_swa_rope2d)
 
     @staticmethod
     def forward(ctx, q, k, v, idx, row_cs_buffer, col_cs_buffer, *win):
@@ -262,7 +255,7 @@ class TiledSwaRope2D(_NativeFunction):
         return (*grads, *(None,) * 9)
 
 
-class TiledSwaPackedQKV(_NativeFunction):
+class TiledSwaPackedQKV(torch.autograd.Function):
     """The op between a packed QKV projection and the output projection, without the
     permute / contiguous copies either side of it.
 
@@ -276,7 +269,7 @@ class TiledSwaPackedQKV(_NativeFunction):
     Same mathematics as ``TiledSwaRope2D`` on the permuted views.
     """
 
-    _native = _native.tiled_swa_packed
+    apply = staticmethod(_native.tiled_swa_packed)
 
     @staticmethod
     def forward(ctx, qkv, idx, row_cs_buffer, col_cs_buffer, *win):
@@ -306,3 +299,6 @@ class TiledSwaPackedQKV(_NativeFunction):
         else:
             swa_backward(q, k, v, *saved, tuple(rest) or None, *ctx.win, out=outs)
         return (dqkv, *(None,) * 9)
+
+
+_native.set_general(*(super(cls, cls).apply for cls in (TiledSwa, TiledSwaRope2D, TiledSwaPackedQKV)))

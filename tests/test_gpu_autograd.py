@@ -66,7 +66,7 @@ def test_general_path_gives_what_the_native_one_gives(entry, monkeypatch):
         try:
             want = step()
             with monkeypatch.context() as m:
-                m.setattr(cls, "_native", staticmethod(lambda *a: None))
+                m.setattr(cls, "apply", super(cls, cls).apply)
                 got = step()
         finally:
             swa.set_rope_mode(prev)
