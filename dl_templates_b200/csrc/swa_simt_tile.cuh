@@ -10,8 +10,8 @@
 // Latency bounds it -- 8 to 12 warps an SM, half of the issue slots and two thirds of the shared-memory wavefronts used --
 // and what the bands cost: their barriers, and warps that wait for the one whose window has most of the band
 // (tile_band_rows in swa_abi.cu).  In vain are scored the columns of the warp's halo beyond a row's own window,
-// (4 + 2 wc) / (2 wc + 1), and one row in 2 wr + 2.  Training steps: 64 x 64, window 21, d = 64, 4 slices 641 -> 500 us, 32 x 32,
-// window 31, d = 128 1091 -> 523 us against one streamed token per lane and four resident rows per warp.
+// (4 + 2 wc) / (2 wc + 1), and one row in 2 wr + 2.  Training steps of 4 slices: 64 x 64, window 21, d = 64 641 -> 499 us, 32 x 32,
+// window 31, d = 128 1091 -> 506 us against one streamed token per lane and four resident rows per warp.
 #pragma once
 
 #include "swa_simt.cuh"
