@@ -235,8 +235,9 @@ bool strip_slides(const swa_geom_t* g, int R4, int KR) {
 // once per chunk), short ones spread a small problem over all SMs; the slowest SM's blocks decide, the taller of two equals.  The
 // height is a multiple of the block height, so that no row's blocks depend on it.
 // A call of a batch size not met before pays for this (three plans: 2 us at 24 x 24, 24 at 128 x 128 with one head, 470 at
-// 4096 x 64; walking every item of every height took 28, 750 and 11100): heights are taken in the order of a bound -- their mean load, their largest item -- and
-// the load of every CTA is put together only for those whose bound is not beyond the best load found.
+// 4096 x 64; walking every item of every height took 28, 750 and 11100): heights are taken in the order of a bound -- their
+// mean load, their largest item -- and the load of every CTA is put together only for those whose bound is not beyond the best
+// load found.
 void choose_chunk(const swa_geom_t* g, Plan* pl) {
   const int quarters = (g->t_height + pl->R4 - 1) / pl->R4;
   const int64_t strips = (int64_t)pl->n_tiles_x * g->B * g->H;
