@@ -207,14 +207,14 @@ bool make_plan_shape(const swa_geom_t* g, int which, int TH, int TW, uint32_t ta
 }
 
 // Shared memory of the strip kernels beside resident rows, ring and tables: alignment pad of the swizzled tiles, barrier /
-// exchange block, row parts of the window mask, dK/dV the lse / delta ring.
+// exchange block, row parts of the window mask, backward the lse / delta of streamed or resident rows.
 uint32_t strip_slack(const swa_geom_t* g, int which, int R4) {
   const uint32_t sh = which == 0 ? (uint32_t)sizeof(Fwd2Shared) : (uint32_t)sizeof(Bwd2Shared);
-  return 1024u + ((sh + 15u) & ~15u) + row_parts_bytes(g->row_size, R4) + (which == 2 ? (kMaskRing + 2) * 1024u : 0u);
+  return 1024u + ((sh + 15u) & ~15u) + row_parts_bytes(g->row_size, R4) + (which == 0 ? 0u : bwd_vec_bytes(which == 2));
 }
 
-// ... and the mask units: three per ring entry, the unused one.
-uint32_t mask_bytes(int N) { return (uint32_t)N * 16u * (3u * kMaskRing + 1u); }
+// ... and the mask units: three per ring entry.
+uint32_t mask_bytes(int N) { return (uint32_t)N * 16u * 3u * kMaskRing; }
 
 // Blocks of a chunk of `nq` quarters whose first row is r0 (the kernels' strip_item).
 int strip_blocks(const swa_geom_t* g, const Plan& pl, int r0, int nq) {
@@ -387,7 +387,8 @@ bool make_strip_shape(const swa_geom_t* g, int which, int TW, Plan* out) {
   while (pl.stages < kMaxStages && rest + (pl.stages + 1) * stage <= kSmemLimit) ++pl.stages;
   if (kn.stages) pl.stages = kn.stages;
   pl.smem_bytes = rest + pl.stages * stage;
-  pl.nsb = 2;
+  // backward: a third score buffer where tensor memory has room beside the two of dP (swa_tc_bwd2.cuh)
+  pl.nsb = which && 5 * pl.N + acc_cols <= 512 ? 3 : 2;
   if (which == 0) {
     // score buffers = look-ahead of the score MMAs: 3, or 4 when the block ring is deep enough to feed them (measured); with
     // columns of their own for P if that leaves three (swa_tc_fwd2.cuh), else P over the scores
@@ -400,7 +401,7 @@ bool make_strip_shape(const swa_geom_t* g, int which, int TW, Plan* out) {
   *out = pl;
   // tensor-memory columns of the final plan (the environment overrides above included): a plan beyond the
   // 512-column allocation is refused here, never launched
-  const uint32_t tmem_cols = (uint32_t)(which == 0 ? pl.nsb * pl.s_stride : 4 * pl.N) + (uint32_t)acc_cols;
+  const uint32_t tmem_cols = (uint32_t)(which == 0 ? pl.nsb * pl.s_stride : (pl.nsb + 2) * pl.N) + (uint32_t)acc_cols;
   return pl.smem_bytes <= kSmemLimit && pl.N % 16 == 0 && pl.N >= 16 && pl.N <= 256 && pl.N <= nmax && pl.stages >= 2 &&
          pl.stages <= kMaxStages && pl.nsb >= 2 && pl.nsb <= 4 && tmem_cols <= 512u;
 }
@@ -675,11 +676,11 @@ bool describe_plan(const swa_geom_t* g, const swa_rope_t* rope, int which, int32
     if (stride < N + (v2 ? pl.p_off / 2 : 0)) tmem = 1u << 30;   // a score buffer would not hold a block
   } else {
     used += pl.nxb * (qch + vch) * 16384u + x_fixed + pl.stages * (N * ((qch + vch) * 128u + xrow) + (v2 ? 0u : 1024u));
-    used += (((v2 ? (uint32_t)sizeof(Bwd2Shared) : (uint32_t)sizeof(BwdShared)) + 15u) & ~15u) + (v2 && kind == 2 ? (kMaskRing + 2) * 1024u : 0u);
-    tmem = 2 * 2 * N + 64u * qch + (kind == 2 ? 64u * vch : 0u);
+    used += (((v2 ? (uint32_t)sizeof(Bwd2Shared) : (uint32_t)sizeof(BwdShared)) + 15u) & ~15u) + (v2 ? bwd_vec_bytes(kind == 2) : 0u);
+    tmem = (v2 ? pl.nsb + 2 : 4) * N + 64u * qch + (kind == 2 ? 64u * vch : 0u);
   }
   used += pl.tab_bytes;
-  const int32_t v[12] = {pl.TH, pl.TW, pl.KR, pl.KW, pl.N, pl.stages, kind == 0 ? pl.nsb : 2, kind == 0 ? 2 : pl.nxb,
+  const int32_t v[12] = {pl.TH, pl.TW, pl.KR, pl.KW, pl.N, pl.stages, kind == 0 || v2 ? pl.nsb : 2, kind == 0 ? 2 : pl.nxb,
                          (int32_t)pl.tab_bytes, (int32_t)pl.smem_bytes, (int32_t)used, (int32_t)tmem};
   for (int i = 0; i < 12; ++i) out[i] = v[i];
   return true;

@@ -23,7 +23,7 @@ int sm_count();
 void refresh_env();
 
 // Resource plan the tensor-core kernel `which` would run with (host-only, no GPU needed): out[0..11] =
-// TH, TW, KR, KW, N, stages, score buffers (forward) / buffer pairs (backward), resident-tile buffers,
+// TH, TW, KR, KW, N, stages, score buffers (backward, streamed rotation: pairs), resident-tile buffers,
 // staged-table bytes, dynamic shared memory requested, shared memory the kernel's layout really uses
 // (with the worst-case alignment pad), tensor-memory columns used.  Returns false when no plan fits.
 bool describe_plan(const swa_geom_t* g, const swa_rope_t* rope, int which, int32_t* out);

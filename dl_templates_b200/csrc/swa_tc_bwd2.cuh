@@ -3,7 +3,7 @@
 // are rotated back to the un-rotated tensors in the epilogue).  Geometry (strips, quarters, slots): swa_tc_strip.cuh.
 //
 //   warp 0        TMA producer: streamed blocks, quarters of the resident side
-//   warp 1        SCORE issuer:  S = X_qk Y_qk^T (+ mask), dP = X_v Y_v^T into the block's (S, dP) pair
+//   warp 1        SCORE issuer:  S = X_qk Y_qk^T (+ mask), dP = X_v Y_v^T into the block's buffers
 //   warp 2        ACCUMULATE issuer: dV += P^T dO, dK += dS^T Q  resp.  dQ += dS K, A operand in tensor memory
 //   warp 3        window-mask units and lse / delta of every streamed block
 //   warps 4-11    two compute groups, one thread per resident row each, on either half of every block's columns
@@ -12,12 +12,12 @@
 // Why two issuers and epilogue warps: one warp that issues every MMA of the kernel runs a dependent scalar instruction
 // stream of about 2000 cycles per block (waits, descriptor arithmetic, commits) next to busy compute warps, while the
 // tensor pipe needs about 850 cycles for the same block; and an epilogue inside the compute groups idles both of them.
-// The order the single issuer gave for free ("the accumulating MMAs of the block that used this pair last were issued
-// before") is one more barrier, pair_free, that the accumulate issuer commits and the score issuer waits for.
+// The order the single issuer gave for free ("the accumulating MMAs of the block that used this buffer last were issued
+// before") is one more barrier, s_free, that the accumulate issuer commits and the score issuer waits for.
 //
-// All waits are bounded by polls, about a second each (umma.cuh).  A warp whose wait gave up runs its loops to the end without waiting
-// for or touching anything; the others run into their own limit, unless they have all they wait for.  At the end any of them
-// raises the CTA's flag: what is in flight is given time to land, TMEM is freed and the status word records it.
+// All waits are bounded by polls, about a second each (umma.cuh).  A warp whose wait gave up leaves its loop; the others run into
+// their own limit, unless they have all they wait for.  At the end any of them raises the CTA's flag: what is in flight is given
+// time to land, TMEM is freed and the status word records it.
 #pragma once
 
 #include "swa_tc_bwd.cuh"
@@ -26,13 +26,19 @@
 namespace swa {
 namespace tc {
 
+constexpr int kBwdRecs = kMaskRing + 3;   // block records (swa_tc_strip.cuh); at most three score buffers
+// Shared memory for the softmax statistics: dK/dV [record][-lse | -delta][128] of the streamed queries, dQ [use parity][slot]
+// [-lse | -delta][32] of the resident ones.
+__host__ __device__ constexpr uint32_t bwd_vec_bytes(bool dkdv) { return dkdv ? kBwdRecs * 1024u : 2048u; }
+
 struct Bwd2Shared {
   uint64_t x_full[2], x_empty[2];
-  uint64_t y_full[kMaxStages], y_empty[kMaxStages], y_ready[kMaskRing], yx_free[kMaskRing];
-  uint64_t sd_full[2], ds_full[2], pair_free[2];
+  uint64_t y_full[kMaxStages], y_empty[kMaxStages], rec_ready[kBwdRecs], yx_free[kMaskRing];
+  uint64_t sd_full[3], ds_full[3], s_free[3];   // per score buffer: S and dP are there; P / dS are; they have been accumulated
   // per slot: the quarter in it is complete; its dV / its dQ, dK accumulators have been read
   uint64_t acc_full[4], v_free[4], qk_free[4];
-  uint64_t vec_ready[kMaskRing + 2];   // dK/dV: the lse / delta slot of a block is written (one barrier per slot)
+  uint64_t xvec_full[2][4];            // dQ: lse / delta of a quarter are written
+  uint32_t rec[kBwdRecs];
   ItemStart start;
   uint32_t tmem_base;
   int abort_flag;
@@ -52,7 +58,7 @@ bwd2_kernel(const __grid_constant__ CUtensorMap tm_xqk, const __grid_constant__ 
   uint8_t* smem = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);   // an offset: the compiler keeps seeing shared memory
   const Plan& pl = p.pl;
   const int N = pl.N, nxb = pl.nxb, qch = ONE ? 1 : p.qch, vch = ONE ? 1 : p.vch;
-  constexpr int nsb = 2;                                         // (S, dP) buffer pairs, used in turn
+  const int nsb = pl.nsb;                                        // score buffers; dP has two, used in turn
   const uint32_t blk_bytes = (uint32_t)N * 128u;               // one 64-wide chunk of a streamed block
   const uint32_t xqk_bytes = qch * 16384u, xv_bytes = vch * 16384u, x_bytes = xqk_bytes + xv_bytes;
   const uint32_t yqk_stage = blk_bytes * qch, yv_stage = blk_bytes * vch;
@@ -61,23 +67,22 @@ bwd2_kernel(const __grid_constant__ CUtensorMap tm_xqk, const __grid_constant__ 
   uint8_t* stg_smem = x_smem + nxb * x_bytes;                   // output staging, pl.stg chunks per epilogue warp
   uint8_t* yqk_smem = stg_smem + 4 * pl.stg * kStageChunk;
   uint8_t* yv_smem = yqk_smem + pl.stages * yqk_stage;
-  uint8_t* xx_smem = yv_smem + pl.stages * yv_stage;            // window mask: indicator units of the resident rows,
-  uint8_t* yr_smem = xx_smem + 8192;                            // ... row units of the mask ring,
+  uint8_t* yr_smem = yv_smem + pl.stages * yv_stage;            // window mask: row units of the mask ring,
   uint8_t* yc_smem = yr_smem + kMaskRing * ub * (pl.TH >> 3);   // ... column units,
-  uint8_t* yz_smem = yc_smem + kMaskRing * ub * (pl.TW >> 3);  // ... the unused unit
-  // -lse / delta of the streamed queries (dK/dV): a ring of kMaskRing + 2 slots [slot][-lse | -delta][128], two deeper
-  // than the ring of mask units because the warp that fills both runs ahead of the compute warps
-  float* vec_smem = reinterpret_cast<float*>(yz_smem + ub);
-  constexpr int vslots = kMaskRing + 2;
-  Bwd2Shared* sh = reinterpret_cast<Bwd2Shared*>(reinterpret_cast<uint8_t*>(vec_smem) + (DKDV ? vslots * 1024 : 0));
+  uint8_t* xx_smem = yc_smem + kMaskRing * ub * (pl.TW >> 3);  // ... indicator units of the resident rows
+  float* vec_smem = reinterpret_cast<float*>(xx_smem + 8192);
+  Bwd2Shared* sh = reinterpret_cast<Bwd2Shared*>(reinterpret_cast<uint8_t*>(vec_smem) + bwd_vec_bytes(DKDV));
   uint8_t* row_parts = reinterpret_cast<uint8_t*>(sh) + ((sizeof(Bwd2Shared) + 15) & ~size_t(15));
-  // tensor memory: buffer pair b = (S at 2N b, dP at 2N b + N), accumulators behind the pairs
-  const uint32_t acc_qk = nsb * 2 * N, acc_v = acc_qk + qch * 64;
+  // Tensor memory: score buffer b at column N b, the two dP buffers behind them, then the accumulators.  P and dS replace the scores,
+  // 16 columns by 16 -- in dK/dV P in the first eight, dS in the others, so that a dP buffer is free once it has been read and the next
+  // block but one's dP need not wait for this one's accumulating MMAs.  With a third score buffer, where there is room, neither need
+  // its scores (31 x 31 window, d = 128, 4 slices: dK/dV, with three, 498 -> 434 us; dQ, with two, 326 -> 309).
+  const uint32_t dp0 = nsb * N, acc_qk = dp0 + 2 * N, acc_v = acc_qk + qch * 64;
 
   const int warp = threadIdx.x >> 5;
 
-  constexpr int n_bars = offsetof(Bwd2Shared, start) / 8, warps4 = offsetof(Bwd2Shared, ds_full) / 8;   // ds_full: one arrival per compute warp
-  for (int i = threadIdx.x; i < n_bars; i += kBwdThreads) mbar_init(reinterpret_cast<uint64_t*>(sh) + i, i == warps4 || i == warps4 + 1 ? 8 : 1);
+  constexpr int n_bars = offsetof(Bwd2Shared, rec) / 8, warps4 = offsetof(Bwd2Shared, ds_full) / 8;   // ds_full: one arrival per compute warp
+  for (int i = threadIdx.x; i < n_bars; i += kBwdThreads) mbar_init(reinterpret_cast<uint64_t*>(sh) + i, i >= warps4 && i < warps4 + 3 ? 8 : 1);
   if (threadIdx.x == 0) {
     sh->abort_flag = 0;
     item_start(p, &sh->start);
@@ -90,7 +95,6 @@ bwd2_kernel(const __grid_constant__ CUtensorMap tm_xqk, const __grid_constant__ 
   build_row_parts<BF16>(row_parts, threadIdx.x, kBwdThreads, p);
   if (threadIdx.x < 128) {
     write_indicator_units<BF16>(xx_smem, threadIdx.x, p);
-    if ((int)threadIdx.x < N) *reinterpret_cast<uint4*>(yz_smem + threadIdx.x * 16) = make_uint4(0u, 0u, 0u, 0u);
   }
   fence_proxy_async_smem();
   tc_fence_before();
@@ -100,14 +104,13 @@ bwd2_kernel(const __grid_constant__ CUtensorMap tm_xqk, const __grid_constant__ 
   pdl_wait();                                                    // from here on: global memory
   const uint32_t tmem = sh->tmem_base;
 
-  bool ok = true;   // warp-uniform: a failed wait does not leave the loops, but nothing is waited for or touched any more
+  bool ok = true;   // warp-uniform: false once a wait has given up
   auto wait_spin = [&](uint64_t* bar, uint32_t parity) {
-    if (ok) ok = __all_sync(0xffffffffu, mbar_wait_polls<0>(smem_u32(bar), parity));
+    ok &= __all_sync(0xffffffffu, mbar_wait_polls<0>(smem_u32(bar), parity)) != 0;
   };
   auto wait_park = [&](uint64_t* bar, uint32_t parity) {
-    if (ok) ok = __all_sync(0xffffffffu, mbar_wait_polls<100>(smem_u32(bar), parity));
+    ok &= __all_sync(0xffffffffu, mbar_wait_polls<100>(smem_u32(bar), parity)) != 0;
   };
-  const int n_mine = sh->start.count;
 
   // Registers follow the work: producer / issuer / mask warpgroup 104, compute 120, epilogue 168:
   // (104 + 2 * 120 + 168) * 128 = 64 Ki.
@@ -121,111 +124,78 @@ bwd2_kernel(const __grid_constant__ CUtensorMap tm_xqk, const __grid_constant__ 
     const uint32_t lane_base = tmem + ((uint32_t)(quarter * 32) << 16);
     const uint64_t c22 = f2_pack(p.scale_log2, p.scale_log2);
     const int ng = N >> 4;
-    uint32_t q0 = 0;                               // quarters before the current item
-    int tn = 0;
-    int buf = 0, buf_par = 0, vslot = 0, vpar = 0;   // buffer pair and lse / delta slot of the next block, their barriers' parities
     const int n1 = (ng + 1) >> 1;                  // first half: n1 steps of 16 columns
-    const int own_r = lane >> pl.tw_log, own_c = lane & (pl.TW - 1);
-    ItemWalk w(sh->start);
+    int buf = 0, buf_par = 0, rs = 0, rpar = 0;    // score buffer and record of the next block, their barriers' parities
+    uint32_t dp = dp0;                             // its dP buffer
+    int tn = 0;
+    bool second = g != 0;
+    float my_nlse = 0.f, my_ndelta = 0.f;          // dQ: of this thread's query
 #pragma unroll 1
-    for (int it = 0; it < n_mine; ++it, w.next(p)) {
-      const StripItem si = strip_item(p, w);
-      // this warp's slot holds the quarters qi, qi + 4, ...; [q_lo, q_hi] = the blocks quarter qi takes part in
-      int qi = (quarter - (int)q0) & 3;
-      int q_lo = quarter_first(p, si, qi), q_hi = quarter_last(p, si, qi);
-      float my_nlse = 0.f, my_delta = 0.f, nx_nlse = 0.f, nx_delta = 0.f;   // dQ: -lse and delta of this thread's query; of the next
-      auto fetch = [&](int i, float& a, float& b) {
-        a = -INFINITY;
-        b = 0.f;
-        if constexpr (!DKDV) {
-          const int tr = si.r0 + i * pl.R4 + own_r, tx = si.x0 + own_c;
-          if (i < si.nq && tr < p.t_h && tx < p.Wtok) {
-            const int64_t at = ((int64_t)(w.bi * p.H + w.hi) * p.t_h + tr) * p.Wtok + tx;
-            a = -lse[at];
-            b = delta[at];
-          }
-        }
-      };
-      fetch(qi, my_nlse, my_delta);
-      fetch(qi + 4, nx_nlse, nx_delta);
-#pragma unroll 1
-      for (int j = 0; j < si.nblk; ++j) {
-        trace_ev(p, 2 + g, tn, m == 0 && it >= p.trace_it, 0 * 16 + (j & 15));
-        const uint32_t s_tm = lane_base + buf * 2 * N, d_tm = s_tm + N;
-        uint64_t* const ds_bar = &sh->ds_full[buf];
-        wait_spin(&sh->sd_full[buf], buf_par);
-        trace_ev(p, 2 + g, tn, m == 0 && it >= p.trace_it, 1 * 16 + (j & 15));
-        const float* vec = vec_smem + vslot * 256;
-        // -lse / delta of the block's queries are staged.  One barrier per slot of that ring, not the stage's
-        // y_ready: the mask warp runs ahead of the block ring and may complete a stage's y_ready twice before this
-        // warp has looked at it, but it cannot refill a slot before this warp has read it.
-        if (DKDV) {
-          wait_spin(&sh->vec_ready[vslot], vpar);
-          if (++vslot == vslots) { vslot = 0; vpar ^= 1; }
-        }
-        buf ^= 1;
-        if (buf == 0) buf_par ^= 1;
-#pragma unroll 1
-        while (qi < si.nq && q_hi < j) {             // the quarter has left the slot: its successor
-          qi += 4;
-          q_lo = quarter_first(p, si, qi);
-          q_hi = quarter_last(p, si, qi);
-          my_nlse = nx_nlse;
-          my_delta = nx_delta;
-          fetch(qi + 4, nx_nlse, nx_delta);
-        }
-        // a quarter that takes no part in the block: its rows of P and dS are never read (umma_ts_slots)
-        const bool seen = qi < si.nq && q_lo <= j;
-        if (ok && seen) {
-          tc_fence_after();
-          // This group's half of the columns, 16 at a time.  P and dS go over the scores and dP already read, from the half's
-          // first column on.
-          const bool second = ((j ^ g) & 1) != 0;
-          const int c_lo = second ? 16 * n1 : 0, c_hi = second ? N : 16 * n1;
-          uint32_t out = c_lo;
-#pragma unroll 1
-          for (int c = c_lo; c < c_hi; c += 16, out += 8) {
-            uint32_t s[16], d[16];
-            tmem_ld16(s_tm + c, s);
-            tmem_ld16(d_tm + c, d);
-            uint32_t wp[8], ws[8];
-            uint64_t nl[8], ndl[8];                        // -lse, -delta of the columns
-#pragma unroll
-            for (int h = 0; h < 4; ++h) {
-              if constexpr (DKDV) {
-                const ulonglong2 a = *reinterpret_cast<const ulonglong2*>(vec + c + 4 * h), b = *reinterpret_cast<const ulonglong2*>(vec + 128 + c + 4 * h);
-                nl[2 * h] = a.x; nl[2 * h + 1] = a.y;
-                ndl[2 * h] = b.x; ndl[2 * h + 1] = b.y;
-              } else {
-                nl[2 * h] = nl[2 * h + 1] = f2_pack(my_nlse, my_nlse);
-                ndl[2 * h] = ndl[2 * h + 1] = f2_pack(-my_delta, -my_delta);
-              }
-            }
-            tmem_wait_ld();
-#pragma unroll
-            for (int h = 0; h < 8; ++h) {
-              const float2 x = f2_unpack(f2_fma(f2_pack(__uint_as_float(s[2 * h]), __uint_as_float(s[2 * h + 1])), c22, nl[h]));
-              const float p0 = exp2f(x.x), p1 = exp2f(x.y);
-              const uint64_t u = f2_add(f2_pack(__uint_as_float(d[2 * h]), __uint_as_float(d[2 * h + 1])), ndl[h]);
-              const float2 ds = f2_unpack(f2_mul(f2_pack(p0, p1), u));
-              ws[h] = pack2<BF16>(ds.x, ds.y);
-              if constexpr (DKDV) wp[h] = pack2<BF16>(p0, p1);
-            }
-            if constexpr (DKDV) {
-              tmem_st8(s_tm + out, wp);      // P^T over S^T
-              tmem_st8(d_tm + out, ws);      // dS^T over dP^T
-            } else {
-              tmem_st8(s_tm + out, ws);      // dS over S
-            }
-          }
-          tmem_wait_st();
-          tc_fence_before();
-          __syncwarp();
-        }
-        if (ok && lane == 0) mbar_arrive(ds_bar);
-        trace_ev(p, 2 + g, tn, m == 0 && it >= p.trace_it, 2 * 16 + (j & 15));
+    while (true) {
+      // what does not depend on the scores comes before the wait for them
+      trace_ev(p, 2 + g, tn, m == 0, 0 * 16 + rs);
+      wait_spin(&sh->rec_ready[rs], rpar);
+      const uint32_t rec = sh->rec[rs];
+      if (!ok || (rec & kRecEnd)) break;
+      // a quarter that takes no part in the block: its rows of P and dS are never read (umma_ts_slots)
+      const bool mine = rec >> (kRecAct + quarter) & 1u;
+      if (!DKDV && (rec >> (kRecFresh + quarter) & 1u)) {
+        const int use = rec >> (kRecUse + quarter) & 1;
+        wait_spin(&sh->xvec_full[use][quarter], rec >> (kRecUse2 + quarter) & 1u);
+        const float* xv = vec_smem + (use * 4 + quarter) * 64 + lane;
+        my_nlse = xv[0];
+        my_ndelta = xv[32];
       }
-      q0 += si.nq;
+      wait_spin(&sh->sd_full[buf], buf_par);
+      if (!ok) break;
+      trace_ev(p, 2 + g, tn, m == 0, 1 * 16 + rs);
+      if (mine) {
+        const uint32_t s_tm = lane_base + buf * N, d_tm = lane_base + dp;
+        [[maybe_unused]] const float* vec = vec_smem + rs * 256;
+        tc_fence_after();
+        // this group's half of the columns, 16 at a time
+        const int c_hi = second ? N : 16 * n1;
+#pragma unroll 1
+        for (int c = second ? 16 * n1 : 0; c < c_hi; c += 16) {
+          uint32_t s[16], d[16];
+          tmem_ld16(s_tm + c, s);
+          tmem_ld16(d_tm + c, d);
+          uint32_t w[DKDV ? 16 : 8];
+          uint64_t nl[8], ndl[8];                          // -lse, -delta of the columns
+#pragma unroll
+          for (int h = 0; h < 4; ++h) {
+            if constexpr (DKDV) {
+              const ulonglong2 a = *reinterpret_cast<const ulonglong2*>(vec + c + 4 * h), b = *reinterpret_cast<const ulonglong2*>(vec + 128 + c + 4 * h);
+              nl[2 * h] = a.x; nl[2 * h + 1] = a.y;
+              ndl[2 * h] = b.x; ndl[2 * h + 1] = b.y;
+            } else {
+              nl[2 * h] = nl[2 * h + 1] = f2_pack(my_nlse, my_nlse);
+              ndl[2 * h] = ndl[2 * h + 1] = f2_pack(my_ndelta, my_ndelta);
+            }
+          }
+          tmem_wait_ld();
+#pragma unroll
+          for (int h = 0; h < 8; ++h) {
+            const float2 x = f2_unpack(f2_fma(f2_pack(__uint_as_float(s[2 * h]), __uint_as_float(s[2 * h + 1])), c22, nl[h]));
+            const float p0 = exp2f(x.x), p1 = exp2f(x.y);
+            const uint64_t u = f2_add(f2_pack(__uint_as_float(d[2 * h]), __uint_as_float(d[2 * h + 1])), ndl[h]);
+            const float2 ds = f2_unpack(f2_mul(f2_pack(p0, p1), u));
+            w[DKDV ? 8 + h : h] = pack2<BF16>(ds.x, ds.y);
+            if constexpr (DKDV) w[h] = pack2<BF16>(p0, p1);
+          }
+          if constexpr (DKDV) tmem_st16(s_tm + c, w);
+          else tmem_st8(s_tm + c, w);
+        }
+        tmem_wait_st();
+        tc_fence_before();
+        __syncwarp();
+      }
+      if (lane == 0) mbar_arrive(&sh->ds_full[buf]);
+      trace_ev(p, 2 + g, tn, m == 0, 2 * 16 + rs);
+      second = !second;                            // the groups take turns with the larger half
+      dp ^= dp0 ^ (dp0 + N);
+      if (++buf == nsb) { buf = 0; buf_par ^= 1; }
+      if (++rs == kBwdRecs) { rs = 0; rpar ^= 1; }
     }
   } else if (warp < 4) {
     setmaxnreg_dec<104>();
@@ -233,7 +203,7 @@ bwd2_kernel(const __grid_constant__ CUtensorMap tm_xqk, const __grid_constant__ 
       // ------------------------------------------------------------------ TMA producer
       const LoadArgs f{x_smem, x_bytes, xqk_bytes, yqk_smem, yv_smem, yqk_stage, yv_stage, blk_bytes, sh->x_full, sh->x_empty,
                        sh->y_full, sh->y_empty, &sh->start, &tm_xqk, &tm_xv, &tm_yqk, &tm_yv};
-      load_warp(p, f, ok);
+      load_warp<ONE, true>(p, f, ok);
     } else if (warp == 1) {
       // ------------------------------------------------------------------ score issuer: S (+ mask) and dP of every block
       const uint32_t fmt = BF16 ? 1u : 0u;
@@ -243,70 +213,71 @@ bwd2_kernel(const __grid_constant__ CUtensorMap tm_xqk, const __grid_constant__ 
                      yqk_desc0 = smem_desc_from(smem_u32(yqk_smem), 16, hi_sw), yv_desc0 = smem_desc_from(smem_u32(yv_smem), 16, hi_sw),
                      xx_desc0 = smem_desc_from(smem_u32(xx_smem), 2048, hi_ns);
       const uint32_t yqk16 = yqk_stage >> 4, yv16 = yv_stage >> 4, blk16 = blk_bytes >> 4, x16 = x_bytes >> 4;
-      const uint32_t yr0 = smem_u32(yr_smem), yc0 = smem_u32(yc_smem), yz0 = smem_u32(yz_smem);
-      int stage = 0, stage_par = 0, buf = 0, xb = nxb - 1, x_par = 1;   // resident buffer in use; parity of its "full" phase
-      uint32_t G = 0;                                  // position in the CTA's stream of blocks
+      const uint32_t yr0 = smem_u32(yr_smem), yc0 = smem_u32(yc_smem), yz0 = smem_u32(xx_smem);
+      int stage = 0, stage_par = 0, buf = 0, buf_par = 1, xb = nxb - 1, x_par = 1;   // resident buffer in use; parity of its "full" phase
+      int rbuf = 0, rbuf_par = 0, started = 0;   // score buffer of the block that read this block's dP buffer last; blocks so far, up to 2
+      uint32_t dp = dp0;
+      int mslot = 0, rs = 0, rpar = 0;
+      const int stages = pl.stages;
+      // units of a ring entry: 0 and 1 of the first step, 2 and (unused) 3 of the second, from where and how far to the next entry
+      const uint32_t row_step = ub * (pl.TH >> 3), col_step = ub * (pl.TW >> 3);
+      const bool tw8 = pl.TW == 8;
+      const uint32_t el = elect_one();
       int tn = 0;
       const bool tl = (threadIdx.x & 31) == 0;
-      ItemWalk w(sh->start);
 #pragma unroll 1
-      for (int it = 0; it < n_mine; ++it, w.next(p)) {
-        const StripItem si = strip_item(p, w);
-        int hi = min(4, si.nq);                          // the first four quarters enter with the item
-        int next_first = hi < si.nq ? quarter_first(p, si, hi) : si.nblk;
-#pragma unroll 1
-        for (int j = 0; j < si.nblk; ++j, ++G) {
-          trace_ev(p, 1, tn, tl && it >= p.trace_it, 2 * 16 + (j & 15));
-          bool enters = j == 0;                          // a quarter enters: the next version of the resident rows
-#pragma unroll 1
-          while (next_first <= j) {
-            enters = true;
-            ++hi;
-            next_first = hi < si.nq ? quarter_first(p, si, hi) : si.nblk;
-          }
-          if (enters) {
-            if (++xb == nxb) { xb = 0; x_par ^= 1; }
-            wait_spin(&sh->x_full[xb], x_par);
-          }
-          wait_spin(&sh->y_full[stage], stage_par);    // the block has landed ...
-          const int mslot = G & (kMaskRing - 1);
-          wait_spin(&sh->y_ready[mslot], (G / kMaskRing) & 1);    // ... and its mask rows (and lse / delta) are written
-          // the pair is free once the accumulating MMAs of the block that used it last have completed
-          if (G >= 2) wait_spin(&sh->pair_free[buf], ((G >> 1) - 1) & 1);
-          if (ok) {
-            tc_fence_after();
-            if (elect_one()) {
-              const uint32_t s_tm = tmem + buf * 2 * N, d_tm = s_tm + N;
-              uint64_t xd = x_desc0 + (uint64_t)(xb * x16), yd = yqk_desc0 + (uint64_t)(stage * yqk16);
-              uint32_t acc = 0u;
-#pragma unroll 1
-              for (int c = 0; c < qch; ++c, xd += 1024 - 8, yd += blk16 - 8) {
-#pragma unroll
-                for (int k = 0; k < 4; ++k, xd += 2, yd += 2, acc = 1u) umma_ss(s_tm, xd, yd, idesc_s, acc);
-              }
-              // + indicator x penalty, the window mask: row units, column units, the unused unit
-              const uint32_t yc = yc0 + mslot * (ub * (pl.TW >> 3));
-              const uint32_t u0 = yr0 + mslot * (ub * (pl.TH >> 3)), u1 = pl.TW == 8 ? u0 + ub : yc, u2 = pl.TW == 8 ? yc : yc + ub;
-              umma_ss(s_tm, xx_desc0, smem_desc_from(u0, u1 - u0, hi_ns), idesc_s, 1u);
-              umma_ss(s_tm, xx_desc0 + 256, smem_desc_from(u2, yz0 - u2, hi_ns), idesc_s, 1u);
-              // xd now points at the v chunks of the resident rows
-              yd = yv_desc0 + (uint64_t)(stage * yv16);
-              acc = 0u;
-#pragma unroll 1
-              for (int c = 0; c < vch; ++c, xd += 1024 - 8, yd += blk16 - 8) {
-#pragma unroll
-                for (int k = 0; k < 4; ++k, xd += 2, yd += 2, acc = 1u) umma_ss(d_tm, xd, yd, idesc_s, acc);
-              }
-              umma_commit(&sh->sd_full[buf]);
-              umma_commit(&sh->yx_free[mslot]);                        // its mask units may be overwritten
-              if (next_first == j + 1 || j == si.nblk - 1) umma_commit(&sh->x_empty[xb]);   // last read of this version
-            }
-            __syncwarp();
-          }
-          trace_ev(p, 1, tn, tl && it >= p.trace_it, 3 * 16 + (j & 15));
-          buf ^= 1;
-          if (++stage == pl.stages) { stage = 0; stage_par ^= 1; }
+      while (true) {
+        trace_ev(p, 1, tn, tl, 2 * 16 + rs);
+        wait_spin(&sh->rec_ready[rs], rpar);         // the block's mask units (and lse / delta) are written
+        const uint32_t rec = sh->rec[rs];
+        if (!ok || (rec & kRecEnd)) break;
+        if (rec & kRecEnters) {                      // a quarter enters: the next version of the resident rows
+          if (++xb == nxb) { xb = 0; x_par ^= 1; }
+          wait_spin(&sh->x_full[xb], x_par);
         }
+        wait_spin(&sh->y_full[stage], stage_par);    // the block has landed
+        // the dP buffer is free once the compute groups are done with the block but one before
+        if (started == 2) {
+          wait_spin(&sh->ds_full[rbuf], rbuf_par);
+          if (++rbuf == nsb) { rbuf = 0; rbuf_par ^= 1; }
+        } else {
+          ++started;
+        }
+        if (!ok) break;
+        tc_fence_after();
+        const uint32_t s_tm = tmem + buf * N, d_tm = tmem + dp;
+        const uint64_t xd = x_desc0 + (uint64_t)(xb * x16), yd = yqk_desc0 + (uint64_t)(stage * yqk16);
+        const uint64_t xv = xd + (uint64_t)(qch * 1024), yv = yv_desc0 + (uint64_t)(stage * yv16);   // the v chunks
+#pragma unroll
+        for (int k = 0; k < 4; ++k) umma_ss_el(el, d_tm, xv + 2 * k, yv + 2 * k, idesc_s, k ? 1u : 0u);
+        if (vch > 1) {
+#pragma unroll
+          for (int k = 0; k < 4; ++k) umma_ss_el(el, d_tm, xv + 1024 + 2 * k, yv + blk16 + 2 * k, idesc_s, 1u);
+        }
+        // the score buffer is free once the accumulating MMAs of the block that used it last have completed
+        wait_spin(&sh->s_free[buf], buf_par);
+        if (!ok) break;
+        tc_fence_after();
+        // window mask, indicator x penalty: row units, column units, the unused unit
+        const uint32_t yc = yc0 + mslot * col_step;
+        const uint32_t u0 = yr0 + mslot * row_step, u1 = tw8 ? u0 + ub : yc, u2 = tw8 ? yc : yc + ub;
+        umma_ss_el(el, s_tm, xx_desc0, smem_desc_from(u0, u1 - u0, hi_ns), idesc_s, 0u);
+        umma_ss_el(el, s_tm, xx_desc0 + 256, smem_desc_from(u2, yz0 - u2, hi_ns), idesc_s, 1u);
+#pragma unroll
+        for (int k = 0; k < 4; ++k) umma_ss_el(el, s_tm, xd + 2 * k, yd + 2 * k, idesc_s, 1u);
+        if (qch > 1) {
+#pragma unroll
+          for (int k = 0; k < 4; ++k) umma_ss_el(el, s_tm, xd + 1024 + 2 * k, yd + blk16 + 2 * k, idesc_s, 1u);
+        }
+        umma_commit_el(el, &sh->sd_full[buf]);
+        umma_commit_el(el, &sh->yx_free[mslot]);                     // its mask units may be overwritten
+        if (rec & kRecLeaves) umma_commit_el(el, &sh->x_empty[xb]);   // last read of this version
+        trace_ev(p, 1, tn, tl, 3 * 16 + rs);
+        dp ^= dp0 ^ (dp0 + N);
+        if (++buf == nsb) { buf = 0; buf_par ^= 1; }
+        if (++stage == stages) { stage = 0; stage_par ^= 1; }
+        if (++mslot == kMaskRing) mslot = 0;
+        if (++rs == kBwdRecs) { rs = 0; rpar ^= 1; }
       }
     } else if (warp == 2) {
       // ------------------------------------------------------------------ accumulate issuer: A operands come from tensor memory
@@ -316,83 +287,49 @@ bwd2_kernel(const __grid_constant__ CUtensorMap tm_xqk, const __grid_constant__ 
       const uint32_t hi_sw = smem_desc_hi(1024, true);
       const uint64_t yqk_mn0 = smem_desc_from(smem_u32(yqk_smem), blk_bytes, hi_sw), yv_mn0 = smem_desc_from(smem_u32(yv_smem), blk_bytes, hi_sw);
       const uint32_t yqk16 = yqk_stage >> 4, yv16 = yv_stage >> 4;
-      const int nks = N >> 4, n1 = (nks + 1) >> 1;           // the second half of P / dS starts at column 16 n1
-      int stage = 0, buf = 0, buf_par = 0;
-      uint32_t q0 = 0;
+      const int stages = pl.stages;
+      const int nks = N >> 4;
+      int stage = 0, buf = 0, buf_par = 0, rs = 0, rpar = 0;
+      const uint32_t el = elect_one();
       int tn = 0;
       const bool tl = (threadIdx.x & 31) == 0;
-      ItemWalk w(sh->start);
 #pragma unroll 1
-      for (int it = 0; it < n_mine; ++it, w.next(p)) {
-        const StripItem si = strip_item(p, w);
-        QuarterCursor qc;
-        qc.begin(p, si);
+      while (true) {
+        trace_ev(p, 6, tn, tl, 0 * 16 + rs);
+        wait_spin(&sh->rec_ready[rs], rpar);
+        const uint32_t rec = sh->rec[rs];
+        if (!ok || (rec & kRecEnd)) break;
+        const uint32_t act = rec >> kRecAct & 15u, fresh = rec >> kRecFresh & 15u;
+        wait_spin(&sh->ds_full[buf], buf_par);
+        trace_ev(p, 6, tn, tl, 3 * 16 + rs);
+        // dV += P^T dO and dK += dS^T Q, resp. dQ += dS K
 #pragma unroll 1
-        for (int j = 0; j < si.nblk; ++j) {
-          trace_ev(p, 6, tn, tl && it >= p.trace_it, 0 * 16 + (j & 15));
-          uint32_t fresh = 0, held = 0, par = 0;           // slots whose quarter starts with this block; that held one before
+        for (int t = DKDV ? 0 : 1; t < 2; ++t) {
 #pragma unroll 1
-          while (qc.hi < si.nq && qc.next_first <= j) {
-            const uint32_t Q = q0 + qc.hi, bit = 1u << (Q & 3);
-            fresh |= bit;
-            if (Q >= 4) held |= bit;
-            if ((Q >> 2) & 1 ^ 1) par |= bit;
-            qc.next_first = quarter_first(p, si, ++qc.hi);
+          for (uint32_t h = fresh; h; h &= h - 1) {  // the accumulators' last quarter has been read
+            const int e = __ffs(h) - 1;
+            wait_spin((t ? sh->qk_free : sh->v_free) + e, (rec >> (kRecUse + e) & 1u) ^ 1u);
           }
-          qc.act |= fresh;
-          // the accumulators of those slots have been read (`bars`)
-          auto wait_read = [&](uint64_t* bars) {
-#pragma unroll 1
-            for (uint32_t h = held; h; h &= h - 1) {
-              const int e = __ffs(h) - 1;
-              wait_spin(bars + e, par >> e & 1);
-            }
-          };
-          wait_spin(&sh->ds_full[buf], buf_par);
-          trace_ev(p, 6, tn, tl && it >= p.trace_it, 3 * 16 + (j & 15));
-          trace_ev(p, 6, tn, tl && it >= p.trace_it, 4 * 16 + (j & 15));
-          uint32_t ends = 0;                               // slots whose quarter is complete with this block
-          const uint32_t act = qc.act;
-#pragma unroll 1
-          while (qc.lo < qc.hi && qc.lo_last <= j) {
-            ends |= 1u << ((q0 + qc.lo) & 3);
-            ++qc.lo;
-            qc.lo_last = quarter_last(p, si, qc.lo);
-          }
-          qc.act &= ~ends;
-          // dV += P^T dO and dK += dS^T Q, resp. dQ += dS K
-#pragma unroll 1
-          for (int t = DKDV ? 0 : 1; t < 2; ++t) {
-            wait_read(t ? sh->qk_free : sh->v_free);
-            if (ok && act) {
-              tc_fence_after();
-              if (elect_one())
-                accumulate_block(tmem + (t ? acc_qk : acc_v), tmem + buf * 2 * N + (DKDV && t ? N : 0),
-                                 t ? yqk_mn0 + (uint64_t)(stage * yqk16) : yv_mn0 + (uint64_t)(stage * yv16), t ? idesc_qk : idesc_v, nks, n1,
-                                 8 * n1, act, fresh);
-              __syncwarp();
-            }
-          }
-          if (ok) {
-            if (elect_one()) {
-              umma_commit(&sh->pair_free[buf]);
-              umma_commit(&sh->y_empty[stage]);
-#pragma unroll
-              for (int e = 0; e < 4; ++e)
-                if (ends & (1u << e)) umma_commit(&sh->acc_full[e]);
-            }
-            __syncwarp();
-          }
-          trace_ev(p, 6, tn, tl && it >= p.trace_it, 1 * 16 + (j & 15));
-          if (++stage == pl.stages) stage = 0;
-          buf ^= 1;
-          if (buf == 0) buf_par ^= 1;
+          if (!ok) break;
+          tc_fence_after();
+          if (act)
+            accumulate_block(el, tmem + (t ? acc_qk : acc_v), tmem + buf * N + (DKDV && t ? 8 : 0),
+                             t ? yqk_mn0 + (uint64_t)(stage * yqk16) : yv_mn0 + (uint64_t)(stage * yv16), t ? idesc_qk : idesc_v, nks, 16,
+                             act, fresh);
         }
-        q0 += si.nq;
+        if (!ok) break;
+        umma_commit_el(el, &sh->s_free[buf]);
+        umma_commit_el(el, &sh->y_empty[stage]);
+#pragma unroll 1
+        for (uint32_t h = rec >> kRecEnds & 15u; h; h &= h - 1) umma_commit_el(el, &sh->acc_full[__ffs(h) - 1]);
+        trace_ev(p, 6, tn, tl, 1 * 16 + rs);
+        if (++stage == stages) stage = 0;
+        if (++buf == nsb) { buf = 0; buf_par ^= 1; }
+        if (++rs == kBwdRecs) { rs = 0; rpar ^= 1; }
       }
     } else {
       // ------------------------------------------------------------------ window mask, lse / delta
-      const MaskArgs f{yr_smem, yc_smem, sh->yx_free, sh->y_ready, vec_smem, vslots, sh->vec_ready, lse, delta, row_parts, &sh->start};
+      const MaskArgs f{yr_smem, yc_smem, sh->yx_free, sh->rec, sh->rec_ready, kBwdRecs, vec_smem, lse, delta, row_parts, &sh->start};
       mask_warp<BF16, DKDV>(p, f, ok, wait_park);
     }
   } else {
@@ -457,67 +394,78 @@ bwd2_kernel(const __grid_constant__ CUtensorMap tm_xqk, const __grid_constant__ 
       }
     };
     int tn = 0;
-    int acc_par = 0;
-    uint32_t q0 = 0;
-    ItemWalk w(sh->start);
+    int use = 0;                                   // how often the slot has been used
+    const int n_mine = sh->start.count;
+    QuarterWalk qw(p, sh->start, slot);
+    // dQ: -lse and -delta of the slot's next quarter, one ahead of the accumulators
+    auto fetch = [&](int u) {
+      if (DKDV || !qw.more) return;
+      const int tr = qw.s.r0 + qw.i * pl.R4 + own_r, tx = qw.s.x0 + own_c;
+      float a = -INFINITY, b = 0.f;
+      if (tr < p.t_h && tx < p.Wtok) {
+        const int64_t at = ((int64_t)(qw.w.bi * p.H + qw.w.hi) * p.t_h + tr) * p.Wtok + tx;
+        a = -lse[at];
+        b = -delta[at];
+      }
+      float* xv = vec_smem + ((u & 1) * 4 + slot) * 64 + lane;
+      xv[0] = a;
+      xv[32] = b;
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&sh->xvec_full[u & 1][slot]);
+    };
+    fetch(0);
 #pragma unroll 1
-    for (int it = 0; it < n_mine; ++it, w.next(p)) {
-      const StripItem si = strip_item(p, w);
-#pragma unroll 1
-      for (int i = (slot - (int)q0) & 3; i < si.nq; i += 4) {
-        const int qr = si.r0 + i * pl.R4;
+    while (qw.more) {
+        const int qr = qw.s.r0 + qw.i * pl.R4, x0 = qw.s.x0, hi = qw.w.hi, bi = qw.w.bi;
+        qw.next(p, n_mine, slot);
+        fetch(use + 1);
         int irow = -1, icol = -1;
         if constexpr (NE > 0) {
-          const int tr = qr + own_r, tx = si.x0 + own_c;
+          const int tr = qr + own_r, tx = x0 + own_c;
           if (rope_on && tr < p.t_h && tx < p.Wtok) decode_idx(p.rope.idx[(int64_t)tr * p.Wtok + tx], p.rope.max_h, p.rope.max_w, irow, icol);
         }
-        trace_ev(p, 5, tn, slot == 0 && lane == 0 && it >= p.trace_it, 0 * 16 + (i & 15));
-        wait_park(&sh->acc_full[slot], acc_par);
-        acc_par ^= 1;
-        trace_ev(p, 5, tn, slot == 0 && lane == 0 && it >= p.trace_it, 1 * 16 + (i & 15));
-        if (!ok) continue;
+        trace_ev(p, 5, tn, slot == 0 && lane == 0, 0 * 16 + (use & 15));
+        wait_park(&sh->acc_full[slot], use & 1);
+        ++use;
+        trace_ev(p, 5, tn, slot == 0 && lane == 0, 1 * 16 + (use & 15));
+        if (!ok) break;
         tc_fence_after();
         if constexpr (ONE) {
           // Heads of at most 64: the accumulators are read at once and handed on before anything else is done with them --
           // where quarters follow each other block by block, the next block's MMAs wait for that.
-          if (lane == 0) tma_store_wait_read();          // the previous quarter's rows have left the staging
-          __syncwarp();
+          uint32_t a[DKDV ? 64 : 1], x[64];
           if constexpr (DKDV) {
-#pragma unroll 1
-            for (int h = 0; h < 2; ++h) {
-              uint32_t a[32];
-              tmem_ld32(lane_base + acc_v + 32 * h, a);
-              tmem_wait_ld();
-              if (h == 1) {
-                tc_fence_before();
-                __syncwarp();
-                if (lane == 0) mbar_arrive(&sh->v_free[slot]);
-              }
-#pragma unroll
-              for (int u = 0; u < 4; ++u) {
-                uint32_t wd[4];
-#pragma unroll
-                for (int e = 0; e < 4; ++e) wd[e] = pack2<BF16>(__uint_as_float(a[8 * u + 2 * e]), __uint_as_float(a[8 * u + 2 * e + 1]));
-                sts128(row0 + (((uint32_t)(4 * h + u) << 4) ^ swz_x), wd[0], wd[1], wd[2], wd[3]);
-              }
-            }
+            tmem_ld32(lane_base + acc_v, a);
+            tmem_ld32(lane_base + acc_v + 32, a + 32);
           }
-          uint32_t x[64];
           tmem_ld32(lane_base + acc_qk, x);
           tmem_ld32(lane_base + acc_qk + 32, x + 32);
           tmem_wait_ld();
           tc_fence_before();
+          if (lane == 0) tma_store_wait_read();          // the previous quarter's rows have left the staging
           __syncwarp();
-          if (lane == 0) mbar_arrive(&sh->qk_free[slot]);
-          trace_ev(p, 5, tn, slot == 0 && lane == 0 && it >= p.trace_it, 2 * 16 + (i & 15));
+          if (lane == 0) {
+            if constexpr (DKDV) mbar_arrive(&sh->v_free[slot]);
+            mbar_arrive(&sh->qk_free[slot]);
+          }
+          trace_ev(p, 5, tn, slot == 0 && lane == 0, 2 * 16 + (use & 15));
+          if constexpr (DKDV) {
+#pragma unroll
+            for (int u = 0; u < 8; ++u) {
+              uint32_t wd[4];
+#pragma unroll
+              for (int e = 0; e < 4; ++e) wd[e] = pack2<BF16>(__uint_as_float(a[8 * u + 2 * e]), __uint_as_float(a[8 * u + 2 * e + 1]));
+              sts128(row0 + (((uint32_t)u << 4) ^ swz_x), wd[0], wd[1], wd[2], wd[3]);
+            }
+          }
           const uint32_t row = row0 + (DKDV ? kStageChunk : 0u);
           put_half(x, 0, 0, p.sm_scale, rope_on, irow, icol, row);
           put_half(x + 32, 1, 0, p.sm_scale, rope_on, irow, icol, row);
           fence_proxy_async_smem();
           __syncwarp();
           if (lane == 0) {
-            if constexpr (DKDV) tma_store_5d(&tm_ov, stg, 0, si.x0, qr, w.hi, w.bi);
-            tma_store_5d(&tm_oqk, stg + (DKDV ? kStageChunk : 0u), 0, si.x0, qr, w.hi, w.bi);
+            if constexpr (DKDV) tma_store_5d(&tm_ov, stg, 0, x0, qr, hi, bi);
+            tma_store_5d(&tm_oqk, stg + (DKDV ? kStageChunk : 0u), 0, x0, qr, hi, bi);
             tma_store_commit();
           }
         } else {
@@ -549,7 +497,7 @@ bwd2_kernel(const __grid_constant__ CUtensorMap tm_xqk, const __grid_constant__ 
             fence_proxy_async_smem();
             __syncwarp();
             if (lane == 0) {
-              tma_store_5d(is_v ? &tm_ov : &tm_oqk, stg + sc * kStageChunk, 64 * c, si.x0, qr, w.hi, w.bi);
+              tma_store_5d(is_v ? &tm_ov : &tm_oqk, stg + sc * kStageChunk, 64 * c, x0, qr, hi, bi);
               tma_store_commit();
             }
             if (++sc == pl.stg && ch + 1 < nch) {
@@ -559,9 +507,7 @@ bwd2_kernel(const __grid_constant__ CUtensorMap tm_xqk, const __grid_constant__ 
             }
           }
         }
-        trace_ev(p, 5, tn, slot == 0 && lane == 0 && it >= p.trace_it, 3 * 16 + (i & 15));
-      }
-      q0 += si.nq;
+        trace_ev(p, 5, tn, slot == 0 && lane == 0, 3 * 16 + (use & 15));
     }
     if (lane == 0) tma_store_wait_all();
   }

@@ -32,7 +32,7 @@ struct Plan {
                        // streamed rotation, for halos wider than one block)
   int n_tiles_x, n_tiles_y;
   int stages;          // streamed-block pipeline depth
-  int nsb, nxb;        // backward: (S, dP) buffer pairs in tensor memory, resident-tile buffers in shared memory
+  int nsb, nxb;        // score buffers in tensor memory (backward, streamed rotation: (S, dP) pairs), resident-tile buffers in shared memory
   // Strip kernels (no streamed rotation, swa_tc_strip.cuh); n_tiles_y is then the number of chunks of a strip:
   int R4, nq;          // grid rows per quarter of the resident tile (32 / TW), quarters per chunk
   int tw_log;          // log2 of TW
@@ -58,7 +58,7 @@ struct KParams {
   int n_items;         // persistent kernels: work items = tiles per head x batch x heads
   int32_t* status;
   long long* trace;    // optional per-role clock64() samples of one CTA (performance debugging), else null
-  int trace_it;        // which work item of that CTA is sampled
+  int trace_it;        // blocks before the log starts
 };
 
 // Position of a resident-tile CTA and the halo it streams.
@@ -445,10 +445,14 @@ __device__ __forceinline__ void trace_mark(const KParams& p, int role, int k) {
 }
 
 // Event log of one CTA (performance debugging, -DSWA_TC_TRACE only): one designated thread of a role
-// appends (clock << 8 | tag) to that role's row of 256 entries; `n` is the thread's own cursor.
+// appends (clock << 8 | tag) to that role's row of 256 entries, from about its trace_it'th block on; `n` counts the events.
 __device__ __forceinline__ void trace_ev(const KParams& p, int role, int& n, bool on, int tag) {
 #ifdef SWA_TC_TRACE
-  if (on && p.trace != nullptr && blockIdx.x == 37 && n < 256) p.trace[128 + role * 256 + n++] = (clock64() << 8) | (long long)(tag & 255);
+  if (on && p.trace != nullptr && blockIdx.x == 37) {
+    constexpr int per_block[7] = {4, 2, 3, 3, 3, 1, 3};          // events a block of each role (about)
+    const int k = n++ - p.trace_it * per_block[role];
+    if (k >= 0 && k < 512) reinterpret_cast<uint32_t*>(p.trace)[256 + role * 512 + k] = (uint32_t)clock() << 8 | (uint32_t)(tag & 255);
+  }
 #endif
 }
 

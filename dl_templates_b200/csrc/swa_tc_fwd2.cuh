@@ -20,9 +20,9 @@
 // query tile in this kernel as well (about 400 dependent instructions per row on the critical path, 1.1 ms per launch
 // at the default workload, against 0.1 ms for a streaming pass over q).
 //
-// All waits are bounded by polls, about a second each (umma.cuh).  A warp whose wait gave up runs its loops to the end without waiting
-// for or touching anything; the others run into their own limit, unless they have all they wait for.  At the end any of them
-// raises the CTA's flag: what is in flight is given time to land, TMEM is freed and the status word records it.
+// All waits are bounded by polls, about a second each (umma.cuh).  A warp whose wait gave up leaves its loop; the others run into
+// their own limit, unless they have all they wait for.  At the end any of them raises the CTA's flag: what is in flight is given
+// time to land, TMEM is freed and the status word records it.
 #pragma once
 
 #include "swa_tc_fwd.cuh"
@@ -31,16 +31,19 @@
 namespace swa {
 namespace tc {
 
+constexpr int kFwdRecs = kMaskRing + 4;   // block records (swa_tc_strip.cuh); at most four score buffers
+
 struct Fwd2Shared {
   uint64_t q_full[2], q_empty[2];
-  uint64_t kv_full[kMaxStages], kv_empty[kMaxStages], k_ready[kMaskRing], kx_free[kMaskRing];
+  uint64_t kv_full[kMaxStages], kv_empty[kMaxStages], rec_ready[kFwdRecs], kx_free[kMaskRing];
   uint64_t s_full[4], p_full[4], s_free[4], pv_done[2];
-  uint64_t o_full[4], o_free[4];        // per slot: the quarter in it is complete / has been read
+  uint64_t o_full[2][4], o_free[2][4];  // per group and slot: the group's part of the quarter in it is complete / has been read
   // [quarter parity][slot]: running maximum and sum handed over, per group; read.  The softmax groups run up to nsb blocks ahead of
   // the PV MMAs -- with small windows that is several quarters of a slot -- so a barrier per slot alone could complete twice
   // before the epilogue warp looks.
   uint64_t ml_full[2][4][2], ml_empty[2][4];
   float ml[2][4][2][2][32];             // [quarter parity][slot][group][maximum | sum][row]
+  uint32_t rec[kFwdRecs];
   ItemStart start;
   uint32_t tmem_base;
   int abort_flag;
@@ -72,11 +75,10 @@ fwd2_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CU
   uint8_t* stg_smem = q_smem + 2 * q_bytes;                     // output staging, pl.stg chunks per epilogue warp
   uint8_t* k_smem = stg_smem + 4 * pl.stg * kStageChunk;
   uint8_t* v_smem = k_smem + pl.stages * k_stage;
-  uint8_t* qx_smem = v_smem + pl.stages * v_stage;              // window mask: indicator units of the query rows,
-  uint8_t* kr_smem = qx_smem + 8192;                            // ... row units of the mask ring,
+  uint8_t* kr_smem = v_smem + pl.stages * v_stage;              // window mask: row units of the mask ring,
   uint8_t* kc_smem = kr_smem + kMaskRing * ub * (pl.TH >> 3);   // ... column units,
-  uint8_t* kz_smem = kc_smem + kMaskRing * ub * (pl.TW >> 3);  // ... the unused unit
-  Fwd2Shared* sh = reinterpret_cast<Fwd2Shared*>(kz_smem + ub);
+  uint8_t* qx_smem = kc_smem + kMaskRing * ub * (pl.TW >> 3);  // ... indicator units of the query rows
+  Fwd2Shared* sh = reinterpret_cast<Fwd2Shared*>(qx_smem + 8192);
   uint8_t* row_parts = reinterpret_cast<uint8_t*>(sh) + ((sizeof(Fwd2Shared) + 15) & ~size_t(15));
 
   const int warp = threadIdx.x >> 5;
@@ -96,7 +98,6 @@ fwd2_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CU
   build_row_parts<BF16>(row_parts, threadIdx.x, kFwdThreads, p);
   if (threadIdx.x < 128) {
     write_indicator_units<BF16>(qx_smem, threadIdx.x, p);
-    if ((int)threadIdx.x < N) *reinterpret_cast<uint4*>(kz_smem + threadIdx.x * 16) = make_uint4(0u, 0u, 0u, 0u);
   }
   fence_proxy_async_smem();
   tc_fence_before();
@@ -106,12 +107,12 @@ fwd2_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CU
   pdl_wait();                                                    // from here on: global memory
   const uint32_t tmem = sh->tmem_base;
 
-  bool ok = true;   // warp-uniform: a failed wait does not leave the loops, but nothing is waited for or touched any more
+  bool ok = true;   // warp-uniform: false once a wait has given up
   auto wait_spin = [&](uint64_t* bar, uint32_t parity) {
-    if (ok) ok = __all_sync(0xffffffffu, mbar_wait_polls<0>(smem_u32(bar), parity));
+    ok &= __all_sync(0xffffffffu, mbar_wait_polls<0>(smem_u32(bar), parity)) != 0;
   };
   auto wait_park = [&](uint64_t* bar, uint32_t parity) {
-    if (ok) ok = __all_sync(0xffffffffu, mbar_wait_polls<100>(smem_u32(bar), parity));
+    ok &= __all_sync(0xffffffffu, mbar_wait_polls<100>(smem_u32(bar), parity)) != 0;
   };
   const int n_mine = sh->start.count;
 
@@ -129,149 +130,137 @@ fwd2_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CU
     const uint32_t o_tm = lane_base + o_base + g * o_cols;
     const float c2 = p.scale_log2;
     const int ng = N >> 4;                        // 16-column granules of a row
-    uint32_t gbase = 0, q0 = 0;                   // stream position of the current item's block 0, quarters before it
-    uint32_t own_next = g, n_own = 0;             // this group's next block in the stream; blocks done so far
-    int sbuf = g % nsb, spar = 0;                 // ... its score buffer and that buffer's barrier parity
+    uint32_t n_own = 0;                           // blocks this group has done
+    int rs = g, rpar = 0;                         // ring entry of this group's next record, its barrier's parity
+    int sbuf = g % nsb, spar = 0;                 // score buffer of that block, the same
     int tn = 0;
     float m_used = -INFINITY, l = 0.f;
-    ItemWalk w(sh->start);
 #pragma unroll 1
-    for (int it = 0; it < n_mine; ++it, w.next(p)) {
-      const StripItem si = strip_item(p, w);
-      // this warp's slot holds the quarters qi, qi + 4, ...; [q_lo, q_hi] = the blocks quarter qi takes part in
-      int qi = (quarter - (int)q0) & 3;
-      int q_lo = quarter_first(p, si, qi), q_hi = quarter_last(p, si, qi);
+    for (;; ++n_own) {
+      // what does not depend on the scores comes before the wait for them
+      wait_spin(&sh->rec_ready[rs], rpar);
+      if (!ok) break;
+      const uint32_t rec = sh->rec[rs] >> quarter;
+      if (sh->rec[rs] & kRecEnd) break;
+      const uint32_t s_tm = lane_base + sbuf * s_stride;
+      trace_ev(p, 2 + g, tn, m == 0, 0 * 16 + rs);
+      wait_spin(&sh->s_full[sbuf], spar);
+      if (!ok) break;
+      trace_ev(p, 2 + g, tn, m == 0, 1 * 16 + rs);
+      // a quarter that takes no part in the block: its rows of P are never read (umma_ts_slots)
+      if (rec >> kRecAct & 1u) {
+        const bool first = rec >> kRecGroupFirst & 1u;        // this group's first block of the quarter
+        if (first) { m_used = -INFINITY; l = 0.f; }
+        tc_fence_after();
+        uint32_t r[16];
+        float mx = -INFINITY, bl;
+        // The row maximum is taken before the exponentials in every block when P overwrites the scores, else only in a group's
+        // first block of a quarter: the others use the running maximum and see afterwards whether it still serves: a row
+        // whose maximum has grown by more than 2^8 is done again, which is rare.  (A load of 16 columns takes 14 cycles.)
+        bool exact = !OWNP || first;
+        tmem_ld16(s_tm, r);
+        if (exact) {
+          float mx4[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
 #pragma unroll 1
-      for (int j = (int)(own_next - gbase); j < si.nblk; j += 2, own_next += 2, ++n_own) {
-        const uint32_t s_tm = lane_base + sbuf * s_stride;
-        uint64_t* const p_bar = &sh->p_full[sbuf];
-        trace_ev(p, 2 + g, tn, m == 0 && it >= p.trace_it, 0 * 16 + (j & 15));
-        wait_spin(&sh->s_full[sbuf], spar);
-        trace_ev(p, 2 + g, tn, m == 0 && it >= p.trace_it, 1 * 16 + (j & 15));
-        sbuf += 2;                                // two positions on in the ring of nsb buffers
-        if (sbuf >= nsb) { sbuf -= nsb; spar ^= 1; }
-#pragma unroll 1
-        while (qi < si.nq && q_hi < j) {          // the quarter has left the slot: its successor
-          qi += 4;
-          q_lo = quarter_first(p, si, qi);
-          q_hi = quarter_last(p, si, qi);
-        }
-        // a quarter that takes no part in the block: its rows of P are never read (umma_ts_slots)
-        const bool seen = qi < si.nq && q_lo <= j;
-        if (ok && seen) {
-          const bool first = j - q_lo < 2;        // this group's first block of the quarter
-          if (first) { m_used = -INFINITY; l = 0.f; }
-          tc_fence_after();
-          uint32_t r[16];
-          float mx = -INFINITY, bl;
-          // The row maximum is taken before the exponentials in every block when P overwrites the scores, else only in a group's
-          // first block of a quarter: the others use the running maximum and see afterwards whether it still serves: a row
-          // whose maximum has grown by more than 2^8 is done again, which is rare.  16 columns at a time, the load of the next
-          // 16 in flight while these are worked on.
-          bool exact = !OWNP || first;
-          tmem_ld16(s_tm, r);
-          if (exact) {
+          for (int i = 0; i < ng; i += 2) {
             uint32_t t[16];
-            float mx4[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
-#pragma unroll 1
-            for (int i = 0; i < ng; i += 2) {
-              tmem_wait_ld();
-              if (i + 1 < ng) tmem_ld16(s_tm + 16 * (i + 1), t);
+            if (i + 1 < ng) tmem_ld16(s_tm + 16 * (i + 1), t);
+            tmem_wait_ld();
 #pragma unroll
-              for (int e = 0; e < 8; ++e) mx4[e & 3] = fmaxf(mx4[e & 3], fmaxf(__uint_as_float(r[2 * e]), __uint_as_float(r[2 * e + 1])));
-              if (i + 1 < ng) {
-                tmem_wait_ld();
-                if (i + 2 < ng) tmem_ld16(s_tm + 16 * (i + 2), r);
+            for (int e = 0; e < 8; ++e) mx4[e & 3] = fmaxf(mx4[e & 3], fmaxf(__uint_as_float(r[2 * e]), __uint_as_float(r[2 * e + 1])));
+            if (i + 1 < ng) {
+              if (i + 2 < ng) tmem_ld16(s_tm + 16 * (i + 2), r);
 #pragma unroll
-                for (int e = 0; e < 8; ++e) mx4[e & 3] = fmaxf(mx4[e & 3], fmaxf(__uint_as_float(t[2 * e]), __uint_as_float(t[2 * e + 1])));
-              }
+              for (int e = 0; e < 8; ++e) mx4[e & 3] = fmaxf(mx4[e & 3], fmaxf(__uint_as_float(t[2 * e]), __uint_as_float(t[2 * e + 1])));
             }
-            mx = fmaxf(fmaxf(mx4[0], mx4[1]), fmaxf(mx4[2], mx4[3]));
-            tmem_ld16(s_tm, r);                             // first 16 columns, in flight during the bookkeeping
           }
-#pragma unroll 1
-          while (true) {
-            if (exact) {
-              if (mx < none_thresh) mx = -INFINITY;
-              // running max with lazy rescale: keep scaling by m_used until the true max exceeds it by 2^8
-              bool need = false;
-              float m_new = m_used;
-              if (mx > m_used) {
-                if (m_used == -INFINITY) m_used = mx;       // nothing accumulated yet for this row
-                else if ((mx - m_used) * c2 > kRescaleThreshold) { need = true; m_new = mx; }
-              }
-              if (__any_sync(0xffffffffu, need) && !first) {
-                // O_g must be at rest: wait for the PV MMA of this group's previous block, then scale the row
-                wait_spin(&sh->pv_done[g], (n_own - 1) & 1);
-                if (ok) {
-                  tc_fence_after();
-                  const float alpha = need ? exp2f((m_used - m_new) * c2) : 1.f;
-                  tmem_wait_ld();
-#pragma unroll 1
-                  for (int c = 0; c < (int)o_cols; c += 16) {
-                    uint32_t t[16];
-                    tmem_ld16(o_tm + c, t);
-                    tmem_wait_ld();
-#pragma unroll
-                    for (int e = 0; e < 16; ++e) t[e] = __float_as_uint(__uint_as_float(t[e]) * alpha);
-                    tmem_st16(o_tm + c, t);
-                  }
-                  if (need) { m_used = m_new; l *= alpha; }
-                }
-              }
-            }
-            const float mc = (m_used == -INFINITY) ? 0.f : m_used * c2;
-            const uint64_t c22 = f2_pack(c2, c2), nmc2 = f2_pack(-mc, -mc);
-            // P = exp2(S*c - m), its row sum, (OWNP) the row maximum of S*c - m; packed, two columns of P per word
-            uint64_t ls[2] = {0ull, 0ull};
-            float mx2[2] = {-INFINITY, -INFINITY};
-#pragma unroll 1
-            for (int i = 0; i < ng; ++i) {
-              uint64_t e[8];
-              uint32_t w[8];
-              tmem_wait_ld();
-#pragma unroll
-              for (int h = 0; h < 8; ++h) e[h] = f2_fma(f2_pack(__uint_as_float(r[2 * h]), __uint_as_float(r[2 * h + 1])), c22, nmc2);
-              if (i + 1 < ng) tmem_ld16(s_tm + 16 * (i + 1), r);
-#pragma unroll
-              for (int h = 0; h < 8; ++h) {
-                const float2 x = f2_unpack(e[h]);
-                if constexpr (OWNP) mx2[h & 1] = fmaxf(mx2[h & 1], fmaxf(x.x, x.y));
-                const float p0 = exp2f(x.x), p1 = exp2f(x.y);
-                ls[h & 1] = f2_add(ls[h & 1], f2_pack(p0, p1));
-                w[h] = pack2<BF16>(p0, p1);
-              }
-              tmem_st8(s_tm + p_off + 8 * i, w);
-            }
-            const float2 l2 = f2_unpack(f2_add(ls[0], ls[1]));
-            bl = l2.x + l2.y;
-            if (exact) break;
-            // rows whose maximum passes the threshold (or that had none yet) are done again with the true one
-            const float emx = fmaxf(mx2[0], mx2[1]);
-            const bool again = m_used == -INFINITY ? emx > none_thresh * c2 : emx > kRescaleThreshold;
-            if (!__any_sync(0xffffffffu, again)) break;
-            mx = again ? (emx + mc) / c2 : m_used;
-            exact = true;
-            tmem_ld16(s_tm, r);
-          }
-          l += bl;
-          const uint32_t Q = q0 + qi;
-          const int qp = (int)(Q >> 2) & 1;
-          if (q_hi - j < 2) {                     // its last one: hand maximum and sum to the epilogue warp
-            if (Q >= 8) wait_spin(&sh->ml_empty[qp][quarter], ((Q >> 3) - 1) & 1);
-            sh->ml[qp][quarter][g][0][lane] = m_used;
-            sh->ml[qp][quarter][g][1][lane] = l;
-          }
-          tmem_wait_st();
-          tc_fence_before();
-          __syncwarp();
-          if (ok && q_hi - j < 2 && lane == 0) mbar_arrive(&sh->ml_full[qp][quarter][g]);
+          mx = fmaxf(fmaxf(mx4[0], mx4[1]), fmaxf(mx4[2], mx4[3]));
+          tmem_ld16(s_tm, r);                             // first 16 columns, in flight during the bookkeeping
         }
-        if (ok && lane == 0) mbar_arrive(p_bar);
-        trace_ev(p, 2 + g, tn, m == 0 && it >= p.trace_it, 2 * 16 + (j & 15));
+#pragma unroll 1
+        while (true) {
+          if (exact) {
+            if (mx < none_thresh) mx = -INFINITY;
+            // running max with lazy rescale: keep scaling by m_used until the true max exceeds it by 2^8
+            bool need = false;
+            float m_new = m_used;
+            if (mx > m_used) {
+              if (m_used == -INFINITY) m_used = mx;       // nothing accumulated yet for this row
+              else if ((mx - m_used) * c2 > kRescaleThreshold) { need = true; m_new = mx; }
+            }
+            if (__any_sync(0xffffffffu, need) && !first) {
+              // O_g must be at rest: wait for the PV MMA of this group's previous block, then scale the row
+              wait_spin(&sh->pv_done[g], (n_own - 1) & 1);
+              if (ok) {
+                tc_fence_after();
+                const float alpha = need ? exp2f((m_used - m_new) * c2) : 1.f;
+                tmem_wait_ld();
+#pragma unroll 1
+                for (int c = 0; c < (int)o_cols; c += 16) {
+                  uint32_t t[16];
+                  tmem_ld16(o_tm + c, t);
+                  tmem_wait_ld();
+#pragma unroll
+                  for (int e = 0; e < 16; ++e) t[e] = __float_as_uint(__uint_as_float(t[e]) * alpha);
+                  tmem_st16(o_tm + c, t);
+                }
+                if (need) { m_used = m_new; l *= alpha; }
+              }
+            }
+          }
+          const float mc = (m_used == -INFINITY) ? 0.f : m_used * c2;
+          const uint64_t c22 = f2_pack(c2, c2), nmc2 = f2_pack(-mc, -mc);
+          // P = exp2(S*c - m), its row sum, (OWNP) the row maximum of S*c - m; packed, two columns of P per word
+          uint64_t ls[2] = {0ull, 0ull};
+          float mx2[2] = {-INFINITY, -INFINITY};
+#pragma unroll 1
+          for (int i = 0; i < ng; ++i) {
+            uint64_t e[8];
+            uint32_t w[8];
+            tmem_wait_ld();
+#pragma unroll
+            for (int h = 0; h < 8; ++h) e[h] = f2_fma(f2_pack(__uint_as_float(r[2 * h]), __uint_as_float(r[2 * h + 1])), c22, nmc2);
+            if (i + 1 < ng) tmem_ld16(s_tm + 16 * (i + 1), r);
+#pragma unroll
+            for (int h = 0; h < 8; ++h) {
+              const float2 x = f2_unpack(e[h]);
+              if constexpr (OWNP) mx2[h & 1] = fmaxf(mx2[h & 1], fmaxf(x.x, x.y));
+              const float p0 = exp2f(x.x), p1 = exp2f(x.y);
+              ls[h & 1] = f2_add(ls[h & 1], f2_pack(p0, p1));
+              w[h] = pack2<BF16>(p0, p1);
+            }
+            tmem_st8(s_tm + p_off + 8 * i, w);
+          }
+          const float2 l2 = f2_unpack(f2_add(ls[0], ls[1]));
+          bl = l2.x + l2.y;
+          if (exact) break;
+          // rows whose maximum passes the threshold (or that had none yet) are done again with the true one
+          const float emx = fmaxf(mx2[0], mx2[1]);
+          const bool again = m_used == -INFINITY ? emx > none_thresh * c2 : emx > kRescaleThreshold;
+          if (!__any_sync(0xffffffffu, again)) break;
+          mx = again ? (emx + mc) / c2 : m_used;
+          exact = true;
+          tmem_ld16(s_tm, r);
+        }
+        l += bl;
+        const bool last = rec >> kRecGroupLast & 1u;
+        const int qp = rec >> kRecUse & 1u;
+        if (last) {                             // hand maximum and sum to the epilogue warp
+          wait_spin(&sh->ml_empty[qp][quarter], (rec >> kRecUse2 & 1u) ^ 1u);
+          sh->ml[qp][quarter][g][0][lane] = m_used;
+          sh->ml[qp][quarter][g][1][lane] = l;
+        }
+        tmem_wait_st();
+        tc_fence_before();
+        __syncwarp();
+        if (last && lane == 0) mbar_arrive(&sh->ml_full[qp][quarter][g]);
       }
-      gbase += si.nblk;
-      q0 += si.nq;
+      if (lane == 0) mbar_arrive(&sh->p_full[sbuf]);
+      trace_ev(p, 2 + g, tn, m == 0, 2 * 16 + rs);
+      sbuf += 2;                                  // two positions on in the ring of nsb buffers
+      if (sbuf >= nsb) { sbuf -= nsb; spar ^= 1; }
+      rs += 2;
+      if (rs >= kFwdRecs) { rs -= kFwdRecs; rpar ^= 1; }
     }
   } else if (warp < 4) {
     setmaxnreg_dec<104>();
@@ -279,73 +268,61 @@ fwd2_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CU
       // ------------------------------------------------------------------ TMA producer
       const LoadArgs f{q_smem, q_bytes, q_bytes, k_smem, v_smem, k_stage, v_stage, blk_bytes, sh->q_full, sh->q_empty,
                        sh->kv_full, sh->kv_empty, &sh->start, &tm_q, nullptr, &tm_k, &tm_v};
-      load_warp(p, f, ok);
+      load_warp<ONE, false>(p, f, ok);
     } else if (warp == 1) {
-      // ------------------------------------------------------------------ score issuer
+      // ------------------------------------------------------------------ score issuer 
       const uint32_t fmt = BF16 ? 1u : 0u;
       const uint32_t idesc_s = instr_desc(fmt, 128, N, 0, 0);
       const uint32_t hi_sw = smem_desc_hi(1024, true), hi_ns = smem_desc_hi(kUnitSbo, false);
       const uint64_t q_desc0 = smem_desc_from(smem_u32(q_smem), 16, hi_sw), k_desc0 = smem_desc_from(smem_u32(k_smem), 16, hi_sw),
                      qx_desc0 = smem_desc_from(smem_u32(qx_smem), 2048, hi_ns);
       const uint32_t k_stage16 = k_stage >> 4, blk16 = blk_bytes >> 4;
-      const uint32_t kr0 = smem_u32(kr_smem), kc0 = smem_u32(kc_smem), kz0 = smem_u32(kz_smem);
-      int stage = 0, stage_par = 0, buf = 0, xb = 1, x_par = 1;   // query buffer in use; parity of its "full" phase
-      int mslot = 0, m_par = 0;
-      uint32_t use = 0;                              // how often the ring of score buffers has wrapped
+      const uint32_t kr0 = smem_u32(kr_smem), kc0 = smem_u32(kc_smem), kz0 = smem_u32(qx_smem);
+      int stage = 0, stage_par = 0, buf = 0, buf_par = 1, xb = 1, x_par = 1;   // query buffer in use; parity of its "full" phase
+      int mslot = 0, rs = 0, rpar = 0;
+      const int stages = pl.stages;
+      // units of a ring entry: 0 and 1 of the first step, 2 and (unused) 3 of the second, from where and how far to the next entry
+      const uint32_t row_step = ub * (pl.TH >> 3), col_step = ub * (pl.TW >> 3);
+      const bool tw8 = pl.TW == 8;
+      const uint32_t el = elect_one();
       int tn = 0;
-      const bool tl = (threadIdx.x & 31) == 0;
-      ItemWalk w(sh->start);
 #pragma unroll 1
-      for (int it = 0; it < n_mine; ++it, w.next(p)) {
-        const StripItem si = strip_item(p, w);
-        int hi = min(4, si.nq);                        // the first four quarters enter with the item
-        int next_first = hi < si.nq ? quarter_first(p, si, hi) : si.nblk;
-#pragma unroll 1
-        for (int j = 0; j < si.nblk; ++j) {
-          trace_ev(p, 1, tn, tl && it >= p.trace_it, 2 * 16 + (j & 15));
-          bool enters = j == 0;                        // a quarter enters: the next version of the query rows
-#pragma unroll 1
-          while (next_first <= j) {
-            enters = true;
-            ++hi;
-            next_first = hi < si.nq ? quarter_first(p, si, hi) : si.nblk;
-          }
-          if (enters) {
-            xb ^= 1;
-            if (xb == 0) x_par ^= 1;
-            wait_spin(&sh->q_full[xb], x_par);
-          }
-          wait_spin(&sh->kv_full[stage], stage_par);    // the block has landed ...
-          wait_spin(&sh->k_ready[mslot], m_par);        // ... and its window-mask units are written
-          // the buffer is free once the PV MMA of the block that used it last has completed
-          if (use >= 1) wait_spin(&sh->s_free[buf], (use - 1) & 1);
-          if (ok) {
-            tc_fence_after();
-            if (elect_one()) {
-              const uint32_t sd = tmem + buf * s_stride;
-              uint64_t qd = q_desc0 + (uint64_t)(xb * (q_bytes >> 4)), kd = k_desc0 + (uint64_t)(stage * k_stage16);
-              uint32_t acc = 0u;
-#pragma unroll 1
-              for (int c = 0; c < qch; ++c, qd += 1024 - 8, kd += blk16 - 8) {
-#pragma unroll
-                for (int k = 0; k < 4; ++k, qd += 2, kd += 2, acc = 1u) umma_ss(sd, qd, kd, idesc_s, acc);
-              }
-              // + indicator x penalty, the window mask: row units, column units, the unused unit
-              const uint32_t yc = kc0 + mslot * (ub * (pl.TW >> 3));
-              const uint32_t u0 = kr0 + mslot * (ub * (pl.TH >> 3)), u1 = pl.TW == 8 ? u0 + ub : yc, u2 = pl.TW == 8 ? yc : yc + ub;
-              umma_ss(sd, qx_desc0, smem_desc_from(u0, u1 - u0, hi_ns), idesc_s, 1u);
-              umma_ss(sd, qx_desc0 + 256, smem_desc_from(u2, kz0 - u2, hi_ns), idesc_s, 1u);
-              umma_commit(&sh->s_full[buf]);
-              umma_commit(&sh->kx_free[mslot]);                        // its mask units may be overwritten
-              if (next_first == j + 1 || j == si.nblk - 1) umma_commit(&sh->q_empty[xb]);   // last read of this version
-            }
-            __syncwarp();
-          }
-          trace_ev(p, 1, tn, tl && it >= p.trace_it, 3 * 16 + (j & 15));
-          if (++stage == pl.stages) { stage = 0; stage_par ^= 1; }
-          if (++mslot == kMaskRing) { mslot = 0; m_par ^= 1; }
-          if (++buf == nsb) { buf = 0; ++use; }
+      while (true) {
+        trace_ev(p, 1, tn, (threadIdx.x & 31) == 0, 2 * 16 + rs);
+        wait_spin(&sh->rec_ready[rs], rpar);          // the block's window-mask units are written
+        const uint32_t rec = sh->rec[rs];
+        if (!ok || (rec & kRecEnd)) break;
+        if (rec & kRecEnters) {                       // a quarter enters: the next version of the query rows
+          xb ^= 1;
+          if (xb == 0) x_par ^= 1;
+          wait_spin(&sh->q_full[xb], x_par);
         }
+        wait_spin(&sh->kv_full[stage], stage_par);    // the block has landed
+        // the buffer is free once the PV MMA of the block that used it last has completed
+        wait_spin(&sh->s_free[buf], buf_par);
+        if (!ok) break;
+        tc_fence_after();
+        const uint32_t sd = tmem + buf * s_stride;
+        // window mask, indicator x penalty: row units, column units, the unused unit
+        const uint32_t yc = kc0 + mslot * col_step;
+        const uint32_t u0 = kr0 + mslot * row_step, u1 = tw8 ? u0 + ub : yc, u2 = tw8 ? yc : yc + ub;
+        umma_ss_el(el, sd, qx_desc0, smem_desc_from(u0, u1 - u0, hi_ns), idesc_s, 0u);
+        umma_ss_el(el, sd, qx_desc0 + 256, smem_desc_from(u2, kz0 - u2, hi_ns), idesc_s, 1u);
+        const uint64_t qd = q_desc0 + (uint64_t)(xb * (q_bytes >> 4)), kd = k_desc0 + (uint64_t)(stage * k_stage16);
+#pragma unroll
+        for (int k = 0; k < 4; ++k) umma_ss_el(el, sd, qd + 2 * k, kd + 2 * k, idesc_s, 1u);
+        if (qch > 1) {
+#pragma unroll
+          for (int k = 0; k < 4; ++k) umma_ss_el(el, sd, qd + 1024 + 2 * k, kd + blk16 + 2 * k, idesc_s, 1u);
+        }
+        umma_commit_el(el, &sh->s_full[buf]);
+        umma_commit_el(el, &sh->kx_free[mslot]);                     // its mask units may be overwritten
+        if (rec & kRecLeaves) umma_commit_el(el, &sh->q_empty[xb]);   // last read of this version
+        trace_ev(p, 1, tn, (threadIdx.x & 31) == 0, 3 * 16 + rs);
+        if (++stage == stages) { stage = 0; stage_par ^= 1; }
+        if (++mslot == kMaskRing) mslot = 0;
+        if (++buf == nsb) { buf = 0; buf_par ^= 1; }
+        if (++rs == kFwdRecs) { rs = 0; rpar ^= 1; }
       }
     } else if (warp == 2) {
       // ------------------------------------------------------------------ PV issuer: O_g += P V, P from tensor memory
@@ -354,67 +331,44 @@ fwd2_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CU
       const uint32_t hi_sw = smem_desc_hi(1024, true);
       const uint64_t v_desc0 = smem_desc_from(smem_u32(v_smem), blk_bytes, hi_sw);
       const uint32_t v_stage16 = v_stage >> 4;
+      const int stages = pl.stages;
       const int nks = N >> 4;
-      int stage = 0, buf = 0, buf_par = 0, grp = 0;
-      uint32_t q0 = 0;
+      int stage = 0, buf = 0, buf_par = 0, grp = 0, rs = 0, rpar = 0;
+      const uint32_t el = elect_one();
       int tn = 0;
-      const bool tl = (threadIdx.x & 31) == 0;
-      ItemWalk w(sh->start);
 #pragma unroll 1
-      for (int it = 0; it < n_mine; ++it, w.next(p)) {
-        const StripItem si = strip_item(p, w);
-        QuarterCursor qc;
-        qc.begin(p, si);
-        uint32_t before = 0;                               // slots whose quarters entered with the previous block
+      while (true) {
+        trace_ev(p, 6, tn, (threadIdx.x & 31) == 0, 0 * 16 + rs);
+        // everything that does not depend on P first: what follows the wait for it is the chain of a score buffer
+        wait_spin(&sh->rec_ready[rs], rpar);
+        const uint32_t rec = sh->rec[rs];
+        if (!ok || (rec & kRecEnd)) break;
+        const uint32_t act = rec >> kRecAct & 15u, fresh = act & rec >> kRecGroupFirst;   // first block of these quarters for this group's O_g
 #pragma unroll 1
-        for (int j = 0; j < si.nblk; ++j) {
-          trace_ev(p, 6, tn, tl && it >= p.trace_it, 0 * 16 + (j & 15));
-          uint32_t entered = 0;                            // slots whose quarter starts with this block
-#pragma unroll 1
-          while (qc.hi < si.nq && qc.next_first <= j) {
-            const uint32_t Q = q0 + qc.hi;
-            if (Q >= 4) wait_spin(&sh->o_free[Q & 3], ((Q >> 2) - 1) & 1);   // its accumulators' last quarter has been read
-            entered |= 1u << (Q & 3);
-            qc.next_first = quarter_first(p, si, ++qc.hi);
-          }
-          qc.act |= entered;
-          wait_spin(&sh->p_full[buf], buf_par);
-          trace_ev(p, 6, tn, tl && it >= p.trace_it, 4 * 16 + (j & 15));
-          const uint32_t act = qc.act, fresh = act & (entered | before);   // first block of these quarters for this group's O_g
-          before = entered;
-          uint32_t ends = 0;                               // slots whose quarter is complete with this block
-#pragma unroll 1
-          while (qc.lo < qc.hi && qc.lo_last <= j) {
-            ends |= 1u << ((q0 + qc.lo) & 3);
-            ++qc.lo;
-            qc.lo_last = quarter_last(p, si, qc.lo);
-          }
-          qc.act &= ~ends;
-          if (ok) {
-            tc_fence_after();
-            if (elect_one()) {
-              if (act)
-                accumulate_block(tmem + o_base + grp * o_cols, tmem + buf * s_stride + p_off, v_desc0 + (uint64_t)(stage * v_stage16), idesc_pv, nks,
-                                 nks, 0, act, fresh);
-              umma_commit(&sh->s_free[buf]);
-              umma_commit(&sh->kv_empty[stage]);
-              umma_commit(&sh->pv_done[grp]);
-#pragma unroll
-              for (int e = 0; e < 4; ++e)
-                if (ends & (1u << e)) umma_commit(&sh->o_full[e]);
-            }
-            __syncwarp();
-          }
-          trace_ev(p, 6, tn, tl && it >= p.trace_it, 1 * 16 + (j & 15));
-          grp ^= 1;
-          if (++stage == pl.stages) stage = 0;
-          if (++buf == nsb) { buf = 0; buf_par ^= 1; }
+        for (uint32_t h = fresh; h; h &= h - 1) {        // the accumulator's last quarter has been read
+          const int e = __ffs(h) - 1;
+          wait_spin(&sh->o_free[grp][e], (rec >> (kRecUse + e) & 1u) ^ 1u);
         }
-        q0 += si.nq;
+        wait_spin(&sh->p_full[buf], buf_par);
+        if (!ok) break;
+        trace_ev(p, 6, tn, (threadIdx.x & 31) == 0, 4 * 16 + rs);
+        tc_fence_after();
+        accumulate_block(el, tmem + o_base + grp * o_cols, tmem + buf * s_stride + p_off, v_desc0 + (uint64_t)(stage * v_stage16), idesc_pv, nks,
+                         8, act, fresh);
+        umma_commit_el(el, &sh->s_free[buf]);
+        umma_commit_el(el, &sh->kv_empty[stage]);
+        umma_commit_el(el, &sh->pv_done[grp]);
+#pragma unroll 1
+        for (uint32_t h = act & rec >> kRecGroupLast; h; h &= h - 1) umma_commit_el(el, &sh->o_full[grp][__ffs(h) - 1]);
+        trace_ev(p, 6, tn, (threadIdx.x & 31) == 0, 1 * 16 + rs);
+        grp ^= 1;
+        if (++stage == stages) stage = 0;
+        if (++buf == nsb) { buf = 0; buf_par ^= 1; }
+        if (++rs == kFwdRecs) { rs = 0; rpar ^= 1; }
       }
     } else {
       // ------------------------------------------------------------------ window mask
-      const MaskArgs f{kr_smem, kc_smem, sh->kx_free, sh->k_ready, nullptr, 0, nullptr, nullptr, nullptr, row_parts, &sh->start};
+      const MaskArgs f{kr_smem, kc_smem, sh->kx_free, sh->rec, sh->rec_ready, kFwdRecs, nullptr, nullptr, nullptr, row_parts, &sh->start};
       mask_warp<BF16, false>(p, f, ok, wait_park);
     }
   } else {
@@ -427,51 +381,63 @@ fwd2_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CU
     uint8_t* const stg = stg_smem + slot * pl.stg * kStageChunk;
     const uint32_t row0 = smem_u32(stg) + lane * 128, swz_x = (uint32_t)(lane & 7) << 4;
     int tn = 0;
-    int o_par = 0, ml_par = 0;                      // barrier parities (ml: bit per quarter parity and group)
+    int o_par = 0, ml_par = 0;                      // barrier parities (o: bit per group; ml: per quarter parity and group)
     uint32_t gb = 0, q0 = 0;
     ItemWalk w(sh->start);
 #pragma unroll 1
     for (int it = 0; it < n_mine; ++it, w.next(p)) {
       const StripItem si = strip_item(p, w);
-      // Blocks are even or odd by their position in the grid.  The two parities' partial results are merged in that order, not
-      // by which group happened to take them: the result of a row must not depend on the work that preceded it.
-      const int a0 = (int)((uint32_t)(si.h0 + p.wr) / (uint32_t)pl.KR) * pl.ncb;     // grid position of the item's block 0
-      const int g_even = (int)((gb + (uint32_t)a0) & 1u);   // the group that took the even blocks
 #pragma unroll 1
       for (int i = (slot - (int)q0) & 3; i < si.nq; i += 4) {
-        const int qr = si.r0 + i * pl.R4;
-        const int b_lo = a0 + quarter_first(p, si, i), b_hi = a0 + quarter_last(p, si, i);
-        const bool has_e = b_hi > b_lo || !(b_lo & 1), has_d = b_hi > b_lo || (b_lo & 1);
+        // The groups' partial results are merged in the order in which they become complete, which the blocks' positions in the grid
+        // decide: the result of a row does not depend on the work that preceded it.  The one that is complete a block earlier is
+        // read -- and its accumulator handed on -- then: where quarters follow each other block by block the next block wants it.
+        const int qr = si.r0 + i * pl.R4, b_lo = quarter_first(p, si, i), b_hi = quarter_last(p, si, i);
+        const int g2 = (int)((gb + (uint32_t)b_hi) & 1u), g1 = g2 ^ 1;      // the group of the last block, the other one
+        const bool both = b_hi > b_lo;
         const int qp = (int)((q0 + i) >> 2) & 1;
-        float m_e = -INFINITY, l_e = 0.f, m_d = -INFINITY, l_d = 0.f;
-        trace_ev(p, 5, tn, slot == 0 && lane == 0 && it >= p.trace_it, 0 * 16 + (i & 15));
-        if (has_e) {
-          wait_park(&sh->ml_full[qp][slot][g_even], (ml_par >> (2 * qp + g_even)) & 1);
-          ml_par ^= 1 << (2 * qp + g_even);
-          m_e = sh->ml[qp][slot][g_even][0][lane];
-          l_e = sh->ml[qp][slot][g_even][1][lane];
+        float m_1 = -INFINITY, l_1 = 0.f;
+        trace_ev(p, 5, tn, slot == 0 && lane == 0, 0 * 16 + (i & 15));
+        const uint32_t o_2 = lane_base + o_base + g2 * o_cols, o_1 = lane_base + o_base + (both ? g1 : g2) * o_cols;
+        [[maybe_unused]] uint32_t x[ONE ? 64 : 1];
+        if (both) {
+          wait_park(&sh->ml_full[qp][slot][g1], (ml_par >> (2 * qp + g1)) & 1);
+          ml_par ^= 1 << (2 * qp + g1);
+          m_1 = sh->ml[qp][slot][g1][0][lane];
+          l_1 = sh->ml[qp][slot][g1][1][lane];
+          wait_spin(&sh->o_full[g1][slot], o_par >> g1 & 1);
+          o_par ^= 1 << g1;
         }
-        if (has_d) {
-          wait_park(&sh->ml_full[qp][slot][g_even ^ 1], (ml_par >> (2 * qp + (g_even ^ 1))) & 1);
-          ml_par ^= 1 << (2 * qp + (g_even ^ 1));
-          m_d = sh->ml[qp][slot][g_even ^ 1][0][lane];
-          l_d = sh->ml[qp][slot][g_even ^ 1][1][lane];
+        if (!ok) break;
+        tc_fence_after();
+        if constexpr (ONE) {
+          if (both) {
+            tmem_ld32(o_1, x);
+            tmem_ld32(o_1 + 32, x + 32);
+            tmem_wait_ld();
+            tc_fence_before();
+          } else {
+#pragma unroll
+            for (int e = 0; e < 64; ++e) x[e] = 0u;
+          }
+          __syncwarp();
+          if (lane == 0) mbar_arrive(&sh->o_free[g1][slot]);
         }
+        wait_park(&sh->ml_full[qp][slot][g2], (ml_par >> (2 * qp + g2)) & 1);
+        ml_par ^= 1 << (2 * qp + g2);
+        const float m_2 = sh->ml[qp][slot][g2][0][lane], l_2 = sh->ml[qp][slot][g2][1][lane];
         __syncwarp();
         if (ok && lane == 0) mbar_arrive(&sh->ml_empty[qp][slot]);
-        const float mm = fmaxf(m_e, m_d);
-        const float w_e = (m_e == -INFINITY) ? 0.f : exp2f((m_e - mm) * c2);
-        const float w_d = (m_d == -INFINITY) ? 0.f : exp2f((m_d - mm) * c2);
-        const float lt = fmaf(l_d, w_d, l_e * w_e);
+        const float mm = fmaxf(m_1, m_2);
+        const float w_1 = (m_1 == -INFINITY) ? 0.f : exp2f((m_1 - mm) * c2);
+        const float w_2 = (m_2 == -INFINITY) ? 0.f : exp2f((m_2 - mm) * c2);
+        const float lt = fmaf(l_2, w_2, l_1 * w_1);
         const float inv = 1.f / lt;
-        const float f_e = w_e * inv, f_d = w_d * inv;
-        // (a parity without blocks has weight 0 and an accumulator that may hold anything: the other one is read twice)
-        const uint32_t o_even = lane_base + o_base + (has_e ? g_even : g_even ^ 1) * o_cols;
-        const uint32_t o_odd = lane_base + o_base + (has_d ? g_even ^ 1 : g_even) * o_cols;
-        wait_park(&sh->o_full[slot], o_par);
-        o_par ^= 1;
-        trace_ev(p, 5, tn, slot == 0 && lane == 0 && it >= p.trace_it, 1 * 16 + (i & 15));
-        if (!ok) continue;
+        const float f_1 = w_1 * inv, f_2 = w_2 * inv;
+        wait_spin(&sh->o_full[g2][slot], o_par >> g2 & 1);
+        o_par ^= 1 << g2;
+        if (!ok) break;
+        trace_ev(p, 5, tn, slot == 0 && lane == 0, 1 * 16 + (i & 15));
         tc_fence_after();
         // Heads of at most 64 leave through the staging by TMA; wider ones, which need the shared memory for larger blocks, are
         // stored by the threads that hold the rows.
@@ -480,35 +446,51 @@ fwd2_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CU
         const int64_t tok = (int64_t)tr * p.Wtok + tx;
         using T = typename std::conditional<BF16, __nv_bfloat16, __half>::type;
         [[maybe_unused]] T* const orow = (T*)o.ptr + w.bi * o.s0 + w.hi * o.s1 + tok * o.s2;
-        if (ONE && lane == 0) tma_store_wait_read();     // the previous quarter's rows have left the staging
-        __syncwarp();
-        const int halves = 2 * vch;
-#pragma unroll 1
-        for (int m = 0; m < halves; ++m) {               // 32 columns
-          uint32_t a[32], b[32];
-          tmem_ld32(o_even + 32 * m, a);
-          tmem_ld32(o_odd + 32 * m, b);
+        if constexpr (ONE) {
+          uint32_t y[64];
+          tmem_ld32(o_2, y);
+          tmem_ld32(o_2 + 32, y + 32);
           tmem_wait_ld();
-          if (m == halves - 1) {                         // the last column has been read
-            tc_fence_before();
-            __syncwarp();
-            if (lane == 0) mbar_arrive(&sh->o_free[slot]);
-            trace_ev(p, 5, tn, slot == 0 && lane == 0 && it >= p.trace_it, 2 * 16 + (i & 15));
-          }
-          [[maybe_unused]] const uint32_t row = row0;
+          tc_fence_before();
+          __syncwarp();
+          if (lane == 0) mbar_arrive(&sh->o_free[g2][slot]);
+          trace_ev(p, 5, tn, slot == 0 && lane == 0, 2 * 16 + (i & 15));
+          if (lane == 0) tma_store_wait_read();          // the previous quarter's rows have left the staging
+          __syncwarp();
 #pragma unroll
-          for (int u = 0; u < 4; ++u) {
+          for (int u = 0; u < 8; ++u) {
             uint32_t wd[4];
 #pragma unroll
             for (int h = 0; h < 4; ++h) {
               const int e = 8 * u + 2 * h;
-              wd[h] = pack2<BF16>(fmaf(__uint_as_float(b[e]), f_d, __uint_as_float(a[e]) * f_e),
-                                  fmaf(__uint_as_float(b[e + 1]), f_d, __uint_as_float(a[e + 1]) * f_e));
+              wd[h] = pack2<BF16>(fmaf(__uint_as_float(y[e]), f_2, __uint_as_float(x[e]) * f_1),
+                                  fmaf(__uint_as_float(y[e + 1]), f_2, __uint_as_float(x[e + 1]) * f_1));
             }
-            if constexpr (ONE) {
-              sts128(row + (((uint32_t)(4 * m + u) << 4) ^ swz_x), wd[0], wd[1], wd[2], wd[3]);
-            } else if (t_in && 32 * m + 8 * u < p.dv) {
-              *reinterpret_cast<uint4*>(orow + 32 * m + 8 * u) = make_uint4(wd[0], wd[1], wd[2], wd[3]);
+            sts128(row0 + (((uint32_t)u << 4) ^ swz_x), wd[0], wd[1], wd[2], wd[3]);
+          }
+        } else {
+          // (a group without blocks has weight 0 and an accumulator that may hold anything: the other one is read twice)
+#pragma unroll 1
+          for (int m = 0; m < 2 * vch; ++m) {              // 32 columns
+            uint32_t a[32], b[32];
+            tmem_ld32(o_1 + 32 * m, a);
+            tmem_ld32(o_2 + 32 * m, b);
+            tmem_wait_ld();
+            if (m == 2 * vch - 1) {                        // the last column has been read
+              tc_fence_before();
+              __syncwarp();
+              if (lane < 2) mbar_arrive(&sh->o_free[lane][slot]);
+            }
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+              uint32_t wd[4];
+#pragma unroll
+              for (int h = 0; h < 4; ++h) {
+                const int e = 8 * u + 2 * h;
+                wd[h] = pack2<BF16>(fmaf(__uint_as_float(b[e]), f_2, __uint_as_float(a[e]) * f_1),
+                                    fmaf(__uint_as_float(b[e + 1]), f_2, __uint_as_float(a[e + 1]) * f_1));
+              }
+              if (t_in && 32 * m + 8 * u < p.dv) *reinterpret_cast<uint4*>(orow + 32 * m + 8 * u) = make_uint4(wd[0], wd[1], wd[2], wd[3]);
             }
           }
         }
@@ -521,7 +503,7 @@ fwd2_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CU
           }
         }
         if (t_in) lse[(int64_t)(w.bi * p.H + w.hi) * p.t_h * p.Wtok + tok] = mm * c2 + log2f(lt);
-        trace_ev(p, 5, tn, slot == 0 && lane == 0 && it >= p.trace_it, 3 * 16 + (i & 15));
+        trace_ev(p, 5, tn, slot == 0 && lane == 0, 3 * 16 + (i & 15));
       }
       gb += si.nblk;
       q0 += si.nq;

@@ -16,16 +16,18 @@
 // Accumulating MMAs write only the lanes of quarters that take part in the block (umma_ts_slots): a quarter that is
 // complete rests untouched until it has been read, however late that is, and a new quarter's first MMA overwrites.
 //
-// What bounds these kernels is the latency of the chain of a buffer pair -- score MMAs, tensor memory to registers,
-// exponentials, back, next MMAs -- and, next to it, the exponentials (16 a clock and SM: 640 cycles for 128 rows x 80
-// columns; the MMAs of such a block take 530 to 1000).  Backward, with two buffer pairs, both compute groups work on every
-// block, each on half of its columns (whole steps of 16; they take turns with the larger half): one group walking 80 columns
-// alone took 1.85 ms per dK/dV launch at the 128 x 128 grid with a 13 x 13 window, d = 64 and 256 slices, two sharing
-// them 1.61.  Forward, with three or four score buffers, the groups alternate blocks (0.94 against 1.03 ms).
-// There the sliding strips run 0.93 / 1.09 / 1.25 ms (forward / dQ / dK/dV) against 1.17 / 1.31 / 2.16 for fixed tiles.
+// What bounds these kernels is how long each role takes for a block, one after the other along the chain of a score buffer --
+// score MMAs, tensor memory to registers, exponentials, back, accumulating MMAs -- and beside it: at the 13 x 13 window with d = 64
+// a block of 128 rows x 80 columns takes 1500 to 1900 cycles, of which the MMAs need 520 to 930 and the exponentials 640 (16 a
+// clock and SM); masking, loading and issuing warps were each busy for most of the rest, as a satisfied wait alone costs 80
+// cycles and an MMA issued under a branch twice one issued by a converged warp (umma.cuh).  Hence block records instead of
+// six walks over items and quarters, written eight blocks at a time, a load order without polling, and scores of the next blocks
+// that wait for as little as possible (swa_tc_bwd2.cuh).  128 x 128 grid, 13 x 13 window, d = 64, 64 slices, bf16: forward / dQ /
+// dK/dV 240 / 273 / 318 us before, 205 / 196 / 253 now; 256 x 256, 31 x 31, d = 128, 4 slices: 329 / 366 / 577, 293 / 306 / 439.
 //
-// Six roles fetch their code anew for every block: the kernels are kept near 50 KB (at 90 KB, with unrolled polling loops
-// and divisions, everything ran at half the speed).
+// Backward both compute groups work on every block, each on half of its columns (whole steps of 16; they take turns with
+// the larger half): one group walking 80 columns alone took 1.85 ms per dK/dV launch at 256 slices, two sharing them 1.61 (first
+// strip kernels).  Forward, with three or four score buffers, the groups alternate blocks (0.94 against 1.03 ms).
 //
 // Rows of the grid: block j of an item covers the rows h0 + band * KR .. with h0 = -wr (mod KR) in every item (chunk heights
 // are multiples of KR), so the blocks a row meets, and with them the order of every sum, depend neither on the chunk height
@@ -92,23 +94,61 @@ __device__ __forceinline__ int strip_hx0(const KParams& p, int x0) {
 }
 
 // First and last block of the item that hold a row of quarter i's window.
-__device__ __forceinline__ int quarter_first(const KParams& p, const StripItem& s, int i) {
-  return div_kr(p.pl, max(i * p.pl.R4 + s.off, 0)) * p.pl.ncb;
-}
-__device__ __forceinline__ int quarter_last(const KParams& p, const StripItem& s, int i) {
-  return div_kr(p.pl, min(i * p.pl.R4 + s.off + p.pl.R4 - 1 + 2 * p.wr, p.t_h - 1 - s.h0)) * p.pl.ncb + p.pl.ncb - 1;
-}
+struct QuarterBlocks {
+  int R4, kr_inv, ncb, reach;    // reach: R4 - 1 + 2 wr
+  __device__ __forceinline__ explicit QuarterBlocks(const KParams& p)
+      : R4(p.pl.R4), kr_inv(p.pl.kr_inv), ncb(p.pl.ncb), reach(p.pl.R4 - 1 + 2 * p.wr) {}
+  __device__ __forceinline__ int band(int x) const { return (int)(((uint32_t)x * (uint32_t)kr_inv) >> 16) * ncb; }
+  __device__ __forceinline__ int first(const StripItem& s, int i) const { return band(max(i * R4 + s.off, 0)); }
+  __device__ __forceinline__ int last(const StripItem& s, int i, int end) const {   // end: the grid's last row, from the first streamed one
+    return band(min(i * R4 + s.off + reach, end)) + ncb - 1;
+  }
+};
+__device__ __forceinline__ int quarter_first(const KParams& p, const StripItem& s, int i) { return QuarterBlocks(p).first(s, i); }
+__device__ __forceinline__ int quarter_last(const KParams& p, const StripItem& s, int i) { return QuarterBlocks(p).last(s, i, p.t_h - 1 - s.h0); }
 
-// The quarters that take part in the blocks of an item, block by block (roles that issue MMAs).
-struct QuarterCursor {
-  int lo, hi;               // quarters lo .. hi - 1 take part
-  int next_first, lo_last;  // first block of quarter hi, last block of quarter lo
-  uint32_t act;             // slots that take part
-  __device__ __forceinline__ void begin(const KParams& p, const StripItem& s) {
-    lo = hi = 0;
-    act = 0u;
-    next_first = 0;
-    lo_last = quarter_last(p, s, 0);
+// What the roles do with a block is put together once, by the masking warp, in one word: the roles that run block by block are
+// loops over these records and know nothing of items and quarters.
+// A ring of kMaskRing + (score buffers) records: a record is overwritten once the score MMAs of the block kMaskRing before the
+// new one are complete, which needed the buffer, and so the accumulating MMAs, of the block whose record it is.
+// Two kRecEnd records follow the last block (the forward kernel's groups read every second one).
+enum : uint32_t {
+  kRecAct = 0,              // 4 bits each, per slot: its quarter takes part in the block,
+  kRecFresh = 4,            // ... starts with it,
+  kRecEnds = 8,             // ... is complete with it;
+  kRecGroupFirst = 12,      // ... starts with it or the block before (the first for one of two groups on alternate blocks),
+  kRecGroupLast = 16,       // ... is complete with it or the next;
+  kRecUse = 20,             // bit 0 and
+  kRecUse2 = 24,            // ... bit 1 of how often the slot had been used before its quarter
+  kRecEnters = 0x10000000u,  // a quarter enters: the next version of the resident rows
+  kRecLeaves = 0x20000000u,  // the last block that reads this version
+  kRecEnd = 0x40000000u,    // no block: the stream has ended
+};
+
+// The quarters of one slot in the order of the stream.
+struct QuarterWalk {
+  ItemWalk w;
+  StripItem s;
+  int it, i;                // item, quarter in the item
+  uint32_t q0;              // quarters before the item
+  bool more;
+  __device__ __forceinline__ QuarterWalk(const KParams& p, const ItemStart& st, int slot) : w(st), it(0), i(slot), q0(0), more(true) {
+    s = strip_item(p, w);
+    settle(p, st.count, slot);
+  }
+  __device__ __forceinline__ void next(const KParams& p, int count, int slot) {
+    i += 4;
+    settle(p, count, slot);
+  }
+  __device__ __forceinline__ void settle(const KParams& p, int count, int slot) {
+#pragma unroll 1
+    while (i >= s.nq && more) {
+      q0 += s.nq;
+      more = ++it < count;
+      w.next(p);
+      s = strip_item(p, w);
+      i = (slot - (int)q0) & 3;
+    }
   }
 };
 
@@ -117,7 +157,8 @@ struct QuarterCursor {
 // column of its ring row (slot * R4 + row in the quarter) and of its token column, a streamed token a penalty in every
 // column it may not interact with.  Every 8 of those columns (a "unit", 16 bytes of a row) are a tile of their own,
 // rows one after the other (8-row core matrices 128 bytes apart), so that what changes at different times lies apart:
-// the row units with the blocks, the column units with the strips, the unused unit never.
+// the row units with the blocks, the column units with the strips.  The fourth unit is unused: the resident rows' is zero, and the
+// streamed side is pointed at their units (any finite numbers behind the others in memory).
 constexpr uint32_t kUnitSbo = 128;
 constexpr int kMaskRing = 4;      // blocks whose units are held; evenly sliding quarters repeat them every four blocks
 __device__ __forceinline__ uint32_t unit_bytes(const Plan& pl) { return (uint32_t)pl.N * 16u; }
@@ -151,33 +192,32 @@ __device__ __forceinline__ void build_row_parts(uint8_t* tab, int t, int nthread
 
 // ---- accumulating MMAs ------------------------------------------------------------------------------------------------
 // D (+)= A B over nks steps of 16 streamed tokens, rows of the quarters that take part (`act`) only; the first step overwrites
-// the rows of quarters that start with this block (`fresh`).  From step n1 on A lies `gap` columns further.  One elected thread.
-__device__ __forceinline__ void accumulate_block(uint32_t d, uint32_t a, uint64_t b, uint32_t idesc, int nks, int n1, uint32_t gap,
+// the rows of quarters that start with this block (`fresh`).  A's steps lie `step` columns apart.
+__device__ __forceinline__ void accumulate_block(uint32_t el, uint32_t d, uint32_t a, uint64_t b, uint32_t idesc, int nks, uint32_t step,
                                                  uint32_t act, uint32_t fresh) {
   using namespace ptx;
+  if (fresh) umma_ts_slots(el, d, a, b, idesc, 0u, SlotMask(fresh));
+  if (act & ~fresh) umma_ts_slots(el, d, a, b, idesc, 1u, SlotMask(act & ~fresh));
   const SlotMask m(act);
-  if (fresh) {
-    umma_ts_slots(d, a, b, idesc, 0u, SlotMask(fresh));
-    act &= ~fresh;
-  }
-  if (act) umma_ts_slots(d, a, b, idesc, 1u, SlotMask(act));
 #pragma unroll 1
   for (int ks = 1; ks < nks; ++ks) {
-    a += 8;
+    a += step;
     b += 128;
-    if (ks == n1) a += gap;
-    umma_ts_slots(d, a, b, idesc, 1u, m);
+    umma_ts_slots(el, d, a, b, idesc, 1u, m);
   }
 }
 
 // ---- loads ----------------------------------------------------------------------------------------------------------
-// The producer warp fills the ring of streamed blocks and the buffers of resident rows, whichever has room first.  A
-// resident buffer holds four quarters; it changes when a quarter slides in, so the blocks alternate between nxb buffers
-// ("versions") and a buffer is brought up to date -- the slots whose quarter has changed since it was last loaded -- as soon as
-// the score MMAs of its previous version are done.  With two buffers a quarter crosses L2 twice (it is fetched into L2 one
-// quarter ahead), and its load has one whole block's time to arrive.
-// Whether a barrier's phase has completed is voted on: two lanes that test it while it completes may see different answers, and
-// the walk's state and elect_one must not part ways.
+// The producer warp fills the ring of streamed blocks and the buffers of resident rows.  A resident buffer holds four quarters;
+// it changes when a quarter slides in, so the blocks alternate between nxb buffers ("versions") and a buffer is brought up to
+// date -- the slots whose quarter has changed since it was last loaded -- when the score MMAs of its previous version are done.
+// With two buffers a quarter crosses L2 twice (it is fetched into L2 one quarter ahead), and its load has one whole block's time
+// to arrive.
+// Blocks and versions are loaded in one fixed order: the version nxb - 1 after the one that block n starts, right before block
+// n + stages - 2.  Its buffer is read last by the score MMAs of block n - 1; the stage of the block loaded before it by the
+// accumulating MMAs of block n - 3, which are complete by then, and the stage of the one after it by those of block n - 2: neither
+// waits long for the other, and what a wait needs has been loaded before.  (Looking at both rings in turn took 2000 cycles per
+// block with the walk that goes with it, more than the other roles needed.)
 struct LoadArgs {
   uint8_t* x_smem;              // nxb buffers of qk chunks, then v chunks (128 rows of 128 bytes each)
   uint32_t x_bytes, xqk_bytes;
@@ -185,39 +225,92 @@ struct LoadArgs {
   uint32_t yqk_stage, yv_stage, blk_bytes;
   uint64_t *x_full, *x_empty, *y_full, *y_empty;
   const ItemStart* start;
-  const CUtensorMap *xqk, *xv, *yqk, *yv;   // xv: null in the forward kernel (no second resident tensor)
+  const CUtensorMap *xqk, *xv, *yqk, *yv;   // (the forward kernel has no second resident tensor: XV)
 };
 
-constexpr uint32_t kLoadPolls = 1u << 23;   // rounds that found no room in a row: 64 ns or more each, 0.5 s and up
-
+template <bool ONE, bool XV>
 __device__ __forceinline__ void load_warp(const KParams& p, const LoadArgs& f, bool& ok) {
   using namespace ptx;
   const Plan& pl = p.pl;
-  const int count = f.start->count;
+  const int count = f.start->count, qch = ONE ? 1 : p.qch, vch = ONE ? 1 : p.vch;
+  const int KR = pl.KR, KW = pl.KW, ncb = pl.ncb, stages = pl.stages, nxb = pl.nxb;
+  const uint32_t y_bytes = f.yqk_stage + f.yv_stage, yqk_stage = f.yqk_stage, yv_stage = f.yv_stage, blk_bytes = f.blk_bytes,
+                 x_bytes = f.x_bytes;
+  QuarterBlocks qb(p);
+  const uint32_t el = elect_one();
+  int tn = 0;
   int stage = 0, stage_par = 1, xb = 0, x_par = 1;
-  bool ring_full = false, x_ring_full = false;
-  uint32_t q0 = 0, stale0 = 0, stale1 = 0, m = 0, polls = 0;
+  uint32_t q0 = 0;
   ItemWalk wy(*f.start), wx(*f.start);
   StripItem sy = strip_item(p, wy), sx = sy;
-  int jy = 0, yrow = sy.h0, ycol = strip_hx0(p, sy.x0), cblk = 0, ity = 0;   // next streamed block
-  int jx = 0, itx = 0, hi = 0;                                               // block the next version is for; quarters in so far
+  int jy = 0, yrow = sy.h0, ycol = strip_hx0(p, sy.x0), cblk = 0, ity = 0, ny = 0;   // next streamed block; blocks loaded
+  int jx = 0, itx = 0, hi = 0, from = 0, bx = 0;   // block the next version is for, in its item; quarters in so far, and before the last version; blocks before the item
+  int due = 0;                                     // the next version is loaded once so many blocks are
 #pragma unroll 1
-  while (ok && (ity < count || itx < count)) {
-    bool idle = true;
-    if (ity < count && (!ring_full || __all_sync(0xffffffffu, mbar_test(smem_u32(f.y_empty + stage), stage_par)))) {
-      idle = false;
-      if (elect_one()) {
-        uint64_t* bar = f.y_full + stage;
-        mbar_arrive_expect_tx(bar, f.yqk_stage + f.yv_stage);
+  while (ity < count || itx < count) {
+    if (itx < count && (ny >= due || ity == count)) {
+      trace_ev(p, 0, tn, el, 0 * 16 + xb);
+      ok = __all_sync(0xffffffffu, mbar_wait_polls<kSleepPoll>(smem_u32(f.x_empty + xb), x_par));
+      trace_ev(p, 0, tn, el, 1 * 16 + xb);
+      if (!ok) break;
+      // The quarters that enter: the first four with the item, the others with the first block that needs them.  This buffer
+      // (of two) lacks those that entered with the version before, too.
+      int i = nxb == 1 ? hi : from;
+      from = hi;
+      const int had = bx + jx;                     // block this version is for
 #pragma unroll 1
-        for (int c = 0; c < p.qch; ++c) tma_load_5d(f.yqk_smem + stage * f.yqk_stage + c * f.blk_bytes, f.yqk, bar, c * 64, ycol, yrow, wy.hi, wy.bi);
+      do {
+        ++hi;
+        jx = hi < sx.nq ? hi < 4 ? 0 : qb.first(sx, hi) : 1 << 30;
+      } while (jx <= had - bx);
+      i = max(i, hi - 4);
+      const uint32_t dst = smem_u32(f.x_smem + xb * x_bytes), bar = smem_u32(f.x_full + xb);
+      mbar_expect_tx_el(el, bar, (uint32_t)(hi - i) * (x_bytes >> 2));
+      int row = sx.r0 + i * qb.R4;
 #pragma unroll 1
-        for (int c = 0; c < p.vch; ++c) tma_load_5d(f.yv_smem + stage * f.yv_stage + c * f.blk_bytes, f.yv, bar, c * 64, ycol, yrow, wy.hi, wy.bi);
+      for (; i < hi; ++i, row += qb.R4) {
+        uint32_t to = dst + ((q0 + i) & 3u) * 4096u;
+#pragma unroll 1
+        for (int c = 0; c < qch; ++c, to += 16384) tma_load_5d_el(el, to, f.xqk, bar, c * 64, sx.x0, row, wx.hi, wx.bi);
+        if constexpr (XV) {
+#pragma unroll 1
+          for (int c = 0; c < vch; ++c, to += 16384) tma_load_5d_el(el, to, f.xv, bar, c * 64, sx.x0, row, wx.hi, wx.bi);
+        }
       }
-      __syncwarp();
-      if (++stage == pl.stages) { stage = 0; stage_par ^= 1; ring_full = true; }
-      ycol += pl.KW;
-      if (++cblk == pl.ncb) { cblk = 0; ycol -= pl.KW * pl.ncb; yrow += pl.KR; }
+      if (hi < sx.nq) {                            // the next quarter on its way into L2
+#pragma unroll 1
+        for (int c = 0; c < qch; ++c) tma_prefetch_5d_el(el, f.xqk, c * 64, sx.x0, row, wx.hi, wx.bi);
+        if constexpr (XV) {
+#pragma unroll 1
+          for (int c = 0; c < vch; ++c) tma_prefetch_5d_el(el, f.xv, c * 64, sx.x0, row, wx.hi, wx.bi);
+        }
+      } else {
+        jx = hi = from = 0;
+        q0 += sx.nq;
+        bx += sx.nblk;
+        wx.next(p);
+        sx = strip_item(p, wx);
+        ++itx;
+      }
+      if (++xb == nxb) { xb = 0; x_par ^= 1; }
+      due = (nxb == 1 ? bx + jx : had) + stages - 2;
+    } else {
+      trace_ev(p, 0, tn, el, 2 * 16 + stage);
+      ok = __all_sync(0xffffffffu, mbar_wait_polls<kSleepPoll>(smem_u32(f.y_empty + stage), stage_par));
+      trace_ev(p, 0, tn, el, 3 * 16 + stage);
+      if (!ok) break;
+      const uint32_t bar = smem_u32(f.y_full + stage);
+      mbar_expect_tx_el(el, bar, y_bytes);
+      uint32_t to = smem_u32(f.yqk_smem) + stage * yqk_stage;
+#pragma unroll 1
+      for (int c = 0; c < qch; ++c, to += blk_bytes) tma_load_5d_el(el, to, f.yqk, bar, c * 64, ycol, yrow, wy.hi, wy.bi);
+      to = smem_u32(f.yv_smem) + stage * yv_stage;
+#pragma unroll 1
+      for (int c = 0; c < vch; ++c, to += blk_bytes) tma_load_5d_el(el, to, f.yv, bar, c * 64, ycol, yrow, wy.hi, wy.bi);
+      ++ny;
+      if (++stage == stages) { stage = 0; stage_par ^= 1; }
+      ycol += KW;
+      if (++cblk == ncb) { cblk = 0; ycol -= KW * ncb; yrow += KR; }
       if (++jy == sy.nblk) {
         jy = 0;
         wy.next(p);
@@ -227,74 +320,22 @@ __device__ __forceinline__ void load_warp(const KParams& p, const LoadArgs& f, b
         ++ity;
       }
     }
-    if (itx < count && (!x_ring_full || __all_sync(0xffffffffu, mbar_test(smem_u32(f.x_empty + xb), x_par)))) {
-      idle = false;
-      if (jx == 0) stale0 = stale1 = 0;
-      // the quarters that enter: the first four with the item, the others with the first block that needs them
-      int lo = hi;
-      m = 0;
-#pragma unroll 1
-      do m |= 1u << ((q0 + hi++) & 3u);
-      while (hi < sx.nq && (hi < 4 || quarter_first(p, sx, hi) <= jx));
-      stale0 |= m;
-      stale1 |= m;
-      m = xb ? stale1 : stale0;
-      if (xb) stale1 = 0; else stale0 = 0;
-      if (elect_one()) {
-        uint8_t* dst = f.x_smem + xb * f.x_bytes;
-        uint64_t* bar = f.x_full + xb;
-        mbar_arrive_expect_tx(bar, __popc(m) * (f.x_bytes >> 2));
-        lo = max(hi - 4, 0);                       // a slot of m holds one of the last four quarters
-#pragma unroll 1
-        for (int i = lo; i < hi; ++i) {
-          const int e = (q0 + i) & 3, row = sx.r0 + i * pl.R4;
-          if (!(m >> e & 1u)) continue;
-#pragma unroll 1
-          for (int c = 0; c < p.qch; ++c) tma_load_5d(dst + c * 16384 + e * 4096, f.xqk, bar, c * 64, sx.x0, row, wx.hi, wx.bi);
-          if (f.xv != nullptr) {
-#pragma unroll 1
-            for (int c = 0; c < p.vch; ++c) tma_load_5d(dst + f.xqk_bytes + c * 16384 + e * 4096, f.xv, bar, c * 64, sx.x0, row, wx.hi, wx.bi);
-          }
-        }
-        if (hi < sx.nq) {                          // the next quarter on its way into L2
-          const int row = sx.r0 + hi * pl.R4;
-#pragma unroll 1
-          for (int c = 0; c < p.qch; ++c) tma_prefetch_5d(f.xqk, c * 64, sx.x0, row, wx.hi, wx.bi);
-          if (f.xv != nullptr) {
-#pragma unroll 1
-            for (int c = 0; c < p.vch; ++c) tma_prefetch_5d(f.xv, c * 64, sx.x0, row, wx.hi, wx.bi);
-          }
-        }
-      }
-      __syncwarp();
-      if (++xb == pl.nxb) { xb = 0; x_par ^= 1; x_ring_full = true; }
-      if (hi < sx.nq) {
-        jx = quarter_first(p, sx, hi);
-      } else {
-        jx = 0;
-        hi = 0;
-        q0 += sx.nq;
-        wx.next(p);
-        sx = strip_item(p, wx);
-        ++itx;
-      }
-    }
-    polls = idle ? polls + 1 : 0;
-    if (idle) __nanosleep(32);
-    if (polls == kLoadPolls) ok = false;
   }
 }
 
 // ---- the masking warp ---------------------------------------------------------------------------------------------
-// One warp writes the mask units (VEC: and -lse / delta) of every streamed block.  A ring entry whose units already are what the
-// block needs is left alone: while quarters slide evenly the row units repeat with the period of their ring, and the strips
-// that the grid does not clip share their column units.
+// One warp writes the record, the mask units (VEC: and -lse / -delta) of every streamed block.  What they are is worked out for eight
+// blocks of an item at a time, by four lanes each: block by block the masking warp was busy for nearly the whole time of a block
+// and bounded the forward kernel (cells of 16 tokens, head dim 32: 40.8 -> 36.9 us).  A ring entry whose units already
+// are what the block needs is left alone: while quarters slide evenly the row units repeat with the period of their ring, and the
+// strips that the grid does not clip share their column units.
 struct MaskArgs {
   uint8_t *yr_smem, *yc_smem;   // row and column units of every ring entry
-  uint64_t *yx_free, *y_ready;
-  float* vec_smem;              // VEC: [slot][-lse | -delta][128]
-  int vslots;
-  uint64_t* vec_ready;
+  uint64_t* yx_free;
+  uint32_t* rec;                // ring of n_rec records
+  uint64_t* rec_ready;          // a block's record, mask units and vec slot are written
+  int n_rec;
+  float* vec_smem;              // VEC: [record][-lse | -delta][128]
   const float *lse, *delta;
   const uint8_t* row_parts;
   const ItemStart* start;
@@ -304,127 +345,155 @@ template <bool BF16, bool VEC, typename Wait>
 __device__ __forceinline__ void mask_warp(const KParams& p, const MaskArgs& f, bool& ok, Wait&& wait) {
   using namespace ptx;
   const Plan& pl = p.pl;
-  const int lane = threadIdx.x & 31, N = pl.N;
+  const int lane = threadIdx.x & 31, slot = lane & 3, N = pl.N;
+  const int t_h = p.t_h, Wtok = p.Wtok, wr = p.wr, KR = pl.KR, KW = pl.KW, ncb = pl.ncb;
+  const int r4_log = 5 - pl.tw_log;
+  QuarterBlocks qb(p);
   const uint32_t ub = unit_bytes(pl), row_stage = ub * (uint32_t)(pl.TH >> 3), col_units = ub * (uint32_t)(pl.TW >> 3);
-  int jrc[4];                                      // block column | block row << 8 of this lane's (up to four) streamed tokens
+  int jr[4], jc[4], to[4];                         // block row and column of this lane's (up to four) streamed tokens, their offsets
 #pragma unroll
   for (int e = 0; e < 4; ++e) {
     const int n = lane + 32 * e, r = (int)((uint32_t)(n * pl.kw_inv) >> 16);
-    jrc[e] = n < N ? r << 8 | (n - r * pl.KW) : 1 << 30;                        // no such token: below every grid
+    jr[e] = n < N ? r : 1 << 30;                   // no such token: below every grid
+    jc[e] = n - r * KW;
+    to[e] = n < N ? r * Wtok + jc[e] : 0;
   }
-  int stage = 0, stage_par = 1, vslot = 0;
-  bool ring_full = false;
-  uint32_t q0 = 0;
-  int xr = 0;                                      // lane s < 4: first grid row of the quarter in slot s
-  uint64_t row_sig = ~0ull;                        // lane l: what the row units of stage l are for
-  uint64_t col_sig = ~0ull;                        // ... and its column units
+  int tn = 0;
+  int stage = 0, stage_par = 1, rs = 0;            // ring entries of units and of records
+  uint32_t q0 = 0;                                 // quarters before the item
+  int old_row = 1 << 31, old_col = -1;             // lane 16 + 4 t + e: what the units of the t'th of the last four blocks are for
   ItemWalk w(*f.start);
-  const int count = f.start->count, none = 2 * p.wr + pl.R4;
+  const int count = f.start->count, none = 2 * wr + qb.R4;
+  constexpr int kNever = 1 << 30;
 #pragma unroll 1
   for (int it = 0; it < count; ++it, w.next(p)) {
     const StripItem s = strip_item(p, w);
-    const int hx0 = strip_hx0(p, s.x0);
-    int hi = 0, next_first = 0, y0 = s.h0, cblk = 0;
-    const int64_t slice = (int64_t)(w.bi * p.H + w.hi) * p.t_h * p.Wtok;
+    const int hx0 = strip_hx0(p, s.x0), end = t_h - 1 - s.h0;
+    const int64_t slice = (int64_t)(w.bi * p.H + w.hi) * t_h * Wtok;
 #pragma unroll 1
-    for (int j = 0; j < s.nblk; ++j) {
-      float nl[4], dl[4];
-      if constexpr (VEC) {                         // (used after the wait below, which covers their latency)
-        const int c0 = hx0 + cblk * pl.KW;
+    for (int j0 = 0; j0 < s.nblk; j0 += 8) {
+      // Lane 4 t + e: slot e in the item's block j0 + t.  Its quarter i is the first of the slot that is not over by then.
+      const int j = j0 + (lane >> 2), band = ncb == 1 ? j : j / ncb, cblk = j - band * ncb;
+      const int over = band * KR - s.off - qb.reach, lo = over <= 0 ? 0 : (over + qb.R4 - 1) >> r4_log;
+      const int i = lo + ((slot - (int)q0 - lo) & 3);
+      const int first = i < s.nq ? qb.first(s, i) : kNever, last = i < s.nq ? qb.last(s, i, end) : kNever,
+                next_first = i + 4 < s.nq ? qb.first(s, i + 4) : kNever;
+      // (The first four quarters of an item enter with it.)
+      uint32_t rec = (q0 + i & 4u) << (kRecUse - 2) | (q0 + i & 8u) << (kRecUse2 - 3);
+      if (first <= j)
+        rec |= 1u << kRecAct | (uint32_t)(first == j) << kRecFresh | (uint32_t)(last == j) << kRecEnds |
+               (uint32_t)(j - first < 2) << kRecGroupFirst | (uint32_t)(last - j < 2) << kRecGroupLast;
+      rec <<= slot;
+      if (j == 0 || (i >= 4 && first == j)) rec |= kRecEnters;
+      if (j == s.nblk - 1 || (i >= 4 && first == j + 1) || next_first == j + 1) rec |= kRecLeaves;
+      rec |= __shfl_xor_sync(0xffffffffu, rec, 1);
+      rec |= __shfl_xor_sync(0xffffffffu, rec, 2);
+      // Row units: the distance of the block's first row from the quarter (beyond the window: all alike), the rows that the grid
+      // cuts off.  Column units: where the block lies relative to the strip, the columns that the grid cuts off.
+      const int y0 = s.h0 + band * KR, c0 = hx0 + cblk * KW, at = y0 + wr - (s.r0 + i * qb.R4);
+      const int want_row = min(max(at, -KR), none) & 0xffff | max(0, -y0) << 16 | min(KR, max(0, t_h - y0)) << 24;
+      const int want_col = (c0 - s.x0) << 20 | cblk << 16 | min(max(0, -c0), 255) << 8 | min(max(0, Wtok - c0), 255);
+      const int row4 = __shfl_sync(0xffffffffu, want_row, lane & 15), col4 = __shfl_sync(0xffffffffu, want_col, lane & 15);
+      const int row4o = __shfl_sync(0xffffffffu, old_row, lane | 16), col4o = __shfl_sync(0xffffffffu, old_col, lane | 16);
+      uint32_t new_row = __ballot_sync(0xffffffffu, want_row != (lane < 16 ? row4o : row4)),
+               new_col = __ballot_sync(0xffffffffu, want_col != (lane < 16 ? col4o : col4));
+      const int nb = min(8, s.nblk - j0);
+      {
+        const int k = nb - 4 + ((lane >> 2) & 3), src = 4 * (k < 0 ? k + 8 : k) + slot;
+        const int a = __shfl_sync(0xffffffffu, want_row, src), b = __shfl_sync(0xffffffffu, old_row, src);
+        const int c = __shfl_sync(0xffffffffu, want_col, src), d = __shfl_sync(0xffffffffu, old_col, src);
+        old_row = k < 0 ? b : a;
+        old_col = k < 0 ? d : c;
+      }
+      [[maybe_unused]] float nl[4], dl[4];
+      auto fetch = [&](int t) {                    // lse and delta of block t's tokens
+        if constexpr (VEC) {
+          const int y = __shfl_sync(0xffffffffu, y0, 4 * t), c = __shfl_sync(0xffffffffu, c0, 4 * t);
+          const int64_t tok = slice + (int64_t)y * Wtok + c;
+          const float *l0 = f.lse + tok, *d0 = f.delta + tok;
 #pragma unroll
-        for (int e = 0; e < 4; ++e) {
-          const int y = y0 + (jrc[e] >> 8), c = c0 + (jrc[e] & 255);
-          nl[e] = INFINITY;
-          dl[e] = 0.f;
-          if ((uint32_t)y < (uint32_t)p.t_h && (uint32_t)c < (uint32_t)p.Wtok) {
-            const int64_t at = slice + y * p.Wtok + c;
-            nl[e] = f.lse[at];
-            dl[e] = f.delta[at];
+          for (int e = 0; e < 4; ++e) {
+            const bool in = (uint32_t)(y + jr[e]) < (uint32_t)t_h && (uint32_t)(c + jc[e]) < (uint32_t)Wtok;
+            nl[e] = ld_if(l0 + to[e], in, INFINITY);
+            dl[e] = ld_if(d0 + to[e], in, 0.f);
           }
         }
-      }
+      };
+      fetch(0);
 #pragma unroll 1
-      while (hi < s.nq && (hi < 4 || next_first <= j)) {       // the first four quarters enter with the item
-        if (lane == ((q0 + hi) & 3)) xr = s.r0 + hi * pl.R4;
-        next_first = quarter_first(p, s, ++hi);
-      }
-      if (ring_full) wait(f.yx_free + stage, stage_par);
-      if (ok) {
-        // Column units: which tile columns a token column may interact with depends on where the block lies relative to the
-        // strip, and on what the grid clips.
-        const int c0 = hx0 + cblk * pl.KW;
-        const uint64_t want_col = (uint64_t)(uint32_t)(c0 - s.x0) << 32 | (uint32_t)cblk << 24 | (uint32_t)min(max(0, -c0), 255) << 12 |
-                                  (uint32_t)min(max(0, p.Wtok - c0), 255);
-        if (__shfl_sync(0xffffffffu, col_sig, stage) != want_col) {
-          if (lane == stage) col_sig = want_col;
+      for (int t = 0; t < nb; ++t, new_row >>= 4, new_col >>= 4) {
+        trace_ev(p, 4, tn, lane == 0, 0 * 16 + rs);
+        wait(f.yx_free + stage, stage_par);
+        trace_ev(p, 4, tn, lane == 0, 1 * 16 + rs);
+        if (!ok) return;
+        if (new_col & 15u) {
+          const int c = __shfl_sync(0xffffffffu, c0, 4 * t);
           uint8_t* col = f.yc_smem + stage * col_units;
 #pragma unroll 1
           for (int n = lane; n < N; n += 32) {
-            const int yx = c0 + n - (int)((uint32_t)(n * pl.kw_inv) >> 16) * pl.KW;
-            int lo = 1, hi_ = 0;
-            if ((uint32_t)yx < (uint32_t)p.Wtok) {
+            const int yx = c + n - (int)((uint32_t)(n * pl.kw_inv) >> 16) * KW;
+            int l = 1, h = 0;
+            if ((uint32_t)yx < (uint32_t)Wtok) {
               const int yc = p.div_b ? (int)__umulhi((uint32_t)yx, p.div_b) : yx;
-              lo = (yc - p.wc) * p.b - s.x0;                         // allowed tile columns, inclusive
-              hi_ = (yc + p.wc + 1) * p.b - s.x0 - 1;
+              l = (yc - p.wc) * p.b - s.x0;                          // allowed tile columns, inclusive
+              h = (yc + p.wc + 1) * p.b - s.x0 - 1;
             }
 #pragma unroll 1
             for (int u = 0; u < (pl.TW >> 3); ++u)
-              *reinterpret_cast<uint4*>(col + u * ub + n * 16) = penalty_unit<BF16>(lo - 8 * u, hi_ - 8 * u, -p.mask_b);
+              *reinterpret_cast<uint4*>(col + u * ub + n * 16) = penalty_unit<BF16>(l - 8 * u, h - 8 * u, -p.mask_b);
           }
+          fence_proxy_async_smem();
         }
-        // distance of the block's first row from every slot's quarter (beyond the window: all alike), rows inside the grid
-        uint32_t at0[4], sig = 0;
-#pragma unroll
-        for (int e = 0; e < 4; ++e) {
-          at0[e] = (uint32_t)(y0 + p.wr - __shfl_sync(0xffffffffu, xr, e));
-          const int d = min(max((int)at0[e], -pl.KR), none);
-          sig = sig << 8 | (uint32_t)(d + 16);             // -16 <= d <= 2 * 64 + 4
-        }
-        const uint32_t clip = (uint32_t)max(0, -y0) << 8 | (uint32_t)min(pl.KR, max(0, p.t_h - y0));
-        const uint64_t want = (uint64_t)clip << 32 | sig;
-        if (__shfl_sync(0xffffffffu, row_sig, stage) != want) {
-          if (lane == stage) row_sig = want;
+        if (new_row & 15u) {
           uint8_t* tile = f.yr_smem + stage * row_stage;
+          const int y = __shfl_sync(0xffffffffu, y0, 4 * t), at0 = __shfl_sync(0xffffffffu, at, 4 * t), at1 = __shfl_sync(0xffffffffu, at, 4 * t + 1),
+                    at2 = __shfl_sync(0xffffffffu, at, 4 * t + 2), at3 = __shfl_sync(0xffffffffu, at, 4 * t + 3);
 #pragma unroll 1
           for (int n = lane; n < N; n += 32) {
             const int r = (int)((uint32_t)(n * pl.kw_inv) >> 16);
-            const bool in = (uint32_t)(y0 + r) < (uint32_t)p.t_h;
-            uint32_t at[4];
-#pragma unroll
-            for (int e = 0; e < 4; ++e) {
-              at[e] = at0[e] + r;
-              if (!in || at[e] > (uint32_t)none) at[e] = none;
-            }
+            const bool in = (uint32_t)(y + r) < (uint32_t)t_h;
+            auto entry = [&](int a) { return in && (uint32_t)(a + r) <= (uint32_t)none ? a + r : none; };
             if (pl.TW == 8) {
-              const uint2* t = reinterpret_cast<const uint2*>(f.row_parts);
-              const uint2 a = t[at[0]], b = t[at[1]], c = t[at[2]], d = t[at[3]];
+              const uint2* u = reinterpret_cast<const uint2*>(f.row_parts);
+              const uint2 a = u[entry(at0)], b = u[entry(at1)], c = u[entry(at2)], d = u[entry(at3)];
               *reinterpret_cast<uint4*>(tile + n * 16) = make_uint4(a.x, a.y, b.x, b.y);
               *reinterpret_cast<uint4*>(tile + ub + n * 16) = make_uint4(c.x, c.y, d.x, d.y);
             } else {
-              const uint32_t* t = reinterpret_cast<const uint32_t*>(f.row_parts);
-              *reinterpret_cast<uint4*>(tile + n * 16) = make_uint4(t[at[0]], t[at[1]], t[at[2]], t[at[3]]);
+              const uint32_t* u = reinterpret_cast<const uint32_t*>(f.row_parts);
+              *reinterpret_cast<uint4*>(tile + n * 16) = make_uint4(u[entry(at0)], u[entry(at1)], u[entry(at2)], u[entry(at3)]);
             }
           }
+          fence_proxy_async_smem();
         }
         if constexpr (VEC) {
+          float* v = f.vec_smem + rs * 256 + lane;
 #pragma unroll
           for (int e = 0; e < 4; ++e) {            // (rows beyond N: written, never read)
-            f.vec_smem[vslot * 256 + lane + 32 * e] = -nl[e];
-            f.vec_smem[vslot * 256 + 128 + lane + 32 * e] = -dl[e];
+            v[32 * e] = -nl[e];
+            v[128 + 32 * e] = -dl[e];
           }
         }
-        fence_proxy_async_smem();
+        if (lane == 4 * t) f.rec[rs] = rec;
         __syncwarp();
-        if (lane == 0) {
-          mbar_arrive(f.y_ready + stage);
-          if constexpr (VEC) mbar_arrive(f.vec_ready + vslot);
-        }
+        if (lane == 4 * t) mbar_arrive(f.rec_ready + rs);
+        trace_ev(p, 4, tn, lane == 0, 2 * 16 + rs);
+        if (++stage == kMaskRing) { stage = 0; stage_par ^= 1; }
+        if (++rs == f.n_rec) rs = 0;
+        if (t + 1 < nb) fetch(t + 1);
       }
-      if (++stage == kMaskRing) { stage = 0; stage_par ^= 1; ring_full = true; }
-      if (VEC && ++vslot == f.vslots) vslot = 0;
-      if (++cblk == pl.ncb) { cblk = 0; y0 += pl.KR; }
     }
     q0 += s.nq;
+  }
+#pragma unroll 1
+  for (int e = 0; e < 2; ++e) {
+    wait(f.yx_free + stage, stage_par);
+    if (!ok) return;
+    if (lane == 0) {
+      f.rec[rs] = kRecEnd;
+      mbar_arrive(f.rec_ready + rs);
+    }
+    if (++stage == kMaskRing) { stage = 0; stage_par ^= 1; }
+    if (++rs == f.n_rec) rs = 0;
   }
 }
 

@@ -30,6 +30,11 @@ __device__ __forceinline__ float lds32(uint32_t saddr) {
   asm volatile("ld.shared.f32 %0, [%1];" : "=f"(v) : "r"(saddr) : "memory");
   return v;
 }
+// *p if `on`, else `other`, without a branch.
+__device__ __forceinline__ float ld_if(const float* p, bool on, float other) {
+  asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %2, 0;\n\t@p ld.global.f32 %0, [%1];\n\t}" : "+f"(other) : "l"(p), "r"((int)on) : "memory");
+  return other;
+}
 // named barrier among `count` threads (count a multiple of 32); id 0 is __syncthreads
 __device__ __forceinline__ void named_bar_sync(uint32_t id, uint32_t count) {
   asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(count) : "memory");
@@ -145,41 +150,6 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, volati
   return true;
 }
 
-// The strip kernels' wait (swa_tc_strip.cuh): six instructions, because they have two dozen of them in code that is fetched
-// again for every block.  False once the poll budget is used up (a second, as above); the caller's warp then skips every
-// later wait, the others run into their own limit, and the kernel's end tells the host.
-template <uint32_t PARK_NS>
-__device__ __forceinline__ bool mbar_wait_polls(uint32_t bar, uint32_t parity) {
-  uint32_t ok;
-  if constexpr (PARK_NS == 0)
-    asm volatile(
-        "{\n\t.reg .pred p, q;\n\t.reg .u32 n;\n\t"
-        "mov.u32 n, %3;\n"
-        "SWA_WAIT:\n\t"
-        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-        "@p bra SWA_DONE;\n\t"
-        "sub.u32 n, n, 1;\n\t"
-        "setp.ne.u32 q, n, 0;\n\t"
-        "@q bra SWA_WAIT;\n"
-        "SWA_DONE:\n\t"
-        "selp.u32 %0, 1, 0, p;\n\t}"
-        : "=r"(ok) : "r"(bar), "r"(parity), "n"(kSpinPolls) : "memory");
-  else
-    asm volatile(
-        "{\n\t.reg .pred p, q;\n\t.reg .u32 n;\n\t"
-        "mov.u32 n, %3;\n"
-        "SWA_WAIT:\n\t"
-        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %4;\n\t"
-        "@p bra SWA_DONE;\n\t"
-        "sub.u32 n, n, 1;\n\t"
-        "setp.ne.u32 q, n, 0;\n\t"
-        "@q bra SWA_WAIT;\n"
-        "SWA_DONE:\n\t"
-        "selp.u32 %0, 1, 0, p;\n\t}"
-        : "=r"(ok) : "r"(bar), "r"(parity), "n"(kParkPolls), "n"(PARK_NS) : "memory");
-  return ok != 0;
-}
-
 // Whether the phase with the given parity has completed; never suspends.
 __device__ __forceinline__ bool mbar_test(uint32_t bar, uint32_t parity) {
   uint32_t ok;
@@ -189,6 +159,48 @@ __device__ __forceinline__ bool mbar_test(uint32_t bar, uint32_t parity) {
       "selp.u32 %0, 1, 0, p;\n\t}"
       : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
   return ok != 0;
+}
+
+// The strip kernels' wait (swa_tc_strip.cuh): one try_wait, which takes some eighty cycles when the phase has completed and suspends
+// the thread for up to two microseconds when it has not; the polling lies out of the way, because they have two dozen waits in
+// code that runs once per block.  False once the poll budget is used up (about a second); the caller's warp then leaves its
+// loop, the others run into their own limit, and the kernel's end tells the host.
+// HOW: 0 spins on try_wait, kSleepPoll looks every 64 ns (kLoadPolls), anything else is the hint in ns of a parked try_wait.
+constexpr uint32_t kLoadPolls = 1u << 23;
+constexpr uint32_t kSleepPoll = ~0u;
+template <uint32_t HOW>
+__device__ __forceinline__ bool mbar_wait_polls(uint32_t bar, uint32_t parity) {
+  auto poll = [&]() {
+    uint32_t ok;
+    if constexpr (HOW == 0)
+      asm volatile(
+          "{\n\t.reg .pred p;\n\t"
+          "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+          "selp.u32 %0, 1, 0, p;\n\t}"
+          : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
+    else
+      asm volatile(
+          "{\n\t.reg .pred p;\n\t"
+          "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\n\t"
+          "selp.u32 %0, 1, 0, p;\n\t}"
+          : "=r"(ok) : "r"(bar), "r"(parity), "n"(HOW) : "memory");
+    return ok != 0;
+  };
+  if constexpr (HOW == kSleepPoll) {
+    if (__builtin_expect(mbar_test(bar, parity), 1)) return true;
+  } else {
+    if (__builtin_expect(poll(), 1)) return true;
+  }
+#pragma unroll 1
+  for (uint32_t n = HOW == kSleepPoll ? kLoadPolls : HOW == 0 ? kSpinPolls : kParkPolls; n != 0; --n) {
+    if constexpr (HOW == kSleepPoll) {
+      __nanosleep(32);
+      if (mbar_test(bar, parity)) return true;
+    } else {
+      if (poll()) return true;
+    }
+  }
+  return false;
 }
 
 __device__ __forceinline__ void fence_barrier_init() { asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory"); }
@@ -210,10 +222,27 @@ __device__ __forceinline__ void tma_load_5d(void* smem_dst, const CUtensorMap* m
       : "memory");
 }
 
-__device__ __forceinline__ void tma_prefetch_5d(const CUtensorMap* m, int c0, int c1, int c2, int c3, int c4) {
-  asm volatile("cp.async.bulk.prefetch.tensor.5d.L2.global [%0, {%1, %2, %3, %4, %5}];" ::"l"(reinterpret_cast<uint64_t>(m)), "r"(c0),
-               "r"(c1), "r"(c2), "r"(c3), "r"(c4)
-               : "memory");
+// The same by one lane of a converged warp (`el` nonzero there, umma_ts_slots).
+__device__ __forceinline__ void tma_load_5d_el(uint32_t el, uint32_t smem_dst, const CUtensorMap* m, uint32_t bar, int c0, int c1, int c2,
+                                               int c3, int c4) {
+  asm volatile(
+      "{\n\t.reg .pred e;\n\tsetp.ne.b32 e, %8, 0;\n\t"
+      "@e cp.async.bulk.tensor.5d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5, %6, %7}], [%2];\n\t}"
+      ::"r"(smem_dst), "l"(reinterpret_cast<uint64_t>(m)), "r"(bar), "r"(c0), "r"(c1), "r"(c2), "r"(c3), "r"(c4), "r"(el)
+      : "memory");
+}
+__device__ __forceinline__ void tma_prefetch_5d_el(uint32_t el, const CUtensorMap* m, int c0, int c1, int c2, int c3, int c4) {
+  asm volatile(
+      "{\n\t.reg .pred e;\n\tsetp.ne.b32 e, %6, 0;\n\t"
+      "@e cp.async.bulk.prefetch.tensor.5d.L2.global [%0, {%1, %2, %3, %4, %5}];\n\t}" ::"l"(reinterpret_cast<uint64_t>(m)), "r"(c0),
+      "r"(c1), "r"(c2), "r"(c3), "r"(c4), "r"(el)
+      : "memory");
+}
+__device__ __forceinline__ void mbar_expect_tx_el(uint32_t el, uint32_t bar, uint32_t bytes) {
+  asm volatile(
+      "{\n\t.reg .pred e;\n\tsetp.ne.b32 e, %2, 0;\n\t"
+      "@e mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;\n\t}" ::"r"(bar), "r"(bytes), "r"(el)
+      : "memory");
 }
 // 5-D tiled store shared memory -> global (bounds clipped by the map); reads of shared memory are complete after
 // tma_store_wait_read of the issuing thread.
@@ -306,19 +335,39 @@ struct SlotMask {
     for (int s = 0; s < 4; ++s) off[s] = (slots >> s & 1u) - 1u;
   }
 };
-__device__ __forceinline__ void umma_ts_slots(uint32_t d_tmem, uint32_t a_tmem, uint64_t b_desc, uint32_t idesc, uint32_t accumulate,
-                                              const SlotMask& m) {
+// The issuing warps stay converged: `el` is nonzero on one lane (always the same), which the instructions are predicated on.
+// Under a branch on elect_one five of these MMAs, 35 cycles each to the tensor pipe, took 190 cycles to issue, 94 in this form.
+__device__ __forceinline__ void umma_ts_slots(uint32_t el, uint32_t d_tmem, uint32_t a_tmem, uint64_t b_desc, uint32_t idesc,
+                                              uint32_t accumulate, const SlotMask& m) {
   asm volatile(
-      "{\n\t.reg .pred p;\n\t"
+      "{\n\t.reg .pred p, e;\n\t"
       "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, {%5, %6, %7, %8}, p;\n\t}"
-      ::"r"(d_tmem), "r"(a_tmem), "l"(b_desc), "r"(idesc), "r"(accumulate), "r"(m.off[0]), "r"(m.off[1]), "r"(m.off[2]), "r"(m.off[3])
+      "setp.ne.b32 e, %9, 0;\n\t"
+      "@e tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, {%5, %6, %7, %8}, p;\n\t}"
+      ::"r"(d_tmem), "r"(a_tmem), "l"(b_desc), "r"(idesc), "r"(accumulate), "r"(m.off[0]), "r"(m.off[1]), "r"(m.off[2]), "r"(m.off[3]),
+      "r"(el)
+      : "memory");
+}
+__device__ __forceinline__ void umma_ss_el(uint32_t el, uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc, uint32_t accumulate) {
+  asm volatile(
+      "{\n\t.reg .pred p, e;\n\t"
+      "setp.ne.b32 p, %4, 0;\n\t"
+      "setp.ne.b32 e, %5, 0;\n\t"
+      "@e tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
+      ::"r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate), "r"(el)
       : "memory");
 }
 // Arrive on `bar` once every MMA issued so far by this thread has completed.
 __device__ __forceinline__ void umma_commit(uint64_t* bar) {
   asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(bar))
                : "memory");
+}
+__device__ __forceinline__ void umma_commit_el(uint32_t el, uint64_t* bar) {
+  asm volatile(
+      "{\n\t.reg .pred e;\n\t"
+      "setp.ne.b32 e, %1, 0;\n\t"
+      "@e tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n\t}" ::"r"(smem_u32(bar)), "r"(el)
+      : "memory");
 }
 
 // ---- tcgen05: TMEM <-> registers (warp w touches lanes 32*(w%4) .. +31) ---------------------
