@@ -202,7 +202,7 @@ bwd2_kernel(const __grid_constant__ CUtensorMap tm_xqk, const __grid_constant__ 
     if (warp == 0) {
       // ------------------------------------------------------------------ TMA producer
       const LoadArgs f{x_smem, x_bytes, xqk_bytes, yqk_smem, yv_smem, yqk_stage, yv_stage, blk_bytes, sh->x_full, sh->x_empty,
-                       sh->y_full, sh->y_empty, &sh->start, &tm_xqk, &tm_xv, &tm_yqk, &tm_yv};
+                       sh->y_full, sh->y_empty, nullptr, nullptr, &sh->start, &tm_xqk, &tm_xv, &tm_yqk, &tm_yv};
       load_warp<ONE, true>(p, f, ok);
     } else if (warp == 1) {
       // ------------------------------------------------------------------ score issuer: S (+ mask) and dP of every block

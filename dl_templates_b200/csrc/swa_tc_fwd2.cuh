@@ -35,7 +35,7 @@ constexpr int kFwdRecs = kMaskRing + 4;   // block records (swa_tc_strip.cuh); a
 
 struct Fwd2Shared {
   uint64_t q_full[2], q_empty[2];
-  uint64_t kv_full[kMaxStages], kv_empty[kMaxStages], rec_ready[kFwdRecs], kx_free[kMaskRing];
+  uint64_t k_full[kMaxStages], k_empty[kMaxStages], v_full[kMaxStages], v_empty[kMaxStages], rec_ready[kFwdRecs], kx_free[kMaskRing];
   uint64_t s_full[4], p_full[4], s_free[4], pv_done[2];
   uint64_t o_full[2][4], o_free[2][4];  // per group and slot: the group's part of the quarter in it is complete / has been read
   // [quarter parity][slot]: running maximum and sum handed over, per group; read.  The softmax groups run up to nsb blocks ahead of
@@ -65,6 +65,11 @@ fwd2_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CU
   const uint32_t k_stage = blk_bytes * qch, v_stage = blk_bytes * vch;
   const uint32_t o_cols = vch * 64u;                           // TMEM columns of one O accumulator
   const int nsb = pl.nsb;                                        // score buffers = look-ahead of the score MMAs
+  // A stage of keys and values is free once the values have been accumulated -- which is also when the score buffer is free that the
+  // third block on takes.  Where shared memory holds three stages (wide heads) that block's load would start when its MMAs could: keys and
+  // values then have rings of their own, and keys are free once they have been scored (31 x 31 window, d = 128, 4 slices: 292 -> 240 us).
+  // Not where the keys are the smaller part (15 x 15, d = 64 and d_v = 128, 32 slices: one ring 236.6 us, two 238.7).
+  const bool split = !ONE && qch > 1 && pl.stages <= 3;
   // Score buffer b at column s_stride * b, O_g behind the buffers.  P gets columns of its own behind the scores when tensor
   // memory allows (p_off = N), so that the scores survive until it is certain that they need not be read again; else P is
   // written over them.
@@ -267,7 +272,7 @@ fwd2_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CU
     if (warp == 0) {
       // ------------------------------------------------------------------ TMA producer
       const LoadArgs f{q_smem, q_bytes, q_bytes, k_smem, v_smem, k_stage, v_stage, blk_bytes, sh->q_full, sh->q_empty,
-                       sh->kv_full, sh->kv_empty, &sh->start, &tm_q, nullptr, &tm_k, &tm_v};
+                       sh->k_full, sh->k_empty, split ? sh->v_full : nullptr, sh->v_empty, &sh->start, &tm_q, nullptr, &tm_k, &tm_v};
       load_warp<ONE, false>(p, f, ok);
     } else if (warp == 1) {
       // ------------------------------------------------------------------ score issuer 
@@ -297,7 +302,7 @@ fwd2_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CU
           if (xb == 0) x_par ^= 1;
           wait_spin(&sh->q_full[xb], x_par);
         }
-        wait_spin(&sh->kv_full[stage], stage_par);    // the block has landed
+        wait_spin(&sh->k_full[stage], stage_par);    // the block has landed
         // the buffer is free once the PV MMA of the block that used it last has completed
         wait_spin(&sh->s_free[buf], buf_par);
         if (!ok) break;
@@ -316,6 +321,7 @@ fwd2_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CU
           for (int k = 0; k < 4; ++k) umma_ss_el(el, sd, qd + 1024 + 2 * k, kd + blk16 + 2 * k, idesc_s, 1u);
         }
         umma_commit_el(el, &sh->s_full[buf]);
+        if (split) umma_commit_el(el, &sh->k_empty[stage]);
         umma_commit_el(el, &sh->kx_free[mslot]);                     // its mask units may be overwritten
         if (rec & kRecLeaves) umma_commit_el(el, &sh->q_empty[xb]);   // last read of this version
         trace_ev(p, 1, tn, (threadIdx.x & 31) == 0, 3 * 16 + rs);
@@ -333,7 +339,7 @@ fwd2_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CU
       const uint32_t v_stage16 = v_stage >> 4;
       const int stages = pl.stages;
       const int nks = N >> 4;
-      int stage = 0, buf = 0, buf_par = 0, grp = 0, rs = 0, rpar = 0;
+      int stage = 0, stage_par = 0, buf = 0, buf_par = 0, grp = 0, rs = 0, rpar = 0;
       const uint32_t el = elect_one();
       int tn = 0;
 #pragma unroll 1
@@ -349,6 +355,7 @@ fwd2_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CU
           const int e = __ffs(h) - 1;
           wait_spin(&sh->o_free[grp][e], (rec >> (kRecUse + e) & 1u) ^ 1u);
         }
+        if (split) wait_spin(&sh->v_full[stage], stage_par);
         wait_spin(&sh->p_full[buf], buf_par);
         if (!ok) break;
         trace_ev(p, 6, tn, (threadIdx.x & 31) == 0, 4 * 16 + rs);
@@ -356,13 +363,13 @@ fwd2_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CU
         accumulate_block(el, tmem + o_base + grp * o_cols, tmem + buf * s_stride + p_off, v_desc0 + (uint64_t)(stage * v_stage16), idesc_pv, nks,
                          8, act, fresh);
         umma_commit_el(el, &sh->s_free[buf]);
-        umma_commit_el(el, &sh->kv_empty[stage]);
+        umma_commit_el(el, split ? &sh->v_empty[stage] : &sh->k_empty[stage]);
         umma_commit_el(el, &sh->pv_done[grp]);
 #pragma unroll 1
         for (uint32_t h = act & rec >> kRecGroupLast; h; h &= h - 1) umma_commit_el(el, &sh->o_full[grp][__ffs(h) - 1]);
         trace_ev(p, 6, tn, (threadIdx.x & 31) == 0, 1 * 16 + rs);
         grp ^= 1;
-        if (++stage == stages) stage = 0;
+        if (++stage == stages) { stage = 0; stage_par ^= 1; }
         if (++buf == nsb) { buf = 0; buf_par ^= 1; }
         if (++rs == kFwdRecs) { rs = 0; rpar ^= 1; }
       }

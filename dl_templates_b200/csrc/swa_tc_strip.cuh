@@ -224,6 +224,7 @@ struct LoadArgs {
   uint8_t *yqk_smem, *yv_smem;  // streamed blocks
   uint32_t yqk_stage, yv_stage, blk_bytes;
   uint64_t *x_full, *x_empty, *y_full, *y_empty;
+  uint64_t *yv_full, *yv_empty; // null, or those of the v chunks, which then have a ring of their own
   const ItemStart* start;
   const CUtensorMap *xqk, *xv, *yqk, *yv;   // (the forward kernel has no second resident tensor: XV)
 };
@@ -245,6 +246,23 @@ __device__ __forceinline__ void load_warp(const KParams& p, const LoadArgs& f, b
   StripItem sy = strip_item(p, wy), sx = sy;
   int jy = 0, yrow = sy.h0, ycol = strip_hx0(p, sy.x0), cblk = 0, ity = 0, ny = 0;   // next streamed block; blocks loaded
   int jx = 0, itx = 0, hi = 0, from = 0, bx = 0;   // block the next version is for, in its item; quarters in so far, and before the last version; blocks before the item
+  // a ring of their own: the v chunks are loaded two blocks behind
+  const bool split = !ONE && !XV && f.yv_full != nullptr;
+  struct At { int col, row, hi, bi; };
+  At v1{}, v2{};                                   // the last two blocks
+  int vstage = 0, vstage_par = 1;
+  auto load_v = [&](const At& b, int st, uint32_t bar) {
+    uint32_t to = smem_u32(f.yv_smem) + st * yv_stage;
+#pragma unroll 1
+    for (int c = 0; c < vch; ++c, to += blk_bytes) tma_load_5d_el(el, to, f.yv, bar, c * 64, b.col, b.row, b.hi, b.bi);
+  };
+  auto load_behind = [&](const At& b) {
+    ok = __all_sync(0xffffffffu, mbar_wait_polls<kSleepPoll>(smem_u32(f.yv_empty + vstage), vstage_par));
+    if (!ok) return;
+    mbar_expect_tx_el(el, smem_u32(f.yv_full + vstage), yv_stage);
+    load_v(b, vstage, smem_u32(f.yv_full + vstage));
+    if (++vstage == stages) { vstage = 0; vstage_par ^= 1; }
+  };
   int due = 0;                                     // the next version is loaded once so many blocks are
 #pragma unroll 1
   while (ity < count || itx < count) {
@@ -300,13 +318,19 @@ __device__ __forceinline__ void load_warp(const KParams& p, const LoadArgs& f, b
       trace_ev(p, 0, tn, el, 3 * 16 + stage);
       if (!ok) break;
       const uint32_t bar = smem_u32(f.y_full + stage);
-      mbar_expect_tx_el(el, bar, y_bytes);
+      mbar_expect_tx_el(el, bar, split ? yqk_stage : y_bytes);
       uint32_t to = smem_u32(f.yqk_smem) + stage * yqk_stage;
 #pragma unroll 1
       for (int c = 0; c < qch; ++c, to += blk_bytes) tma_load_5d_el(el, to, f.yqk, bar, c * 64, ycol, yrow, wy.hi, wy.bi);
-      to = smem_u32(f.yv_smem) + stage * yv_stage;
-#pragma unroll 1
-      for (int c = 0; c < vch; ++c, to += blk_bytes) tma_load_5d_el(el, to, f.yv, bar, c * 64, ycol, yrow, wy.hi, wy.bi);
+      const At now{ycol, yrow, wy.hi, wy.bi};
+      if (split) {
+        if (ny >= 2) load_behind(v2);
+        if (!ok) break;
+        v2 = v1;
+        v1 = now;
+      } else {
+        load_v(now, stage, bar);
+      }
       ++ny;
       if (++stage == stages) { stage = 0; stage_par ^= 1; }
       ycol += KW;
@@ -321,6 +345,8 @@ __device__ __forceinline__ void load_warp(const KParams& p, const LoadArgs& f, b
       }
     }
   }
+  if (split && ok && ny >= 2) load_behind(v2);
+  if (split && ok) load_behind(v1);
 }
 
 // ---- the masking warp ---------------------------------------------------------------------------------------------
