@@ -305,8 +305,9 @@ bwd2_kernel(const __grid_constant__ CUtensorMap tm_xqk, const __grid_constant__ 
         // dV += P^T dO and dK += dS^T Q, resp. dQ += dS K
 #pragma unroll 1
         for (int t = DKDV ? 0 : 1; t < 2; ++t) {
+          // the accumulators' last quarter has been read (heads of at most 64: dV and dK at once; 251.9 -> 245.0 us, dK/dV, 64 slices)
 #pragma unroll 1
-          for (uint32_t h = fresh; h; h &= h - 1) {  // the accumulators' last quarter has been read
+          for (uint32_t h = ONE && DKDV && t ? 0u : fresh; h; h &= h - 1) {
             const int e = __ffs(h) - 1;
             wait_spin((t ? sh->qk_free : sh->v_free) + e, (rec >> (kRecUse + e) & 1u) ^ 1u);
           }

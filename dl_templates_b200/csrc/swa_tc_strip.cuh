@@ -311,7 +311,9 @@ __device__ __forceinline__ void load_warp(const KParams& p, const LoadArgs& f, b
         ++itx;
       }
       if (++xb == nxb) { xb = 0; x_par ^= 1; }
-      due = (nxb == 1 ? bx + jx : had) + stages - 2;
+      // (deep rings: one block earlier, since score MMAs then run further ahead of the accumulating ones: 201.9 -> 199.5 us, forward, 64 slices
+      // of 128 x 128 x 64; with three stages, 31 x 31 and d = 128, it would cost 3 %)
+      due = (nxb == 1 ? bx + jx : had) + stages - (stages >= 6 ? 3 : 2);
     } else {
       trace_ev(p, 0, tn, el, 2 * 16 + stage);
       ok = __all_sync(0xffffffffu, mbar_wait_polls<kSleepPoll>(smem_u32(f.y_empty + stage), stage_par));
@@ -367,6 +369,18 @@ struct MaskArgs {
   const ItemStart* start;
 };
 
+// Eight 16-bit penalties (`nb2`: two of them), one for every set bit of the low eight.
+__device__ __forceinline__ uint4 penalties(uint32_t bits, uint32_t nb2) {
+  uint32_t w[4];
+#pragma unroll
+  for (int k = 0; k < 2; ++k) {
+    const uint32_t x = (((bits >> (4 * k) & 15u) * 0x00204081u) & 0x01010101u) << 7;      // bit t -> the top bit of byte t, whose sign fills two bytes
+    asm("prmt.b32 %0, %1, %1, 0x9988;" : "=r"(w[2 * k]) : "r"(x));
+    asm("prmt.b32 %0, %1, %1, 0xbbaa;" : "=r"(w[2 * k + 1]) : "r"(x));
+  }
+  return make_uint4(w[0] & nb2, w[1] & nb2, w[2] & nb2, w[3] & nb2);
+}
+
 template <bool BF16, bool VEC, typename Wait>
 __device__ __forceinline__ void mask_warp(const KParams& p, const MaskArgs& f, bool& ok, Wait&& wait) {
   using namespace ptx;
@@ -374,6 +388,7 @@ __device__ __forceinline__ void mask_warp(const KParams& p, const MaskArgs& f, b
   const int lane = threadIdx.x & 31, slot = lane & 3, N = pl.N;
   const int t_h = p.t_h, Wtok = p.Wtok, wr = p.wr, KR = pl.KR, KW = pl.KW, ncb = pl.ncb;
   const int r4_log = 5 - pl.tw_log;
+  const uint32_t nb2 = pack2<BF16>(-p.mask_b, -p.mask_b);
   QuarterBlocks qb(p);
   const uint32_t ub = unit_bytes(pl), row_stage = ub * (uint32_t)(pl.TH >> 3), col_units = ub * (uint32_t)(pl.TW >> 3);
   int jr[4], jc[4], to[4];                         // block row and column of this lane's (up to four) streamed tokens, their offsets
@@ -458,15 +473,14 @@ __device__ __forceinline__ void mask_warp(const KParams& p, const MaskArgs& f, b
 #pragma unroll 1
           for (int n = lane; n < N; n += 32) {
             const int yx = c + n - (int)((uint32_t)(n * pl.kw_inv) >> 16) * KW;
-            int l = 1, h = 0;
+            uint32_t seen = 0u;                            // bit t: tile column t may interact with the token
             if ((uint32_t)yx < (uint32_t)Wtok) {
               const int yc = p.div_b ? (int)__umulhi((uint32_t)yx, p.div_b) : yx;
-              l = (yc - p.wc) * p.b - s.x0;                          // allowed tile columns, inclusive
-              h = (yc + p.wc + 1) * p.b - s.x0 - 1;
+              const int l = min(max((yc - p.wc) * p.b - s.x0, 0), 16), h = min(max((yc + p.wc + 1) * p.b - s.x0, 0), 16);
+              seen = (1u << h) - (1u << min(l, h));
             }
 #pragma unroll 1
-            for (int u = 0; u < (pl.TW >> 3); ++u)
-              *reinterpret_cast<uint4*>(col + u * ub + n * 16) = penalty_unit<BF16>(l - 8 * u, h - 8 * u, -p.mask_b);
+            for (int u = 0; u < (pl.TW >> 3); ++u) *reinterpret_cast<uint4*>(col + u * ub + n * 16) = penalties(~(seen >> (8 * u)), nb2);
           }
           fence_proxy_async_smem();
         }
@@ -474,20 +488,39 @@ __device__ __forceinline__ void mask_warp(const KParams& p, const MaskArgs& f, b
           uint8_t* tile = f.yr_smem + stage * row_stage;
           const int y = __shfl_sync(0xffffffffu, y0, 4 * t), at0 = __shfl_sync(0xffffffffu, at, 4 * t), at1 = __shfl_sync(0xffffffffu, at, 4 * t + 1),
                     at2 = __shfl_sync(0xffffffffu, at, 4 * t + 2), at3 = __shfl_sync(0xffffffffu, at, 4 * t + 3);
-#pragma unroll 1
-          for (int n = lane; n < N; n += 32) {
-            const int r = (int)((uint32_t)(n * pl.kw_inv) >> 16);
-            const bool in = (uint32_t)(y + r) < (uint32_t)t_h;
-            auto entry = [&](int a) { return in && (uint32_t)(a + r) <= (uint32_t)none ? a + r : none; };
-            if (pl.TW == 8) {
-              const uint2* u = reinterpret_cast<const uint2*>(f.row_parts);
-              const uint2 a = u[entry(at0)], b = u[entry(at1)], c = u[entry(at2)], d = u[entry(at3)];
-              *reinterpret_cast<uint4*>(tile + n * 16) = make_uint4(a.x, a.y, b.x, b.y);
-              *reinterpret_cast<uint4*>(tile + ub + n * 16) = make_uint4(c.x, c.y, d.x, d.y);
-            } else {
-              const uint32_t* u = reinterpret_cast<const uint32_t*>(f.row_parts);
-              *reinterpret_cast<uint4*>(tile + n * 16) = make_uint4(u[entry(at0)], u[entry(at1)], u[entry(at2)], u[entry(at3)]);
+          // All table entries of this lane's tokens before the first store: token by token this took most of the time of a block where the
+          // pattern does not repeat with the ring (15 x 15 window, d = 64, d_v = 128, 32 slices: forward kernel 235 -> 221 us, and with the
+          // column units from bits instead of comparisons 213).
+          auto entry = [&](int a, int e) {
+            const int d = a + jr[e];
+            return (uint32_t)(y + jr[e]) < (uint32_t)t_h && (uint32_t)d <= (uint32_t)none ? d : none;
+          };
+          if (pl.TW == 8) {
+            const uint2* u = reinterpret_cast<const uint2*>(f.row_parts);
+            uint2 a[4], b[4], c[4], d[4];
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+              a[e] = u[entry(at0, e)];
+              b[e] = u[entry(at1, e)];
+              c[e] = u[entry(at2, e)];
+              d[e] = u[entry(at3, e)];
             }
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+              uint8_t* to_ = tile + (lane + 32 * e) * 16;
+              if (lane + 32 * e < N) {
+                *reinterpret_cast<uint4*>(to_) = make_uint4(a[e].x, a[e].y, b[e].x, b[e].y);
+                *reinterpret_cast<uint4*>(to_ + ub) = make_uint4(c[e].x, c[e].y, d[e].x, d[e].y);
+              }
+            }
+          } else {
+            const uint32_t* u = reinterpret_cast<const uint32_t*>(f.row_parts);
+            uint4 a[4];
+#pragma unroll
+            for (int e = 0; e < 4; ++e) a[e] = make_uint4(u[entry(at0, e)], u[entry(at1, e)], u[entry(at2, e)], u[entry(at3, e)]);
+#pragma unroll
+            for (int e = 0; e < 4; ++e)
+              if (lane + 32 * e < N) *reinterpret_cast<uint4*>(tile + (lane + 32 * e) * 16) = a[e];
           }
           fence_proxy_async_smem();
         }
