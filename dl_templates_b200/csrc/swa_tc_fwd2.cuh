@@ -159,24 +159,28 @@ fwd2_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CU
         tc_fence_after();
         uint32_t r[16];
         float mx = -INFINITY, bl;
-        // Where P overwrites the scores the row maximum is taken before the exponentials in every block.  Else the running maximum
-        // is used, in a group's first block of a quarter that of the last 16 columns (the part of the block that most of the quarter's
-        // rows see), and afterwards it shows whether it served: a row whose maximum is beyond it by more than 2^8, or that had none,
-        // is done again, which is rare.  (All of a first block's scores read twice: 205 instead of 201 us, 64 slices of 128 x 128 x 64.)
-        bool exact = !OWNP;
+        // The row maximum is taken before the exponentials in every block when P overwrites the scores, else only in a group's
+        // first block of a quarter: the others use the running maximum and see afterwards whether it still serves: a row
+        // whose maximum has grown by more than 2^8 is done again, which is rare.  (A load of 16 columns takes 14 cycles.)
+        bool exact = !OWNP || first;
         tmem_ld16(s_tm, r);
-        if (!OWNP || first) {
+        if (exact) {
           float mx4[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
 #pragma unroll 1
-          for (int i = OWNP ? ng - 1 : 0; i < ng; ++i) {
+          for (int i = 0; i < ng; i += 2) {
             uint32_t t[16];
-            tmem_ld16(s_tm + 16 * i, t);
+            if (i + 1 < ng) tmem_ld16(s_tm + 16 * (i + 1), t);
             tmem_wait_ld();
 #pragma unroll
-            for (int e = 0; e < 8; ++e) mx4[e & 3] = fmaxf(mx4[e & 3], fmaxf(__uint_as_float(t[2 * e]), __uint_as_float(t[2 * e + 1])));
+            for (int e = 0; e < 8; ++e) mx4[e & 3] = fmaxf(mx4[e & 3], fmaxf(__uint_as_float(r[2 * e]), __uint_as_float(r[2 * e + 1])));
+            if (i + 1 < ng) {
+              if (i + 2 < ng) tmem_ld16(s_tm + 16 * (i + 2), r);
+#pragma unroll
+              for (int e = 0; e < 8; ++e) mx4[e & 3] = fmaxf(mx4[e & 3], fmaxf(__uint_as_float(t[2 * e]), __uint_as_float(t[2 * e + 1])));
+            }
           }
           mx = fmaxf(fmaxf(mx4[0], mx4[1]), fmaxf(mx4[2], mx4[3]));
-          if (OWNP && mx >= none_thresh) m_used = mx;
+          tmem_ld16(s_tm, r);                             // first 16 columns, in flight during the bookkeeping
         }
 #pragma unroll 1
         while (true) {
@@ -186,7 +190,7 @@ fwd2_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CU
             bool need = false;
             float m_new = m_used;
             if (mx > m_used) {
-              if (m_used == -INFINITY || first) m_used = mx;   // nothing accumulated yet for this row
+              if (m_used == -INFINITY) m_used = mx;       // nothing accumulated yet for this row
               else if ((mx - m_used) * c2 > kRescaleThreshold) { need = true; m_new = mx; }
             }
             if (__any_sync(0xffffffffu, need) && !first) {
