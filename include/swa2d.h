@@ -184,7 +184,8 @@ int swa_select_impl(const swa_geom_t* g, const swa_rope_t* rope, int32_t which);
  * would launch; 3, 4, 5: what swa_fwd_rot, swa_bwd_dq_rot, swa_bwd_dkdv_rot would launch); host-only, needs no
  * GPU.  A diagnostic without counterpart in the reference: tests use it to check that every plan stays inside
  * 227 KB of shared memory and 512 tensor-memory columns.  out[12] = tile rows, tile columns, block rows, block
- * columns, block tokens N, ring stages, score buffers (fwd) or (S, dP) pairs (bwd), resident-tile buffers,
+ * columns, block tokens N, ring stages, score buffers (strip kernels; two dP buffers beside them, bwd) or (S, dP) pairs (streamed
+ * rotation, bwd), resident-tile buffers,
  * staged cos/sin table bytes, dynamic shared memory requested, shared memory used by the layout (worst-case
  * alignment pad included), tensor-memory columns used.  Negative return: the shape runs on the SIMT kernels. */
 int swa_describe_plan(const swa_geom_t* g, const swa_rope_t* rope, int32_t which, int32_t* out);
