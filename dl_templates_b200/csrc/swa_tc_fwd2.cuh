@@ -37,7 +37,11 @@ struct Fwd2Shared {
   uint64_t q_full[2], q_empty[2];
   uint64_t k_full[kMaxStages], k_empty[kMaxStages], v_full[kMaxStages], v_empty[kMaxStages], rec_ready[kFwdRecs], kx_free[kMaskRing];
   uint64_t s_full[4], p_full[4], s_free[4], pv_done[2];
-  uint64_t o_full[2][4], o_free[2][4];  // per group and slot: the group's part of the quarter in it is complete / has been read
+  // Per group and slot: the group's part of the quarter in it is complete / has been read.  Both count only the quarters that the
+  // group has a part in -- one that lies in a single block is one group's alone -- and whoever waits for them keeps a parity bit of its own for
+  // each and turns it over at every wait.  With a parity from the uses of the slot, uses that the group is not part of go by without a
+  // wait, the barrier may be two phases behind at the next one, and the wait passes (tests/test_strip_handover.py walks the plans).
+  uint64_t o_full[2][4], o_free[2][4];
   // [quarter parity][slot]: running maximum and sum handed over, per group; read.  The softmax groups run up to nsb blocks ahead of
   // the PV MMAs -- with small windows that is several quarters of a slot -- so a barrier per slot alone could complete twice
   // before the epilogue warp looks.
@@ -340,6 +344,7 @@ fwd2_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CU
       const int stages = pl.stages;
       const int nks = N >> 4;
       int stage = 0, stage_par = 0, buf = 0, buf_par = 0, grp = 0, rs = 0, rpar = 0;
+      uint32_t free_par = 0xffu;                           // parity of the next wait for o_free, bit 4 * group + slot
       const uint32_t el = elect_one();
       int tn = 0;
 #pragma unroll 1
@@ -353,8 +358,9 @@ fwd2_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CU
 #pragma unroll 1
         for (uint32_t h = fresh; h; h &= h - 1) {        // the accumulator's last quarter has been read
           const int e = __ffs(h) - 1;
-          wait_spin(&sh->o_free[grp][e], (rec >> (kRecUse + e) & 1u) ^ 1u);
+          wait_spin(&sh->o_free[grp][e], free_par >> (4 * grp + e) & 1u);
         }
+        free_par ^= fresh << (4 * grp);
         if (split) wait_spin(&sh->v_full[stage], stage_par);
         wait_spin(&sh->p_full[buf], buf_par);
         if (!ok) break;
@@ -423,12 +429,12 @@ fwd2_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CU
             tmem_ld32(o_1 + 32, x + 32);
             tmem_wait_ld();
             tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&sh->o_free[g1][slot]);
           } else {
 #pragma unroll
             for (int e = 0; e < 64; ++e) x[e] = 0u;
           }
-          __syncwarp();
-          if (lane == 0) mbar_arrive(&sh->o_free[g1][slot]);
         }
         wait_park(&sh->ml_full[qp][slot][g2], (ml_par >> (2 * qp + g2)) & 1);
         ml_par ^= 1 << (2 * qp + g2);
@@ -486,7 +492,7 @@ fwd2_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CU
             if (m == 2 * vch - 1) {                        // the last column has been read
               tc_fence_before();
               __syncwarp();
-              if (lane < 2) mbar_arrive(&sh->o_free[lane][slot]);
+              if (lane == g2 || (both && lane == g1)) mbar_arrive(&sh->o_free[lane][slot]);
             }
 #pragma unroll
             for (int u = 0; u < 4; ++u) {

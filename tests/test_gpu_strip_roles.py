@@ -1,7 +1,11 @@
 """The roles of the strip kernels at the ends of what they hand each other: streams of blocks shorter and longer than the
 batch the masking warp works out, the record rings and the rings of keys and values."""
 import pytest
+import torch
+from test_gpu_strips import DEV
 from test_gpu_strips import test_strips_against_simt as against_simt
+
+import dl_templates_b200 as swa
 
 pytestmark = pytest.mark.gpu
 
@@ -12,3 +16,24 @@ pytestmark = pytest.mark.gpu
     (70, 20, 1, 12, 12, 128, 128, 16, 60), (19, 31, 1, 7, 7, 128, 64, 16, 9), (40, 17, 1, 15, 15, 96, 96, 8, 40), (8, 8, 16, 1, 1, 32, 32, 0, 2)])
 def test_streams_of_any_length(th, tw, b, wr, wc, dqk, dv, R, BH):
     against_simt(th, tw, b, wr, wc, dqk, dv, R, BH)
+
+
+@pytest.mark.parametrize("dtype,bound", [(torch.bfloat16, 1e-2), (torch.float16, 1.25e-3)])   # P and o rounded: 2^-9, 2^-12 of a value each
+@pytest.mark.parametrize("th,tw,b,wr,wc,BH", [(5, 24, 1, 2, 0, 700), (7, 24, 1, 0, 0, 900), (6, 24, 1, 1, 0, 600), (13, 24, 1, 2, 5, 500), (9, 12, 4, 2, 1, 300),
+                                              (81, 65, 1, 1, 0, 150), (9, 93, 1, 7, 0, 120), (63, 33, 1, 1, 1, 150)])
+def test_quarters_that_one_group_does_alone(th, tw, b, wr, wc, BH, dtype, bound):
+    """Windows at which one of the two softmax groups has no part in some quarters, many items per CTA: every row against the
+    CUDA-core kernels, and the same bits every time."""
+    N, win = th * tw * b, (b, th, tw, wr, wc)
+    g = torch.Generator(device=DEV).manual_seed(th * 1000 + tw)
+    q, k, v = (torch.randn(1, BH, N, 64, device=DEV, generator=g).to(dtype) for _ in range(3))
+    o, lse = swa.swa_forward(q, k, v, None, *win, 0.125, impl="tc")
+    o1, l1 = swa.swa_forward(q, k, v, None, *win, 0.125, impl="simt")
+    swa.check_status()
+    assert (lse - l1).abs().max().item() < 1e-3
+    row = (o.float() - o1.float()).norm(dim=-1) / (o1.float().norm(dim=-1) + 0.3 * 8 * o1.float().pow(2).mean().sqrt())
+    assert row.max().item() < 6 * bound, f"row {int(row.argmax())} off by {row.max().item():.2e}"
+    assert ((o.float() - o1.float()).norm() / o1.float().norm()).item() < bound
+    for _ in range(3):
+        again, l2 = swa.swa_forward(q, k, v, None, *win, 0.125, impl="tc")
+        assert torch.equal(again, o) and torch.equal(l2, lse)

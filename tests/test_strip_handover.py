@@ -1,0 +1,165 @@
+"""Hand-over between the softmax groups, the PV issuer and the epilogue of the forward strip kernel, checked on the planner's own
+block streams without a GPU.
+
+A wait on a barrier knows its phase by parity only: with k completions to wait for it passes at k, and also at k - 2.  It is right if k - 1
+of them are certain when it starts, whatever the roles' speed.  What is certain is worked out here with vector clocks: every
+event knows the latest event of every role that must have come before it (program order, and the waits)."""
+import ctypes as C
+import random
+import re
+
+import pytest
+import torch
+
+from test_kernel_sources import source
+
+from dl_templates_b200 import _lib
+
+
+def o_free_rule():
+    """How the kernel's source takes the parity of its waits for O_g: from the uses of the slot, or from its own waits for that
+    barrier, in which case the epilogue arrives for groups that had a part in the quarter only."""
+    text = re.sub(r"\s+", " ", source("swa_tc_fwd2.cuh"))
+    parity = re.search(r"wait_spin\(&sh->o_free\[grp\]\[e\], ([^;]*)\);", text).group(1)
+    if "kRec" in parity:
+        return "slot"
+    assert "free_par >> (4 * grp + e) & 1u" in parity and "free_par ^= fresh << (4 * grp);" in text and "uint32_t free_par = 0xffu;" in text
+    arrivals = re.findall(r"if \(([^()]*(?:\([^()]*\))?[^()]*)\) mbar_arrive\(&sh->o_free\[(\w+)\]\[slot\]\)", text)
+    assert sorted(arrivals) == [("lane == 0", "g1"), ("lane == 0", "g2"), ("lane == g2 || (both && lane == g1)", "lane")]
+    head = text[:text.index("mbar_arrive(&sh->o_free[g1][slot])")]
+    assert head.rindex("if (both) {") > head.rindex("if constexpr (ONE) {")
+    return "group"
+
+
+class Clock(dict):
+    def join(self, other):
+        for k, v in other.items():
+            if self.get(k, -1) < v:
+                self[k] = v
+
+
+class Walk:
+    """The roles of one CTA over a stream of blocks: `quarters` = (slot, use of the slot, first block, last block)."""
+
+    def __init__(self, o_rule):
+        self.o_rule, self.at, self.n, self.arrivals, self.own, self.early = o_rule, {}, {}, {}, {}, []
+
+    def event(self, role, *after):
+        c = Clock(self.at.get(role, {}))
+        for a in after:
+            if a is not None:
+                c.join(a)
+        self.n[role] = c[role] = self.n.get(role, -1) + 1
+        self.at[role] = c
+        return c
+
+    def count(self, *key):
+        self.own[key] = self.own.get(key, -1) + 1
+        return self.own[key]
+
+    def wait(self, role, bar, k, by):
+        """`role` waits for k arrivals on `bar`, all by role `by`."""
+        c, a = self.event(role), self.arrivals.get(bar, [])
+        known = sum(1 for x in a[:k] if c.get(by, -1) >= x[by])
+        if k - known >= 2:
+            self.early.append((bar, k, known))
+            k = known
+        if k > 0:
+            c.join(a[k - 1])
+
+    def run(self, quarters, n_blocks, nsb, stages, one):
+        pv, scores, handed, act, starts = [], [], {}, {}, {}
+        for q in quarters:
+            starts.setdefault(q[2], []).append(q)
+        for n in range(n_blocks):
+            for q in starts.get(n, []):
+                act[q[0]] = q
+            live, g = [q for q in act.values() if q[2] <= n <= q[3]], n & 1
+            scores.append(self.event("score", pv[n - nsb] if n >= nsb else None, pv[n - stages] if n >= stages else None))
+            masks = []
+            for slot in range(4):
+                masks.append(self.event(("softmax", g, slot), scores[n]))
+                for q in live:
+                    if q[0] == slot and q[3] - n < 2:
+                        masks[-1] = handed[slot, q[1], g] = self.event(("softmax", g, slot))
+            for q in live:
+                if n - q[2] < 2:
+                    own = self.count("pv", g, q[0])
+                    self.wait("pv", ("o_free", g, q[0]), q[1] if self.o_rule == "slot" else own, ("epilogue", q[0]))
+            self.event("pv", *masks)
+            pv.append(self.event("pv"))
+            for slot, use, first, last in (q for q in live if q[3] == n):
+                role, both = ("epilogue", slot), last > first
+                if both:
+                    self.event(role, handed[slot, use, g ^ 1], pv[n - 1])
+                if one and (both or self.o_rule == "slot"):
+                    self.arrivals.setdefault(("o_free", g ^ 1, slot), []).append(self.event(role))
+                self.event(role, handed[slot, use, g])
+                self.event(role, pv[n])
+                for h in (g, g ^ 1) if not one and (both or self.o_rule == "slot") else (g,):
+                    self.arrivals.setdefault(("o_free", h, slot), []).append(self.event(role))
+        return self.early
+
+
+def plan(th, tw, b, wr, wc, dqk, dv):
+    g = _lib.make_geom(torch.bfloat16, 1, 64, b, th, tw, wr, wc, dqk, dv, 1.0)
+    out = (C.c_int32 * 12)()
+    return list(out) if _lib.lib.swa_describe_plan(C.byref(g), None, 0, out) == 0 else None
+
+
+def streams(th, tw, b, wr, wc, p, items=12):
+    """Quarters and block count of a CTA's first items, for chunks of several heights and items taken in several strides."""
+    TW, KR, KW = p[1], p[2], p[3]
+    R4, Wtok = 32 // TW, tw * b
+    total, strips = -(-th // R4), -(-Wtok // TW)
+    halo = max(((x + TW - 1) // b + wc + 1) * b - (x // b - wc) * b for x in range(0, Wtok, TW))
+    ncb, unit = -(-halo // KW), next(u for u in range(1, 17) if u * R4 % KR == 0)
+    slides = all((i * R4 + R4 - 1 + 2 * wr) // KR < (i + 4) * R4 // KR for i in range(KR))
+    for nq in sorted({unit, 2 * unit, 3 * unit, -(-total // unit) * unit}) if slides else [4]:
+        for stride in (1, 37, 148):
+            quarters, blocks, before = [], 0, 0
+            for it in range(0, items * stride, stride):
+                r0 = it // strips % -(-total // nq) * nq * R4
+                n, h0 = min(nq, -(-(th - r0) // R4)), r0 - wr + KR * (max(0, wr - r0) // KR)
+                off, end = r0 - wr - h0, th - 1 - h0
+                for i in range(n):
+                    first, last = max(i * R4 + off, 0) // KR * ncb, min(i * R4 + off + R4 - 1 + 2 * wr, end) // KR * ncb + ncb - 1
+                    quarters.append((before + i & 3, before + i >> 2, blocks + first, blocks + last))
+                blocks += (min(n * R4 - 1 + r0 + wr - h0, end) // KR + 1) * ncb
+                before += n
+            yield quarters, blocks
+
+
+# one-cell and one-column windows, quarters that one group does alone, items whose borders break the alternation
+KNOWN = [(5, 24, 1, 2, 0), (7, 24, 1, 0, 0), (6, 24, 1, 1, 0), (13, 24, 1, 2, 5), (9, 12, 4, 2, 1), (64, 64, 1, 0, 0), (63, 33, 1, 1, 1),
+         (81, 65, 1, 1, 0), (9, 93, 1, 7, 0), (83, 127, 1, 3, 1)]
+
+
+def early_waits(rule, n_random):
+    rng, found = random.Random(11), {}
+    for t in range(len(KNOWN) + n_random):
+        if t < len(KNOWN):
+            th, tw, b, wr, wc = KNOWN[t]
+            dqk = dv = 64
+        else:
+            b, th, wr = rng.choice([1, 1, 1, 2, 4, 16]), rng.randint(1, 140), rng.randint(0, 7)
+            tw, wc = max(1, rng.randint(1, 100) // b), rng.choice([wr, rng.randint(0, 7)])
+            dqk, dv = rng.choice([(64, 64), (64, 64), (32, 32), (128, 128), (128, 64), (64, 128)])
+        wr, wc = min(wr, th - 1), min(wc, tw - 1)
+        p = plan(th, tw, b, wr, wc, dqk, dv)
+        assert p is not None
+        for quarters, blocks in streams(th, tw, b, wr, wc, p):
+            early = Walk(rule).run(quarters, blocks, p[6], p[5], dqk <= 64 and dv <= 64)
+            if early:
+                found.setdefault((th, tw, b, wr, wc, dqk, dv), early[0])
+    return found
+
+
+def test_no_wait_of_the_forward_kernel_can_pass_two_phases_early():
+    assert early_waits(o_free_rule(), 150) == {}
+
+
+def test_the_walk_sees_a_parity_taken_from_the_uses_of_the_slot():
+    """The walk is worth something: with the barriers of O_g counted by the uses of the slot, waits pass early."""
+    found = early_waits("slot", 0)
+    assert (7, 24, 1, 0, 0, 64, 64) in found and (13, 24, 1, 2, 5, 64, 64) in found and len(found) >= 6
