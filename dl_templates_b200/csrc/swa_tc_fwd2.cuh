@@ -398,7 +398,7 @@ fwd2_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CU
     uint32_t gb = 0, q0 = 0;
     ItemWalk w(sh->start);
 #pragma unroll 1
-    for (int it = 0; it < n_mine; ++it, w.next(p)) {
+    for (int it = 0; ok && it < n_mine; ++it, w.next(p)) {
       const StripItem si = strip_item(p, w);
 #pragma unroll 1
       for (int i = (slot - (int)q0) & 3; i < si.nq; i += 4) {

@@ -69,3 +69,39 @@ def test_waits_give_up_after_about_a_second():
         assert 0.5 <= polls[name] * ns * 1e-9 <= 1.5, name
     for f in ("umma.cuh", "swa_tc_strip.cuh", "swa_tc_fwd2.cuh", "swa_tc_bwd2.cuh"):          # ... and no wait has a budget of its own
         assert not re.search(r"(?<!Polls = )1u? << 2\d", source(f)), f
+
+
+def test_a_wait_that_gave_up_ends_every_loop_around_it():
+    """In the strip kernels a wait polls for about a second whether or not one before it gave up.  A loop that waits, itself or in one
+    inside it, is therefore left once `ok` is false: else a warp would give up once per work item.  (Not the loops over the slots of a
+    block, four rounds at most, nor the forward kernel's second look at a row, which ends with `if (exact) break`.)"""
+    wait = re.compile(r"\b(wait_spin|wait_park|wait|take_ml|load_behind|mbar_wait_polls(?:<\w+>)?)\(")
+    left = re.compile(r"if \(!ok(?: \|\| [^;{}]*)?\) (?:break|return);|if \(exact\) break;")
+    loops = re.compile(r"\b(?:for|while) \(|\bdo \{")
+    seen = 0
+
+    def headers(text):
+        for m in loops.finditer(text):
+            if m.group().startswith("do"):
+                yield m.start(), "", body_at(text, m.start())
+                continue
+            depth, j = 0, m.end() - 1
+            while True:
+                depth += {"(": 1, ")": -1}.get(text[j], 0)
+                if depth == 0:
+                    break
+                j += 1
+            if text[j + 1:].lstrip().startswith("{"):
+                yield m.start(), text[m.end():j], body_at(text, j + 1)
+
+    for f in ("swa_tc_strip.cuh", "swa_tc_fwd2.cuh", "swa_tc_bwd2.cuh"):
+        text = re.sub(r"\s+", " ", source(f))
+        for at, head, block in headers(text):
+            if not wait.search(block) or re.search(r"\w+ &= \w+ - 1$", head.strip()):
+                continue
+            own = block
+            for _, _, inner in headers(block[1:]):
+                own = own.replace(inner, "if (!ok) return;" if "if (!ok) return;" in inner else "")
+            seen += 1
+            assert re.match(r"[^;]*;\s*ok && ", head) or left.search(own), (f, text[at:at + 120])
+    assert seen >= 10
