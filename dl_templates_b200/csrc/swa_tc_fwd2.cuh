@@ -44,7 +44,10 @@ struct Fwd2Shared {
   uint64_t o_full[2][4], o_free[2][4];
   // [quarter parity][slot]: running maximum and sum handed over, per group; read.  The softmax groups run up to nsb blocks ahead of
   // the PV MMAs -- with small windows that is several quarters of a slot -- so a barrier per slot alone could complete twice
-  // before the epilogue warp looks.
+  // before the epilogue warp looks.  A group that has no part in a quarter skips a wait for ml_empty too.  The next one is no phase short
+  // because the PV MMAs of a quarter that lies in a single block wait for both groups' o_free: the slot's quarter before the skipped
+  // one, four blocks or more before the group's present one, has then been accumulated, which the one before it in the
+  // ring has been read for.
   uint64_t ml_full[2][4][2], ml_empty[2][4];
   float ml[2][4][2][2][32];             // [quarter parity][slot][group][maximum | sum][row]
   uint32_t rec[kFwdRecs];
@@ -355,10 +358,11 @@ fwd2_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CU
         const uint32_t rec = sh->rec[rs];
         if (!ok || (rec & kRecEnd)) break;
         const uint32_t act = rec >> kRecAct & 15u, fresh = act & rec >> kRecGroupFirst;   // first block of these quarters for this group's O_g
+        const uint32_t alone = rec >> kRecFresh & rec >> kRecEnds & 15u;    // quarters of this block only: the other group's as well (ml_empty)
 #pragma unroll 1
-        for (uint32_t h = fresh; h; h &= h - 1) {        // the accumulator's last quarter has been read
-          const int e = __ffs(h) - 1;
-          wait_spin(&sh->o_free[grp][e], free_par >> (4 * grp + e) & 1u);
+        for (uint32_t h = fresh | alone << 4; h; h &= h - 1) {              // the accumulators' last quarter has been read
+          const int e = (__ffs(h) - 1) ^ 4 * grp;
+          wait_spin(&sh->o_free[0][e], free_par >> e & 1u);
         }
         free_par ^= fresh << (4 * grp);
         if (split) wait_spin(&sh->v_full[stage], stage_par);

@@ -1,9 +1,10 @@
 """Hand-over between the softmax groups, the PV issuer and the epilogue of the forward strip kernel, checked on the planner's own
 block streams without a GPU.
 
-A wait on a barrier knows its phase by parity only: with k completions to wait for it passes at k, and also at k - 2.  It is right if k - 1
-of them are certain when it starts, whatever the roles' speed.  What is certain is worked out here with vector clocks: every
-event knows the latest event of every role that must have come before it (program order, and the waits)."""
+A wait on a barrier knows its phase by parity only: with k completions to wait for it passes at k, and also at k - 2, but not at k + 1.
+It is right if k - 1 of them are certain when it starts, and the one after the k'th cannot come before it has passed, whatever the
+roles' speed.  What is certain is worked out here with vector clocks: every event knows the latest event of every role that
+must have come before it (program order, and the waits)."""
 import ctypes as C
 import random
 import re
@@ -16,19 +17,26 @@ from test_kernel_sources import source
 from dl_templates_b200 import _lib
 
 
-def o_free_rule():
-    """How the kernel's source takes the parity of its waits for O_g: from the uses of the slot, or from its own waits for that
-    barrier, in which case the epilogue arrives for groups that had a part in the quarter only."""
+def rules():
+    """How the kernel's source takes the parity of its waits for O_g, whether a quarter that lies in one block waits for both groups,
+    and where the hand-over of maximum and sum takes its phase from."""
     text = re.sub(r"\s+", " ", source("swa_tc_fwd2.cuh"))
-    parity = re.search(r"wait_spin\(&sh->o_free\[grp\]\[e\], ([^;]*)\);", text).group(1)
+    index, parity = re.search(r"wait_spin\(&sh->o_free((?:\[\w+\])+), ([^;]*)\);", text).groups()
+    assert "wait_spin(&sh->ml_empty[qp][quarter], (rec >> kRecUse2 & 1u) ^ 1u);" in text
+    assert text.count("mbar_arrive(&sh->ml_empty[qp][slot])") == 1
     if "kRec" in parity:
-        return "slot"
-    assert "free_par >> (4 * grp + e) & 1u" in parity and "free_par ^= fresh << (4 * grp);" in text and "uint32_t free_par = 0xffu;" in text
+        return "slot", False
     arrivals = re.findall(r"if \(([^()]*(?:\([^()]*\))?[^()]*)\) mbar_arrive\(&sh->o_free\[(\w+)\]\[slot\]\)", text)
     assert sorted(arrivals) == [("lane == 0", "g1"), ("lane == 0", "g2"), ("lane == g2 || (both && lane == g1)", "lane")]
     head = text[:text.index("mbar_arrive(&sh->o_free[g1][slot])")]
     assert head.rindex("if (both) {") > head.rindex("if constexpr (ONE) {")
-    return "group"
+    assert "uint32_t free_par = 0xffu;" in text and "free_par ^= fresh << (4 * grp);" in text
+    if index == "[grp][e]" and parity == "free_par >> (4 * grp + e) & 1u":
+        return "group", False
+    assert index == "[0][e]" and parity == "free_par >> e & 1u"
+    assert "for (uint32_t h = fresh | alone << 4; h; h &= h - 1) { const int e = (__ffs(h) - 1) ^ 4 * grp;" in text
+    assert "alone = rec >> kRecFresh & rec >> kRecEnds & 15u;" in text
+    return "group", True
 
 
 class Clock(dict):
@@ -41,8 +49,9 @@ class Clock(dict):
 class Walk:
     """The roles of one CTA over a stream of blocks: `quarters` = (slot, use of the slot, first block, last block)."""
 
-    def __init__(self, o_rule):
-        self.o_rule, self.at, self.n, self.arrivals, self.own, self.early = o_rule, {}, {}, {}, {}, []
+    def __init__(self, o_rule, both_groups):
+        self.o_rule, self.both_groups = o_rule, both_groups
+        self.at, self.n, self.arrivals, self.waits, self.own, self.wrong = {}, {}, {}, {}, {}, []
 
     def event(self, role, *after):
         c = Clock(self.at.get(role, {}))
@@ -53,19 +62,28 @@ class Walk:
         self.at[role] = c
         return c
 
-    def count(self, *key):
-        self.own[key] = self.own.get(key, -1) + 1
-        return self.own[key]
+    def own_parts(self, role, g, slot):
+        return self.own.get((role, g, slot), 0)
 
     def wait(self, role, bar, k, by):
         """`role` waits for k arrivals on `bar`, all by role `by`."""
         c, a = self.event(role), self.arrivals.get(bar, [])
         known = sum(1 for x in a[:k] if c.get(by, -1) >= x[by])
         if k - known >= 2:
-            self.early.append((bar, k, known))
-            k = known
-        if k > 0:
-            c.join(a[k - 1])
+            self.wrong.append(("early", bar, k, known))
+        if len(a) > k:
+            self.wrong.append(("late", bar, k, len(a)))
+        m = known if k - known >= 2 else k
+        if m > 0:
+            c.join(a[m - 1])
+        self.waits.setdefault((bar, k), []).append((role, self.event(role)[role]))
+
+    def arrive(self, role, bar):
+        c, a = self.event(role), self.arrivals.setdefault(bar, [])
+        for r, n in self.waits.get((bar, len(a)), []):
+            if c.get(r, -1) < n:
+                self.wrong.append(("late", bar, len(a), r))
+        a.append(c)
 
     def run(self, quarters, n_blocks, nsb, stages, one):
         pv, scores, handed, act, starts = [], [], {}, {}, {}
@@ -81,24 +99,31 @@ class Walk:
                 masks.append(self.event(("softmax", g, slot), scores[n]))
                 for q in live:
                     if q[0] == slot and q[3] - n < 2:
+                        self.wait(("softmax", g, slot), ("ml_empty", q[1] & 1, slot), q[1] >> 1, ("epilogue", slot))
                         masks[-1] = handed[slot, q[1], g] = self.event(("softmax", g, slot))
-            for q in live:
-                if n - q[2] < 2:
-                    own = self.count("pv", g, q[0])
-                    self.wait("pv", ("o_free", g, q[0]), q[1] if self.o_rule == "slot" else own, ("epilogue", q[0]))
+            for slot, use, first, last in live:
+                for h in (g, g ^ 1) if first == last and self.both_groups else (g,) if n - first < 2 else ():
+                    k = use if self.o_rule == "slot" else self.own_parts("pv", h, slot)
+                    self.wait("pv", ("o_free", h, slot), k, ("epilogue", slot))
+            for slot, use, first, last in live:
+                if n - first < 2:
+                    self.own["pv", g, slot] = self.own_parts("pv", g, slot) + 1
             self.event("pv", *masks)
             pv.append(self.event("pv"))
             for slot, use, first, last in (q for q in live if q[3] == n):
                 role, both = ("epilogue", slot), last > first
+                other = both or self.o_rule == "slot"               # also arrives for the group of the block before
                 if both:
                     self.event(role, handed[slot, use, g ^ 1], pv[n - 1])
-                if one and (both or self.o_rule == "slot"):
-                    self.arrivals.setdefault(("o_free", g ^ 1, slot), []).append(self.event(role))
+                if one and other:
+                    self.arrive(role, ("o_free", g ^ 1, slot))
                 self.event(role, handed[slot, use, g])
+                self.arrive(role, ("ml_empty", use & 1, slot))
                 self.event(role, pv[n])
-                for h in (g, g ^ 1) if not one and (both or self.o_rule == "slot") else (g,):
-                    self.arrivals.setdefault(("o_free", h, slot), []).append(self.event(role))
-        return self.early
+                self.arrive(role, ("o_free", g, slot))
+                if not one and other:
+                    self.arrive(role, ("o_free", g ^ 1, slot))
+        return self.wrong
 
 
 def plan(th, tw, b, wr, wc, dqk, dv):
@@ -135,7 +160,7 @@ KNOWN = [(5, 24, 1, 2, 0), (7, 24, 1, 0, 0), (6, 24, 1, 1, 0), (13, 24, 1, 2, 5)
          (81, 65, 1, 1, 0), (9, 93, 1, 7, 0), (83, 127, 1, 3, 1)]
 
 
-def early_waits(rule, n_random):
+def wrong_waits(o_rule, both_groups, n_random):
     rng, found = random.Random(11), {}
     for t in range(len(KNOWN) + n_random):
         if t < len(KNOWN):
@@ -149,17 +174,27 @@ def early_waits(rule, n_random):
         p = plan(th, tw, b, wr, wc, dqk, dv)
         assert p is not None
         for quarters, blocks in streams(th, tw, b, wr, wc, p):
-            early = Walk(rule).run(quarters, blocks, p[6], p[5], dqk <= 64 and dv <= 64)
-            if early:
-                found.setdefault((th, tw, b, wr, wc, dqk, dv), early[0])
+            wrong = Walk(o_rule, both_groups).run(quarters, blocks, p[6], p[5], dqk <= 64 and dv <= 64)
+            if wrong:
+                found.setdefault((th, tw, b, wr, wc, dqk, dv), wrong)
     return found
 
 
-def test_no_wait_of_the_forward_kernel_can_pass_two_phases_early():
-    assert early_waits(o_free_rule(), 150) == {}
+def test_every_wait_of_the_forward_kernel_knows_its_phase():
+    assert wrong_waits(*rules(), 150) == {}
 
 
-def test_the_walk_sees_a_parity_taken_from_the_uses_of_the_slot():
-    """The walk is worth something: with the barriers of O_g counted by the uses of the slot, waits pass early."""
-    found = early_waits("slot", 0)
-    assert (7, 24, 1, 0, 0, 64, 64) in found and (13, 24, 1, 2, 5, 64, 64) in found and len(found) >= 6
+@pytest.mark.parametrize("o_rule,both_groups,bar,where", [
+    ("slot", False, "o_free", [(7, 24, 1, 0, 0), (13, 24, 1, 2, 5), (63, 33, 1, 1, 1)]), ("group", False, "ml_empty", [(81, 65, 1, 1, 0)])])
+def test_the_walk_sees_phases_that_are_not_certain(o_rule, both_groups, bar, where):
+    """The walk is worth something: waits pass early where the phases of O_g are counted by the uses of the slot, and those of the maxima do
+    where a quarter in one block waits for its own group only."""
+    found = wrong_waits(o_rule, both_groups, 0)
+    for w in where:
+        assert any(kind == "early" and b[0] == bar for kind, b, _, _ in found[*w, 64, 64]), w
+
+
+def test_the_walk_sees_waits_that_come_too_late():
+    """... and waits that may never end: the uses of the slot counted, both groups waited for, and the epilogue early for a group without a part."""
+    found = wrong_waits("slot", True, 0)
+    assert any(kind == "late" and b[0] == "o_free" for kind, b, _, _ in found[7, 24, 1, 0, 0, 64, 64])
