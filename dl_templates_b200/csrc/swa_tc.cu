@@ -207,14 +207,16 @@ bool make_plan_shape(const swa_geom_t* g, int which, int TH, int TW, uint32_t ta
 }
 
 // Shared memory of the strip kernels beside resident rows, ring and tables: alignment pad of the swizzled tiles, barrier /
-// exchange block, row parts of the window mask, backward the lse / delta of streamed or resident rows.
+// exchange block, row parts of the window mask, dK/dV the lse / delta of streamed rows.
 uint32_t strip_slack(const swa_geom_t* g, int which, int R4) {
   const uint32_t sh = which == 0 ? (uint32_t)sizeof(Fwd2Shared) : (uint32_t)sizeof(Bwd2Shared);
   return 1024u + ((sh + 15u) & ~15u) + row_parts_bytes(g->row_size, R4) + (which == 0 ? 0u : bwd_vec_bytes(which == 2));
 }
 
-// ... and the mask units: three per ring entry.
-uint32_t mask_bytes(int N) { return (uint32_t)N * 16u * 3u * kMaskRing; }
+// ... and the mask units: three per ring entry.  In dQ the room of one more is left free: with it one plan in seven would be another, with a
+// second resident buffer or strips of the other width, and not all of them a faster one (188 x 100 grid, 9 x 61 window, d = 96, d_v = 32,
+// 21 slices: 338 -> 370 us; 59 x 208, 3 x 61, d = 128, d_v = 64: 252 -> 209).
+uint32_t mask_bytes(int N, int which) { return (uint32_t)N * 16u * (3u * kMaskRing + (which == 1 ? 1u : 0u)); }
 
 // Blocks of a chunk of `nq` quarters whose first row is r0 (the kernels' strip_item).
 int strip_blocks(const swa_geom_t* g, const Plan& pl, int r0, int nq) {
@@ -340,7 +342,7 @@ bool make_strip_shape(const swa_geom_t* g, int which, int TW, Plan* out) {
   // output staging for a whole quarter; for wide heads, whose quarters never follow each other block by block, one chunk (the
   // forward kernel: none)
   pl.stg = which == 0 ? (qch == 1 && vch == 1) : qch == 1 && vch == 1 ? out_chunks : 1;
-  const uint32_t fixed = 8192u + 4u * pl.stg * kStageChunk + slack;
+  const uint32_t fixed = kIndicatorBytes + 4u * pl.stg * kStageChunk + slack;
   long best_cost = -1;
   for (int ncb = 1; ncb <= 16 && best_cost < 0; ++ncb)
     for (int KW = (hw + ncb - 1) / ncb; KW <= 128 && (ncb == 1 || KW * (ncb - 1) < hw); ++KW)
@@ -360,7 +362,7 @@ bool make_strip_shape(const swa_geom_t* g, int which, int TW, Plan* out) {
         // One resident buffer leaves room for larger blocks, but nothing overlaps the load of an item's resident rows (about
         // 3000 cycles, the time of 250 columns); sliding strips need two.
         for (int nxb = kn.nxb && which ? kn.nxb : 2; nxb >= (kn.nxb || slides || which == 0 ? 2 : 1) && nxb >= 1; --nxb) {
-          if (fixed + nxb * x_bytes + min_stages * (uint32_t)N * row_bytes + mask_bytes(N) > kSmemLimit) continue;
+          if (fixed + nxb * x_bytes + min_stages * (uint32_t)N * row_bytes + mask_bytes(N, which) > kSmemLimit) continue;
           // executed columns + what a block costs beside them: backward the latency chain of a buffer pair, as much as a
           // hundred columns; forward the groups' work per block
           const long cost = (blocks * (N + (which == 0 ? 40 : 100)) + (nxb == 1 ? items * 250 : 0)) * pl.n_tiles_x;
@@ -379,7 +381,7 @@ bool make_strip_shape(const swa_geom_t* g, int which, int TW, Plan* out) {
     if (pl.KW < hw || pl.KW > 128 || pl.KR > 16) return false;      // an override must still hold a whole halo row
     pl.nxb = 2;
   }
-  const uint32_t stage = (uint32_t)pl.N * row_bytes, rest = fixed + pl.nxb * x_bytes + mask_bytes(pl.N);
+  const uint32_t stage = (uint32_t)pl.N * row_bytes, rest = fixed + pl.nxb * x_bytes + mask_bytes(pl.N, which);
   pl.kr_inv = (65536 + pl.KR - 1) / pl.KR;
   pl.kw_inv = (65536 + pl.KW - 1) / pl.KW;
   pl.tw_log = TW == 8 ? 3 : 4;
@@ -665,7 +667,7 @@ bool describe_plan(const swa_geom_t* g, const swa_rope_t* rope, int which, int32
   if (!(v2 ? make_plan_prerot(g, kind, &pl) : make_plan(g, rope, kind, &pl))) return false;
   const uint32_t qch = (g->d_qk + 63) / 64, vch = (g->d_v + 63) / 64, N = pl.N;
   const uint32_t xrow = v2 ? 0u : kXRowBytes;                               // window-mask bytes per streamed token of a stage
-  const uint32_t x_fixed = v2 ? 8192u + 4u * pl.stg * kStageChunk + mask_bytes(pl.N) + row_parts_bytes(g->row_size, pl.R4) : 128u * kXRowBytes;
+  const uint32_t x_fixed = v2 ? kIndicatorBytes + 4u * pl.stg * kStageChunk + mask_bytes(pl.N, kind) + row_parts_bytes(g->row_size, pl.R4) : 128u * kXRowBytes;
   uint32_t used = 1023, tmem = 0;   // worst-case pad to the 1024-byte alignment of the swizzled tiles
   if (kind == 0) {
     used += 2 * qch * 16384u + x_fixed + pl.stages * N * ((qch + vch) * 128u + xrow);

@@ -27,9 +27,11 @@ namespace swa {
 namespace tc {
 
 constexpr int kBwdRecs = kMaskRing + 3;   // block records (swa_tc_strip.cuh); at most three score buffers
-// Shared memory for the softmax statistics: dK/dV [record][-lse | -delta][128] of the streamed queries, dQ [use parity][slot]
-// [-lse | -delta][32] of the resident ones.
-__host__ __device__ constexpr uint32_t bwd_vec_bytes(bool dkdv) { return dkdv ? kBwdRecs * 1024u : 2048u; }
+// Shared memory for the softmax statistics: dK/dV [record][-lse | -delta][128] of the streamed queries, behind the indicator units;
+// dQ [use parity][slot][-lse | -delta][32] of the resident ones, in the place of the fourth of them.  (In 2 KB of their own they cost dQ
+// plans of tall windows their block size: 256 x 256, 57 x 31 window, d = 128, 6 slices, blocks of 48 tokens 952 us, of 80 669.)
+__host__ __device__ constexpr uint32_t bwd_vec_bytes(bool dkdv) { return dkdv ? kBwdRecs * 1024u : 0u; }
+static_assert(kIndicatorUnit >= 2 * 4 * 2 * 32 * sizeof(float), "lse / delta of the dQ kernel");
 
 struct Bwd2Shared {
   uint64_t x_full[2], x_empty[2];
@@ -70,8 +72,9 @@ bwd2_kernel(const __grid_constant__ CUtensorMap tm_xqk, const __grid_constant__ 
   uint8_t* yr_smem = yv_smem + pl.stages * yv_stage;            // window mask: row units of the mask ring,
   uint8_t* yc_smem = yr_smem + kMaskRing * ub * (pl.TH >> 3);   // ... column units,
   uint8_t* xx_smem = yc_smem + kMaskRing * ub * (pl.TW >> 3);  // ... indicator units of the resident rows
-  float* vec_smem = reinterpret_cast<float*>(xx_smem + 8192);
-  Bwd2Shared* sh = reinterpret_cast<Bwd2Shared*>(reinterpret_cast<uint8_t*>(vec_smem) + bwd_vec_bytes(DKDV));
+  constexpr int xx_units = DKDV ? 4 : 3;
+  float* vec_smem = reinterpret_cast<float*>(xx_smem + xx_units * kIndicatorUnit);
+  Bwd2Shared* sh = reinterpret_cast<Bwd2Shared*>(xx_smem + kIndicatorBytes + bwd_vec_bytes(DKDV));
   uint8_t* row_parts = reinterpret_cast<uint8_t*>(sh) + ((sizeof(Bwd2Shared) + 15) & ~size_t(15));
   // Tensor memory: score buffer b at column N b, the two dP buffers behind them, then the accumulators.  P and dS replace the scores,
   // 16 columns by 16 -- in dK/dV P in the first eight, dS in the others, so that a dP buffer is free once it has been read and the next
@@ -94,7 +97,7 @@ bwd2_kernel(const __grid_constant__ CUtensorMap tm_xqk, const __grid_constant__ 
   }
   build_row_parts<BF16>(row_parts, threadIdx.x, kBwdThreads, p);
   if (threadIdx.x < 128) {
-    write_indicator_units<BF16>(xx_smem, threadIdx.x, p);
+    write_indicator_units<BF16, xx_units>(xx_smem, threadIdx.x, p);
   }
   fence_proxy_async_smem();
   tc_fence_before();
@@ -211,15 +214,16 @@ bwd2_kernel(const __grid_constant__ CUtensorMap tm_xqk, const __grid_constant__ 
       const uint32_t hi_sw = smem_desc_hi(1024, true), hi_ns = smem_desc_hi(kUnitSbo, false);
       const uint64_t x_desc0 = smem_desc_from(smem_u32(x_smem), 16, hi_sw),
                      yqk_desc0 = smem_desc_from(smem_u32(yqk_smem), 16, hi_sw), yv_desc0 = smem_desc_from(smem_u32(yv_smem), 16, hi_sw),
-                     xx_desc0 = smem_desc_from(smem_u32(xx_smem), 2048, hi_ns);
+                     xx_desc0 = smem_desc_from(smem_u32(xx_smem), kIndicatorUnit, hi_ns);
       const uint32_t yqk16 = yqk_stage >> 4, yv16 = yv_stage >> 4, blk16 = blk_bytes >> 4, x16 = x_bytes >> 4;
-      const uint32_t yr0 = smem_u32(yr_smem), yc0 = smem_u32(yc_smem), yz0 = smem_u32(xx_smem);
+      const uint32_t yr0 = smem_u32(yr_smem), yc0 = smem_u32(yc_smem);
+      [[maybe_unused]] const uint32_t yz0 = smem_u32(xx_smem);
       int stage = 0, stage_par = 0, buf = 0, buf_par = 1, xb = nxb - 1, x_par = 1;   // resident buffer in use; parity of its "full" phase
       int rbuf = 0, rbuf_par = 0, started = 0;   // score buffer of the block that read this block's dP buffer last; blocks so far, up to 2
       uint32_t dp = dp0;
       int mslot = 0, rs = 0, rpar = 0;
       const int stages = pl.stages;
-      // units of a ring entry: 0 and 1 of the first step, 2 and (unused) 3 of the second, from where and how far to the next entry
+      // units of a ring entry: 0 and 1 of the first step, 2 and (unused) 3 of the second (dQ: 1 and 2), from where and how far to the next entry
       const uint32_t row_step = ub * (pl.TH >> 3), col_step = ub * (pl.TW >> 3);
       const bool tw8 = pl.TW == 8;
       const uint32_t el = elect_one();
@@ -262,7 +266,8 @@ bwd2_kernel(const __grid_constant__ CUtensorMap tm_xqk, const __grid_constant__ 
         const uint32_t yc = yc0 + mslot * col_step;
         const uint32_t u0 = yr0 + mslot * row_step, u1 = tw8 ? u0 + ub : yc, u2 = tw8 ? yc : yc + ub;
         umma_ss_el(el, s_tm, xx_desc0, smem_desc_from(u0, u1 - u0, hi_ns), idesc_s, 0u);
-        umma_ss_el(el, s_tm, xx_desc0 + 256, smem_desc_from(u2, yz0 - u2, hi_ns), idesc_s, 1u);
+        if constexpr (DKDV) umma_ss_el(el, s_tm, xx_desc0 + 256, smem_desc_from(u2, yz0 - u2, hi_ns), idesc_s, 1u);
+        else umma_ss_el(el, s_tm, xx_desc0 + 128, smem_desc_from(u1, u2 - u1, hi_ns), idesc_s, 1u);
 #pragma unroll
         for (int k = 0; k < 4; ++k) umma_ss_el(el, s_tm, xd + 2 * k, yd + 2 * k, idesc_s, 1u);
         if (qch > 1) {

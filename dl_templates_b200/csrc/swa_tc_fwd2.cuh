@@ -90,7 +90,7 @@ fwd2_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CU
   uint8_t* kr_smem = v_smem + pl.stages * v_stage;              // window mask: row units of the mask ring,
   uint8_t* kc_smem = kr_smem + kMaskRing * ub * (pl.TH >> 3);   // ... column units,
   uint8_t* qx_smem = kc_smem + kMaskRing * ub * (pl.TW >> 3);  // ... indicator units of the query rows
-  Fwd2Shared* sh = reinterpret_cast<Fwd2Shared*>(qx_smem + 8192);
+  Fwd2Shared* sh = reinterpret_cast<Fwd2Shared*>(qx_smem + kIndicatorBytes);
   uint8_t* row_parts = reinterpret_cast<uint8_t*>(sh) + ((sizeof(Fwd2Shared) + 15) & ~size_t(15));
 
   const int warp = threadIdx.x >> 5;
@@ -287,7 +287,7 @@ fwd2_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CU
       const uint32_t idesc_s = instr_desc(fmt, 128, N, 0, 0);
       const uint32_t hi_sw = smem_desc_hi(1024, true), hi_ns = smem_desc_hi(kUnitSbo, false);
       const uint64_t q_desc0 = smem_desc_from(smem_u32(q_smem), 16, hi_sw), k_desc0 = smem_desc_from(smem_u32(k_smem), 16, hi_sw),
-                     qx_desc0 = smem_desc_from(smem_u32(qx_smem), 2048, hi_ns);
+                     qx_desc0 = smem_desc_from(smem_u32(qx_smem), kIndicatorUnit, hi_ns);
       const uint32_t k_stage16 = k_stage >> 4, blk16 = blk_bytes >> 4;
       const uint32_t kr0 = smem_u32(kr_smem), kc0 = smem_u32(kc_smem), kz0 = smem_u32(qx_smem);
       int stage = 0, stage_par = 0, buf = 0, buf_par = 1, xb = 1, x_par = 1;   // query buffer in use; parity of its "full" phase

@@ -158,19 +158,22 @@ struct QuarterWalk {
 // column it may not interact with.  Every 8 of those columns (a "unit", 16 bytes of a row) are a tile of their own,
 // rows one after the other (8-row core matrices 128 bytes apart), so that what changes at different times lies apart:
 // the row units with the blocks, the column units with the strips.  The fourth unit is unused: the resident rows' is zero, and the
-// streamed side is pointed at their units (any finite numbers behind the others in memory).
+// streamed side is pointed at their units (any finite numbers behind the others in memory).  The dQ kernel has its lse / delta in that
+// unit's place and contracts the middle one of the three twice instead, which adds nothing to allowed pairs and one penalty more to
+// others.
 constexpr uint32_t kUnitSbo = 128;
+constexpr uint32_t kIndicatorUnit = 128 * 16, kIndicatorBytes = 4 * kIndicatorUnit;
 constexpr int kMaskRing = 4;      // blocks whose units are held; evenly sliding quarters repeat them every four blocks
 __device__ __forceinline__ uint32_t unit_bytes(const Plan& pl) { return (uint32_t)pl.N * 16u; }
 
-// Indicator units of the resident rows (4 x 128 rows), the same for every item.
-template <bool BF16>
+// Indicator units of the resident rows (128 rows each), the same for every item.
+template <bool BF16, int UNITS = 4>
 __device__ __forceinline__ void write_indicator_units(uint8_t* xx, int row, const KParams& p) {
   const int hot_r = row >> p.pl.tw_log, hot_c = p.pl.TH + (row & (p.pl.TW - 1));
   const uint16_t one = (uint16_t)(pack2<BF16>(p.mask_a, 0.f) & 0xffffu);
 #pragma unroll 1
-  for (int e = 0; e < 32; ++e)
-    reinterpret_cast<uint16_t*>(xx + (e >> 3) * 2048 + row * 16)[e & 7] = (e == hot_r || e == hot_c) ? one : (uint16_t)0;
+  for (int e = 0; e < 8 * UNITS; ++e)
+    reinterpret_cast<uint16_t*>(xx + (e >> 3) * kIndicatorUnit + row * 16)[e & 7] = (e == hot_r || e == hot_c) ? one : (uint16_t)0;
 }
 
 // The row part of a streamed token depends on which quarter holds each slot: it is put together per block from the entries

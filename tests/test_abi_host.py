@@ -233,6 +233,15 @@ def test_head_dims_the_tensor_core_kernels_take():
             assert (_lib.lib.swa_describe_plan(C.byref(g), C.byref(r), 3, out) == 0) == plain, d
 
 
+@pytest.mark.parametrize("th,tw,b,wr,wc,dqk,dv", [(256, 256, 1, 28, 15, 128, 128), (184, 37, 1, 57, 4, 96, 128), (242, 139, 1, 31, 0, 96, 96),
+                                                  (244, 3, 16, 59, 2, 96, 96), (154, 153, 1, 51, 15, 96, 128)])
+def test_dq_keeps_its_block_size_where_windows_are_tall(th, tw, b, wr, wc, dqk, dv):
+    """The softmax statistics of resident rows take no shared memory that these plans need: blocks of 80 tokens (48 or 64 without)."""
+    g = _geom(t_height=th, t_width=tw, b_size=b, row_size=wr, col_size=wc, d_qk=dqk, d_v=dv)
+    code, p = _plan(g, None, 1)
+    assert code == 0 and p[4] == 80
+
+
 def test_describe_plan_rejects_bad_arguments():
     g = _geom()
     assert _lib.lib.swa_describe_plan(C.byref(g), None, 0, None) < 0

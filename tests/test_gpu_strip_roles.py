@@ -37,3 +37,9 @@ def test_quarters_that_one_group_does_alone(th, tw, b, wr, wc, BH, dtype, bound)
     for _ in range(3):
         again, l2 = swa.swa_forward(q, k, v, None, *win, 0.125, impl="tc")
         assert torch.equal(again, o) and torch.equal(l2, lse)
+
+
+@pytest.mark.parametrize("th,tw,b,wr,wc,dqk,dv,R,BH", [(70, 33, 1, 28, 15, 128, 128, 32, 3), (64, 21, 1, 31, 0, 96, 96, 16, 4), (61, 3, 16, 29, 2, 96, 96, 0, 2)])
+def test_tall_windows_of_wide_heads(th, tw, b, wr, wc, dqk, dv, R, BH):
+    """Largest blocks beside the softmax statistics of the resident rows: not a byte of shared memory to spare."""
+    against_simt(th, tw, b, wr, wc, dqk, dv, R, BH)
