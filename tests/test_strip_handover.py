@@ -12,6 +12,7 @@ import re
 import pytest
 import torch
 
+from test_gpu_strip_roles import STREAMS
 from test_kernel_sources import source
 
 from dl_templates_b200 import _lib
@@ -126,10 +127,10 @@ class Walk:
         return self.wrong
 
 
-def plan(th, tw, b, wr, wc, dqk, dv):
+def plan(th, tw, b, wr, wc, dqk, dv, which=0):
     g = _lib.make_geom(torch.bfloat16, 1, 64, b, th, tw, wr, wc, dqk, dv, 1.0)
     out = (C.c_int32 * 12)()
-    return list(out) if _lib.lib.swa_describe_plan(C.byref(g), None, 0, out) == 0 else None
+    return list(out) if _lib.lib.swa_describe_plan(C.byref(g), None, which, out) == 0 else None
 
 
 def streams(th, tw, b, wr, wc, p, items=12):
@@ -198,3 +199,14 @@ def test_the_walk_sees_waits_that_come_too_late():
     """... and waits that may never end: the uses of the slot counted, both groups waited for, and the epilogue early for a group without a part."""
     found = wrong_waits("slot", True, 0)
     assert any(kind == "late" and b[0] == "o_free" for kind, b, _, _ in found[7, 24, 1, 0, 0, 64, 64])
+
+
+def test_the_streams_that_run_on_a_gpu_have_every_kind_of_plan():
+    """Keys and values in one ring and in rings of their own (d_qk > 64, three stages), two to four score buffers, one and two resident
+    buffers, strips of either width: a change of the planner that loses one of them shows here."""
+    plans = [[(dqk, plan(th, tw, b, wr, wc, dqk, dv, which)) for th, tw, b, wr, wc, dqk, dv, _, _ in STREAMS] for which in range(3)]
+    assert {p[5] <= 3 for d, p in plans[0] if d > 64} == {True, False}
+    assert {p[6] for _, p in plans[0]} >= {3, 4}
+    for kernel in plans[1:]:
+        assert {p[6] for _, p in kernel} == {2, 3} and {p[7] for _, p in kernel} == {1, 2}
+    assert {p[1] for kernel in plans for _, p in kernel} == {8, 16}
