@@ -363,8 +363,11 @@ bool make_strip_shape(const swa_geom_t* g, int which, int TW, Plan* out) {
         // 3000 cycles, the time of 250 columns); sliding strips need two.
         for (int nxb = kn.nxb && which ? kn.nxb : 2; nxb >= (kn.nxb || slides || which == 0 ? 2 : 1) && nxb >= 1; --nxb) {
           if (fixed + nxb * x_bytes + min_stages * (uint32_t)N * row_bytes + mask_bytes(N, which) > kSmemLimit) continue;
-          // executed columns + what a block costs beside them: backward the latency chain of a buffer pair, as much as a
-          // hundred columns; forward the groups' work per block
+          // executed columns + what a block costs beside them: backward as much as a hundred columns, forward forty.  (Fitted on kernels
+          // whose blocks took a quarter longer; the number of score buffers, two or three, is not in it.  On the present ones, 49 plans of 17
+          // geometries against those of the other strip width and of smaller blocks and either resident buffer count: the fastest
+          // or within 3 % of it in 44, 5 to 8 % off in five -- 60 x 60, 7 x 7, d = 128, all three kernels; 100 x 75, 5 x 5, forward; 80 x 80,
+          // 13 x 13, d = 128 / 64, dK/dV.)
           const long cost = (blocks * (N + (which == 0 ? 40 : 100)) + (nxb == 1 ? items * 250 : 0)) * pl.n_tiles_x;
           if (best_cost < 0 || cost < best_cost) {
             best_cost = cost;

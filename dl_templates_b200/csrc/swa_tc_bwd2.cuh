@@ -15,7 +15,7 @@
 // The order the single issuer gave for free ("the accumulating MMAs of the block that used this buffer last were issued
 // before") is one more barrier, s_free, that the accumulate issuer commits and the score issuer waits for.
 //
-// All waits are bounded by polls, about a second each (umma.cuh).  A warp whose wait gave up leaves its loop; the others run into
+// All waits are bounded by polls, a second or (the producer's) half of one each (umma.cuh).  A warp whose wait gave up leaves its loop; the others run into
 // their own limit, unless they have all they wait for.  At the end any of them raises the CTA's flag: what is in flight is given
 // time to land, TMEM is freed and the status word records it.
 #pragma once
@@ -62,7 +62,7 @@ bwd2_kernel(const __grid_constant__ CUtensorMap tm_xqk, const __grid_constant__ 
   const int N = pl.N, nxb = pl.nxb, qch = ONE ? 1 : p.qch, vch = ONE ? 1 : p.vch;
   const int nsb = pl.nsb;                                        // score buffers; dP has two, used in turn
   const uint32_t blk_bytes = (uint32_t)N * 128u;               // one 64-wide chunk of a streamed block
-  const uint32_t xqk_bytes = qch * 16384u, xv_bytes = vch * 16384u, x_bytes = xqk_bytes + xv_bytes;
+  const uint32_t x_bytes = qch * 16384u + vch * 16384u;
   const uint32_t yqk_stage = blk_bytes * qch, yv_stage = blk_bytes * vch;
   const uint32_t ub = unit_bytes(pl);
   uint8_t* x_smem = smem;                                        // nxb buffers of (qk chunks, v chunks)
@@ -79,7 +79,7 @@ bwd2_kernel(const __grid_constant__ CUtensorMap tm_xqk, const __grid_constant__ 
   // Tensor memory: score buffer b at column N b, the two dP buffers behind them, then the accumulators.  P and dS replace the scores,
   // 16 columns by 16 -- in dK/dV P in the first eight, dS in the others, so that a dP buffer is free once it has been read and the next
   // block but one's dP need not wait for this one's accumulating MMAs.  With a third score buffer, where there is room, neither need
-  // its scores (31 x 31 window, d = 128, 4 slices: dK/dV, with three, 498 -> 434 us; dQ, with two, 326 -> 309).
+  // its scores (31 x 31 window, d = 128, 4 slices, when it was built: dK/dV, with three, 498 -> 434 us; dQ, with two, 326 -> 309).
   const uint32_t dp0 = nsb * N, acc_qk = dp0 + 2 * N, acc_v = acc_qk + qch * 64;
 
   const int warp = threadIdx.x >> 5;
@@ -204,7 +204,7 @@ bwd2_kernel(const __grid_constant__ CUtensorMap tm_xqk, const __grid_constant__ 
     setmaxnreg_dec<104>();
     if (warp == 0) {
       // ------------------------------------------------------------------ TMA producer
-      const LoadArgs f{x_smem, x_bytes, xqk_bytes, yqk_smem, yv_smem, yqk_stage, yv_stage, blk_bytes, sh->x_full, sh->x_empty,
+      const LoadArgs f{x_smem, x_bytes, yqk_smem, yv_smem, yqk_stage, yv_stage, blk_bytes, sh->x_full, sh->x_empty,
                        sh->y_full, sh->y_empty, nullptr, nullptr, &sh->start, &tm_xqk, &tm_xv, &tm_yqk, &tm_yv};
       load_warp<ONE, true>(p, f, ok);
     } else if (warp == 1) {

@@ -20,7 +20,7 @@
 // query tile in this kernel as well (about 400 dependent instructions per row on the critical path, 1.1 ms per launch
 // at the default workload, against 0.1 ms for a streaming pass over q).
 //
-// All waits are bounded by polls, about a second each (umma.cuh).  A warp whose wait gave up leaves its loop; the others run into
+// All waits are bounded by polls, a second or (the producer's) half of one each (umma.cuh).  A warp whose wait gave up leaves its loop; the others run into
 // their own limit, unless they have all they wait for.  At the end any of them raises the CTA's flag: what is in flight is given
 // time to land, TMEM is freed and the status word records it.
 #pragma once
@@ -278,11 +278,11 @@ fwd2_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CU
     setmaxnreg_dec<104>();
     if (warp == 0) {
       // ------------------------------------------------------------------ TMA producer
-      const LoadArgs f{q_smem, q_bytes, q_bytes, k_smem, v_smem, k_stage, v_stage, blk_bytes, sh->q_full, sh->q_empty,
+      const LoadArgs f{q_smem, q_bytes, k_smem, v_smem, k_stage, v_stage, blk_bytes, sh->q_full, sh->q_empty,
                        sh->k_full, sh->k_empty, split ? sh->v_full : nullptr, sh->v_empty, &sh->start, &tm_q, nullptr, &tm_k, &tm_v};
       load_warp<ONE, false>(p, f, ok);
     } else if (warp == 1) {
-      // ------------------------------------------------------------------ score issuer 
+      // ------------------------------------------------------------------ score issuer
       const uint32_t fmt = BF16 ? 1u : 0u;
       const uint32_t idesc_s = instr_desc(fmt, 128, N, 0, 0);
       const uint32_t hi_sw = smem_desc_hi(1024, true), hi_ns = smem_desc_hi(kUnitSbo, false);

@@ -27,7 +27,8 @@
 //
 // Backward both compute groups work on every block, each on half of its columns (whole steps of 16; they take turns with
 // the larger half): one group walking 80 columns alone took 1.85 ms per dK/dV launch at 256 slices, two sharing them 1.61 (first
-// strip kernels).  Forward, with three or four score buffers, the groups alternate blocks (0.94 against 1.03 ms).
+// strip kernels).  Forward, with two to four score buffers (two where d_v > 64 and a block has more than 85 columns), the groups
+// alternate blocks (0.94 against 1.03 ms).
 //
 // Rows of the grid: block j of an item covers the rows h0 + band * KR .. with h0 = -wr (mod KR) in every item (chunk heights
 // are multiples of KR), so the blocks a row meets, and with them the order of every sum, depend neither on the chunk height
@@ -223,7 +224,7 @@ __device__ __forceinline__ void accumulate_block(uint32_t el, uint32_t d, uint32
 // block with the walk that goes with it, more than the other roles needed.)
 struct LoadArgs {
   uint8_t* x_smem;              // nxb buffers of qk chunks, then v chunks (128 rows of 128 bytes each)
-  uint32_t x_bytes, xqk_bytes;
+  uint32_t x_bytes;
   uint8_t *yqk_smem, *yv_smem;  // streamed blocks
   uint32_t yqk_stage, yv_stage, blk_bytes;
   uint64_t *x_full, *x_empty, *y_full, *y_empty;

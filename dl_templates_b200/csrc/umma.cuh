@@ -163,9 +163,10 @@ __device__ __forceinline__ bool mbar_test(uint32_t bar, uint32_t parity) {
 
 // The strip kernels' wait (swa_tc_strip.cuh): one try_wait, which takes some eighty cycles when the phase has completed and suspends
 // the thread for up to two microseconds when it has not; the polling lies out of the way, because they have two dozen waits in
-// code that runs once per block.  False once the poll budget is used up (about a second); the caller's warp then leaves its
-// loop, the others run into their own limit, and the kernel's end tells the host.
-// HOW: 0 spins on try_wait, kSleepPoll looks every 64 ns (kLoadPolls), anything else is the hint in ns of a parked try_wait.
+// code that runs once per block.  False once the poll budget is used up; the caller's warp then leaves its loop, the others run into
+// their own limit, and the kernel's end tells the host.
+// HOW: 0 spins on try_wait, anything else is the hint in ns of a parked try_wait (a second each, above), kSleepPoll looks and sleeps:
+// __nanosleep(32) takes anything from 0 to 64 ns, a round 64 ns as measured, so that kLoadPolls come to half a second.
 constexpr uint32_t kLoadPolls = 1u << 23;
 constexpr uint32_t kSleepPoll = ~0u;
 template <uint32_t HOW>
