@@ -501,21 +501,27 @@ __device__ __forceinline__ void mask_warp(const KParams& p, const MaskArgs& f, b
           };
           if (pl.TW == 8) {
             const uint2* u = reinterpret_cast<const uint2*>(f.row_parts);
-            uint2 a[4], b[4], c[4], d[4];
+            // (In dK/dV, whose warp holds lse and delta as well, in two halves: at once its kernels for wide heads spill.  dK/dV, 56 x 56, 7 x 7
+            // window, 96 slices 71.4 -> 70.8 us, 45 x 77, 9 x 9, 24 slices 28.2 -> 27.7; d_v = 128 as above, by its registers alone, 305 -> 302.
+            // In halves in the forward kernel, 128 x 128, 13 x 13, 64 slices: 204 -> 208.5.)
+            const int d4[4] = {at0, at1, at2, at3};
+            constexpr int kUnits = VEC ? 1 : 2;
 #pragma unroll
-            for (int e = 0; e < 4; ++e) {
-              a[e] = u[entry(at0, e)];
-              b[e] = u[entry(at1, e)];
-              c[e] = u[entry(at2, e)];
-              d[e] = u[entry(at3, e)];
-            }
+            for (int h = 0; h < 2; h += kUnits) {
+              uint2 a[kUnits][4], b[kUnits][4];
 #pragma unroll
-            for (int e = 0; e < 4; ++e) {
-              uint8_t* to_ = tile + (lane + 32 * e) * 16;
-              if (lane + 32 * e < N) {
-                *reinterpret_cast<uint4*>(to_) = make_uint4(a[e].x, a[e].y, b[e].x, b[e].y);
-                *reinterpret_cast<uint4*>(to_ + ub) = make_uint4(c[e].x, c[e].y, d[e].x, d[e].y);
-              }
+              for (int e = 0; e < 4; ++e)
+#pragma unroll
+                for (int k = 0; k < kUnits; ++k) {
+                  a[k][e] = u[entry(d4[2 * (h + k)], e)];
+                  b[k][e] = u[entry(d4[2 * (h + k) + 1], e)];
+                }
+#pragma unroll
+              for (int e = 0; e < 4; ++e)
+                if (lane + 32 * e < N)
+#pragma unroll
+                  for (int k = 0; k < kUnits; ++k)
+                    *reinterpret_cast<uint4*>(tile + (h + k) * ub + (lane + 32 * e) * 16) = make_uint4(a[k][e].x, a[k][e].y, b[k][e].x, b[k][e].y);
             }
           } else {
             const uint32_t* u = reinterpret_cast<const uint32_t*>(f.row_parts);
