@@ -23,7 +23,8 @@
 // cycles and an MMA issued under a branch twice one issued by a converged warp (umma.cuh).  Hence block records instead of
 // six walks over items and quarters, written eight blocks at a time, a load order without polling, and scores of the next blocks
 // that wait for as little as possible (swa_tc_bwd2.cuh).  128 x 128 grid, 13 x 13 window, d = 64, 64 slices, bf16: forward / dQ /
-// dK/dV 240 / 273 / 318 us before, 203 / 192 / 245 now; 256 x 256, 31 x 31, d = 128, 4 slices: 329 / 366 / 577, 240 / 307 / 449.
+// dK/dV 240 / 273 / 318 us before, 204 / 191 / 243 now; 256 x 256, 31 x 31, d = 128, 4 slices: 329 / 366 / 577, 239 / 306 / 439 (CUDA events,
+// 1965 MHz, kernels one at a time with pauses).
 //
 // Backward both compute groups work on every block, each on half of its columns (whole steps of 16; they take turns with
 // the larger half): one group walking 80 columns alone took 1.85 ms per dK/dV launch at 256 slices, two sharing them 1.61 (first
